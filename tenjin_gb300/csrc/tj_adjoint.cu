@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(NT) k_adj_face(AG G, int d, const double* X, c
     const int nfx = G.nx + (d == 0);
     const long long nf = (long long)nfx * (G.ny + (d == 1));
     const int n = d == 0 ? G.nx : G.ny;
-    const double dtdx = dt / G.dx[d];
+    const double dtdx = quot(dt, G.dx[d]);
     tja::GradEos gr;
     tja::zero(gr);
     for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < nf; f += (long long)gridDim.x * blockDim.x) {
@@ -421,9 +421,9 @@ __global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const 
         double dS = 0.0;
         {
             const long long f0 = i + (long long)(G.nx + 1) * j;
-            dS += dt / G.dx[0] * (sstar0[f0] - sstar0[f0 + 1]);
+            dS += quot(dt, G.dx[0]) * (sstar0[f0] - sstar0[f0 + 1]);
             const long long h0 = i + (long long)G.nx * j;
-            dS += dt / G.dx[1] * (sstar1[h0] - sstar1[h0 + G.nx]);
+            dS += quot(dt, G.dx[1]) * (sstar1[h0] - sstar1[h0 + G.nx]);
         }
         for (int m = 0; m < M; ++m) acc[m] -= dS * mu[(long long)m * N + g];
         // MUSCL: cells ip = pos-1..pos+1 along d read this cell

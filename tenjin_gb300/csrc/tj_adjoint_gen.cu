@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kGT) k_gen_upd_rev_lin(DevParams P, Fp64Bufs f
     const long long nt = fb.ntot, nf = fb.nftot[d];
     const int NS = P.NS, NX = P.NX;
     const DevDomain D = fb.doms[0];
-    const double dtdx = fb.scal->dt / D.dx[d];
+    const double dtdx = quot(fb.scal->dt, D.dx[d]);
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nt; g += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         split3(g - D.off, D.n[0], D.n[1], i, j, k);
@@ -398,11 +398,11 @@ __global__ void __launch_bounds__(kGT) k_gen_recon_rev(DevParams P, Fp64Bufs fb,
                     const double v = X[src * nt + gs[q]];
                     u[q] = (vd && rf[q][d]) ? -v : v;
                 }
-                double rr = (u[1] - u[0]) / (u[2] - u[1]);
+                double rr = quot(u[1] - u[0], u[2] - u[1]);
                 if (isinf(rr) || isnan(rr)) rr = 0.0;
                 double b1 = 0.0, b2 = 0.0;
                 if (rr > 0.0) {
-                    const double a = 2.0 / (1.0 + rr), b = 2.0 * rr / (1.0 + rr);
+                    const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);
                     if (b < a) b1 = 1.0;
                     else b2 = 1.0;
                 }

@@ -26,6 +26,8 @@
 
 #include <cmath>
 
+#include "tj_quot.h"
+
 #ifdef __CUDACC__
 #define TJA_HD __host__ __device__ inline
 #define TJA_NOTFINITE(x) (isinf(x) || isnan(x))
@@ -35,6 +37,9 @@
 #endif
 
 namespace tja {
+
+using tj::quot;
+using tj::root;
 
 constexpr int MM = 4;  // materials
 
@@ -105,7 +110,7 @@ TJA_HD void cleanup_fwd(int M, const double* a, double* out)
         c[m] = v;
         tot += v;
     }
-    for (int m = 0; m < M; ++m) out[m] = c[m] * (1.0 / tot);
+    for (int m = 0; m < M; ++m) out[m] = c[m] * (quot(1.0, tot));
 }
 
 // lam_in = (d cleanup / d a)^T lam_out
@@ -121,7 +126,7 @@ TJA_HD void cleanup_rev(int M, const double* a, const double* lam_out, double* l
     }
     double s = 0.0;
     for (int m = 0; m < M; ++m) s += lam_out[m] * c[m];
-    const double it = 1.0 / tot;
+    const double it = quot(1.0, tot);
     for (int m = 0; m < M; ++m) {
         const bool in = !(a[m] < 0.0) && !(a[m] > 1.0);
         lam_in[m] = in ? (lam_out[m] * it - s * it * it) : 0.0;
@@ -151,21 +156,21 @@ TJA_HD void face_state_fwd(const Eos& E, const Prim& x, bool clean, FS& s)
     s.p = x.p;
     double invG = 0.0, ent = 0.0, pnt = 0.0;
     for (int m = 0; m < M; ++m) {
-        invG += s.a[m] / E.G[m];
+        invG += quot(s.a[m], E.G[m]);
         ent += E.er[m] * s.ar[m];
-        pnt += E.pr[m] * s.a[m] / E.G[m];
+        pnt += quot(E.pr[m] * s.a[m], E.G[m]);
     }
     s.E = x.p * invG + ent - pnt + ke;
     double A = 0.0, xit = 0.0;
     for (int m = 0; m < M; ++m) {
-        const double xi = 1.0 / E.G[m];
-        const double c2 = x.p * (E.G[m] + 1.0) / x.rk[m] - E.pr[m] / x.rk[m];
-        const double v = xi * c2 * s.ar[m] / s.rho;
+        const double xi = quot(1.0, E.G[m]);
+        const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
+        const double v = quot(xi * c2 * s.ar[m], s.rho);
         A += (0.0 < v) ? v : 0.0;
         xit += xi * s.a[m];
     }
     if (A <= 0.0) A = 1E-6;
-    s.c = sqrt(A / xit);
+    s.c = root(quot(A, xit));
 }
 
 TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l, Prim& lx, GradEos& g)
@@ -184,30 +189,30 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
     {
         double A = 0.0, xit = 0.0;
         for (int m = 0; m < M; ++m) {
-            const double xi = 1.0 / E.G[m];
-            const double c2 = x.p * (E.G[m] + 1.0) / x.rk[m] - E.pr[m] / x.rk[m];
-            const double v = xi * c2 * s.ar[m] / s.rho;
+            const double xi = quot(1.0, E.G[m]);
+            const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
+            const double v = quot(xi * c2 * s.ar[m], s.rho);
             A += (0.0 < v) ? v : 0.0;
             xit += xi * s.a[m];
         }
         const bool floored = A <= 0.0;
-        const double lA = floored ? 0.0 : l.c / (2.0 * s.c * xit);
-        const double lxit = -l.c * s.c / (2.0 * xit);
+        const double lA = floored ? 0.0 : quot(l.c, 2.0 * s.c * xit);
+        const double lxit = quot(-l.c * s.c, 2.0 * xit);
         for (int m = 0; m < M; ++m) {
-            const double xi = 1.0 / E.G[m];
-            const double c2 = x.p * (E.G[m] + 1.0) / x.rk[m] - E.pr[m] / x.rk[m];
-            const double v = xi * c2 * s.ar[m] / s.rho;
+            const double xi = quot(1.0, E.G[m]);
+            const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
+            const double v = quot(xi * c2 * s.ar[m], s.rho);
             double lxi = lxit * s.a[m];
             la[m] += lxit * xi;
             if (0.0 < v) {
-                const double lc2 = lA * xi * s.ar[m] / s.rho;
-                lar[m] += lA * xi * c2 / s.rho;
-                lrho += -lA * v / s.rho;
-                lxi += lA * c2 * s.ar[m] / s.rho;
-                lp += lc2 * (E.G[m] + 1.0) / x.rk[m];
-                lrk[m] += -lc2 * c2 / x.rk[m];
-                g.G[m] += lc2 * x.p / x.rk[m];
-                g.pr[m] += -lc2 / x.rk[m];
+                const double lc2 = quot(lA * xi * s.ar[m], s.rho);
+                lar[m] += quot(lA * xi * c2, s.rho);
+                lrho += -quot(lA * v, s.rho);
+                lxi += quot(lA * c2 * s.ar[m], s.rho);
+                lp += quot(lc2 * (E.G[m] + 1.0), x.rk[m]);
+                lrk[m] += -quot(lc2 * c2, x.rk[m]);
+                g.G[m] += quot(lc2 * x.p, x.rk[m]);
+                g.pr[m] += -quot(lc2, x.rk[m]);
             }
             g.G[m] += -lxi * xi * xi;
         }
@@ -216,12 +221,12 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
     {
         const double lE = l.E;
         double invG = 0.0;
-        for (int m = 0; m < M; ++m) invG += s.a[m] / E.G[m];
+        for (int m = 0; m < M; ++m) invG += quot(s.a[m], E.G[m]);
         lp += lE * invG;
         for (int m = 0; m < M; ++m) {
-            la[m] += lE * (x.p - E.pr[m]) / E.G[m];
-            g.G[m] += -lE * (x.p - E.pr[m]) * s.a[m] / (E.G[m] * E.G[m]);
-            g.pr[m] += -lE * s.a[m] / E.G[m];
+            la[m] += quot(lE * (x.p - E.pr[m]), E.G[m]);
+            g.G[m] += -quot(lE * (x.p - E.pr[m]) * s.a[m], E.G[m] * E.G[m]);
+            g.pr[m] += -quot(lE * s.a[m], E.G[m]);
             g.er[m] += lE * s.ar[m];
             lar[m] += lE * E.er[m];
         }
@@ -258,7 +263,7 @@ TJA_HD void hllc_fwd(int M, const FS& L, const FS& R, int d, HllcOut& o)
     const double x1 = fabs(uL) + L.c, x2 = fabs(uR) + R.c;
     const double SR = (x1 < x2) ? x2 : x1;
     const double SL = -SR;
-    const double Ss = (R.p - L.p + L.ru[d] * (SL - uL) - R.ru[d] * (SR - uR)) / (L.rho * (SL - uL) - R.rho * (SR - uR));
+    const double Ss = quot(R.p - L.p + L.ru[d] * (SL - uL) - R.ru[d] * (SR - uR), L.rho * (SL - uL) - R.rho * (SR - uR));
     o.Ss = Ss;
     int side;
     bool hllc;
@@ -269,7 +274,7 @@ TJA_HD void hllc_fwd(int M, const FS& L, const FS& R, int d, HllcOut& o)
     o.side = side;
     const FS& K = side ? R : L;
     const double SK = side ? SR : SL, uK = K.u[d];
-    const double mult = (fabs((Ss - uK) / Ss) < 1E-20) ? 1.0 : (SK - uK) / (SK - Ss);
+    const double mult = (Ss - uK == 0.0 && Ss != 0.0) ? 1.0 : quot(SK - uK, SK - Ss);
     double ars[MM], rs = 0.0;
     for (int m = 0; m < M; ++m) {
         ars[m] = mult * K.ar[m];
@@ -278,8 +283,8 @@ TJA_HD void hllc_fwd(int M, const FS& L, const FS& R, int d, HllcOut& o)
     double rus[2];
     rus[d] = mult * K.rho * Ss;
     rus[1 - d] = mult * K.ru[1 - d];
-    const double vsd = rus[d] / rs;
-    const double Es = mult * K.rho * (K.E / K.rho + (Ss - uK) * (Ss + K.p / (K.rho * (SK - uK))));
+    const double vsd = quot(rus[d], rs);
+    const double Es = mult * K.rho * (quot(K.E, K.rho) + (Ss - uK) * (Ss + quot(K.p, K.rho * (SK - uK))));
     const double w = hllc ? SK : 0.0;
     for (int m = 0; m < M; ++m) {
         o.Fa[m] = K.a[m] * vsd;
@@ -299,7 +304,7 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     const double SL = -SR;
     const double Num = R.p - L.p + L.ru[d] * (SL - uL) - R.ru[d] * (SR - uR);
     const double Den = L.rho * (SL - uL) - R.rho * (SR - uR);
-    const double Ss = Num / Den;
+    const double Ss = quot(Num, Den);
     int side;
     bool hllc;
     if (SL >= 0.0) { side = 0; hllc = false; }
@@ -309,8 +314,8 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     const FS& K = side ? R : L;
     FS& lK = side ? lR : lL;
     const double SK = side ? SR : SL, uK = K.u[d];
-    const bool guard = fabs((Ss - uK) / Ss) < 1E-20;
-    const double mult = guard ? 1.0 : (SK - uK) / (SK - Ss);
+    const bool guard = Ss - uK == 0.0 && Ss != 0.0;
+    const double mult = guard ? 1.0 : quot(SK - uK, SK - Ss);
     double ars[MM], rs = 0.0;
     for (int m = 0; m < M; ++m) {
         ars[m] = mult * K.ar[m];
@@ -319,8 +324,8 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     double rus[2];
     rus[d] = mult * K.rho * Ss;
     rus[1 - d] = mult * K.ru[1 - d];
-    const double vsd = rus[d] / rs;
-    const double D1 = Ss - uK, D2 = K.rho * Ss + K.p / (SK - uK);
+    const double vsd = quot(rus[d], rs);
+    const double D1 = Ss - uK, D2 = K.rho * Ss + quot(K.p, SK - uK);
     const double W = K.E + D1 * D2;
     const double Es = mult * W;
     const double w = hllc ? SK : 0.0;
@@ -354,8 +359,8 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     lEs = lF.FE * w;
     if (hllc) lSK += lF.FE * (Es - K.E);
     // vsd = rus_d / rs
-    lrus[d] += lvsd / rs;
-    const double lrs = -lvsd * vsd / rs;
+    lrus[d] += quot(lvsd, rs);
+    const double lrs = quot(-lvsd * vsd, rs);
     for (int m = 0; m < M; ++m) lars[m] += lrs;
     // ars = mult K.ar; rus_d = mult K.rho Ss; rus_o = mult K.ru_o
     for (int m = 0; m < M; ++m) {
@@ -376,22 +381,22 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     luK -= lD1;
     lK.rho += lD2 * Ss;
     lSs += lD2 * K.rho;
-    lK.p += lD2 / (SK - uK);
-    lSK += -lD2 * K.p / ((SK - uK) * (SK - uK));
-    luK += lD2 * K.p / ((SK - uK) * (SK - uK));
+    lK.p += quot(lD2, SK - uK);
+    lSK += -quot(lD2 * K.p, (SK - uK) * (SK - uK));
+    luK += quot(lD2 * K.p, (SK - uK) * (SK - uK));
     // mult = (SK - uK) / (SK - Ss)
     if (!guard) {
         const double den = SK - Ss;
-        lSK += lmult * (uK - Ss) / (den * den);
-        luK += -lmult / den;
-        lSs += lmult * mult / den;
+        lSK += quot(lmult * (uK - Ss), den * den);
+        luK += -quot(lmult, den);
+        lSs += quot(lmult * mult, den);
     }
     double lSL = 0.0, lSR = 0.0;
     if (side) lSR += lSK;
     else lSL += lSK;
     lK.u[d] += luK;
     // Ss = Num / Den
-    const double lNum = lSs / Den, lDen = -lSs * Ss / Den;
+    const double lNum = quot(lSs, Den), lDen = quot(-lSs * Ss, Den);
     lR.p += lNum;
     lL.p -= lNum;
     lL.ru[d] += lNum * (SL - uL);
@@ -430,23 +435,23 @@ TJA_HD void c2p_fwd(const Eos& E, const Cons& c, Carried& o)
     for (int m = 0; m < M; ++m) {
         o.a[m] = c.a[m];
         o.ar[m] = c.ar[m];
-        o.rk[m] = c.ar[m] / c.a[m];
+        o.rk[m] = quot(c.ar[m], c.a[m]);
         o.rho += c.ar[m];
     }
     double ke = 0.0;
     for (int r = 0; r < 2; ++r) {
         o.ru[r] = c.ru[r];
-        o.u[r] = c.ru[r] / o.rho;
+        o.u[r] = quot(c.ru[r], o.rho);
         ke += 0.5 * o.rho * o.u[r] * o.u[r];
     }
     o.E = c.E;
     double invG = 0.0, ent = 0.0, pnt = 0.0;
     for (int m = 0; m < M; ++m) {
-        invG += c.a[m] / E.G[m];
+        invG += quot(c.a[m], E.G[m]);
         ent += E.er[m] * c.ar[m];
-        pnt += E.pr[m] * c.a[m] / E.G[m];
+        pnt += quot(E.pr[m] * c.a[m], E.G[m]);
     }
-    o.p = (c.E - ke - ent + pnt) / invG;
+    o.p = quot(c.E - ke - ent + pnt, invG);
 }
 
 TJA_HD void c2p_rev(const Eos& E, const Cons& c, const Carried& lam, Cons& mu, GradEos& g)
@@ -455,13 +460,13 @@ TJA_HD void c2p_rev(const Eos& E, const Cons& c, const Carried& lam, Cons& mu, G
     Carried o;
     c2p_fwd(E, c, o);
     double D = 0.0;
-    for (int m = 0; m < M; ++m) D += c.a[m] / E.G[m];
-    const double lN = lam.p / D, lD = -lam.p * o.p / D;
+    for (int m = 0; m < M; ++m) D += quot(c.a[m], E.G[m]);
+    const double lN = quot(lam.p, D), lD = quot(-lam.p * o.p, D);
     for (int m = 0; m < M; ++m) {
-        mu.a[m] = lam.a[m] - lam.rk[m] * o.rk[m] / c.a[m] + lN * E.pr[m] / E.G[m] + lD / E.G[m];
-        mu.ar[m] = lam.ar[m] + lam.rk[m] / c.a[m] - lN * E.er[m];
-        g.G[m] += -(lN * E.pr[m] + lD) * c.a[m] / (E.G[m] * E.G[m]);
-        g.pr[m] += lN * c.a[m] / E.G[m];
+        mu.a[m] = lam.a[m] - quot(lam.rk[m] * o.rk[m], c.a[m]) + quot(lN * E.pr[m], E.G[m]) + quot(lD, E.G[m]);
+        mu.ar[m] = lam.ar[m] + quot(lam.rk[m], c.a[m]) - lN * E.er[m];
+        g.G[m] += -quot((lN * E.pr[m] + lD) * c.a[m], E.G[m] * E.G[m]);
+        g.pr[m] += quot(lN * c.a[m], E.G[m]);
         g.er[m] += -lN * c.ar[m];
     }
     mu.E = lam.E + lN;
@@ -470,8 +475,8 @@ TJA_HD void c2p_rev(const Eos& E, const Cons& c, const Carried& lam, Cons& mu, G
         // ke = 0.5 rho u^2 with u = ru / rho
         const double lu = lam.u[r] - lN * o.rho * o.u[r];
         lrho += -lN * 0.5 * o.u[r] * o.u[r];
-        mu.ru[r] = lam.ru[r] + lu / o.rho;
-        lrho += -lu * o.u[r] / o.rho;
+        mu.ru[r] = lam.ru[r] + quot(lu, o.rho);
+        lrho += -quot(lu * o.u[r], o.rho);
     }
     for (int m = 0; m < M; ++m) mu.ar[m] += lrho;
 }
@@ -500,9 +505,9 @@ TJA_HD void p2c_state_fwd(const Eos& E, const Prim& x, Carried& o)
     o.p = x.p;
     double invG = 0.0, ent = 0.0, pnt = 0.0;
     for (int m = 0; m < M; ++m) {
-        invG += x.a[m] / E.G[m];
+        invG += quot(x.a[m], E.G[m]);
         ent += E.er[m] * o.ar[m];
-        pnt += E.pr[m] * x.a[m] / E.G[m];
+        pnt += quot(E.pr[m] * x.a[m], E.G[m]);
     }
     o.E = x.p * invG + ent - pnt + ke;
 }
@@ -513,7 +518,7 @@ TJA_HD void p2c_state_rev(const Eos& E, const Prim& x, const Carried& lam, Prim&
     Carried o;
     p2c_state_fwd(E, x, o);
     double invG = 0.0;
-    for (int m = 0; m < M; ++m) invG += x.a[m] / E.G[m];
+    for (int m = 0; m < M; ++m) invG += quot(x.a[m], E.G[m]);
     const double lE = lam.E;
     double lar[MM];
     lx.p = lam.p + lE * invG;
@@ -524,10 +529,10 @@ TJA_HD void p2c_state_rev(const Eos& E, const Prim& x, const Carried& lam, Prim&
     }
     for (int m = 0; m < M; ++m) {
         lar[m] = lam.ar[m] + lE * E.er[m] + lrho;
-        lx.a[m] = lam.a[m] + lE * (x.p - E.pr[m]) / E.G[m] + lar[m] * x.rk[m];
+        lx.a[m] = lam.a[m] + quot(lE * (x.p - E.pr[m]), E.G[m]) + lar[m] * x.rk[m];
         lx.rk[m] = lam.rk[m] + lar[m] * x.a[m];
-        g.G[m] += -lE * (x.p - E.pr[m]) * x.a[m] / (E.G[m] * E.G[m]);
-        g.pr[m] += -lE * x.a[m] / E.G[m];
+        g.G[m] += -quot(lE * (x.p - E.pr[m]) * x.a[m], E.G[m] * E.G[m]);
+        g.pr[m] += -quot(lE * x.a[m], E.G[m]);
         g.er[m] += lE * o.ar[m];
     }
 }
@@ -553,21 +558,21 @@ TJA_HD bool thinc_cand_fwd(const double s[3][3], int d, double beta0, double dx,
     const double mn = (aR < aL) ? aR : aL;
     const double mx = ((aL < aR) ? aR : aL) - mn;
     const double theta = (double)((0.0 < aR - aL) - (aR - aL < 0.0));
-    const double C = (mx < eps) ? 0.0 : (a0 - mn + eps) / (mx + eps);
+    const double C = (mx < eps) ? 0.0 : quot(a0 - mn + eps, mx + eps);
     const double delta = 1E-4;
     const bool mixed = (C > delta) && (C < (0.999999 - delta)) && ((aR - a0) * (a0 - aL) >= 0.0);
     L = R = 0.0;
     if (!mixed) return false;
-    const double nx = -1.0 / (8.0 * dx) * (s[2][2] + 2.0 * s[2][1] + s[2][0] - s[0][2] - 2.0 * s[0][1] - s[0][0]);
-    const double ny = -1.0 / (8.0 * dy) * (s[2][2] + 2.0 * s[1][2] + s[0][2] - s[0][0] - 2.0 * s[1][0] - s[2][0]);
-    const double norm = sqrt(nx * nx + ny * ny);
-    const double nvc = (norm < 1E-20) ? 0.0 : fabs((d == 0 ? nx : ny) / norm);
+    const double nx = quot(-1.0, 8.0 * dx) * (s[2][2] + 2.0 * s[2][1] + s[2][0] - s[0][2] - 2.0 * s[0][1] - s[0][0]);
+    const double ny = quot(-1.0, 8.0 * dy) * (s[2][2] + 2.0 * s[1][2] + s[0][2] - s[0][0] - 2.0 * s[1][0] - s[2][0]);
+    const double norm = root(nx * nx + ny * ny);
+    const double nvc = (norm < 1E-20) ? 0.0 : fabs(quot(d == 0 ? nx : ny, norm));
     const double beta = nvc * beta0 + 0.01;
     const double coshB = ch(beta), tanhB = th(beta);
     const double B = ex(theta * beta * ((2.0 * C) - 1.0));
-    const double A = ((B / coshB) - 1.0) / tanhB;
-    R = mn + (mx / 2.0) * (1.0 + theta * ((tanhB + A) / (1.0 + A * tanhB)));
-    L = mn + (mx / 2.0) * (1.0 + theta * A);
+    const double A = quot((quot(B, coshB)) - 1.0, tanhB);
+    R = mn + (0.5 * mx) * (1.0 + theta * (quot(tanhB + A, 1.0 + A * tanhB)));
+    L = mn + (0.5 * mx) * (1.0 + theta * A);
     return true;
 }
 
@@ -581,38 +586,38 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
     const double mn = (aR < aL) ? aR : aL;
     const double mx = ((aL < aR) ? aR : aL) - mn;
     const double theta = (double)((0.0 < aR - aL) - (aR - aL < 0.0));
-    const double C = (a0 - mn + eps) / (mx + eps);
-    const double nx = -1.0 / (8.0 * dx) * (s[2][2] + 2.0 * s[2][1] + s[2][0] - s[0][2] - 2.0 * s[0][1] - s[0][0]);
-    const double ny = -1.0 / (8.0 * dy) * (s[2][2] + 2.0 * s[1][2] + s[0][2] - s[0][0] - 2.0 * s[1][0] - s[2][0]);
-    const double norm = sqrt(nx * nx + ny * ny);
+    const double C = quot(a0 - mn + eps, mx + eps);
+    const double nx = quot(-1.0, 8.0 * dx) * (s[2][2] + 2.0 * s[2][1] + s[2][0] - s[0][2] - 2.0 * s[0][1] - s[0][0]);
+    const double ny = quot(-1.0, 8.0 * dy) * (s[2][2] + 2.0 * s[1][2] + s[0][2] - s[0][0] - 2.0 * s[1][0] - s[2][0]);
+    const double norm = root(nx * nx + ny * ny);
     const bool flat = norm < 1E-20;
     const double nd = d == 0 ? nx : ny;
     const double nvc = flat ? 0.0 : fabs(nd / norm);
     const double beta = nvc * beta0 + 0.01;
     const double coshB = ch(beta), tanhB = th(beta);
     const double B = ex(theta * beta * ((2.0 * C) - 1.0));
-    const double A = ((B / coshB) - 1.0) / tanhB;
+    const double A = quot((quot(B, coshB)) - 1.0, tanhB);
     const double q = 1.0 + A * tanhB;
-    const double T = (tanhB + A) / q;
+    const double T = quot(tanhB + A, q);
 
     double lmn = lL + lR;
     double lmx = lL * 0.5 * (1.0 + theta * A) + lR * 0.5 * (1.0 + theta * T);
-    double lA = lL * (mx / 2.0) * theta;
-    const double lT = lR * (mx / 2.0) * theta;
-    double lt = lT * (1.0 - A * A) / (q * q);
-    lA += lT * (1.0 - tanhB * tanhB) / (q * q);
-    const double lB = lA / (coshB * tanhB);
-    const double lch = -lA * B / (coshB * coshB * tanhB);
-    lt += -lA * A / tanhB;
+    double lA = lL * (0.5 * mx) * theta;
+    const double lT = lR * (0.5 * mx) * theta;
+    double lt = quot(lT * (1.0 - A * A), q * q);
+    lA += quot(lT * (1.0 - tanhB * tanhB), q * q);
+    const double lB = quot(lA, coshB * tanhB);
+    const double lch = quot(-lA * B, coshB * coshB * tanhB);
+    lt += -quot(lA * A, tanhB);
     double lbeta = lB * B * theta * (2.0 * C - 1.0);
     const double lC = lB * B * theta * beta * 2.0;
     lbeta += lch * tanhB * coshB;  // d cosh = sinh = tanh cosh
     lbeta += lt * (1.0 - tanhB * tanhB);
     const double lnvc = lbeta * beta0;
     // C = (a0 - mn + eps) / (mx + eps)
-    double la0 = lC / (mx + eps);
-    lmn -= lC / (mx + eps);
-    lmx -= lC * C / (mx + eps);
+    double la0 = quot(lC, mx + eps);
+    lmn -= quot(lC, mx + eps);
+    lmx -= quot(lC * C, mx + eps);
     // mx = max - mn
     const double lmax = lmx;
     lmn -= lmx;
@@ -635,9 +640,9 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
     if (!flat) {
         const double sg = (double)((nd > 0.0) - (nd < 0.0));
         const double n3 = norm * norm * norm;
-        const double lnx = lnvc * sg * ((d == 0 ? 1.0 : 0.0) / norm - nd * nx / n3);
-        const double lny = lnvc * sg * ((d == 1 ? 1.0 : 0.0) / norm - nd * ny / n3);
-        const double cx = -1.0 / (8.0 * dx) * lnx, cy = -1.0 / (8.0 * dy) * lny;
+        const double lnx = lnvc * sg * (quot(d == 0 ? 1.0 : 0.0, norm) - quot(nd * nx, n3));
+        const double lny = lnvc * sg * (quot(d == 1 ? 1.0 : 0.0, norm) - quot(nd * ny, n3));
+        const double cx = quot(-1.0, 8.0 * dx) * lnx, cy = quot(-1.0, 8.0 * dy) * lny;
         ls[2][2] += cx + cy;
         ls[2][1] += 2.0 * cx;
         ls[2][0] += cx - cy;
@@ -656,11 +661,11 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
 // ---------------------------------------------------------------------------
 TJA_HD void muscl_fwd(double um, double u0, double up, double& l, double& r)
 {
-    double rr = (u0 - um) / (up - u0);
+    double rr = quot(u0 - um, up - u0);
     if (TJA_NOTFINITE(rr)) rr = 0.0;
     double phi = 0.0;
     if (rr > 0.0) {
-        const double a = 2.0 / (1.0 + rr), b = 2.0 * rr / (1.0 + rr);
+        const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);
         phi = (b < a) ? b : a;
     }
     const double grad = phi * 0.5 * (up - um);
@@ -670,10 +675,10 @@ TJA_HD void muscl_fwd(double um, double u0, double up, double& l, double& r)
 
 TJA_HD int muscl_branch(double um, double u0, double up)
 {
-    double rr = (u0 - um) / (up - u0);
+    double rr = quot(u0 - um, up - u0);
     if (TJA_NOTFINITE(rr)) rr = 0.0;
     if (rr <= 0.0) return 0;
-    const double a = 2.0 / (1.0 + rr), b = 2.0 * rr / (1.0 + rr);
+    const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);
     return (b < a) ? 1 : 2;
 }
 

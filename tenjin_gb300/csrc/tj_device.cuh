@@ -12,6 +12,7 @@
 
 #include <cstdint>
 
+#include "tj_quot.h"
 #include "tj_math.cuh"
 #include "tj_types.h"
 
@@ -80,7 +81,7 @@ __device__ __forceinline__ typename PT::real mix_gamma_term(const PT& P, int m, 
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
-    return (lam * q[0] * q[3] + (R(1.0) - lam) * q[4] * q[7]) / (lam * q[3] + (R(1.0) - lam) * q[7]) - R(1.0);
+    return quot(lam * q[0] * q[3] + (R(1.0) - lam) * q[4] * q[7], lam * q[3] + (R(1.0) - lam) * q[7]) - R(1.0);
 }
 
 template <typename PT>
@@ -92,18 +93,18 @@ __device__ inline typename PT::real eos_e_cold(const PT& P, int m, const ECellT<
         case TJ_EOS_MIEGRUNEISEN: return q[2] * e.arho;  // equationofstate.cpp:37-40
         case TJ_EOS_MIXTURE: return e.lam * (q[2] * e.arho) + (R(1.0) - e.lam) * (q[6] * e.arho);  // :161-165
         case TJ_EOS_ROMENSKII: {                         // :418-423
-            R a = q[6], K0 = q[5], r0 = q[4], x = e.rhok / r0;
-            return e.arho * (((K0 / (R(2.0) * r0 * a * a)) * (tjm_pow(x, a) - R(1.0))) * (tjm_pow(x, a) - R(1.0)));
+            R a = q[6], K0 = q[5], r0 = q[4], x = quot(e.rhok, r0);
+            return e.arho * (((quot(K0, R(2.0) * r0 * a * a)) * (tjm_pow(x, a) - R(1.0))) * (tjm_pow(x, a) - R(1.0)));
         }
         case TJ_EOS_WILKINS: {  // :519-524
-            R r0 = q[4], x = e.rhok / r0;
-            return e.arho * ((q[5] + q[6] * x * x + q[7] * x + q[8] / x - q[9] * tjm_log(x)) / r0);
+            R r0 = q[4], x = quot(e.rhok, r0);
+            return e.arho * (quot(q[5] + q[6] * x * x + q[7] * x + quot(q[8], x) - q[9] * tjm_log(x), r0));
         }
         default: {  // Hugoniot reference curve (copper; no reference class)
             R r0 = q[4], c0 = q[5], sl = q[6];
-            R et = R(1.0) - r0 / e.rhok, dd = R(1.0) - sl * et;
-            R ph = r0 * c0 * c0 * et / (dd * dd);
-            return e.arho * (ph * et / (R(2.0) * r0));
+            R et = R(1.0) - quot(r0, e.rhok), dd = R(1.0) - sl * et;
+            R ph = quot(r0 * c0 * c0 * et, dd * dd);
+            return e.arho * (quot(ph * et, R(2.0) * r0));
         }
     }
 }
@@ -115,23 +116,23 @@ __device__ inline typename PT::real eos_p_cold(const PT& P, int m, const ECellT<
     const R* q = P.prm[m];
     R G = gam(P, m);
     switch (P.eos[m]) {
-        case TJ_EOS_MIEGRUNEISEN: return q[1] * e.alpha / G;  // :42-45
+        case TJ_EOS_MIEGRUNEISEN: return quot(q[1] * e.alpha, G);  // :42-45
         case TJ_EOS_MIXTURE:                                  // :167-171
-            return (q[1] * e.alpha / (q[0] - R(1.0))) * e.lam * e.rhok / (e.rm0) +
-                   (q[5] * e.alpha / (q[4] - R(1.0))) * (R(1.0) - e.lam) * e.rhok / (e.rm1);
+            return quot((quot(q[1] * e.alpha, q[0] - R(1.0))) * e.lam * e.rhok, e.rm0) +
+                   quot((quot(q[5] * e.alpha, q[4] - R(1.0))) * (R(1.0) - e.lam) * e.rhok, e.rm1);
         case TJ_EOS_ROMENSKII: {                              // :425-430
-            R a = q[6], K0 = q[5], r0 = q[4], x = e.rhok / r0;
-            return (e.alpha / G) * ((K0 / a) * tjm_pow(x, a + R(1.0)) * (tjm_pow(x, a) - R(1.0)));
+            R a = q[6], K0 = q[5], r0 = q[4], x = quot(e.rhok, r0);
+            return (quot(e.alpha, G)) * ((quot(K0, a)) * tjm_pow(x, a + R(1.0)) * (tjm_pow(x, a) - R(1.0)));
         }
         case TJ_EOS_WILKINS: {  // :526-531
-            R r0 = q[4], x = e.rhok / r0;
-            return (e.alpha / G) * ((R(2.0) * q[6] * x * x * x + q[7] * x * x - q[8] - q[9] * x));
+            R r0 = q[4], x = quot(e.rhok, r0);
+            return (quot(e.alpha, G)) * ((R(2.0) * q[6] * x * x * x + q[7] * x * x - q[8] - q[9] * x));
         }
         default: {
             R r0 = q[4], c0 = q[5], sl = q[6];
-            R et = R(1.0) - r0 / e.rhok, dd = R(1.0) - sl * et;
-            R ph = r0 * c0 * c0 * et / (dd * dd);
-            return (e.alpha / G) * ph;
+            R et = R(1.0) - quot(r0, e.rhok), dd = R(1.0) - sl * et;
+            R ph = quot(r0 * c0 * c0 * et, dd * dd);
+            return (quot(e.alpha, G)) * ph;
         }
     }
 }
@@ -144,7 +145,7 @@ __device__ inline typename PT::real eos_G(const PT& P, int m, const ECellT<typen
     switch (P.eos[m]) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;                           // :81-84
         case TJ_EOS_MIXTURE: return R(0.0);                                          // :146-149
-        case TJ_EOS_ROMENSKII: return q[8] * tjm_pow((e.rhok / q[4]), q[7] + R(1.0));  // :437-440
+        case TJ_EOS_ROMENSKII: return q[8] * tjm_pow((quot(e.rhok, q[4])), q[7] + R(1.0));  // :437-440
         case TJ_EOS_WILKINS: return q[10];                                           // :538-541
         default: return q[7];
     }
@@ -157,7 +158,7 @@ __device__ inline typename PT::real eos_dGdrho(const PT& P, int m, const ECellT<
     const R* q = P.prm[m];
     switch (P.eos[m]) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;
-        case TJ_EOS_ROMENSKII: return q[8] * (q[7] + R(1.0)) * tjm_pow((e.rhok / q[4]), q[7]) / q[4];  // :442-445
+        case TJ_EOS_ROMENSKII: return quot(q[8] * (q[7] + R(1.0)) * tjm_pow((quot(e.rhok, q[4])), q[7]), q[4]);  // :442-445
         default: return R(0.0);
     }
 }
@@ -170,7 +171,7 @@ __device__ inline typename PT::real eos_dG2drho2(const PT& P, int m, const ECell
     switch (P.eos[m]) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;
         case TJ_EOS_ROMENSKII:  // :447-450
-            return q[8] * (q[7] + R(1.0)) * (q[7]) * tjm_pow((e.rhok / q[4]), q[7] - R(1.0)) / (q[4] * q[4]);
+            return quot(q[8] * (q[7] + R(1.0)) * (q[7]) * tjm_pow((quot(e.rhok, q[4])), q[7] - R(1.0)), q[4] * q[4]);
         default: return R(0.0);
     }
 }
@@ -195,16 +196,16 @@ __device__ inline typename PT::real eos_p_shear(const PT& P, int m, const ECellT
     switch (P.eos[m]) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;  // :106-109
         case TJ_EOS_MIXTURE: return R(0.0);                 // :141-144
-        case TJ_EOS_HUGONIOT: return (e.alpha / G) * ((e.rhok * R(0.0) - P.prm[m][7]) * e.hj2);
-        default: return (e.alpha / G) * ((e.rhok * eos_dGdrho(P, m, e) - eos_G(P, m, e)) * e.hj2);  // :462-465
+        case TJ_EOS_HUGONIOT: return (quot(e.alpha, G)) * ((e.rhok * R(0.0) - P.prm[m][7]) * e.hj2);
+        default: return (quot(e.alpha, G)) * ((e.rhok * eos_dGdrho(P, m, e) - eos_G(P, m, e)) * e.hj2);  // :462-465
     }
 }
 
 template <typename PT>
 __device__ __forceinline__ typename PT::real eos_invG(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
-    if (P.eos[m] == TJ_EOS_MIXTURE) return e.alpha / mix_gamma_term(P, m, e.lam);  // :173-178
-    return e.alpha / gam(P, m);
+    if (P.eos[m] == TJ_EOS_MIXTURE) return quot(e.alpha, mix_gamma_term(P, m, e.lam));  // :173-178
+    return quot(e.alpha, gam(P, m));
 }
 
 // xi (equationofstate.cpp:72-75, 222-225)
@@ -212,8 +213,8 @@ template <typename PT>
 __device__ __forceinline__ typename PT::real eos_xi(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
-    if (P.eos[m] == TJ_EOS_MIXTURE) return R(1.0) / mix_gamma_term(P, m, e.lam);
-    return R(1.0) / gam(P, m);
+    if (P.eos[m] == TJ_EOS_MIXTURE) return quot(R(1.0), mix_gamma_term(P, m, e.lam));
+    return quot(R(1.0), gam(P, m));
 }
 
 // Sound-speed contribution c^2_m (getSoundSpeedContribution).
@@ -224,36 +225,36 @@ __device__ inline typename PT::real eos_c2(const PT& P, int m, const ECellT<type
     const R* q = P.prm[m];
     R G = gam(P, m);
     switch (P.eos[m]) {
-        case TJ_EOS_MIEGRUNEISEN: return e.p * (G + R(1.0)) / e.rhok - q[1] / e.rhok;  // :61-64
+        case TJ_EOS_MIEGRUNEISEN: return quot(e.p * (G + R(1.0)), e.rhok) - quot(q[1], e.rhok);  // :61-64
         case TJ_EOS_MIXTURE: {  // mixtureSoundSpeed (:208-220)
             const R G1 = q[0] - R(1.0), G2 = q[4] - R(1.0);
-            R dedrho = (e.lam) * ((q[1] - e.p) / (G1 * e.rhok * e.rhok));
-            dedrho += (R(1.0) - e.lam) * ((q[5] - e.p) / (G2 * e.rhok * e.rhok));
-            return (e.p / (e.rhok * e.rhok) - dedrho) / (e.lam / (e.rm0 * G1) + (R(1.0) - e.lam) / (e.rm1 * G2));
+            R dedrho = (e.lam) * (quot(q[1] - e.p, G1 * e.rhok * e.rhok));
+            dedrho += (R(1.0) - e.lam) * (quot(q[5] - e.p, G2 * e.rhok * e.rhok));
+            return quot(quot(e.p, e.rhok * e.rhok) - dedrho, quot(e.lam, e.rm0 * G1) + quot(R(1.0) - e.lam, e.rm1 * G2));
         }
         case TJ_EOS_ROMENSKII: {                                                       // :432-435
-            R a = q[6], K0 = q[5], r0 = q[4], x = e.rhok / r0;
-            R dpc = (K0 / (a * r0)) * tjm_pow(x, a) * ((R(2.0) * a + R(1.0)) * tjm_pow(x, a) - (a + R(1.0)));
+            R a = q[6], K0 = q[5], r0 = q[4], x = quot(e.rhok, r0);
+            R dpc = (quot(K0, a * r0)) * tjm_pow(x, a) * ((R(2.0) * a + R(1.0)) * tjm_pow(x, a) - (a + R(1.0)));
             R dps = e.rhok * eos_dG2drho2(P, m, e) * e.hj2;
-            return (e.p * (G + R(1.0)) - (eos_p_cold(P, m, e) + eos_p_shear(P, m, e)) * (G + R(1.0))) / e.rhok + dpc +
-                   dps + R(4.0 / 3.0) * eos_G(P, m, e) / e.rhok;
+            return quot(e.p * (G + R(1.0)) - (eos_p_cold(P, m, e) + eos_p_shear(P, m, e)) * (G + R(1.0)), e.rhok) + dpc +
+                   dps + quot(R(4.0 / 3.0) * eos_G(P, m, e), e.rhok);
         }
         case TJ_EOS_WILKINS: {  // :533-536
-            R r0 = q[4], x = e.rhok / r0;
-            R dpc = (R(6.0) * q[6] * x * x + R(2.0) * q[7] * x - q[9]) / r0;
+            R r0 = q[4], x = quot(e.rhok, r0);
+            R dpc = quot(R(6.0) * q[6] * x * x + R(2.0) * q[7] * x - q[9], r0);
             R dps = e.rhok * eos_dG2drho2(P, m, e) * e.hj2;
-            return (e.p * (G + R(1.0)) - (eos_p_cold(P, m, e) + eos_p_shear(P, m, e)) * (G + R(1.0))) / e.rhok + dpc +
-                   dps + R(4.0 / 3.0) * eos_G(P, m, e) / e.rhok;
+            return quot(e.p * (G + R(1.0)) - (eos_p_cold(P, m, e) + eos_p_shear(P, m, e)) * (G + R(1.0)), e.rhok) + dpc +
+                   dps + quot(R(4.0 / 3.0) * eos_G(P, m, e), e.rhok);
         }
         default: {  // Mie-Gruneisen sound speed on the Hugoniot reference curve
             R r0 = q[4], c0 = q[5], sl = q[6], G0 = q[7];
-            R rho = e.rhok, et = R(1.0) - r0 / rho, dd = R(1.0) - sl * et;
-            R ph = r0 * c0 * c0 * et / (dd * dd);
-            R dph = r0 * c0 * c0 * (R(1.0) + sl * et) / (dd * dd * dd);
-            R detadrho = r0 / (rho * rho);
+            R rho = e.rhok, et = R(1.0) - quot(r0, rho), dd = R(1.0) - sl * et;
+            R ph = quot(r0 * c0 * c0 * et, dd * dd);
+            R dph = quot(r0 * c0 * c0 * (R(1.0) + sl * et), dd * dd * dd);
+            R detadrho = quot(r0, rho * rho);
             R dp = dph * detadrho;
-            R de = (ph + et * dph) / (R(2.0) * r0) * detadrho;
-            return dp - G * rho * de + (e.p * (G + R(1.0)) - ph) / rho + R(4.0 / 3.0) * G0 / rho;
+            R de = quot(ph + et * dph, R(2.0) * r0) * detadrho;
+            return dp - G * rho * de + quot(e.p * (G + R(1.0)) - ph, rho) + quot(R(4.0 / 3.0) * G0, rho);
         }
     }
 }
@@ -289,9 +290,9 @@ __device__ inline void invert3(const R* M, R* Minv)
       c12 = R(-1.0) * det2(M[0], M[1], M[6], M[7]);
     R c20 = det2(M[1], M[2], M[4], M[5]), c21 = R(-1.0) * det2(M[0], M[2], M[3], M[5]),
       c22 = det2(M[0], M[1], M[3], M[4]);
-    Minv[0] = c00 / D; Minv[1] = c10 / D; Minv[2] = c20 / D;
-    Minv[3] = c01 / D; Minv[4] = c11 / D; Minv[5] = c21 / D;
-    Minv[6] = c02 / D; Minv[7] = c12 / D; Minv[8] = c22 / D;
+    Minv[0] = quot(c00, D); Minv[1] = quot(c10, D); Minv[2] = quot(c20, D);
+    Minv[3] = quot(c01, D); Minv[4] = quot(c11, D); Minv[5] = quot(c21, D);
+    Minv[6] = quot(c02, D); Minv[7] = quot(c12, D); Minv[8] = quot(c22, D);
 }
 
 // Row-major product, k summed innermost in increasing order (the reference
@@ -354,9 +355,9 @@ __device__ inline void sym3_eig(const R* a_in, R* w, R* q)
             R apr = a[p * 3 + r];
             if (apr == R(0.0)) continue;
             R app = a[p * 3 + p], arr = a[r * 3 + r];
-            R theta = (arr - app) / (R(2.0) * apr);
-            R t = (theta >= R(0.0) ? R(1.0) : R(-1.0)) / (fabs(theta) + sqrt(theta * theta + R(1.0)));
-            R c = R(1.0) / sqrt(t * t + R(1.0));
+            R theta = quot(arr - app, R(2.0) * apr);
+            R t = quot(theta >= R(0.0) ? R(1.0) : R(-1.0), fabs(theta) + root(theta * theta + R(1.0)));
+            R c = quot(R(1.0), root(t * t + R(1.0)));
             R s = t * c;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -415,7 +416,7 @@ __device__ inline void sqrtm3(const R* A, R* Rm)
         for (int j = 0; j < 3; ++j) {
             L[i * 3 + j] = q[i * 3 + j];
             RT[i * 3 + j] = q[j * 3 + i];
-            S[i * 3 + j] = sqrt(w[i]) * (R)(i == j);
+            S[i * 3 + j] = root(w[i]) * (R)(i == j);
         }
     mm3(L, S, tmp);
     mm3(tmp, RT, Rm);
@@ -483,7 +484,7 @@ __device__ inline void stress(const PT& P, CellT<typename PT::real>& c)
             solid = 1;
             Gt += eos_G(P, m, e) * (eos_invG(P, m, e));
         }
-    Gt = Gt / eff_invG(P, c);
+    Gt = quot(Gt, eff_invG(P, c));
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -504,7 +505,7 @@ constexpr int kMaxBisect = 200;
 
 __device__ __forceinline__ double mix_rhob(const CellT<double>& c, double rhoa)  // rhobFunc (:243-246)
 {
-    return (1.0 - c.lam) / (1.0 / c.rhok[0] - c.lam / rhoa);
+    return quot(1.0 - c.lam, quot(1.0, c.rhok[0]) - quot(c.lam, rhoa));
 }
 
 __device__ __forceinline__ int sgn_d(double v) { return (0.0 < v) - (v < 0.0); }
@@ -514,10 +515,10 @@ __device__ inline double mix_bisect_f(const PD& P, CellT<double>& c, double rho_
 {
     c.rm0 = rho_try;
     c.rm1 = mix_rhob(c, rho_try);
-    const double p = (c.E - ke - eff_e_nonthermal(P, c) + eff_p_nonthermal(P, c)) / (eff_invG(P, c));
+    const double p = quot(c.E - ke - eff_e_nonthermal(P, c) + eff_p_nonthermal(P, c), eff_invG(P, c));
     const double* q = P.prm[0];
     // pressureFunction (:251-260)
-    return ((p - q[1]) / (c.rm0 * (q[0] - 1.0) * q[3])) - ((p - q[5]) / (c.rm1 * (q[4] - 1.0) * q[7]));
+    return (quot(p - q[1], c.rm0 * (q[0] - 1.0) * q[3])) - (quot(p - q[5], c.rm1 * (q[4] - 1.0) * q[7]));
 }
 
 template <typename PD>
@@ -526,7 +527,7 @@ __device__ inline int mix_root_find(const PD& P, CellT<double>& c, double ke)
     const double* q = P.prm[0];
     const double lam = c.lam, rk = c.rhok[0];
     if (q[1] == 0.0 && q[5] == 0.0) {
-        c.rm0 = rk * (lam + (1.0 - lam) * ((q[4] - 1.0) * q[7]) / ((q[0] - 1.0) * q[3]));
+        c.rm0 = rk * (lam + quot((1.0 - lam) * ((q[4] - 1.0) * q[7]), (q[0] - 1.0) * q[3]));
         c.rm1 = mix_rhob(c, c.rm0);
         return 0;
     }
@@ -555,7 +556,7 @@ __device__ inline int mix_root_find(const PD& P, CellT<double>& c, double ke)
         if (sgn_d(mix_bisect_f(P, c, mid, ke)) == sgn_d(mix_bisect_f(P, c, A, ke))) A = mid;
         else B = mid;
         mid = 0.5 * (A + B);
-        if (fabs(A - B) / (A + B) < 1E-7) {
+        if (quot(fabs(A - B), A + B) < 1E-7) {
             c.rm0 = mid;
             c.rm1 = mix_rhob(c, c.rm0);
             return 0;
@@ -587,8 +588,8 @@ __device__ __forceinline__ void closure_terms64(const P32& P, int m, const ECell
         case TJ_EOS_HUGONIOT: {
             const double aG = e.alpha * P.rG[m];
             const double r0 = q[4], c0 = q[5], sl = q[6];
-            const double et = 1.0 - r0 / e.rhok, dd = 1.0 - sl * et;
-            const double ph = r0 * c0 * c0 * et / (dd * dd);
+            const double et = 1.0 - quot(r0, e.rhok), dd = 1.0 - sl * et;
+            const double ph = quot(r0 * c0 * c0 * et, dd * dd);
             ent += e.arho * (ph * et * P.rR0h[m]) + e.alpha * (q[7] * e.hj2);
             pnt += aG * ph - aG * (q[7] * e.hj2);
             ig += aG;
@@ -620,15 +621,15 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
     int err = 0;
     c.rho = 0;
     for (int m = 0; m < P.M; ++m) {
-        c.rhok[m] = c.arho[m] / c.alpha[m];
+        c.rhok[m] = quot(c.arho[m], c.alpha[m]);
         c.rho += c.arho[m];
-        if (P.plastic && P.phase[m] == TJ_PHASE_SOLID) c.eps[m] = c.are[m] / c.arho[m];
+        if (P.plastic && P.phase[m] == TJ_PHASE_SOLID) c.eps[m] = quot(c.are[m], c.arho[m]);
     }
     hencky(P, c);
     R ke = R(0.0);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        c.vel[r] = c.rhou[r] / c.rho;
+        c.vel[r] = quot(c.rhou[r], c.rho);
         ke += R(0.5) * c.rho * c.vel[r] * c.vel[r];
     }
     if constexpr (sizeof(R) == 4) {
@@ -642,7 +643,7 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
             acc_pair32(sh, sl, -ke);
             acc_pair32(sh, sl, -ent);
             acc_pair32(sh, sl, pnt);
-            c.p = __fadd_rn(sh, sl) / ig;
+            c.p = quot(__fadd_rn(sh, sl), ig);
             stress(P, c);
             return err;
         }
@@ -652,10 +653,10 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
         double rho = 0.0, ent = 0.0, pnt = 0.0, ig = 0.0;
         for (int m = 0; m < P.M; ++m) rho += (double)c.arho[m];
         const double ru0 = c.rhou[0], ru1 = c.rhou[1], ru2 = c.rhou[2];
-        const double ked = 0.5 * (ru0 * ru0 + ru1 * ru1 + ru2 * ru2) / rho;
+        const double ked = quot(0.5 * (ru0 * ru0 + ru1 * ru1 + ru2 * ru2), rho);
         double lam = 0.0, rm0 = 0.0, rm1 = 0.0;
         if (P.nmix) {
-            lam = (double)c.arl / (double)c.arho[0];
+            lam = quot((double)c.arl, (double)c.arho[0]);
             CellT<double> cd;
             for (int m = 0; m < P.M; ++m) {
                 cd.alpha[m] = c.alpha[m];
@@ -693,14 +694,14 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
                 closure_terms64(P, m, e, ent, pnt, ig);
             }
         }
-        c.p = (R)(((double)c.E + (double)c.Elo - ked - ent + pnt) / ig);
+        c.p = (R)(quot((double)c.E + (double)c.Elo - ked - ent + pnt, ig));
     } else {
         if (P.nmix) {  // :104-113
-            c.lam = c.arl / c.arho[0];
+            c.lam = quot(c.arl, c.arho[0]);
             // binary64 only: the tangent instance takes no mixtures
             if constexpr (std::is_same<R, double>::value) err = mix_root_find(P, c, ke);
         }
-        c.p = (c.E - ke - eff_e_nonthermal(P, c) + eff_p_nonthermal(P, c)) / (eff_invG(P, c));
+        c.p = quot(c.E - ke - eff_e_nonthermal(P, c) + eff_p_nonthermal(P, c), eff_invG(P, c));
     }
     stress(P, c);
     return err;
@@ -719,9 +720,9 @@ __device__ inline void p2c(const PT& P, CellT<typename PT::real>& c)
             c.arl = c.lam * c.alpha[0] * c.rhok[0];
             // defineMixtureDensities (equationofstate.cpp:390-396)
             const R* q = P.prm[0];
-            c.rm0 = c.rhok[0] * (c.lam + (R(1.0) - c.lam) * ((c.p - q[1]) / (c.p - q[5])) *
-                                             ((q[7] * (q[4] - R(1.0))) / (q[3] * (q[0] - R(1.0)))));
-            c.rm1 = (R(1.0) - c.lam) / (R(1.0) / c.rhok[0] - c.lam / c.rm0);
+            c.rm0 = c.rhok[0] * (c.lam + (R(1.0) - c.lam) * (quot(c.p - q[1], c.p - q[5])) *
+                                             (quot(q[7] * (q[4] - R(1.0)), q[3] * (q[0] - R(1.0)))));
+            c.rm1 = quot(R(1.0) - c.lam, quot(R(1.0), c.rhok[0]) - quot(c.lam, c.rm0));
         }
         if (P.plastic && P.phase[m] == TJ_PHASE_SOLID) c.are[m] = c.eps[m] * c.arho[m];
     }
@@ -745,12 +746,12 @@ __device__ inline typename PT::real sound_speed(const PT& P, const CellT<typenam
     for (int m = 0; m < P.M; ++m) {
         ECellT<R> e = ecell_of(c, m);
         R xi = eos_xi(P, m, e);
-        R v = xi * eos_c2(P, m, e) * c.arho[m] / c.rho;
+        R v = quot(xi * eos_c2(P, m, e) * c.arho[m], c.rho);
         a += (R(0.0) < v) ? v : R(0.0);
         xit += xi * c.alpha[m];
     }
     if (a <= R(0.0)) a = R(1E-6);
-    return sqrt(a / xit);
+    return root(quot(a, xit));
 }
 
 // cleanUpAlpha on one cell (:530-599). Returns TJ_ERR_ALPHA on the
@@ -773,11 +774,13 @@ __device__ inline int cleanup_alpha(const PT& P, typename PT::real* alpha)
         tot += a;
     }
     if (nan > 0) {
-        alpha[nan] = R(1.0) - tot;
-        tot += alpha[nan];
+        const R a = R(1.0) - tot;
+        for (int m = 0; m < P.M; ++m)  // no index that is not a constant: alpha stays in registers
+            if (m == nan) alpha[m] = a;
+        tot += a;
     }
     if (tot <= R(0.0)) return TJ_ERR_ALPHA;
-    for (int m = 0; m < P.M; ++m) alpha[m] *= R(1.0) / tot;
+    for (int m = 0; m < P.M; ++m) alpha[m] *= quot(R(1.0), tot);
     return 0;
 }
 
@@ -791,10 +794,10 @@ __device__ inline typename PT::real transverse_speed(const PT& P, CellT<typename
     for (int m = 0; m < P.M; ++m)
         if (P.phase[m] == TJ_PHASE_SOLID) {
             ECellT<R> e = ecell_of(c, m);
-            b += eos_invG(P, m, e) * eos_G(P, m, e) / (c.rhok[m]);
+            b += quot(eos_invG(P, m, e) * eos_G(P, m, e), c.rhok[m]);
         }
     if (isnan(b) || b < R(0.0)) b = R(0.0);
-    R t = sqrt(b / eff_invG(P, c));
+    R t = root(quot(b, eff_invG(P, c)));
     if (isnan(t)) t = R(0.0);
     return t;
 }

@@ -35,8 +35,8 @@ __device__ __forceinline__ Dual operator-(Dual a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, dmul(a.d, b.v) + dmul(b.d, a.v)); }
 __device__ __forceinline__ Dual operator/(Dual a, Dual b)
 {
-    const double q = a.v / b.v;
-    return Dual(q, (b.d != 0.0 ? (a.d - q * b.d) / b.v : (a.d != 0.0 ? a.d / b.v : 0.0)));
+    const double q = quot(a.v, b.v);
+    return Dual(q, (b.d != 0.0 ? quot(a.d - q * b.d, b.v) : (a.d != 0.0 ? quot(a.d, b.v) : 0.0)));
 }
 __device__ __forceinline__ Dual operator+(Dual a, double b) { return Dual(a.v + b, a.d); }
 __device__ __forceinline__ Dual operator+(double a, Dual b) { return Dual(a + b.v, b.d); }
@@ -44,11 +44,11 @@ __device__ __forceinline__ Dual operator-(Dual a, double b) { return Dual(a.v - 
 __device__ __forceinline__ Dual operator-(double a, Dual b) { return Dual(a - b.v, -b.d); }
 __device__ __forceinline__ Dual operator*(Dual a, double b) { return Dual(a.v * b, dmul(a.d, b)); }
 __device__ __forceinline__ Dual operator*(double a, Dual b) { return Dual(a * b.v, dmul(b.d, a)); }
-__device__ __forceinline__ Dual operator/(Dual a, double b) { return Dual(a.v / b, a.d != 0.0 ? a.d / b : 0.0); }
+__device__ __forceinline__ Dual operator/(Dual a, double b) { return Dual(quot(a.v, b), a.d != 0.0 ? quot(a.d, b) : 0.0); }
 __device__ __forceinline__ Dual operator/(double a, Dual b)
 {
-    const double q = a / b.v;
-    return Dual(q, b.d != 0.0 ? -q * b.d / b.v : 0.0);
+    const double q = quot(a, b.v);
+    return Dual(q, b.d != 0.0 ? quot(-q * b.d, b.v) : 0.0);
 }
 __device__ __forceinline__ Dual& operator+=(Dual& a, Dual b) { return a = a + b; }
 __device__ __forceinline__ Dual& operator-=(Dual& a, Dual b) { return a = a - b; }
@@ -78,22 +78,25 @@ __device__ __forceinline__ bool isinf(Dual a) { return ::isinf(a.v); }
 __device__ __forceinline__ Dual fabs(Dual a) { return a.v < 0.0 ? -a : a; }
 // d sqrt(x) = dx / (2 sqrt(x)); a zero direction stays zero at x = 0 (the
 // Hencky J2 of an undeformed cell)
-__device__ __forceinline__ Dual sqrt(Dual a)
+__device__ __forceinline__ Dual root(Dual a)
 {
-    const double s = ::sqrt(a.v);
-    return Dual(s, a.d == 0.0 ? 0.0 : a.d / (2.0 * s));
+    const double s = root(a.v);
+    return Dual(s, a.d == 0.0 ? 0.0 : quot(a.d, 2.0 * s));
 }
+__device__ __forceinline__ Dual quot(Dual a, Dual b) { return a / b; }
+// a constant argument
+__device__ __forceinline__ Dual sqrt(Dual a) { return root(a); }
 __device__ __forceinline__ Dual tjm_exp(Dual a)
 {
     const double e = tjm_exp(a.v);
     return Dual(e, dmul(a.d, e));
 }
-__device__ __forceinline__ Dual tjm_log(Dual a) { return Dual(tjm_log(a.v), a.d != 0.0 ? a.d / a.v : 0.0); }
+__device__ __forceinline__ Dual tjm_log(Dual a) { return Dual(tjm_log(a.v), a.d != 0.0 ? quot(a.d, a.v) : 0.0); }
 __device__ __forceinline__ Dual tjm_pow(Dual x, Dual y)
 {
     const double p = tjm_pow(x.v, y.v);
     double d = 0.0;
-    if (x.d != 0.0) d += p * y.v * x.d / x.v;
+    if (x.d != 0.0) d += quot(p * y.v * x.d, x.v);
     if (y.d != 0.0) d += p * ::log(x.v) * y.d;
     return Dual(p, d);
 }
@@ -141,14 +144,14 @@ __device__ inline void sqrtm3(const Dual* A, Dual* Rm)
         for (int j = 0; j < 3; ++j) t[i * 3 + j] = da[i * 3 + 0] * q[0 * 3 + j] + da[i * 3 + 1] * q[1 * 3 + j] + da[i * 3 + 2] * q[2 * 3 + j];
     double sw[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) sw[i] = ::sqrt(w[i] > 0.0 ? w[i] : 0.0);
+    for (int i = 0; i < 3; ++i) sw[i] = root(w[i] > 0.0 ? w[i] : 0.0);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const double v = q[0 * 3 + i] * t[0 * 3 + j] + q[1 * 3 + i] * t[1 * 3 + j] + q[2 * 3 + i] * t[2 * 3 + j];
             const double den = sw[i] + sw[j];
-            dp[i * 3 + j] = den > 0.0 ? v / den : 0.0;
+            dp[i * 3 + j] = den > 0.0 ? quot(v, den) : 0.0;
         }
     // dS = Q dS' Q^T
 #pragma unroll

@@ -19,11 +19,11 @@ __device__ inline void muscl1(Dual um, Dual u0, Dual up, Dual& l, Dual& r)
 {
     double lv, rv;
     muscl1(um.v, u0.v, up.v, lv, rv);
-    double rr = (u0.v - um.v) / (up.v - u0.v);
+    double rr = quot(u0.v - um.v, up.v - u0.v);
     if (isinf(rr) || isnan(rr)) rr = 0.0;
     double dg = 0.0;
     if (rr > 0.0) {
-        const double a = 2.0 / (1.0 + rr), b = 2.0 * rr / (1.0 + rr);
+        const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);
         dg = (b < a) ? u0.d - um.d : up.d - u0.d;
     }
     l = Dual(lv, u0.d - 0.5 * dg);

@@ -17,6 +17,8 @@
 //   tanh:  t/(t+2), t = expm1(2|x|), with the sign of x.
 #pragma once
 
+#include "tj_quot.h"
+
 namespace tj {
 
 #define TJM_LN2_HI 0x1.62e42fee00000p-1
@@ -76,7 +78,7 @@ __device__ inline double tjm_log(double x)
         e = e - 1;
     }
     double f = m - 1.0;
-    double s = f / (2.0 + f);
+    double s = quot(f, 2.0 + f);
     double z = s * s;
     // 1/(2k+1), k = 12 .. 0, rounded to nearest
     double q = 0x1.47ae147ae147bp-5;
@@ -116,7 +118,7 @@ __device__ inline double tjm_cosh(double x)
         return (0.5 * t) * t;
     }
     double t = tjm_exp(a);
-    return 0.5 * t + 0.5 / t;
+    return 0.5 * t + quot(0.5, t);
 }
 
 __device__ inline double tjm_tanh(double x)
@@ -127,7 +129,7 @@ __device__ inline double tjm_tanh(double x)
     if (a > 22.0) r = 1.0;
     else {
         double t = tjm_expm1(2.0 * a);
-        r = t / (t + 2.0);
+        r = quot(t, t + 2.0);
     }
     return copysign(r, x);
 }

@@ -373,18 +373,39 @@ template <typename R>
 __device__ __forceinline__ R vanleer(R r)  // hllc.cpp:527-537
 {
     if (r <= R(0.0)) return R(0.0);
-    R a = R(2.0) / (R(1.0) + r), b = R(2.0) * r / (R(1.0) + r);
+    R a = quot(R(2.0), R(1.0) + r), b = quot(R(2.0) * r, R(1.0) + r);
     return (b < a) ? b : a;
 }
 
 template <typename R>
 __device__ __forceinline__ void muscl1(R um, R u0, R up, R& l, R& r)  // hllc.cpp:557-568
 {
-    R rr = (u0 - um) / (up - u0);
+    R rr = quot(u0 - um, up - u0);
     if (isinf(rr) || isnan(rr)) rr = R(0.0);
     R grad = vanleer(rr) * R(0.5) * (up - um);
     l = u0 - R(0.5) * grad;
     r = u0 + R(0.5) * grad;
+}
+
+// The same in binary64 with the same bits and fewer operations of that pipe:
+// a ratio that is not positive and finite gives slope 0 without a division;
+// of the limiter's two quotients 2 / (1 + r) and 2 r / (1 + r) the smaller is
+// the one with the smaller numerator (rounding is monotonic), so one is formed;
+// and the factors of one half are exact, so they go into that quotient and
+// into the fused multiply-adds (7 binary64 operations instead of about 45).
+__device__ __forceinline__ void muscl1(double um, double u0, double up, double& l, double& r)
+{
+    const double num = u0 - um, den = up - u0;
+    const int hn = __double2hiint(num), hd = __double2hiint(den);
+    double half = 0.0;
+    if ((hn ^ hd) >= 0 && ((hn << 1) | __double2loint(num)) != 0 && ((hd << 1) | __double2loint(den)) != 0) {
+        const double rr = quot(num, den);
+        if ((__double2hiint(rr) & 0x7ff00000) != 0x7ff00000)  // finite
+            half = quot(__double2hiint(rr) < 0x3ff00000 ? rr : 1.0, 1.0 + rr);
+    }
+    const double grad = half * (up - um);
+    l = fma(-0.5, grad, u0);
+    r = fma(0.5, grad, u0);
 }
 
 // One carried word at a possibly-ghost cell.
@@ -416,10 +437,10 @@ __device__ inline R youngs(const PT& P, const DevDomain& D, const R* X, long lon
 {
     int a = P.S_ALPHA + m;
 #define NB(di, dj) gv(P, D, X, nt, a, i + (di), j + (dj), k)
-    R nx = -R(1.0) / (R(8.0) * (R)D.dx[0]) * (NB(1, 1) + R(2.0) * NB(1, 0) + NB(1, -1) - NB(-1, 1) - R(2.0) * NB(-1, 0) - NB(-1, -1));
-    R ny = -R(1.0) / (R(8.0) * (R)D.dx[1]) * (NB(1, 1) + R(2.0) * NB(0, 1) + NB(-1, 1) - NB(-1, -1) - R(2.0) * NB(0, -1) - NB(1, -1));
+    R nx = quot(-R(1.0), R(8.0) * (R)D.dx[0]) * (NB(1, 1) + R(2.0) * NB(1, 0) + NB(1, -1) - NB(-1, 1) - R(2.0) * NB(-1, 0) - NB(-1, -1));
+    R ny = quot(-R(1.0), R(8.0) * (R)D.dx[1]) * (NB(1, 1) + R(2.0) * NB(0, 1) + NB(-1, 1) - NB(-1, -1) - R(2.0) * NB(0, -1) - NB(1, -1));
 #undef NB
-    R norm = sqrt(nx * nx + ny * ny);
+    R norm = root(nx * nx + ny * ny);
     if (norm < R(1E-20)) return 0;
     return d == 0 ? fabs(nx / norm) : fabs(ny / norm);
 }
@@ -440,7 +461,7 @@ __device__ inline void thinc_cand(const PT& P, const DevDomain& D, const R* X, l
         R mn = (aR < aL) ? aR : aL;
         R mx = ((aL < aR) ? aR : aL) - mn;
         R theta = (R)((R(0.0) < aR - aL) - (aR - aL < R(0.0)));
-        R C = (mx < eps) ? R(0.0) : (a0 - mn + eps) / (mx + eps);
+        R C = (mx < eps) ? R(0.0) : quot(a0 - mn + eps, mx + eps);
         R delta = R(1E-4);
         int mixed = (C > delta) && (C < (R(0.999999) - delta)) && ((aR - a0) * (a0 - aL) >= R(0.0));
         t.mixed[m] = mixed;
@@ -452,9 +473,9 @@ __device__ inline void thinc_cand(const PT& P, const DevDomain& D, const R* X, l
             R beta = nvc * beta0 + R(0.01);
             R coshB = tjm_cosh(beta), tanhB = tjm_tanh(beta);
             R B = tjm_exp(theta * beta * ((R(2.0) * C) - R(1.0)));
-            R A = ((B / coshB) - R(1.0)) / tanhB;
-            t.Rv[m] = mn + (mx / R(2.0)) * (R(1.0) + theta * ((tanhB + A) / (R(1.0) + A * tanhB)));
-            t.L[m] = mn + (mx / R(2.0)) * (R(1.0) + theta * A);
+            R A = quot((quot(B, coshB)) - R(1.0), tanhB);
+            t.Rv[m] = mn + (mx * R(0.5)) * (R(1.0) + theta * (quot(tanhB + A, R(1.0) + A * tanhB)));
+            t.L[m] = mn + (mx * R(0.5)) * (R(1.0) + theta * A);
         }
     }
 }
@@ -607,14 +628,19 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
 template <typename PT, typename R = typename PT::real>
 __device__ inline void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, R SK, R Ss, int d)  // :12-73
 {
-    const R tol = R(1E-20);
     R ud = U.vel[d];
-    R mult = (fabs((Ss - ud) / Ss) < tol ? R(1.0) : (SK - ud) / (SK - Ss));
+    // |(Ss - ud) / Ss| < 1e-20: the difference of two binary64 numbers that
+    // differ is not smaller than 2^-54 of either, so the quotient is that small
+    // only when they are equal (and not zero)
+    bool contact;
+    if constexpr (sizeof(R) == 4) contact = fabs((Ss - ud) / Ss) < R(1E-20);
+    else contact = Ss - ud == R(0.0) && Ss != R(0.0);
+    R mult = contact ? R(1.0) : quot(SK - ud, SK - Ss);
     Us.rho = R(0.0);
     for (int m = 0; m < P.M; ++m) {
         Us.alpha[m] = U.alpha[m];
         Us.arho[m] = mult * U.arho[m];
-        Us.rhok[m] = Us.arho[m] / Us.alpha[m];
+        Us.rhok[m] = quot(Us.arho[m], Us.alpha[m]);
         if (P.nmix && m == 0) Us.arl = mult * U.arl;
         // a fluid carries no plastic strain: its alphaRhoEps star value is 0
         // (the reference writes only the plastic materials' and resets the
@@ -626,13 +652,13 @@ __device__ inline void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, 
     for (int row = 0; row < 3; ++row) {
         if (row == d) Us.rhou[row] = mult * U.rho * Ss;
         else Us.rhou[row] = mult * U.rhou[row];
-        Us.vel[row] = Us.rhou[row] / Us.rho;
+        Us.vel[row] = quot(Us.rhou[row], Us.rho);
         if (P.solid)
 #pragma unroll
             for (int col = 0; col < 3; ++col)
                 Us.V[3 * row + col] = (row == d) ? U.V[3 * row + col] : mult * U.V[3 * row + col];
     }
-    Us.E = mult * U.rho * (U.E / U.rho + (Ss - ud) * (Ss - (U.sigma[4 * d]) / (U.rho * (SK - ud))));
+    Us.E = mult * U.rho * (quot(U.E, U.rho) + (Ss - ud) * (Ss - quot(U.sigma[4 * d], U.rho * (SK - ud))));
 }
 
 // The conservative variables of one state, or their fluxes, by name: kept in
@@ -754,8 +780,7 @@ __device__ inline int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& 
     R x1 = fabs(L.vel[d]) + L.a, x2 = fabs(Rc.vel[d]) + Rc.a;
     R SR = (x1 < x2) ? x2 : x1;
     R SL = -SR;
-    Ss = (-Rc.sigma[4 * d] + L.sigma[4 * d] + L.rhou[d] * (SL - L.vel[d]) - Rc.rhou[d] * (SR - Rc.vel[d])) /
-         (L.rho * (SL - L.vel[d]) - Rc.rho * (SR - Rc.vel[d]));  // getSstar, hllc.cpp:5-8
+    Ss = quot(-Rc.sigma[4 * d] + L.sigma[4 * d] + L.rhou[d] * (SL - L.vel[d]) - Rc.rhou[d] * (SR - Rc.vel[d]), L.rho * (SL - L.vel[d]) - Rc.rho * (SR - Rc.vel[d]));  // getSstar, hllc.cpp:5-8
     if (!P.solid) {
         // the state K of the upwind side and its star state (no pointer or
         // reference selects between L and Rc: both stay in registers)
@@ -797,22 +822,21 @@ __device__ inline int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& 
 #pragma unroll
         for (int i = 0; i < 3; ++i)  // getSigmaStar, hllc.cpp:75-83
             UKs.sigma[3 * i + d] =
-                (Ls.rho * (Ss - SLT) * Rs.rho * (Ss - SRT) * (L.vel[i] - Rc.vel[i]) + Ls.rho * (Ss - SLT) * Rc.sigma[3 * i + d] -
-                 Rs.rho * (Ss - SRT) * L.sigma[3 * i + d]) /
-                (Ls.rho * (Ss - SLT) - Rs.rho * (Ss - SRT));
+                quot(Ls.rho * (Ss - SLT) * Rs.rho * (Ss - SRT) * (L.vel[i] - Rc.vel[i]) + Ls.rho * (Ss - SLT) * Rc.sigma[3 * i + d] -
+                 Rs.rho * (Ss - SRT) * L.sigma[3 * i + d], Ls.rho * (Ss - SLT) - Rs.rho * (Ss - SRT));
 #pragma unroll
         for (int row = 0; row < 3; ++row) {
             if (row == d) continue;
-            Uss.rhou[row] += (UKs.sigma[3 * row + d] - UK.sigma[3 * row + d]) / (Ss - SKT);
-            Uss.vel[row] = Uss.rhou[row] / Uss.rho;
+            Uss.rhou[row] += quot(UKs.sigma[3 * row + d] - UK.sigma[3 * row + d], Ss - SKT);
+            Uss.vel[row] = quot(Uss.rhou[row], Uss.rho);
         }
 #pragma unroll
         for (int row = 0; row < 3; ++row) {
             if (row == d) continue;
-            Uss.E += (Uss.vel[row] * UKs.sigma[3 * row + d] - UK.vel[row] * UK.sigma[3 * row + d]) / (Ss - SKT);
+            Uss.E += quot(Uss.vel[row] * UKs.sigma[3 * row + d] - UK.vel[row] * UK.sigma[3 * row + d], Ss - SKT);
 #pragma unroll
             for (int col = 0; col < 3; ++col)
-                Uss.V[3 * row + col] += (Uss.V[3 * d + col] * (Uss.vel[row] - UK.vel[row])) / (Ss - SKT);
+                Uss.V[3 * row + col] += quot(Uss.V[3 * d + col] * (Uss.vel[row] - UK.vel[row]), Ss - SKT);
         }
     };
     if (SL >= R(0.0)) {
@@ -938,9 +962,9 @@ __device__ inline int plastic_cell(const PT& P, CellT<R>& c)
     for (int m = 0; m < P.M; ++m) {
         ECellT<R> e = ecell_of(c, m);
         if (P.phase[m] == TJ_PHASE_SOLID) {
-            J = sqrt(c.hj2);
+            J = root(c.hj2);
             R G = eos_G(P, m, e);
-            if (G * J * sqrt(R(3.0)) > P.yield[m]) Jn = P.yield[m] / (sqrt(R(3.0)) * G);
+            if (G * J * sqrt(R(3.0)) > P.yield[m]) Jn = quot(P.yield[m], sqrt(R(3.0)) * G);
             else Jn = J;
             c.eps[m] += sqrt(R(2.0) / R(3.0)) * (J - Jn);
             c.are[m] = c.eps[m] * c.arho[m];
@@ -954,8 +978,8 @@ __device__ inline int plastic_cell(const PT& P, CellT<R>& c)
         JT += (eos_invG(P, m, e)) * Jn;
         norm += (eos_invG(P, m, e));
     }
-    JB *= R(1.0) / norm;
-    JT *= R(1.0) / norm;
+    JB *= quot(R(1.0), norm);
+    JT *= quot(R(1.0), norm);
     if (JB == R(0.0) && JT == R(0.0)) { JB = R(1.0); JT = R(1.0); }
     R t1[9], t2[9], t2i[9];
 #pragma unroll
@@ -964,7 +988,7 @@ __device__ inline int plastic_cell(const PT& P, CellT<R>& c)
         for (int q = 0; q < 3; ++q) {
             R& dv = c.devH[3 * r + q];
             if (dv != R(0.0) && JB == R(0.0) && JT != R(0.0)) return TJ_ERR_PLASTIC;
-            dv *= JT / JB;
+            dv *= quot(JT, JB);
             t1[3 * r + q] = (R)(r == q) + R(0.5) * dv;
             t2[3 * r + q] = (R)(r == q) - R(0.5) * dv;
         }
@@ -1006,9 +1030,9 @@ __device__ inline int plastic_cell_proj64(const PT& P, CellT<R>& c)
         e.rm1 = c.rm1;
         double J, Jn;
         if (P.phase[m] == TJ_PHASE_SOLID) {
-            J = sqrt(hj2);
+            J = root(hj2);
             const double G = eos_G(PD, m, e);
-            Jn = (G * J * sqrt(3.0) > PD.yield[m]) ? PD.yield[m] / (sqrt(3.0) * G) : J;
+            Jn = (G * J * sqrt(3.0) > PD.yield[m]) ? quot(PD.yield[m], sqrt(3.0) * G) : J;
             const double eps = (double)c.eps[m] + sqrt(2.0 / 3.0) * (J - Jn);
             c.eps[m] = (R)eps;
             c.are[m] = (R)(eps * (double)c.arho[m]);
@@ -1023,8 +1047,8 @@ __device__ inline int plastic_cell_proj64(const PT& P, CellT<R>& c)
         JT += ig * Jn;
         norm += ig;
     }
-    JB *= 1.0 / norm;
-    JT *= 1.0 / norm;
+    JB *= quot(1.0, norm);
+    JT *= quot(1.0, norm);
     if (JB == 0.0 && JT == 0.0) { JB = 1.0; JT = 1.0; }
     R t1[9], t2[9], t2i[9];
 #pragma unroll
@@ -1033,7 +1057,7 @@ __device__ inline int plastic_cell_proj64(const PT& P, CellT<R>& c)
         for (int q = 0; q < 3; ++q) {
             R& dv = c.devH[3 * r + q];
             if (dv != R(0.0) && JB == 0.0 && JT != 0.0) return TJ_ERR_PLASTIC;
-            dv = (R)((double)dv * (JT / JB));
+            dv = (R)((double)dv * (quot(JT, JB)));
             t1[3 * r + q] = (R)(r == q) + R(0.5) * dv;
             t2[3 * r + q] = (R)(r == q) - R(0.5) * dv;
         }
@@ -1057,7 +1081,7 @@ __device__ inline void cleanup_v_cell(const PT& P, CellT<R>& c)
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) c.V[3 * r + q] = ((Sq[3 * r + q] * norm * ts) + (R)(r == q) * (ta - ts)) / ta;
+        for (int q = 0; q < 3; ++q) c.V[3 * r + q] = quot((Sq[3 * r + q] * norm * ts) + (R)(r == q) * (ta - ts), ta);
 }
 
 // contains_nan over the conservative and primitive lists of one cell.
@@ -1087,7 +1111,7 @@ __device__ __forceinline__ R reactive_euler(R arl, R arho, R p, R alpha, R dt)
 {
     const R sigma = R(20.0), nu = R(0.5), n = R(1.2);
     if (alpha < R(0.5)) return arl;
-    R r = arl - (dt) * (sigma * tjm_pow(arho, R(1.0) - nu) * tjm_pow(arl, nu) * tjm_pow((p / R(1E6)), n));
+    R r = arl - (dt) * (sigma * tjm_pow(arho, R(1.0) - nu) * tjm_pow(arl, nu) * tjm_pow((quot(p, R(1E6))), n));
     if (r < R(0.0)) r = R(0.0);
     return r;
 }
@@ -1114,7 +1138,7 @@ __device__ inline int reactive_cell(const PT& P, CellT<R>& c, R dt)
 template <typename PT, typename R = typename PT::real>
 __device__ inline void radial_source(const PT& P, CellT<R>& c, const R* sg, int i, double dx0, R dt)
 {
-    const R inv_r = R(P.dim == 1 ? -2.0 : -1.0) / (((R)i + R(0.5)) * (R)dx0);
+    const R inv_r = quot(R(P.dim == 1 ? -2.0 : -1.0), ((R)i + R(0.5)) * (R)dx0);
     const R s = dt * inv_r;
     const R u = c.vel[0];
     for (int m = 0; m < P.M; ++m) {
@@ -1167,7 +1191,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
     load_state(P, X, nt, g, nullptr, U);
     if (first) Yc = U;
     else load_state(P, Y, nt, g, nullptr, Yc);
-    const R dtdx = dtdx_num / (R)D.dx[d];
+    const R dtdx = quot(dtdx_num, (R)D.dx[d]);
     for (int m = 0; m < P.M; ++m) {
         Yc.alpha[m] += dtdx * (FXW(P.X_ALPHA + m, 0) - FXW(P.X_ALPHA + m, 1) - U.alpha[m] * (FXW(P.X_SSTAR, 0) - FXW(P.X_SSTAR, 1)));
         Yc.arho[m] += dtdx * (FXW(P.X_ARHO + m, 0) - FXW(P.X_ARHO + m, 1));
@@ -1308,7 +1332,7 @@ __global__ void k_cfl(PT P, PathBufs<typename PT::real> b, const R* __restrict__
         load_state(P, X, nt, g, nullptr, c);
         R a = sound_speed(P, c);
         for (int n = 0; n < P.dim; ++n) {
-            R v = (R)D.dx[n] / (a + fabs(c.vel[n]));
+            R v = quot((R)D.dx[n], a + fabs(c.vel[n]));
             if (v < mn) mn = v;
         }
     }
