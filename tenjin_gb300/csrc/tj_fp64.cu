@@ -24,13 +24,6 @@ namespace tj {
 
 static constexpr int kThreads = 256;
 
-static inline int nblocks(long long n, int cap = 152 * 16)
-{
-    long long b = (n + kThreads - 1) / kThreads;
-    if (b < 1) b = 1;
-    if (b > cap) b = cap;
-    return (int)b;
-}
 
 
 __global__ void k_dt_finalize(DevParams P, DevScalars* s, int clamp)
@@ -396,7 +389,8 @@ int fp64_set_dt(const Fp64Bufs& b, double dt, cudaStream_t st)
 
 int fp64_cell_op(const DevParams& P, const Fp64Bufs& b, double* X, const double* X2, int op, cudaStream_t st, double dt)
 {
-    k_cell_op<<<nblocks(b.ntot), kThreads, 0, st>>>(P, b, X, X2, op, dt);
+    const LaunchShape sh = launch_shape(b.ntot, 64);
+    k_cell_op<<<sh.blocks, sh.threads, 0, st>>>(P, b, X, X2, op, dt);
     return 1;
 }
 
@@ -405,7 +399,8 @@ int fp64_ap_to_state(const DevParams& P, const Fp64Bufs& b, int dom, const int* 
 {
     (void)ld_k;
     int nx = bx[3] - bx[0] + 1, ny = bx[4] - bx[1] + 1, nz = bx[5] - bx[2] + 1;
-    k_ap_to_state<<<nblocks((long long)nx * ny * nz), kThreads, 0, st>>>(P, b, dom, bx[0], bx[1], bx[2], nx, ny, nz, ap, ld_i,
+    const LaunchShape sh = launch_shape((long long)nx * ny * nz, 64);
+    k_ap_to_state<<<sh.blocks, sh.threads, 0, st>>>(P, b, dom, bx[0], bx[1], bx[2], nx, ny, nz, ap, ld_i,
                                                                          ld_j, cs, go, X);
     return 1;
 }
@@ -417,14 +412,16 @@ int fp64_state_to_ap(const DevParams& P, const Fp64Bufs& b, int dom, const int* 
     int nx = bx[3] - bx[0] + 1, ny = bx[4] - bx[1] + 1, nz = bx[5] - bx[2] + 1;
     if (t1 < 0) t1 = (long long)nx * ny * nz;
     if (t1 <= t0) return 0;
-    k_state_to_ap<<<nblocks(t1 - t0), kThreads, 0, st>>>(P, b, dom, bx[0], bx[1], bx[2], nx, ny, nz, X, ap, ld_i, ld_j,
+    const LaunchShape sh = launch_shape(t1 - t0, 64);
+    k_state_to_ap<<<sh.blocks, sh.threads, 0, st>>>(P, b, dom, bx[0], bx[1], bx[2], nx, ny, nz, X, ap, ld_i, ld_j,
                                                          cs, go, t0, t1);
     return 1;
 }
 
 int fp64_prim_to_state(const DevParams& P, const Fp64Bufs& b, int dom, const double* prim, double* X, cudaStream_t st)
 {
-    k_prim_to_state<<<nblocks(b.ntot), kThreads, 0, st>>>(P, b, dom, prim, X);
+    const LaunchShape sh = launch_shape(b.ntot, 64);
+    k_prim_to_state<<<sh.blocks, sh.threads, 0, st>>>(P, b, dom, prim, X);
     return 1;
 }
 
@@ -438,7 +435,8 @@ int fp64_conservation(const DevParams& P, const Fp64Bufs& b, const double* X, do
 int fp64_state_component(const DevParams& P, const Fp64Bufs& b, int dom, const double* X, int comp, double* out,
                          cudaStream_t st)
 {
-    k_state_component<<<nblocks(b.ntot), kThreads, 0, st>>>(P, b, dom, X, comp, out);
+    const LaunchShape sh = launch_shape(b.ntot, 64);
+    k_state_component<<<sh.blocks, sh.threads, 0, st>>>(P, b, dom, X, comp, out);
     return 1;
 }
 

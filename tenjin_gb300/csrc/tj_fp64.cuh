@@ -28,6 +28,26 @@ struct PathBufs {
 };
 using Fp64Bufs = PathBufs<double>;
 
+// Launch shape of a per-cell (or per-face) grid-stride kernel over n entries.
+// A binary64 warp instruction holds its SM's pipe for 16 cycles, so what
+// counts is that every SM has the same number of warps: blocks of 256 put a
+// 1000-cell line on 4 SMs (eight warps taking turns on each) and 65536 cells on
+// 152 SMs as one or two blocks each. The block is halved, from `most` down to
+// one warp, until there are four blocks an SM.
+struct LaunchShape {
+    int blocks, threads;
+};
+inline LaunchShape launch_shape(long long n, int most)
+{
+    constexpr long long kSMs = 152;
+    int t = most;
+    while (t > 32 && n < t * kSMs * 4) t /= 2;
+    long long b = (n + t - 1) / t;
+    if (b < 1) b = 1;
+    if (b > kSMs * 16 * 256 / t) b = kSMs * 16 * 256 / t;
+    return {(int)b, t};
+}
+
 // The binary32 parameter block of a binary64 one (tj_fp32.cu).
 DevParams32 make_params32(const DevParams& P);
 

@@ -30,6 +30,13 @@
 
 namespace tj {
 
+// Registers of the binary64 instances: 128 a thread, so that 16 warps share an
+// SM. With the divisions on the integer units the kernels wait for their own
+// serial chains, and two warps a scheduler (255 registers) hide less of them
+// than four, spills included: bubble 256^2, 20 steps 21.6 / 17.2 / 18.0 ms and
+// copper 40^3, 10 steps 24.6 / 19.5 / 20.3 ms with 4 / 8 / 12 blocks of 64.
+constexpr int kBlocks64 = 8;
+
 // Error-free accumulation of b into the pair (hi, lo) (binary32 energy).
 __device__ __forceinline__ void dd_add32(float& hi, float& lo, float b)
 {
@@ -485,7 +492,7 @@ __device__ inline void thinc_cand(const PT& P, const DevDomain& D, const R* X, l
 // ---------------------------------------------------------------------------
 // DC >= 0: the direction as a compile-time constant (d is then ignored).
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
     k_recon(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
@@ -897,7 +904,7 @@ __device__ inline int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& 
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_flux(PT P, PathBufs<typename PT::real> b, int dyn_d)
+__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64) k_flux(PT P, PathBufs<typename PT::real> b, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
     if (b.scal->done) return;
@@ -1295,7 +1302,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
     k_update(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, R* Y, int dyn_d, int first, int last,
              int finish)
 {

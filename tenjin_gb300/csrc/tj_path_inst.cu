@@ -20,13 +20,12 @@
 namespace tj {
 
 namespace {
-constexpr int kPathThreads = 256;
-inline int path_blocks(long long n, int cap = 152 * 16)
+// binary64 kernels keep eight warps an SM (up to 255 registers): blocks of two
+// warps balance best; binary32 ones hold two blocks of eight.
+template <class PT>
+inline LaunchShape path_shape(long long n)
 {
-    long long b = (n + kPathThreads - 1) / kPathThreads;
-    if (b < 1) b = 1;
-    if (b > cap) b = cap;
-    return (int)b;
+    return launch_shape(n, sizeof(typename PT::real) == 4 ? 256 : 64);
 }
 }  // namespace
 
@@ -38,14 +37,15 @@ int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     const char* nr = f64 ? "tj_recon_fp64" : "tj_recon_fp32";
     const char* nf = f64 ? "tj_flux_fp64" : "tj_flux_fp32";
     const char* nu = f64 ? "tj_update_fp64" : "tj_update_fp32";
+    const LaunchShape cells = path_shape<PT>(b.ntot), faces = path_shape<PT>(b.nftot[d]);
     if (pr) pr->begin(nr, st);
-    k_recon<PT, DC><<<path_blocks(b.ntot), kPathThreads, 0, st>>>(P, b, X, d);
+    k_recon<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, d);
     if (pr) pr->end(nr, st);
     if (pr) pr->begin(nf, st);
-    k_flux<PT, DC><<<path_blocks(b.nftot[d]), kPathThreads, 0, st>>>(P, b, d);
+    k_flux<PT, DC><<<faces.blocks, faces.threads, 0, st>>>(P, b, d);
     if (pr) pr->end(nf, st);
     if (pr) pr->begin(nu, st);
-    k_update<PT, DC><<<path_blocks(b.ntot), kPathThreads, 0, st>>>(P, b, X, Y, d, first, last, finish);
+    k_update<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, d, first, last, finish);
     if (pr) pr->end(nu, st);
     return 3;
 }
@@ -55,7 +55,8 @@ int path_cfl(const PT& P, const PathBufs<typename PT::real>& b, const typename P
 {
     const char* nc = sizeof(typename PT::real) == 8 ? "tj_cfl_fp64" : "tj_cfl_fp32";
     if (pr) pr->begin(nc, st);
-    k_cfl<<<path_blocks(b.ntot), kPathThreads, 0, st>>>(P, b, X);
+    const LaunchShape s = path_shape<PT>(b.ntot);
+    k_cfl<<<s.blocks, s.threads, 0, st>>>(P, b, X);
     if (pr) pr->end(nc, st);
     return 1;
 }
