@@ -54,30 +54,32 @@ inline int gblocks(long long n)
     return (int)std::max(1LL, std::min(b, 152LL * 32));
 }
 
-struct FacePairLocal {
-    const Dual* F0;
-    const Dual* F1;
-    __device__ __forceinline__ Dual operator()(int w, int s) const { return s ? F1[w] : F0[w]; }
+// Flux words of a cell's two faces, read in place; the word `seed` carries
+// direction 1 on face 0.
+struct FacePairSeed {
+    const double* FX;
+    long long nf, f0, f1;
+    int seed;
+    __device__ __forceinline__ Dual operator()(int w, int s) const
+    {
+        return Dual(FX[(long long)w * nf + (s ? f1 : f0)], (!s && w == seed) ? 1.0 : 0.0);
+    }
 };
 
-// One forward-mode pass of a cell's update: the output's tangent dotted with
-// the output adjoint lo. Yw / Aw are work copies of the accumulator and U^n.
-__device__ __noinline__ double upd_pass(const DevParamsT& P, const PathBufs<Dual>& lb, const Dual* X, const Dual* Y,
-                                        const Dual* A, Dual* Yw, Dual* Aw, const Dual* F0, const Dual* F1,
-                                        const double* lo, const DevDomain& D, int i, int d, int first, int last,
-                                        int finish, Dual dtv)
-{
-    for (int w = 0; w < P.NS; ++w) {
-        Yw[w] = Y[w];
-        Aw[w] = A[w];
-    }
-    update_cell(P, lb, X, Yw, 0LL, D, i, d, first, last, finish, dtv, FacePairLocal{F0, F1});
-    const Dual* out = finish ? Aw : Yw;
-    double s = 0.0;
-    for (int w = 0; w < P.NS; ++w)
-        if (lo[w] != 0.0) s += lo[w] * out[w].d;  // a zero adjoint takes no part
-    return s;
-}
+// The inputs of a cell's update whose derivatives are formed, one pass each
+// (the others have none: conservativeToPrimitive and the radial return
+// overwrite the words they would come from, and a face flux enters as the
+// difference of the two faces, so face 1's adjoint is the negative of face
+// 0's). kind 0: accumulator, 1: stage input, 2: flux of face 0, 3: U^n,
+// 4: EOS parameter (word = material * npar + parameter).
+struct UpdPass {
+    short kind, word;
+};
+constexpr int kMaxPass = 3 * kNS + kNX + TJ_MAX_MAT * TJ_MAX_EOS_PARAMS;
+struct UpdPasses {
+    int n;
+    UpdPass p[kMaxPass];
+};
 
 // ---------------------------------------------------------------------------
 // Update of one direction, reversed per cell. Inputs: the accumulator Yin
@@ -85,78 +87,72 @@ __device__ __noinline__ double upd_pass(const DevParamsT& P, const PathBufs<Dual
 // U, the two face fluxes F0 / F1 and, with the finish, U^n (A0). The output
 // adjoint lamOut is that of the direction's output (the next accumulator, or
 // U^{n+1} for the finish). Writes the adjoints of Yin and of the two fluxes
-// (per cell: F0 of the face below, F1 of the face above), adds those of U and
-// A0, and adds each EOS parameter's part into geos (per cell).
+// (per cell: F0 of the face below, F1 of the face above; the words without a
+// pass are zeroed by the host), adds those of U and A0, and adds each EOS
+// parameter's part into geos (per cell).
+//
+// One thread per cell and pass, cells fastest: the passes are independent
+// forward-mode evaluations of the cell's update whose values are the same and
+// whose direction is one input's. (One thread per cell running its ~110
+// passes in turn left 32 blocks for the 16^3 copper plate and spent its time in
+// the latency of one serial chain: backward 580 ms for 4 steps.) A warp's
+// lanes share the pass, so zero directions are skipped together.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kGT) k_gen_upd_rev(DevParamsT P, Fp64Bufs fb, const double* Yin, const double* U,
-                                                     const double* A0, const double* lamOut, double* lamYin,
-                                                     double* lamU, double* lamA0, double* lamF0, double* lamF1,
-                                                     double* geos, int d, int first, int last, int finish, int npar)
+__global__ void __launch_bounds__(kGT) k_gen_upd_rev(const __grid_constant__ DevParamsT P, Fp64Bufs fb,
+                                                     const UpdPasses* __restrict__ passes,
+                                                     const double* Yin, const double* U, const double* A0,
+                                                     const double* lamOut, double* lamYin, double* lamU, double* lamA0,
+                                                     double* lamF0, double* lamF1, double* geos, int d, int first,
+                                                     int last, int finish, int npar)
 {
-    const long long nt = fb.ntot, nf = fb.nftot[d];
-    const int NS = P.NS, NX = P.NX;
+    const long long nt = fb.ntot, all = nt * passes->n;
+    const int NS = P.NS;
     const DevDomain D = fb.doms[0];
     const Dual dtv(fb.scal->dt);
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nt; g += (long long)gridDim.x * blockDim.x) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
+        const int pass = (int)(e / nt);
+        const long long g = e - (long long)pass * nt;
+        const int kind = passes->p[pass].kind, word = passes->p[pass].word;
         int i, j, k;
         split3(g - D.off, D.n[0], D.n[1], i, j, k);
         int o[3] = {0, 0, 0};
         o[d] = 1;
-        const long long f0 = face_index(D, d, i, j, k), f1 = face_index(D, d, i + o[0], j + o[1], k + o[2]);
-        Dual X[kNS], Y[kNS], A[kNS], Yw[kNS], Aw[kNS], F0[kNX], F1[kNX];
-        double lo[kNS];
+        const FacePairSeed fx{fb.FX, fb.nftot[d], face_index(D, d, i, j, k),
+                              face_index(D, d, i + o[0], j + o[1], k + o[2]), kind == 2 ? word : -1};
+        Dual X[kNS], Y[kNS], A[kNS];
         for (int w = 0; w < NS; ++w) {
-            X[w] = Dual(U[w * nt + g]);
-            Y[w] = Dual(first ? 0.0 : Yin[w * nt + g]);
-            A[w] = Dual(finish ? A0[w * nt + g] : 0.0);
-            lo[w] = lamOut[w * nt + g];
-        }
-        for (int w = 0; w < NX; ++w) {
-            F0[w] = Dual(fb.FX[w * nf + f0]);
-            F1[w] = Dual(fb.FX[w * nf + f1]);
+            X[w] = Dual(U[w * nt + g], (kind == 1 && w == word) ? 1.0 : 0.0);
+            Y[w] = first ? Dual(0.0) : Dual(Yin[w * nt + g], (kind == 0 && w == word) ? 1.0 : 0.0);
+            A[w] = finish ? Dual(A0[w * nt + g], (kind == 3 && w == word) ? 1.0 : 0.0) : Dual(0.0);
         }
         int cb = fb.cell_box[g];
         PathBufs<Dual> lb{};
         lb.ntot = 1;
-        lb.A = Aw;
+        lb.A = A;
         lb.cell_box = &cb;
         lb.scal = fb.scal;
-#define TJ_PASS(PP) upd_pass(PP, lb, X, Y, A, Yw, Aw, F0, F1, lo, D, i, d, first, last, finish, dtv)
-        if (!first)
-            for (int w = 0; w < NS; ++w) {
-                Y[w].d = 1.0;
-                lamYin[w * nt + g] = TJ_PASS(P);
-                Y[w].d = 0.0;
-            }
+        DevParamsT Q;
+        const DevParamsT* par = &P;
+        if (kind == 4) {  // an EOS parameter's direction: a copy of the block with it
+            Q = P;
+            Q.prm[word / npar][word % npar].d = 1.0;
+            par = &Q;
+        }
+        update_cell(*par, lb, X, Y, 0LL, D, i, d, first, last, finish, dtv, fx);
+        const Dual* out = finish ? A : Y;
+        double s = 0.0;
         for (int w = 0; w < NS; ++w) {
-            X[w].d = 1.0;
-            lamU[w * nt + g] += TJ_PASS(P);
-            X[w].d = 0.0;
+            const double lo = lamOut[w * nt + g];
+            if (lo != 0.0) s += lo * out[w].d;  // a zero adjoint takes no part
         }
-        for (int w = 0; w < NX; ++w) {
-            F0[w].d = 1.0;
-            lamF0[w * nt + g] = TJ_PASS(P);
-            F0[w].d = 0.0;
-            F1[w].d = 1.0;
-            lamF1[w * nt + g] = TJ_PASS(P);
-            F1[w].d = 0.0;
-        }
-        if (finish)
-            for (int w = 0; w < NS; ++w) {
-                A[w].d = 1.0;
-                lamA0[w * nt + g] += TJ_PASS(P);
-                A[w].d = 0.0;
-            }
-        if (geos && npar > 0) {
-            DevParamsT Q = P;
-            for (int m = 0; m < P.M; ++m)
-                for (int q = 0; q < npar; ++q) {
-                    Q.prm[m][q].d = 1.0;
-                    geos[(long long)(m * npar + q) * nt + g] += TJ_PASS(Q);
-                    Q.prm[m][q].d = 0.0;
-                }
-        }
-#undef TJ_PASS
+        const long long at = (long long)word * nt + g;
+        if (kind == 0) lamYin[at] = s;
+        else if (kind == 1) lamU[at] += s;
+        else if (kind == 2) {
+            lamF0[at] = s;
+            lamF1[at] = -s;
+        } else if (kind == 3) lamA0[at] += s;
+        else geos[at] += s;
     }
 }
 
@@ -237,39 +233,27 @@ __global__ void __launch_bounds__(kGT) k_gen_upd_rev_lin(DevParams P, Fp64Bufs f
     }
 }
 
-// One forward-mode pass of a face's Riemann problem from its two stored
-// states: the flux's tangent dotted with the flux adjoint lF.
-__device__ __noinline__ double flux_pass(const DevParamsT& P, const Dual* Lp, const Dual* Rp, Dual* Fo, const double* lF,
-                                         int oddl, int oddr, int d, DevScalars* scal)
-{
-    CellT<Dual> L, R;
-    load_prim_face(P, Lp, 1LL, 0LL, oddl, L);
-    load_prim_face(P, Rp, 1LL, 0LL, oddr, R);
-    FluxV<Dual> F;
-    Dual Ss, vstar[3] = {Dual(0.0), Dual(0.0), Dual(0.0)};
-    face_flux(P, L, R, d, F, Ss, vstar, scal);
-    for (int w = 0; w < P.NX; ++w) Fo[w] = Dual(0.0);
-    store_flux(P, Fo, 1LL, 0LL, F, Ss, vstar);
-    double s = 0.0;
-    for (int w = 0; w < P.NX; ++w)
-        if (lF[w] != 0.0) s += lF[w] * Fo[w].d;
-    return s;
-}
-
 // ---------------------------------------------------------------------------
 // Riemann problem of one face, reversed: the face's flux adjoint is gathered
 // from the cell above (its F0) and the cell below (its F1); one pass per
 // word of the two stored face states (UR of the cell below, UL of the cell
-// above, boundary images as k_flux maps them) gives their adjoints, per face.
+// above, boundary images as k_flux maps them) gives their adjoints, per face,
+// one per EOS parameter in use those of the parameters: one thread per face
+// and pass, faces fastest, as in k_gen_upd_rev.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kGT) k_gen_flux_rev(DevParamsT P, Fp64Bufs fb, const double* lamF0,
-                                                      const double* lamF1, double* lamLf, double* lamRf,
-                                                      double* geos_f, int d, int npar, int nfw)
+__global__ void __launch_bounds__(kGT) k_gen_flux_rev(const __grid_constant__ DevParamsT P, Fp64Bufs fb,
+                                                      const UpdPasses* __restrict__ passes,
+                                                      const double* lamF0, const double* lamF1, double* lamLf,
+                                                      double* lamRf, double* geos_f, int d, int npar, int nfw)
 {
     const long long nt = fb.ntot, nf = fb.nftot[d];
     const int NX = P.NX;
     const DevDomain D = fb.doms[0];
-    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < nf; f += (long long)gridDim.x * blockDim.x) {
+    const long long all = nf * passes->n;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
+        const int pass = (int)(e / nf);
+        const long long f = e - (long long)pass * nf;
+        const int kind = passes->p[pass].kind, word = passes->p[pass].word;
         int nfv[3] = {D.n[0], D.n[1], D.n[2]};
         nfv[d] += 1;
         int i, j, k;
@@ -280,37 +264,36 @@ __global__ void __launch_bounds__(kGT) k_gen_flux_rev(DevParamsT P, Fp64Bufs fb,
         int rl[3], rr[3];
         const long long gl = map_cell(P, D, i - o[0], j - o[1], k - o[2], rl);
         const long long gr = map_cell(P, D, i, j, k, rr);
-        double lF[kNX];
-        for (int w = 0; w < NX; ++w) {
-            double s = 0.0;
-            if (idx[d] >= 1) s += lamF1[w * nt + D.off + (i - o[0]) + (long long)D.n[0] * ((j - o[1]) + (long long)D.n[1] * (k - o[2]))];
-            if (idx[d] < D.n[d]) s += lamF0[w * nt + D.off + i + (long long)D.n[0] * (j + (long long)D.n[1] * k)];
-            lF[w] = s;
-        }
         Dual Lp[kNF], Rp[kNF], Fo[kNX];
         for (int w = 0; w < nfw; ++w) {
-            Lp[w] = Dual(fb.UR[w * nt + gl]);
-            Rp[w] = Dual(fb.UL[w * nt + gr]);
+            Lp[w] = Dual(fb.UR[w * nt + gl], (kind == 0 && w == word) ? 1.0 : 0.0);
+            Rp[w] = Dual(fb.UL[w * nt + gr], (kind == 1 && w == word) ? 1.0 : 0.0);
         }
-#define TJ_PASS(PP) flux_pass(PP, Lp, Rp, Fo, lF, rl[d] ? d : -1, rr[d] ? d : -1, d, fb.scal)
-        for (int w = 0; w < nfw; ++w) {
-            Lp[w].d = 1.0;
-            lamLf[w * nf + f] = TJ_PASS(P);
-            Lp[w].d = 0.0;
-            Rp[w].d = 1.0;
-            lamRf[w * nf + f] = TJ_PASS(P);
-            Rp[w].d = 0.0;
+        CellT<Dual> L, R;
+        FluxV<Dual> F;
+        Dual Ss, vstar[3] = {Dual(0.0), Dual(0.0), Dual(0.0)};
+        DevParamsT Q;
+        const DevParamsT* par = &P;
+        if (kind == 4) {
+            Q = P;
+            Q.prm[word / npar][word % npar].d = 1.0;
+            par = &Q;
         }
-        if (geos_f && npar > 0) {
-            DevParamsT Q = P;
-            for (int m = 0; m < P.M; ++m)
-                for (int q = 0; q < npar; ++q) {
-                    Q.prm[m][q].d = 1.0;
-                    geos_f[(long long)(m * npar + q) * nf + f] += TJ_PASS(Q);
-                    Q.prm[m][q].d = 0.0;
-                }
+        load_prim_face(*par, Lp, 1LL, 0LL, rl[d] ? d : -1, L);
+        load_prim_face(*par, Rp, 1LL, 0LL, rr[d] ? d : -1, R);
+        face_flux(*par, L, R, d, F, Ss, vstar, fb.scal);
+        for (int w = 0; w < NX; ++w) Fo[w] = Dual(0.0);
+        store_flux(P, Fo, 1LL, 0LL, F, Ss, vstar);
+        double s = 0.0;
+        for (int w = 0; w < NX; ++w) {
+            double lF = 0.0;
+            if (idx[d] >= 1) lF += lamF1[w * nt + D.off + (i - o[0]) + (long long)D.n[0] * ((j - o[1]) + (long long)D.n[1] * (k - o[2]))];
+            if (idx[d] < D.n[d]) lF += lamF0[w * nt + D.off + i + (long long)D.n[0] * (j + (long long)D.n[1] * k)];
+            if (lF != 0.0) s += lF * Fo[w].d;
         }
-#undef TJ_PASS
+        if (kind == 0) lamLf[word * nf + f] = s;
+        else if (kind == 1) lamRf[word * nf + f] = s;
+        else geos_f[(long long)word * nf + f] += s;
     }
 }
 
@@ -545,6 +528,7 @@ struct GenAdj {
     double *lamF0 = nullptr, *lamF1 = nullptr, *lamLf = nullptr, *lamRf = nullptr, *geos = nullptr, *geosf = nullptr;
     double *prim0 = nullptr, *gsum = nullptr;
     int* a_to_s = nullptr;
+    UpdPasses* passes = nullptr;  // device: first, middle, last, finish updates, faces
     long long made[8] = {};  // the sizes the buffers were made for (gen_alloc)
 };
 
@@ -557,6 +541,8 @@ static void gen_free(GenAdj* a)
     a->bufs.clear();
     if (a->a_to_s) cudaFree(a->a_to_s);
     a->a_to_s = nullptr;
+    if (a->passes) cudaFree(a->passes);
+    a->passes = nullptr;
     for (long long& m : a->made) m = 0;
 }
 
@@ -576,6 +562,57 @@ const char* gen_unsupported(const DevParams& P, int ndom)
     if (P.thinc) return "the general adjoint covers MUSCL without BVD-THINC (2-D fluids with THINC: the 2-D adjoint)";
     if (P.nmix) return "the adjoint covers no mixtures";
     return nullptr;
+}
+
+// EOS parameters a material's equation of state reads ([gamma, pref, eref, CV,
+// ...]): the others have no derivative.
+static bool eos_reads(int eos, int q)
+{
+    switch (eos) {
+        case TJ_EOS_MIEGRUNEISEN: return q <= 2;
+        case TJ_EOS_ROMENSKII: return q == 0 || (q >= 4 && q <= 8);
+        case TJ_EOS_WILKINS: return q == 0 || (q >= 4 && q <= 10);
+        default: return q == 0 || (q >= 4 && q <= 7);
+    }
+}
+
+// The passes of a last direction's update (first: it is the only direction
+// too), with or without the second stage's finish, and of a face.
+enum PassList { PL_LAST = 0, PL_LAST_FIRST, PL_FINISH, PL_FINISH_FIRST, PL_FACE, kPassLists };
+
+static void list_passes(const DevParams& P, int npar, int nfw, UpdPasses* L)
+{
+    const auto in = [](int w, int w0, int n) { return w0 >= 0 && w >= w0 && w < w0 + n; };
+    for (int k = 0; k < kPassLists; ++k) {
+        UpdPasses& u = L[k];
+        u.n = 0;
+        const auto add = [&](int kind, int word) { u.p[u.n++] = {(short)kind, (short)word}; };
+        if (k == PL_FACE) {
+            for (int w = 0; w < nfw; ++w) {
+                add(0, w);
+                add(1, w);
+            }
+        } else {
+            const bool first = k == PL_LAST_FIRST || k == PL_FINISH_FIRST, finish = k >= PL_FINISH;
+            for (int w = 0; w < P.NS; ++w) {
+                // overwritten by the last direction's conservativeToPrimitive
+                const bool closed = in(w, P.S_RHOK, P.M) || w == P.S_RHO || in(w, P.S_VEL, 3) || w == P.S_P ||
+                                    (P.any_solid && w == P.S_HJ2);
+                // the non-conservative terms read alpha, V and the velocity
+                const bool noncons = in(w, P.S_ALPHA, P.M) || (P.solid && (in(w, P.S_V, 9) || in(w, P.S_VEL, 3)));
+                if (!first && !closed) add(0, w);
+                if (noncons || (first && !closed)) add(1, w);
+                // the return map's conservativeToPrimitive again overwrites the averaged ones
+                const bool mapped = P.plastic && (w == P.S_RHO || in(w, P.S_VEL, 3) || w == P.S_P ||
+                                                  (P.any_solid && w == P.S_HJ2));
+                if (finish && !mapped) add(3, w);
+            }
+            for (int w = 0; w < P.NX; ++w) add(2, w);
+        }
+        for (int m = 0; m < P.M; ++m)
+            for (int q = 0; q < npar; ++q)
+                if (eos_reads(P.eos[m], q)) add(4, m * npar + q);
+    }
 }
 
 static int gen_alloc(GenAdj* a, const DevParams& P, const Fp64Bufs& b, int nsteps, int stride)
@@ -601,7 +638,8 @@ static int gen_alloc(GenAdj* a, const DevParams& P, const Fp64Bufs& b, int nstep
               al(&a->lamF1, (size_t)P.NX * N) && al(&a->lamLf, (size_t)P.NF * nfmax) &&
               al(&a->lamRf, (size_t)P.NF * nfmax) && al(&a->geos, (size_t)mp * N) &&
               al(&a->geosf, (size_t)mp * nfmax) && al(&a->prim0, (size_t)P.NS * N) && al(&a->gsum, mp);
-    ok = ok && cudaMalloc(&a->a_to_s, sizeof(int) * 64) == cudaSuccess;
+    ok = ok && cudaMalloc(&a->a_to_s, sizeof(int) * 64) == cudaSuccess &&
+         cudaMalloc(&a->passes, sizeof(UpdPasses) * kPassLists) == cudaSuccess;
     if (!ok) {
         gen_free(a);
         return TJ_ERR_CUDA;
@@ -672,6 +710,9 @@ long long gen_backward(GenAdj* a, const DevParams& P, const Fp64Bufs& b, const d
         map(P.A_ARE, P.S_ARE, P.M);
     }
     cudaMemcpyAsync(a->a_to_s, a2s, sizeof(int) * P.NCOMP, cudaMemcpyHostToDevice, st);
+    std::vector<UpdPasses> lists(kPassLists);
+    list_passes(P, npar, nfw, lists.data());
+    cudaMemcpyAsync(a->passes, lists.data(), sizeof(UpdPasses) * kPassLists, cudaMemcpyHostToDevice, st);
     k_gen_ap_to_lam<<<gblocks(N), kGT, 0, st>>>(grad_ap, a->a_to_s, P.NCOMP, N, a->lamA, P.NS);
     ++launches;
     cudaMemsetAsync(a->geos, 0, sizeof(double) * std::max(mp, 1) * N, st);
@@ -698,13 +739,20 @@ long long gen_backward(GenAdj* a, const DevParams& P, const Fp64Bufs& b, const d
         Fp64Bufs f2 = fb;
         launches += path_dir_any(P, f2, U, a->yscr2, d, 1, 0, 0, st, nullptr);
         if (mp > 0) cudaMemsetAsync(a->geosf, 0, sizeof(double) * mp * b.nftot[d], st);
+        const int pl = finish ? (first ? PL_FINISH_FIRST : PL_FINISH) : (first ? PL_LAST_FIRST : PL_LAST);
         if (!last && !finish)
             k_gen_upd_rev_lin<<<gblocks(N), kGT, 0, st>>>(P, fb, U, lamOut, lamYin, lamU, a->lamF0, a->lamF1, d, first);
-        else
-            k_gen_upd_rev<<<gblocks(N), kGT, 0, st>>>(PT, fb, Yin, U, A0, lamOut, lamYin, lamU, lamA0, a->lamF0,
-                                                      a->lamF1, mp > 0 ? a->geos : nullptr, d, first, last, finish, npar);
-        k_gen_flux_rev<<<gblocks(b.nftot[d]), kGT, 0, st>>>(PT, fb, a->lamF0, a->lamF1, a->lamLf, a->lamRf,
-                                                            mp > 0 ? a->geosf : nullptr, d, npar, nfw);
+        else {
+            // the accumulator words without a pass
+            if (!first) cudaMemsetAsync(lamYin, 0, sizeof(double) * S, st);
+            const LaunchShape sh = launch_shape(N * lists[pl].n, kGT);
+            k_gen_upd_rev<<<sh.blocks, sh.threads, 0, st>>>(PT, fb, a->passes + pl, Yin, U, A0, lamOut, lamYin, lamU,
+                                                            lamA0, a->lamF0, a->lamF1, a->geos, d, first, last, finish,
+                                                            npar);
+        }
+        const LaunchShape sf = launch_shape(b.nftot[d] * lists[PL_FACE].n, kGT);
+        k_gen_flux_rev<<<sf.blocks, sf.threads, 0, st>>>(PT, fb, a->passes + PL_FACE, a->lamF0, a->lamF1, a->lamLf,
+                                                         a->lamRf, a->geosf, d, npar, nfw);
         k_gen_recon_rev<<<gblocks(N), kGT, 0, st>>>(P, fb, U, a->lamLf, a->lamRf, lamU, d, nfw);
         launches += 3;
         fold_faces(d);
