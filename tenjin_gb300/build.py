@@ -49,6 +49,13 @@ INSTANCES = {
                              "-fmad=false" if r == 64 else "-use_fast_math"])
     for r in (64, 32) for m, d in _INST
 }
+# fluids (kind 1, binary64) and plastic solids (kind 2): ParamKind in tj_types.h
+INSTANCES.update({
+    f"tj_path_{r}_m{m}_d{d}_k{k}.o":
+        ("tj_path_inst.cu", [f"-DTJ_INST_R={r}", f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", f"-DTJ_INST_K={k}",
+                             "-fmad=false" if r == 64 else "-use_fast_math"])
+    for r, k in ((64, 1), (64, 2), (32, 2)) for m in (1, 2) for d in (0, 1, 2)
+})
 # the tangent instance (tj_dual.cuh): two materials along x and y, and the
 # generic instance for every other material count and direction
 INSTANCES.update({

@@ -16,6 +16,13 @@
 #include "tj_math.cuh"
 #include "tj_types.h"
 
+// A function left out of line takes its cells through local memory: the
+// per-direction kernels of one kind inline them all (tj_path_inst.cu); where
+// every configuration's code is in one kernel it is left to the compiler.
+#ifndef TJ_DEV
+#define TJ_DEV __device__ inline
+#endif
+
 namespace tj {
 
 // ---------------------------------------------------------------------------
@@ -67,6 +74,19 @@ __device__ __forceinline__ ECellT<R> ecell_of(const CellT<R>& c, int m)
 // Parameter vectors as getMaterialParameters builds them (initialise.cpp:125-235).
 // ---------------------------------------------------------------------------
 template <typename PT>
+__device__ __forceinline__ int eos_of(const PT& P, int m)
+{
+    if constexpr (PT::kKind == KIND_FLUID) return TJ_EOS_MIEGRUNEISEN;
+    else return P.eos[m];
+}
+template <typename PT>
+__device__ __forceinline__ int phase_of(const PT& P, int m)
+{
+    if constexpr (PT::kKind == KIND_FLUID) return TJ_PHASE_FLUID;
+    else return P.phase[m];
+}
+
+template <typename PT>
 __device__ __forceinline__ typename PT::real gam(const PT& P, int m)
 {
     using R = typename PT::real;
@@ -85,11 +105,11 @@ __device__ __forceinline__ typename PT::real mix_gamma_term(const PT& P, int m, 
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_e_cold(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_e_cold(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return q[2] * e.arho;  // equationofstate.cpp:37-40
         case TJ_EOS_MIXTURE: return e.lam * (q[2] * e.arho) + (R(1.0) - e.lam) * (q[6] * e.arho);  // :161-165
         case TJ_EOS_ROMENSKII: {                         // :418-423
@@ -110,12 +130,12 @@ __device__ inline typename PT::real eos_e_cold(const PT& P, int m, const ECellT<
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_p_cold(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_p_cold(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
     R G = gam(P, m);
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return quot(q[1] * e.alpha, G);  // :42-45
         case TJ_EOS_MIXTURE:                                  // :167-171
             return quot((quot(q[1] * e.alpha, q[0] - R(1.0))) * e.lam * e.rhok, e.rm0) +
@@ -138,11 +158,11 @@ __device__ inline typename PT::real eos_p_cold(const PT& P, int m, const ECellT<
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_G(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_G(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;                           // :81-84
         case TJ_EOS_MIXTURE: return R(0.0);                                          // :146-149
         case TJ_EOS_ROMENSKII: return q[8] * tjm_pow((quot(e.rhok, q[4])), q[7] + R(1.0));  // :437-440
@@ -152,11 +172,11 @@ __device__ inline typename PT::real eos_G(const PT& P, int m, const ECellT<typen
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_dGdrho(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_dGdrho(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;
         case TJ_EOS_ROMENSKII: return quot(q[8] * (q[7] + R(1.0)) * tjm_pow((quot(e.rhok, q[4])), q[7]), q[4]);  // :442-445
         default: return R(0.0);
@@ -164,11 +184,11 @@ __device__ inline typename PT::real eos_dGdrho(const PT& P, int m, const ECellT<
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_dG2drho2(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_dG2drho2(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;
         case TJ_EOS_ROMENSKII:  // :447-450
             return quot(q[8] * (q[7] + R(1.0)) * (q[7]) * tjm_pow((quot(e.rhok, q[4])), q[7] - R(1.0)), q[4] * q[4]);
@@ -177,10 +197,10 @@ __device__ inline typename PT::real eos_dG2drho2(const PT& P, int m, const ECell
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_e_shear(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_e_shear(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;  // :101-104
         case TJ_EOS_MIXTURE: return R(0.0);                 // :136-139
         case TJ_EOS_HUGONIOT: return e.alpha * (P.prm[m][7] * e.hj2);
@@ -189,11 +209,11 @@ __device__ inline typename PT::real eos_e_shear(const PT& P, int m, const ECellT
 }
 
 template <typename PT>
-__device__ inline typename PT::real eos_p_shear(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_p_shear(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     R G = gam(P, m);
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return R(0.0) * e.alpha;  // :106-109
         case TJ_EOS_MIXTURE: return R(0.0);                 // :141-144
         case TJ_EOS_HUGONIOT: return (quot(e.alpha, G)) * ((e.rhok * R(0.0) - P.prm[m][7]) * e.hj2);
@@ -204,7 +224,7 @@ __device__ inline typename PT::real eos_p_shear(const PT& P, int m, const ECellT
 template <typename PT>
 __device__ __forceinline__ typename PT::real eos_invG(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
-    if (P.eos[m] == TJ_EOS_MIXTURE) return quot(e.alpha, mix_gamma_term(P, m, e.lam));  // :173-178
+    if (eos_of(P, m) == TJ_EOS_MIXTURE) return quot(e.alpha, mix_gamma_term(P, m, e.lam));  // :173-178
     return quot(e.alpha, gam(P, m));
 }
 
@@ -213,18 +233,18 @@ template <typename PT>
 __device__ __forceinline__ typename PT::real eos_xi(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
-    if (P.eos[m] == TJ_EOS_MIXTURE) return quot(R(1.0), mix_gamma_term(P, m, e.lam));
+    if (eos_of(P, m) == TJ_EOS_MIXTURE) return quot(R(1.0), mix_gamma_term(P, m, e.lam));
     return quot(R(1.0), gam(P, m));
 }
 
 // Sound-speed contribution c^2_m (getSoundSpeedContribution).
 template <typename PT>
-__device__ inline typename PT::real eos_c2(const PT& P, int m, const ECellT<typename PT::real>& e)
+TJ_DEV typename PT::real eos_c2(const PT& P, int m, const ECellT<typename PT::real>& e)
 {
     using R = typename PT::real;
     const R* q = P.prm[m];
     R G = gam(P, m);
-    switch (P.eos[m]) {
+    switch (eos_of(P, m)) {
         case TJ_EOS_MIEGRUNEISEN: return quot(e.p * (G + R(1.0)), e.rhok) - quot(q[1], e.rhok);  // :61-64
         case TJ_EOS_MIXTURE: {  // mixtureSoundSpeed (:208-220)
             const R G1 = q[0] - R(1.0), G2 = q[4] - R(1.0);
@@ -270,7 +290,7 @@ __device__ __forceinline__ R det2(R a, R b, R c, R d)
 
 // Cofactor expansion along the first row (tensor.cpp:296-333).
 template <typename R>
-__device__ inline R det3(const R* M)
+TJ_DEV R det3(const R* M)
 {
     R det = R(0.0);
     det += (R(1.0) * M[0]) * det2(M[4], M[5], M[7], M[8]);
@@ -281,7 +301,7 @@ __device__ inline R det3(const R* M)
 
 // Transposed cofactors over the determinant (tensor.cpp:187-233).
 template <typename R>
-__device__ inline void invert3(const R* M, R* Minv)
+TJ_DEV void invert3(const R* M, R* Minv)
 {
     R D = det3(M);
     R c00 = det2(M[4], M[5], M[7], M[8]), c01 = R(-1.0) * det2(M[3], M[5], M[6], M[8]),
@@ -298,7 +318,7 @@ __device__ inline void invert3(const R* M, R* Minv)
 // Row-major product, k summed innermost in increasing order (the reference
 // BLAS order for each element, tensor.cpp:81-115).
 template <typename R>
-__device__ inline void mm3(const R* A, const R* B, R* C)
+TJ_DEV void mm3(const R* A, const R* B, R* C)
 {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -312,7 +332,7 @@ __device__ inline void mm3(const R* A, const R* B, R* C)
         }
 }
 template <typename R>
-__device__ inline void mmT3(const R* A, const R* B, R* C)  // A B^T
+TJ_DEV void mmT3(const R* A, const R* B, R* C)  // A B^T
 {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -339,7 +359,7 @@ __device__ __forceinline__ R trace3(const R* M)
 // Loan, Matrix Computations, sec. 8.5). w decreasing; q holds the
 // eigenvectors as columns. Bounded at 50 sweeps.
 template <typename R>
-__device__ inline void sym3_eig(const R* a_in, R* w, R* q)
+TJ_DEV void sym3_eig(const R* a_in, R* w, R* q)
 {
     R a[9];
 #pragma unroll
@@ -406,7 +426,7 @@ __device__ inline void sym3_eig(const R* a_in, R* w, R* q)
 
 // matrixSquareRoot (tensor.cpp:452-475): L S^(1/2) RT with L = Q, RT = Q^T.
 template <typename R>
-__device__ inline void sqrtm3(const R* A, R* Rm)
+TJ_DEV void sqrtm3(const R* A, R* Rm)
 {
     R w[3], q[9], L[9], RT[9], S[9], tmp[9];
     sym3_eig(A, w, q);
@@ -426,18 +446,20 @@ __device__ inline void sqrtm3(const R* A, R* Rm)
 // BoxAccessCellArray per-cell operations (boxaccesscellarray.cpp).
 // ---------------------------------------------------------------------------
 template <typename PT>
-__device__ inline typename PT::real eff_invG(const PT& P, const CellT<typename PT::real>& c)  // :218-228
+TJ_DEV typename PT::real eff_invG(const PT& P, const CellT<typename PT::real>& c)  // :218-228
 {
     using R = typename PT::real;
     R tot = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) tot += eos_invG(P, m, ecell_of(c, m));
     return tot;
 }
 template <typename PT>
-__device__ inline typename PT::real eff_e_nonthermal(const PT& P, const CellT<typename PT::real>& c)  // :230-240
+TJ_DEV typename PT::real eff_e_nonthermal(const PT& P, const CellT<typename PT::real>& c)  // :230-240
 {
     using R = typename PT::real;
     R tot = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         ECellT<R> e = ecell_of(c, m);
         tot += (eos_e_cold(P, m, e) + eos_e_shear(P, m, e));
@@ -445,10 +467,11 @@ __device__ inline typename PT::real eff_e_nonthermal(const PT& P, const CellT<ty
     return tot;
 }
 template <typename PT>
-__device__ inline typename PT::real eff_p_nonthermal(const PT& P, const CellT<typename PT::real>& c)  // :242-252
+TJ_DEV typename PT::real eff_p_nonthermal(const PT& P, const CellT<typename PT::real>& c)  // :242-252
 {
     using R = typename PT::real;
     R tot = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         ECellT<R> e = ecell_of(c, m);
         tot += eos_p_cold(P, m, e) + eos_p_shear(P, m, e);
@@ -458,7 +481,7 @@ __device__ inline typename PT::real eff_p_nonthermal(const PT& P, const CellT<ty
 
 // getDeviatoricHenckyStrain + getHenckyJ2 (:326-380); solids only.
 template <typename PT>
-__device__ inline void hencky(const PT& P, CellT<typename PT::real>& c)
+TJ_DEV void hencky(const PT& P, CellT<typename PT::real>& c)
 {
     using R = typename PT::real;
     if (!P.any_solid) return;
@@ -473,13 +496,14 @@ __device__ inline void hencky(const PT& P, CellT<typename PT::real>& c)
 
 // stressTensor (:176-216)
 template <typename PT>
-__device__ inline void stress(const PT& P, CellT<typename PT::real>& c)
+TJ_DEV void stress(const PT& P, CellT<typename PT::real>& c)
 {
     using R = typename PT::real;
     R Gt = R(0.0);
     int solid = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m)
-        if (P.phase[m] == TJ_PHASE_SOLID) {
+        if (phase_of(P, m) == TJ_PHASE_SOLID) {
             ECellT<R> e = ecell_of(c, m);
             solid = 1;
             Gt += eos_G(P, m, e) * (eos_invG(P, m, e));
@@ -511,7 +535,7 @@ __device__ __forceinline__ double mix_rhob(const CellT<double>& c, double rhoa) 
 __device__ __forceinline__ int sgn_d(double v) { return (0.0 < v) - (v < 0.0); }
 
 template <typename PD>
-__device__ inline double mix_bisect_f(const PD& P, CellT<double>& c, double rho_try, double ke)  // :262-272
+TJ_DEV double mix_bisect_f(const PD& P, CellT<double>& c, double rho_try, double ke)  // :262-272
 {
     c.rm0 = rho_try;
     c.rm1 = mix_rhob(c, rho_try);
@@ -522,7 +546,7 @@ __device__ inline double mix_bisect_f(const PD& P, CellT<double>& c, double rho_
 }
 
 template <typename PD>
-__device__ inline int mix_root_find(const PD& P, CellT<double>& c, double ke)
+TJ_DEV int mix_root_find(const PD& P, CellT<double>& c, double ke)
 {
     const double* q = P.prm[0];
     const double lam = c.lam, rk = c.rhok[0];
@@ -620,10 +644,11 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
     using R = typename PT::real;
     int err = 0;
     c.rho = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         c.rhok[m] = quot(c.arho[m], c.alpha[m]);
         c.rho += c.arho[m];
-        if (P.plastic && P.phase[m] == TJ_PHASE_SOLID) c.eps[m] = quot(c.are[m], c.arho[m]);
+        if (P.plastic && phase_of(P, m) == TJ_PHASE_SOLID) c.eps[m] = quot(c.are[m], c.arho[m]);
     }
     hencky(P, c);
     R ke = R(0.0);
@@ -651,6 +676,7 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
         // (and of the mixture densities) in binary64, from the compensated
         // energy (E, Elo) and binary64 cold terms
         double rho = 0.0, ent = 0.0, pnt = 0.0, ig = 0.0;
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) rho += (double)c.arho[m];
         const double ru0 = c.rhou[0], ru1 = c.rhou[1], ru2 = c.rhou[2];
         const double ked = quot(0.5 * (ru0 * ru0 + ru1 * ru1 + ru2 * ru2), rho);
@@ -658,6 +684,7 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
         if (P.nmix) {
             lam = quot((double)c.arl, (double)c.arho[0]);
             CellT<double> cd;
+            #pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m) {
                 cd.alpha[m] = c.alpha[m];
                 cd.arho[m] = c.arho[m];
@@ -676,6 +703,7 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
             c.rm0 = (R)rm0;
             c.rm1 = (R)rm1;
         }
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             ECellT<double> e;
             e.alpha = c.alpha[m];
@@ -709,10 +737,11 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
 
 // primitiveToConservative (:124-174)
 template <typename PT>
-__device__ inline void p2c(const PT& P, CellT<typename PT::real>& c)
+TJ_DEV void p2c(const PT& P, CellT<typename PT::real>& c)
 {
     using R = typename PT::real;
     c.rho = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         c.arho[m] = c.alpha[m] * c.rhok[m];
         c.rho += c.arho[m];
@@ -724,7 +753,7 @@ __device__ inline void p2c(const PT& P, CellT<typename PT::real>& c)
                                              (quot(q[7] * (q[4] - R(1.0)), q[3] * (q[0] - R(1.0)))));
             c.rm1 = quot(R(1.0) - c.lam, quot(R(1.0), c.rhok[0]) - quot(c.lam, c.rm0));
         }
-        if (P.plastic && P.phase[m] == TJ_PHASE_SOLID) c.are[m] = c.eps[m] * c.arho[m];
+        if (P.plastic && phase_of(P, m) == TJ_PHASE_SOLID) c.are[m] = c.eps[m] * c.arho[m];
     }
     hencky(P, c);
     R ke = R(0.0);
@@ -739,10 +768,11 @@ __device__ inline void p2c(const PT& P, CellT<typename PT::real>& c)
 
 // getSoundSpeed (:254-285)
 template <typename PT>
-__device__ inline typename PT::real sound_speed(const PT& P, const CellT<typename PT::real>& c)
+TJ_DEV typename PT::real sound_speed(const PT& P, const CellT<typename PT::real>& c)
 {
     using R = typename PT::real;
     R a = R(0.0), xit = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         ECellT<R> e = ecell_of(c, m);
         R xi = eos_xi(P, m, e);
@@ -757,11 +787,12 @@ __device__ inline typename PT::real sound_speed(const PT& P, const CellT<typenam
 // cleanUpAlpha on one cell (:530-599). Returns TJ_ERR_ALPHA on the
 // reference's fatal conditions.
 template <typename PT>
-__device__ inline int cleanup_alpha(const PT& P, typename PT::real* alpha)
+TJ_DEV int cleanup_alpha(const PT& P, typename PT::real* alpha)
 {
     using R = typename PT::real;
     R tot = R(0.0);
     int nan = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         R a = alpha[m];
         if (isnan(a)) {
@@ -775,24 +806,27 @@ __device__ inline int cleanup_alpha(const PT& P, typename PT::real* alpha)
     }
     if (nan > 0) {
         const R a = R(1.0) - tot;
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m)  // no index that is not a constant: alpha stays in registers
             if (m == nan) alpha[m] = a;
         tot += a;
     }
     if (tot <= R(0.0)) return TJ_ERR_ALPHA;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) alpha[m] *= quot(R(1.0), tot);
     return 0;
 }
 
 // transverseWaveSpeed on a star state (:287-324).
 template <typename PT>
-__device__ inline typename PT::real transverse_speed(const PT& P, CellT<typename PT::real>& c)
+TJ_DEV typename PT::real transverse_speed(const PT& P, CellT<typename PT::real>& c)
 {
     using R = typename PT::real;
     hencky(P, c);
     R b = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m)
-        if (P.phase[m] == TJ_PHASE_SOLID) {
+        if (phase_of(P, m) == TJ_PHASE_SOLID) {
             ECellT<R> e = ecell_of(c, m);
             b += quot(eos_invG(P, m, e) * eos_G(P, m, e), c.rhok[m]);
         }

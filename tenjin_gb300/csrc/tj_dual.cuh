@@ -171,6 +171,7 @@ __device__ inline void sqrtm3(const Dual* A, Dual* Rm)
 // derivatives along the EOS parameters come out of the same run.
 struct DevParamsT {
     using real = Dual;
+    static constexpr int kKind = KIND_ANY;
     int dim, M, solid, thinc, plastic, muscl, any_solid;
     int fused64;
     int radial;

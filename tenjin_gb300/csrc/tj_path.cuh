@@ -136,9 +136,10 @@ __device__ __forceinline__ long long face_index(const DevDomain& D, int d, int i
 
 // Carried-state load with the reflect_odd sign applied.
 template <typename PT, typename R = typename PT::real>
-__device__ inline void load_state(const PT& P, const R* X, long long nt, long long g, const int* refl,
+TJ_DEV void load_state(const PT& P, const R* X, long long nt, long long g, const int* refl,
                                   CellT<R>& c)
 {
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         c.alpha[m] = X[(P.S_ALPHA + m) * nt + g];
         c.arho[m] = X[(P.S_ARHO + m) * nt + g];
@@ -162,6 +163,7 @@ __device__ inline void load_state(const PT& P, const R* X, long long nt, long lo
         c.hj2 = X[P.S_HJ2 * nt + g];
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             c.eps[m] = X[(P.S_EPS + m) * nt + g];
             c.are[m] = X[(P.S_ARE + m) * nt + g];
@@ -179,8 +181,9 @@ __device__ inline void load_state(const PT& P, const R* X, long long nt, long lo
 // each face state): the primitives with the reflect_odd sign, the cell's own
 // HJ2 (SOLID) and alphaRhoEps (PLASTIC), and lambda (mixtures).
 template <typename PT, typename R = typename PT::real>
-__device__ inline void load_prims(const PT& P, const R* X, long long nt, long long g, const int* refl, CellT<R>& c)
+TJ_DEV void load_prims(const PT& P, const R* X, long long nt, long long g, const int* refl, CellT<R>& c)
 {
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         c.alpha[m] = X[(P.S_ALPHA + m) * nt + g];
         c.rhok[m] = X[(P.S_RHOK + m) * nt + g];
@@ -199,6 +202,7 @@ __device__ inline void load_prims(const PT& P, const R* X, long long nt, long lo
         c.hj2 = X[P.S_HJ2 * nt + g];
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             c.eps[m] = X[(P.S_EPS + m) * nt + g];
             c.are[m] = X[(P.S_ARE + m) * nt + g];
@@ -207,8 +211,9 @@ __device__ inline void load_prims(const PT& P, const R* X, long long nt, long lo
 }
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline void store_state(const PT& P, R* X, long long nt, long long g, const CellT<R>& c)
+TJ_DEV void store_state(const PT& P, R* X, long long nt, long long g, const CellT<R>& c)
 {
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         X[(P.S_ALPHA + m) * nt + g] = c.alpha[m];
         X[(P.S_ARHO + m) * nt + g] = c.arho[m];
@@ -229,6 +234,7 @@ __device__ inline void store_state(const PT& P, R* X, long long nt, long long g,
         X[P.S_HJ2 * nt + g] = c.hj2;
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             X[(P.S_EPS + m) * nt + g] = c.eps[m];
             X[(P.S_ARE + m) * nt + g] = c.are[m];
@@ -242,8 +248,9 @@ __device__ inline void store_state(const PT& P, R* X, long long nt, long long g,
 }
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline void store_face(const PT& P, R* F, long long nt, long long g, const CellT<R>& c)
+TJ_DEV void store_face(const PT& P, R* F, long long nt, long long g, const CellT<R>& c)
 {
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         F[(P.F_ALPHA + m) * nt + g] = c.alpha[m];
         F[(P.F_ARHO + m) * nt + g] = c.arho[m];
@@ -265,13 +272,15 @@ __device__ inline void store_face(const PT& P, R* F, long long nt, long long g, 
         }
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) F[(P.F_ARE + m) * nt + g] = c.are[m];
     if (P.nmix) F[P.F_ARL * nt + g] = c.arl;
 }
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline void load_face(const PT& P, const R* F, long long nt, long long g, int oddir, CellT<R>& c)
+TJ_DEV void load_face(const PT& P, const R* F, long long nt, long long g, int oddir, CellT<R>& c)
 {
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         c.alpha[m] = F[(P.F_ALPHA + m) * nt + g];
         c.arho[m] = F[(P.F_ARHO + m) * nt + g];
@@ -302,6 +311,7 @@ __device__ inline void load_face(const PT& P, const R* F, long long nt, long lon
             for (int q = 0; q < 3; ++q) c.sigma[3 * r + q] = -c.p * (R)(r == q);  // stressTensor, fluid
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) c.are[m] = F[(P.F_ARE + m) * nt + g];
     if (P.nmix) c.arl = F[P.F_ARL * nt + g];
 }
@@ -320,10 +330,12 @@ __device__ __forceinline__ bool compact_faces(const PT& P)
 }
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline void store_prim_face(const PT& P, R* F, long long nt, long long g, const CellT<R>& c)
+TJ_DEV void store_prim_face(const PT& P, R* F, long long nt, long long g, const CellT<R>& c)
 {
     int w = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = c.alpha[m];
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = c.rhok[m];
 #pragma unroll
     for (int r = 0; r < 3; ++r) F[(long long)(w++) * nt + g] = c.vel[r];
@@ -334,17 +346,20 @@ __device__ inline void store_prim_face(const PT& P, R* F, long long nt, long lon
         if (!P.any_solid) F[(long long)(w++) * nt + g] = c.hj2;  // getHenckyJ2 does not run: the cell's own
     }
     if (P.plastic)  // epsilon of a solid closes alphaRhoEps; a fluid's alphaRhoEps is the cell's own
-        for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = P.phase[m] == TJ_PHASE_SOLID ? c.eps[m] : c.are[m];
+        #pragma unroll UnrollM<PT>::n
+        for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = phase_of(P, m) == TJ_PHASE_SOLID ? c.eps[m] : c.are[m];
 }
 
 // The closed face state of load_face from stored primitives: the closures
 // of the reconstruction, then the fields load_face leaves at zero, then the
 // reflect_odd sign of a boundary image.
 template <typename PT, typename R = typename PT::real>
-__device__ inline void load_prim_face(const PT& P, const R* F, long long nt, long long g, int oddir, CellT<R>& c)
+TJ_DEV void load_prim_face(const PT& P, const R* F, long long nt, long long g, int oddir, CellT<R>& c)
 {
     int w = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) c.alpha[m] = F[(long long)(w++) * nt + g];
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) c.rhok[m] = F[(long long)(w++) * nt + g];
 #pragma unroll
     for (int r = 0; r < 3; ++r) c.vel[r] = F[(long long)(w++) * nt + g];
@@ -356,13 +371,15 @@ __device__ inline void load_prim_face(const PT& P, const R* F, long long nt, lon
         if (!P.any_solid) c.hj2 = F[(long long)(w++) * nt + g];
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             const R v = F[(long long)(w++) * nt + g];
-            if (P.phase[m] == TJ_PHASE_SOLID) c.eps[m] = v;
+            if (phase_of(P, m) == TJ_PHASE_SOLID) c.eps[m] = v;
             else c.are[m] = v;
         }
     p2c(P, c);
     c.a = sound_speed(P, c);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) c.rhok[m] = R(0.0);
     c.hj2 = R(0.0);
     if (!P.solid)
@@ -423,8 +440,9 @@ __device__ __forceinline__ R gv(const PT& P, const DevDomain& D, const R* X, lon
     int refl[3];
     long long g = map_cell(P, D, i, j, k, refl);
     R v = X[word * nt + g];
-    for (int d = 0; d < P.dim; ++d)
-        if (refl[d] && (word == P.S_VEL + d || word == P.S_RHOU + d)) v = -v;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        if (d < P.dim && refl[d] && (word == P.S_VEL + d || word == P.S_RHOU + d)) v = -v;
     return v;
 }
 
@@ -439,7 +457,7 @@ struct ThincCand {
 };
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline R youngs(const PT& P, const DevDomain& D, const R* X, long long nt, int m, int i,
+TJ_DEV R youngs(const PT& P, const DevDomain& D, const R* X, long long nt, int m, int i,
                                 int j, int k, int d)  // thinc.cpp:28-53
 {
     int a = P.S_ALPHA + m;
@@ -453,13 +471,14 @@ __device__ inline R youngs(const PT& P, const DevDomain& D, const R* X, long lon
 }
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline void thinc_cand(const PT& P, const DevDomain& D, const R* X, long long nt, int i, int j,
+TJ_DEV void thinc_cand(const PT& P, const DevDomain& D, const R* X, long long nt, int i, int j,
                                   int k, int d, ThincCand<R>& t)
 {
     const R eps = R(1E-20), beta0 = P.beta;
     int o[3] = {0, 0, 0};
     o[d] = 1;
     t.flag = 0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         int a = P.S_ALPHA + m;
         R aL = gv(P, D, X, nt, a, i - o[0], j - o[1], k - o[2]);
@@ -516,6 +535,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
         L = u0;
         Rc = u0;
         if (P.muscl) {  // MUSCLextrapolate over the primitive list
+            #pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m) {
                 muscl1(um.alpha[m], u0.alpha[m], up.alpha[m], L.alpha[m], Rc.alpha[m]);
                 muscl1(um.rhok[m], u0.rhok[m], up.rhok[m], L.rhok[m], Rc.rhok[m]);
@@ -527,6 +547,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
 #pragma unroll
                 for (int qq = 0; qq < 9; ++qq) muscl1(um.V[qq], u0.V[qq], up.V[qq], L.V[qq], Rc.V[qq]);
             if (P.plastic)
+                #pragma unroll UnrollM<PT>::n
                 for (int m = 0; m < P.M; ++m) muscl1(um.eps[m], u0.eps[m], up.eps[m], L.eps[m], Rc.eps[m]);
             if (P.nmix) muscl1(um.lam, u0.lam, up.lam, L.lam, Rc.lam);
         }
@@ -543,6 +564,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
             const long long gmm = D.off + (i - o[0]) + (long long)D.n[0] * ((j - o[1]) + (long long)D.n[1] * (k - o[2]));
             const long long gpp = D.off + (i + o[0]) + (long long)D.n[0] * ((j + o[1]) + (long long)D.n[1] * (k + o[2]));
             int code = 0;
+            #pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m) {
                 const int a = P.S_ALPHA + m;
                 R urm, ulp, trm, tlp;
@@ -584,6 +606,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
                 }
             }
             if (b.rec) {
+                #pragma unroll UnrollM<PT>::n
                 for (int m = 0; m < P.M; ++m) {
                     b.rec[((long long)(d * 2) * P.M + m) * nt + g] = L.alpha[m];
                     b.rec[((long long)(d * 2 + 1) * P.M + m) * nt + g] = Rc.alpha[m];
@@ -591,6 +614,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
                 b.rec_code[(long long)d * nt + g] = code;
             }
             // THINC pass 1 writes its candidates into the persistent scratch.
+            #pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m)
                 if (tc.mixed[m]) {
                     b.ulstar[(long long)m * nt + g] = tc.L[m];
@@ -615,10 +639,12 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
             S.a = sound_speed(P, S);
             for (int r = 1; r < reps; ++r) {
                 R before[TJ_MAX_MAT];
+                #pragma unroll UnrollM<PT>::n
                 for (int m = 0; m < P.M; ++m) before[m] = S.alpha[m];
                 int e = cleanup_alpha(P, S.alpha);
                 if (e) set_status(b.scal, e);
                 bool same = true;
+                #pragma unroll UnrollM<PT>::n
                 for (int m = 0; m < P.M; ++m)
                     same &= same_bits(before[m], S.alpha[m]);
                 if (same) break;
@@ -633,7 +659,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
 // Riemann solvers (hllc.cpp:1-487, flux.cpp:5-47).
 // ---------------------------------------------------------------------------
 template <typename PT, typename R = typename PT::real>
-__device__ inline void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, R SK, R Ss, int d)  // :12-73
+TJ_DEV void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, R SK, R Ss, int d)  // :12-73
 {
     R ud = U.vel[d];
     // |(Ss - ud) / Ss| < 1e-20: the difference of two binary64 numbers that
@@ -644,6 +670,7 @@ __device__ inline void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, 
     else contact = Ss - ud == R(0.0) && Ss != R(0.0);
     R mult = contact ? R(1.0) : quot(SK - ud, SK - Ss);
     Us.rho = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         Us.alpha[m] = U.alpha[m];
         Us.arho[m] = mult * U.arho[m];
@@ -652,7 +679,7 @@ __device__ inline void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, 
         // a fluid carries no plastic strain: its alphaRhoEps star value is 0
         // (the reference writes only the plastic materials' and resets the
         // fluids' after every step, so no result depends on it)
-        if (P.plastic) Us.are[m] = P.phase[m] == TJ_PHASE_SOLID ? mult * U.are[m] : R(0.0);
+        if (P.plastic) Us.are[m] = phase_of(P, m) == TJ_PHASE_SOLID ? mult * U.are[m] : R(0.0);
         Us.rho += Us.arho[m];
     }
 #pragma unroll
@@ -677,9 +704,10 @@ struct FluxV {
 
 // Physical flux of the conservative variables (flux.cpp:33-47).
 template <typename PT, typename R = typename PT::real>
-__device__ inline void phys_flux(const PT& P, const CellT<R>& U, int d, FluxV<R>& F)
+TJ_DEV void phys_flux(const PT& P, const CellT<R>& U, int d, FluxV<R>& F)
 {
     R ud = U.vel[d];
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         F.alpha[m] = U.alpha[m] * ud;
         F.arho[m] = U.arho[m] * ud;
@@ -697,14 +725,16 @@ __device__ inline void phys_flux(const PT& P, const CellT<R>& U, int d, FluxV<R>
             F.V[q] = U.V[q] * ud - U.V[3 * d + col] * U.vel[row];
         }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) F.are[m] = U.are[m] * ud;
     if (P.nmix) F.arl = U.arl * ud;
 }
 
 // Conservative values of a state.
 template <typename PT, typename R = typename PT::real>
-__device__ inline void cons_vals(const PT& P, const CellT<R>& U, FluxV<R>& Q)
+TJ_DEV void cons_vals(const PT& P, const CellT<R>& U, FluxV<R>& Q)
 {
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         Q.alpha[m] = U.alpha[m];
         Q.arho[m] = U.arho[m];
@@ -716,6 +746,7 @@ __device__ inline void cons_vals(const PT& P, const CellT<R>& U, FluxV<R>& Q)
 #pragma unroll
         for (int q = 0; q < 9; ++q) Q.V[q] = U.V[q];
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) Q.are[m] = U.are[m];
     if (P.nmix) Q.arl = U.arl;
 }
@@ -727,7 +758,7 @@ __device__ inline void cons_vals(const PT& P, const CellT<R>& U, FluxV<R>& Q)
 //   NT = 2: FK + S1 (Q1 - Q0) + S2 (Q2 - Q1)
 // alpha takes the flux of the star state FA.
 template <int NT, typename PT, typename R = typename PT::real>
-__device__ inline void flux_combine(const PT& P, FluxV<R>& F, const FluxV<R>& FA, const FluxV<R>& FK,
+TJ_DEV void flux_combine(const PT& P, FluxV<R>& F, const FluxV<R>& FA, const FluxV<R>& FK,
                                     const FluxV<R>& Q0, const FluxV<R>& Q1, const FluxV<R>& Q2, R S1, R S2)
 {
     auto one = [&](R fk, R q0, R q1, R q2) -> R {
@@ -735,6 +766,7 @@ __device__ inline void flux_combine(const PT& P, FluxV<R>& F, const FluxV<R>& FA
         else if constexpr (NT == 1) return fk + S1 * (q1 - q0);
         else return fk + S1 * (q1 - q0) + S2 * (q2 - q1);
     };
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         F.alpha[m] = FA.alpha[m];
         F.arho[m] = one(FK.arho[m], Q0.arho[m], Q1.arho[m], Q2.arho[m]);
@@ -746,16 +778,18 @@ __device__ inline void flux_combine(const PT& P, FluxV<R>& F, const FluxV<R>& FA
 #pragma unroll
         for (int q = 0; q < 9; ++q) F.V[q] = one(FK.V[q], Q0.V[q], Q1.V[q], Q2.V[q]);
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) F.are[m] = one(FK.are[m], Q0.are[m], Q1.are[m], Q2.are[m]);
     if (P.nmix) F.arl = one(FK.arl, Q0.arl, Q1.arl, Q2.arl);
 }
 
 // One face into the flux-word layout (nf faces per word).
 template <typename PT, typename R = typename PT::real>
-__device__ inline void store_flux(const PT& P, R* FX, long long nf, long long f, const FluxV<R>& F, R Ss,
+TJ_DEV void store_flux(const PT& P, R* FX, long long nf, long long f, const FluxV<R>& F, R Ss,
                                   const R* vstar)
 {
 #define FXS(w) FX[(long long)(w) * nf + f]
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         FXS(P.X_ALPHA + m) = F.alpha[m];
         FXS(P.X_ARHO + m) = F.arho[m];
@@ -770,6 +804,7 @@ __device__ inline void store_flux(const PT& P, R* FX, long long nf, long long f,
         for (int col = 0; col < 3; ++col) FXS(P.X_VSTAR + col) = vstar[col];
     }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) FXS(P.X_ARE + m) = F.are[m];
     if (P.nmix) FXS(P.X_ARL) = F.arl;
     FXS(P.X_SSTAR) = Ss;
@@ -781,7 +816,7 @@ __device__ inline void store_flux(const PT& P, R* FX, long long nf, long long f,
 // values (solids). Returns the side whose star alpha the face carries: 0
 // left, 1 right.
 template <typename PT, typename R = typename PT::real>
-__device__ inline int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& Rc, int d, FluxV<R>& F, R& Ss,
+TJ_DEV int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& Rc, int d, FluxV<R>& F, R& Ss,
                                 R* vstar, DevScalars* scal)
 {
     R x1 = fabs(L.vel[d]) + L.a, x2 = fabs(Rc.vel[d]) + Rc.a;
@@ -935,17 +970,18 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
         int side = face_flux(P, L, Rc, d, F, Ss, vstar, b.scal);
         store_flux(P, b.FX, nf, f, F, Ss, vstar);
         if (P.thinc) {
-            const CellT<R>& src = side ? Rc : L;
             int idx[3] = {i, j, k};
             if (idx[d] < D.n[d]) {  // ULStar alpha at the valid cell of this face
                 long long g = D.off + i + (long long)D.n[0] * (j + (long long)D.n[1] * k);
-                for (int m = 0; m < P.M; ++m) b.ulstar[(long long)m * nt + g] = src.alpha[m];
+                #pragma unroll UnrollM<PT>::n
+                for (int m = 0; m < P.M; ++m) b.ulstar[(long long)m * nt + g] = (side ? Rc.alpha[m] : L.alpha[m]);
             }
             if (idx[d] >= 1) {  // the ghost hi+1 of the box to the left, if this is its hi face
                 long long gL = D.off + (i - o[0]) + (long long)D.n[0] * ((j - o[1]) + (long long)D.n[1] * (k - o[2]));
                 const int* bx = b.boxes + 6 * (D.box_off + b.cell_box[gL]);
                 if (bx[3 + d] == idx[d] - 1)
-                    for (int m = 0; m < P.M; ++m) b.gstar[d][(long long)m * nf + f] = src.alpha[m];
+                    #pragma unroll UnrollM<PT>::n
+                    for (int m = 0; m < P.M; ++m) b.gstar[d][(long long)m * nf + f] = (side ? Rc.alpha[m] : L.alpha[m]);
             }
         }
     }
@@ -955,20 +991,23 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
 // Plastic radial return (plastic.cpp:83-223) and cleanUpV (:476-528).
 // ---------------------------------------------------------------------------
 template <typename PT, typename R = typename PT::real>
-__device__ inline int plastic_cell(const PT& P, CellT<R>& c)
+TJ_DEV int plastic_cell(const PT& P, CellT<R>& c)
 {
     R tsolid = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m)
-        if (P.phase[m] == TJ_PHASE_SOLID) tsolid += c.alpha[m];
+        if (phase_of(P, m) == TJ_PHASE_SOLID) tsolid += c.alpha[m];
     if (tsolid <= R(0.5)) {  // cellIsMostlyFluid
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) { c.eps[m] = R(0.0); c.are[m] = R(0.0); }
         return 0;
     }
     hencky(P, c);
     R JT = R(0.0), JB = R(0.0), norm = R(0.0), J, Jn;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         ECellT<R> e = ecell_of(c, m);
-        if (P.phase[m] == TJ_PHASE_SOLID) {
+        if (phase_of(P, m) == TJ_PHASE_SOLID) {
             J = root(c.hj2);
             R G = eos_G(P, m, e);
             if (G * J * sqrt(R(3.0)) > P.yield[m]) Jn = quot(P.yield[m], sqrt(R(3.0)) * G);
@@ -1012,19 +1051,22 @@ __device__ inline int plastic_cell(const PT& P, CellT<R>& c)
 // once; the reconstruction of V from devH and the conservativeToPrimitive
 // that follows are binary32 (pressure closure in binary64).
 template <typename PT, typename R = typename PT::real>
-__device__ inline int plastic_cell_proj64(const PT& P, CellT<R>& c)
+TJ_DEV int plastic_cell_proj64(const PT& P, CellT<R>& c)
 {
     const DevParams& PD = P.d;
     R tsolid = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m)
-        if (P.phase[m] == TJ_PHASE_SOLID) tsolid += c.alpha[m];
+        if (phase_of(P, m) == TJ_PHASE_SOLID) tsolid += c.alpha[m];
     if (tsolid <= R(0.5)) {  // cellIsMostlyFluid
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) { c.eps[m] = R(0.0); c.are[m] = R(0.0); }
         return 0;
     }
     hencky(P, c);
     const double hj2 = c.hj2;
     double JT = 0.0, JB = 0.0, norm = 0.0;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         ECellT<double> e;
         e.alpha = c.alpha[m];
@@ -1036,7 +1078,7 @@ __device__ inline int plastic_cell_proj64(const PT& P, CellT<R>& c)
         e.rm0 = c.rm0;
         e.rm1 = c.rm1;
         double J, Jn;
-        if (P.phase[m] == TJ_PHASE_SOLID) {
+        if (phase_of(P, m) == TJ_PHASE_SOLID) {
             J = root(hj2);
             const double G = eos_G(PD, m, e);
             Jn = (G * J * sqrt(3.0) > PD.yield[m]) ? quot(PD.yield[m], sqrt(3.0) * G) : J;
@@ -1074,12 +1116,13 @@ __device__ inline int plastic_cell_proj64(const PT& P, CellT<R>& c)
 }
 
 template <typename PT, typename R = typename PT::real>
-__device__ inline void cleanup_v_cell(const PT& P, CellT<R>& c)
+TJ_DEV void cleanup_v_cell(const PT& P, CellT<R>& c)
 {
     R ta = R(0.0), ts = R(0.0);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         ta += c.alpha[m];
-        if (P.phase[m] == TJ_PHASE_SOLID) ts += c.alpha[m];
+        if (phase_of(P, m) == TJ_PHASE_SOLID) ts += c.alpha[m];
     }
     R B[9], Sq[9];
     mmT3(c.V, c.V, B);
@@ -1093,9 +1136,10 @@ __device__ inline void cleanup_v_cell(const PT& P, CellT<R>& c)
 
 // contains_nan over the conservative and primitive lists of one cell.
 template <typename PT, typename R = typename PT::real>
-__device__ inline bool cell_has_nan(const PT& P, const CellT<R>& c)
+TJ_DEV bool cell_has_nan(const PT& P, const CellT<R>& c)
 {
     bool n = false;
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) n |= isnan(c.alpha[m]) || isnan(c.arho[m]) || isnan(c.rhok[m]);
 #pragma unroll
     for (int r = 0; r < 3; ++r) n |= isnan(c.rhou[r]) || isnan(c.vel[r]);
@@ -1104,6 +1148,7 @@ __device__ inline bool cell_has_nan(const PT& P, const CellT<R>& c)
 #pragma unroll
         for (int q = 0; q < 9; ++q) n |= isnan(c.V[q]);
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) n |= isnan(c.eps[m]) || isnan(c.are[m]);
     if (P.nmix) n |= isnan(c.lam) || isnan(c.arl);
     return n;
@@ -1127,7 +1172,7 @@ __device__ __forceinline__ R reactive_euler(R arl, R arho, R p, R alpha, R dt)
 // same alphaRho, pressure and alpha, averaged with the start value, then
 // conservativeToPrimitive. Returns the c2p status.
 template <typename PT, typename R = typename PT::real>
-__device__ inline int reactive_cell(const PT& P, CellT<R>& c, R dt)
+TJ_DEV int reactive_cell(const PT& P, CellT<R>& c, R dt)
 {
     const R a0 = c.arl;
     const R a1 = reactive_euler(a0, c.arho[0], c.p, c.alpha[0], dt);
@@ -1143,11 +1188,12 @@ __device__ inline int reactive_cell(const PT& P, CellT<R>& c, R dt)
 // point and the velocity is the cell's; neither changes while the conservative
 // variables are updated, so the per-cell order is the reference's.
 template <typename PT, typename R = typename PT::real>
-__device__ inline void radial_source(const PT& P, CellT<R>& c, const R* sg, int i, double dx0, R dt)
+TJ_DEV void radial_source(const PT& P, CellT<R>& c, const R* sg, int i, double dx0, R dt)
 {
     const R inv_r = quot(R(P.dim == 1 ? -2.0 : -1.0), ((R)i + R(0.5)) * (R)dx0);
     const R s = dt * inv_r;
     const R u = c.vel[0];
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         c.alpha[m] += s * R(0.0);
         c.arho[m] += s * (c.arho[m] * u);
@@ -1168,6 +1214,7 @@ __device__ inline void radial_source(const PT& P, CellT<R>& c, const R* sg, int 
             c.V[q] += s * g;
         }
         if (P.plastic)
+            #pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m) c.are[m] += s * (c.are[m] * u);
     }
 }
@@ -1199,6 +1246,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
     if (first) Yc = U;
     else load_state(P, Y, nt, g, nullptr, Yc);
     const R dtdx = quot(dtdx_num, (R)D.dx[d]);
+    #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         Yc.alpha[m] += dtdx * (FXW(P.X_ALPHA + m, 0) - FXW(P.X_ALPHA + m, 1) - U.alpha[m] * (FXW(P.X_SSTAR, 0) - FXW(P.X_SSTAR, 1)));
         Yc.arho[m] += dtdx * (FXW(P.X_ARHO + m, 0) - FXW(P.X_ARHO + m, 1));
@@ -1216,6 +1264,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
                                 U.vel[row] * (FXW(P.X_VSTAR + col, 0) - FXW(P.X_VSTAR + col, 1)));
         }
     if (P.plastic)
+        #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) Yc.are[m] += dtdx * (FXW(P.X_ARE + m, 0) - FXW(P.X_ARE + m, 1));
     if (P.nmix) Yc.arl += dtdx * (FXW(P.X_ARL, 0) - FXW(P.X_ARL, 1));
     if (last) {
@@ -1226,6 +1275,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
             // U1 = U*0.5 + U2*0.5 over every carried component (hllc.cpp:705)
             CellT<R> A0;
             load_state(P, b.A, nt, g, nullptr, A0);
+            #pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m) {
                 Yc.alpha[m] = (A0.alpha[m] * (R(1.0) / R(2.0))) + (Yc.alpha[m] * (R(1.0) / R(2.0)));
                 Yc.arho[m] = (A0.arho[m] * (R(1.0) / R(2.0))) + (Yc.arho[m] * (R(1.0) / R(2.0)));
@@ -1338,10 +1388,12 @@ __global__ void k_cfl(PT P, PathBufs<typename PT::real> b, const R* __restrict__
         CellT<R> c;
         load_state(P, X, nt, g, nullptr, c);
         R a = sound_speed(P, c);
-        for (int n = 0; n < P.dim; ++n) {
-            R v = quot((R)D.dx[n], a + fabs(c.vel[n]));
-            if (v < mn) mn = v;
-        }
+#pragma unroll
+        for (int n = 0; n < 3; ++n)
+            if (n < P.dim) {
+                R v = quot((R)D.dx[n], a + fabs(c.vel[n]));
+                if (v < mn) mn = v;
+            }
     }
     for (int s = 16; s > 0; s >>= 1) {
         R o = __shfl_down_sync(0xffffffffu, mn, s);

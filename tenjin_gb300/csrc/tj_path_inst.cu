@@ -1,11 +1,14 @@
 // One instance of the per-direction launchers (tj_path_launch.cuh), selected
 // at compile time: TJ_INST_R = 64 (binary64, DevParams) or 32 (binary32,
 // DevParams32); TJ_INST_M = material count, 0 for the generic instance;
+// TJ_INST_K = its ParamKind (0 if not given);
 // TJ_INST_D = direction, -1 for the generic instance; TJ_INST_R = 128 is the
 // tangent instance (DevParamsT, tj_dual.cuh), which has no CFL pass. The CFL
 // pass is instantiated with the first direction of each material count.
 #if defined(TJ_INST_R) && TJ_INST_R == 128
 #include "tj_dual.cuh"
+#elif defined(TJ_INST_K) && TJ_INST_K > 0
+#define TJ_DEV __device__ __forceinline__
 #endif
 #include "tj_path.cuh"
 #include "tj_path_launch.cuh"
@@ -69,7 +72,10 @@ using InstBase = DevParamsT;
 using InstBase = DevParams32;
 #endif
 #if TJ_INST_M > 0
-using InstPT = WithM<InstBase, TJ_INST_M>;
+#ifndef TJ_INST_K
+#define TJ_INST_K 0
+#endif
+using InstPT = WithM<InstBase, TJ_INST_M, TJ_INST_K>;
 #else
 using InstPT = InstBase;
 #endif

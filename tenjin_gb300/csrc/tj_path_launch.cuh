@@ -3,12 +3,16 @@
 // in which both are compile-time constants: the per-material loops unroll,
 // the cell structures stay in registers and every direction-indexed access
 // is static. M = 3 and 4 use the generic instance (runtime M and direction).
+// In binary64 the fluids and the plastic solids have instances of their own
+// (ParamKind), without the code and the registers of the rest.
 // The instances are compiled in separate translation units
 // (tj_path_inst.cu, once per type, M and direction) so that they build in
 // parallel.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "tj_fp64.cuh"
 
@@ -24,28 +28,60 @@ template <class PT>
 int path_cfl(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, cudaStream_t st,
              Prof* pr);
 
+// Whether a working type has instances of its own for a kind: binary64 for
+// both, binary32 for the plastic solids (its fluids have the fused kernels),
+// the tangent for none.
+template <class Base, int K>
+constexpr bool kHasKind = K == KIND_FLUID ? std::is_same<Base, DevParams>::value
+                                          : std::is_same<Base, DevParams>::value ||
+                                                std::is_same<Base, DevParams32>::value;
+
+template <class Base, int K>
+inline int path_dir_kind(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
+                         typename Base::real* Y, int d, int first, int last, int finish, cudaStream_t st, Prof* pr)
+{
+#define TJ_DIR(MC, DC) path_dir<WithM<Base, MC, K>, DC>(WithM<Base, MC, K>(P), b, X, Y, d, first, last, finish, st, pr)
+    switch (P.M * 4 + d) {
+        case 4: return TJ_DIR(1, 0);
+        case 5: return TJ_DIR(1, 1);
+        case 6: return TJ_DIR(1, 2);
+        case 8: return TJ_DIR(2, 0);
+        case 9: return TJ_DIR(2, 1);
+        case 10: return TJ_DIR(2, 2);
+        default: return path_dir<Base, -1>(P, b, X, Y, d, first, last, finish, st, pr);
+    }
+#undef TJ_DIR
+}
+
 template <class Base>
 inline int path_dir_any(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
                         typename Base::real* Y, int d, int first, int last, int finish, cudaStream_t st, Prof* pr)
 {
-    switch (P.M * 4 + d) {
-        case 4: return path_dir<WithM<Base, 1>, 0>(WithM<Base, 1>(P), b, X, Y, d, first, last, finish, st, pr);
-        case 5: return path_dir<WithM<Base, 1>, 1>(WithM<Base, 1>(P), b, X, Y, d, first, last, finish, st, pr);
-        case 6: return path_dir<WithM<Base, 1>, 2>(WithM<Base, 1>(P), b, X, Y, d, first, last, finish, st, pr);
-        case 8: return path_dir<WithM<Base, 2>, 0>(WithM<Base, 2>(P), b, X, Y, d, first, last, finish, st, pr);
-        case 9: return path_dir<WithM<Base, 2>, 1>(WithM<Base, 2>(P), b, X, Y, d, first, last, finish, st, pr);
-        case 10: return path_dir<WithM<Base, 2>, 2>(WithM<Base, 2>(P), b, X, Y, d, first, last, finish, st, pr);
-        default: return path_dir<Base, -1>(P, b, X, Y, d, first, last, finish, st, pr);
-    }
+    if constexpr (kHasKind<Base, KIND_FLUID>)
+        if (param_kind(P) == KIND_FLUID) return path_dir_kind<Base, KIND_FLUID>(P, b, X, Y, d, first, last, finish, st, pr);
+    if constexpr (kHasKind<Base, KIND_PLASTIC>)
+        if (param_kind(P) == KIND_PLASTIC) return path_dir_kind<Base, KIND_PLASTIC>(P, b, X, Y, d, first, last, finish, st, pr);
+    return path_dir_kind<Base, KIND_ANY>(P, b, X, Y, d, first, last, finish, st, pr);
+}
+
+template <class Base, int K>
+inline int path_cfl_kind(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
+                         cudaStream_t st, Prof* pr)
+{
+    if (P.M == 1) return path_cfl<WithM<Base, 1, K>>(WithM<Base, 1, K>(P), b, X, st, pr);
+    if (P.M == 2) return path_cfl<WithM<Base, 2, K>>(WithM<Base, 2, K>(P), b, X, st, pr);
+    return path_cfl<Base>(P, b, X, st, pr);
 }
 
 template <class Base>
 inline int path_cfl_any(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
                         cudaStream_t st, Prof* pr)
 {
-    if (P.M == 1) return path_cfl<WithM<Base, 1>>(WithM<Base, 1>(P), b, X, st, pr);
-    if (P.M == 2) return path_cfl<WithM<Base, 2>>(WithM<Base, 2>(P), b, X, st, pr);
-    return path_cfl<Base>(P, b, X, st, pr);
+    if constexpr (kHasKind<Base, KIND_FLUID>)
+        if (param_kind(P) == KIND_FLUID) return path_cfl_kind<Base, KIND_FLUID>(P, b, X, st, pr);
+    if constexpr (kHasKind<Base, KIND_PLASTIC>)
+        if (param_kind(P) == KIND_PLASTIC) return path_cfl_kind<Base, KIND_PLASTIC>(P, b, X, st, pr);
+    return path_cfl_kind<Base, KIND_ANY>(P, b, X, st, pr);
 }
 
 }  // namespace tj

@@ -7,10 +7,18 @@
 
 namespace tj {
 
+// What a parameter block's type says about its materials (WithM below).
+enum ParamKind {
+    KIND_ANY = 0,
+    KIND_FLUID = 1,   // stiffened gases only: no solid, plasticity, mixture or reaction
+    KIND_PLASTIC = 2  // SOLID with PLASTIC, no THINC, mixture or reaction
+};
+
 // Device copy of the solver parameters plus the layouts of the device
 // arrays (component offsets). Passed to kernels by value.
 struct DevParams {
     using real = double;
+    static constexpr int kKind = KIND_ANY;
     int dim, M, solid, thinc, plastic, muscl, any_solid;
     int fused64;  // fused kernels in binary64 (TJ_PRECISION_FUSED64)
     int radial;   // RADIAL: geometric source term after the plastic update
@@ -42,6 +50,7 @@ struct DevParams {
 // the binary64 block for the pressure closure and the yield projection.
 struct DevParams32 {
     using real = float;
+    static constexpr int kKind = KIND_ANY;
     int dim, M, solid, thinc, plastic, muscl, any_solid;
     int fused64;
     int radial;
@@ -64,15 +73,51 @@ struct DevParams32 {
     double rG[TJ_MAX_MAT], rR0h[TJ_MAX_MAT];
 };
 
-// A parameter block whose material count is a compile-time constant: the
-// static member M hides the base's runtime M, so that the per-material loops
-// of the kernels unroll and their per-material arrays stay in registers.
-template <class Base, int MC>
+// A parameter block whose material count, and with a kind what the
+// configuration holds, are compile-time constants: the static members hide the
+// base's runtime ones, so that the per-material loops of the kernels unroll,
+// their per-material arrays stay in registers, and a fluid's kernels hold no
+// code and no registers for solids, other equations of state or mixtures.
+template <class Base, int MC, int K = KIND_ANY>
 struct WithM : Base {
     static constexpr int M = MC;
     WithM() = default;
     explicit WithM(const Base& b) : Base(b) {}
 };
+template <class Base, int MC>
+struct WithM<Base, MC, KIND_FLUID> : Base {
+    static constexpr int M = MC, kKind = KIND_FLUID;
+    static constexpr int solid = 0, plastic = 0, any_solid = 0, nmix = 0, reactive = 0;
+    WithM() = default;
+    explicit WithM(const Base& b) : Base(b) {}
+};
+template <class Base, int MC>
+struct WithM<Base, MC, KIND_PLASTIC> : Base {
+    static constexpr int M = MC, kKind = KIND_PLASTIC;
+    static constexpr int solid = 1, plastic = 1, any_solid = 1, nmix = 0, reactive = 0, thinc = 0;
+    WithM() = default;
+    explicit WithM(const Base& b) : Base(b) {}
+};
+// Unroll count of a loop over the materials: all of them where the block's
+// type knows how many. A loop left rolled indexes its cells' arrays with a
+// variable, which puts the whole cell into local memory.
+template <class PT>
+struct UnrollM {
+    static constexpr int n = 1;
+};
+template <class Base, int MC, int K>
+struct UnrollM<WithM<Base, MC, K>> {
+    static constexpr int n = MC;
+};
+template <class Base>
+inline int param_kind(const Base& P)
+{
+    bool gases = true;
+    for (int m = 0; m < P.M; ++m) gases = gases && P.eos[m] == TJ_EOS_MIEGRUNEISEN && P.phase[m] == TJ_PHASE_FLUID;
+    if (P.nmix || P.reactive) return KIND_ANY;
+    if (gases && !P.solid && !P.plastic && !P.any_solid) return KIND_FLUID;
+    return P.solid && P.plastic && P.any_solid && !P.thinc ? KIND_PLASTIC : KIND_ANY;
+}
 
 // One independent domain: valid cells [0,n) per axis, stored contiguously
 // from cell offset `off` (i fastest) in every state block.
