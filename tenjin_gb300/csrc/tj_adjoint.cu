@@ -49,8 +49,10 @@ namespace tj {
 
 namespace {
 
-constexpr int NT = 256;
-constexpr int NBLK = 152 * 4;  // grid of the kernels that accumulate EOS-parameter adjoints
+// Blocks of two warps, as the forward's kernels (tj_fp64.cuh): at 192^2 cells
+// blocks of 256 left SMs with one block or none.
+constexpr int NT = 64;
+constexpr int NBLK = 152 * 16;  // grid of the kernels that accumulate EOS-parameter adjoints
 constexpr int NG = 3 * tja::MM;
 
 struct AG {
@@ -62,6 +64,19 @@ struct AG {
     int sa, sar, srk, srho, sru, su, sE, sp, ns;
     int NW;  // words of a reconstructed state: alpha[M], rho_k[M], u0, u1, p
     int nl;  // lines of the image arrays: max(nx, ny)
+};
+
+// The parameters with the material count a compile-time constant (MC > 0):
+// the loops over materials unroll and the states stay in registers.
+template <int MC>
+struct AGM : AG {
+    static constexpr int M = MC, NW = 2 * MC + 3;
+    tja::EosM<MC> E;
+    __device__ __forceinline__ explicit AGM(const AG& g) : AG(g), E(g.E) {}
+};
+template <>
+struct AGM<0> : AG {
+    __device__ __forceinline__ explicit AGM(const AG& g) : AG(g) {}
 };
 
 __device__ __forceinline__ int mapi(int i, int n, int lo, int hi, bool& refl)
@@ -79,7 +94,8 @@ __device__ __forceinline__ int mapi(int i, int n, int lo, int hi, bool& refl)
 }
 
 // carried-state word of reconstructed variable q
-__device__ __forceinline__ int qword(const AG& G, int q)
+template <class GT>
+__device__ __forceinline__ int qword(const GT& G, int q)
 {
     if (q < G.M) return G.sa + q;
     if (q < 2 * G.M) return G.srk + q - G.M;
@@ -89,7 +105,8 @@ __device__ __forceinline__ int qword(const AG& G, int q)
 
 // reconstructed variable q at cell (i, j) + s * o_d (s in -1, 0, 1), ghosts
 // mapped, the normal velocity negated in a reflected ghost
-__device__ __forceinline__ double qat(const AG& G, const double* X, int i, int j, int d, int s, int q)
+template <class GT>
+__device__ __forceinline__ double qat(const GT& G, const double* X, int i, int j, int d, int s, int q)
 {
     bool refl;
     if (d == 0) i = mapi(i + s, G.nx, G.lo_bc[0], G.hi_bc[0], refl);
@@ -107,9 +124,11 @@ __device__ __forceinline__ double& pw(tja::Prim& x, int M, int q)
 }
 
 // reconstructed state of valid cell (i, j) on side (0 UL, 1 UR) along d
-__device__ void face_prim(const AG& G, const double* X, const double* rec, int i, int j, int d, int side, tja::Prim& x)
+template <class GT>
+__device__ __forceinline__ void face_prim(const GT& G, const double* X, const double* rec, int i, int j, int d, int side, tja::Prim& x)
 {
     const long long g = i + (long long)G.nx * j;
+#pragma unroll
     for (int q = 0; q < G.NW; ++q) {
         const double u0 = qat(G, X, i, j, d, 0, q);
         double v = u0;
@@ -121,20 +140,26 @@ __device__ void face_prim(const AG& G, const double* X, const double* rec, int i
         pw(x, G.M, q) = v;
     }
     if (G.thinc)
+#pragma unroll
         for (int m = 0; m < G.M; ++m) x.a[m] = rec[((long long)(d * 2 + side) * G.M + m) * G.N + g];
 }
 
 // Adds the block's sum of g to its slot gpart[blockIdx.x][k], k = m (G),
 // MM + m (p_ref), 2 MM + m (e_ref).
-__device__ void block_add_grad(const tja::GradEos& g, int M, double* gpart)
+__device__ __forceinline__ void block_add_grad(const tja::GradEos& g, int M, double* gpart)
 {
     __shared__ double red[NT / 32][NG];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
     for (int k = 0; k < NG; ++k) {
         const int m = k % tja::MM, kind = k / tja::MM;
-        double v = m >= M ? 0.0 : (kind == 0 ? g.G[m] : (kind == 1 ? g.pr[m] : g.er[m]));
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[warp][k] = v;
+        if (m < M) {  // the slots of absent materials stay zero
+            double v = kind == 0 ? g.G[m] : (kind == 1 ? g.pr[m] : g.er[m]);
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[warp][k] = v;
+        } else if (lane == 0) {
+            red[warp][k] = 0.0;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -155,9 +180,11 @@ __global__ void k_adj_avg(DevParams P, AG G, const double* S0, const double* S2,
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
         for (int w = 0; w < G.ns; ++w) out[w * N + g] = (S0[w * N + g] * (1.0 / 2.0)) + (S2[w * N + g] * (1.0 / 2.0));
         double a[TJ_MAX_MAT];
+#pragma unroll
         for (int m = 0; m < G.M; ++m) a[m] = out[(G.sa + m) * N + g];
         const int e = cleanup_alpha(P, a);
         if (e) atomicCAS(&scal->status, 0, e);
+#pragma unroll
         for (int m = 0; m < G.M; ++m) out[(G.sa + m) * N + g] = a[m];
     }
 }
@@ -166,11 +193,14 @@ __global__ void k_adj_avg(DevParams P, AG G, const double* S0, const double* S2,
 // Reverse of the average and cleanUpAlpha: lam <- lam_avg / 2 (the S0 part),
 // lamA <- lam_avg / 2 (the S2 part).
 // ---------------------------------------------------------------------------
-__global__ void k_adj_finish(AG G, double* lam, double* lamA, const double* S0, const double* S2)
+template <int MC>
+__global__ void __launch_bounds__(NT, 8) k_adj_finish(AG G0, double* lam, double* lamA, const double* S0, const double* S2)
 {
+    const AGM<MC> G(G0);
     const long long N = G.N;
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
         double aavg[tja::MM], la[tja::MM], li[tja::MM];
+#pragma unroll
         for (int m = 0; m < G.M; ++m) {
             aavg[m] = (S0[(G.sa + m) * N + g] * (1.0 / 2.0)) + (S2[(G.sa + m) * N + g] * (1.0 / 2.0));
             la[m] = lam[(G.sa + m) * N + g];
@@ -190,8 +220,10 @@ __global__ void k_adj_finish(AG G, double* lam, double* lamA, const double* S0, 
 // mu = adjoint of the conserved words of a stage output Y, from the adjoint of
 // all its carried words (conservativeToPrimitive reversed).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(NT) k_adj_c2p(AG G, const double* lamY, const double* Y, double* mu, double* gpart)
+template <int MC>
+__global__ void __launch_bounds__(NT, 8) k_adj_c2p(AG G0, const double* lamY, const double* Y, double* mu, double* gpart)
 {
+    const AGM<MC> G(G0);
     const long long N = G.N;
     const int M = G.M;
     tja::GradEos gr;
@@ -201,6 +233,7 @@ __global__ void __launch_bounds__(NT) k_adj_c2p(AG G, const double* lamY, const 
         tja::Carried l;
         tja::zero(c);
         tja::zero(l);
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             c.a[m] = Y[(G.sa + m) * N + g];
             c.ar[m] = Y[(G.sar + m) * N + g];
@@ -219,6 +252,7 @@ __global__ void __launch_bounds__(NT) k_adj_c2p(AG G, const double* lamY, const 
         l.rho = lamY[G.srho * N + g];
         tja::Cons o;
         tja::c2p_rev(G.E, c, l, o, gr);
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             mu[(long long)m * N + g] = o.a[m];
             mu[(long long)(M + m) * N + g] = o.ar[m];
@@ -233,10 +267,12 @@ __global__ void __launch_bounds__(NT) k_adj_c2p(AG G, const double* lamY, const 
 // ---------------------------------------------------------------------------
 // Per face along d: adjoint of the two reconstructed states that meet there.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(NT) k_adj_face(AG G, int d, const double* X, const double* rec, const double* mu,
+template <int MC, int d>
+__global__ void __launch_bounds__(NT, 8) k_adj_face(AG G0, const double* X, const double* rec, const double* mu,
                                                  double* lface, double* limg, double* sstar, double dt, double* gpart,
                                                  double* sul)
 {
+    const AGM<MC> G(G0);
     const int M = G.M, NW = G.NW;
     const long long N = G.N;
     const int nfx = G.nx + (d == 0);
@@ -270,6 +306,7 @@ __global__ void __launch_bounds__(NT) k_adj_face(AG G, int d, const double* X, c
                                                                 : line + (long long)G.nx * (pos - 1))
                                                       : 0;
         double lS = 0.0;
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             const double muRa = hasR ? mu[(long long)m * N + cR] : 0.0, muLa = hasL ? mu[(long long)m * N + cL] : 0.0;
             const double muRr = hasR ? mu[(long long)(M + m) * N + cR] : 0.0,
@@ -297,6 +334,7 @@ __global__ void __launch_bounds__(NT) k_adj_face(AG G, int d, const double* X, c
             const double x1 = fabs(L.u[d]) + L.c, x2 = fabs(R.u[d]) + R.c;
             const double SL = -((x1 < x2) ? x2 : x1);
             const bool left = (SL >= 0.0) || (Ss >= 0.0);
+#pragma unroll
             for (int m = 0; m < M; ++m) {
                 const double v = sul[(long long)m * N + gR];
                 if (left) lL.a[m] += v;
@@ -311,6 +349,7 @@ __global__ void __launch_bounds__(NT) k_adj_face(AG G, int d, const double* X, c
         tja::face_state_rev(G.E, xr, G.thinc != 0, lR, pR, gr);
         if (reflL) pL.u[d] = -pL.u[d];
         if (reflR) pR.u[d] = -pR.u[d];
+#pragma unroll
         for (int q = 0; q < NW; ++q) {
             if (!imgL) lface[((long long)(d * 2 + 1) * NW + q) * N + gL] = pw(pL, M, q);
             else limg[((long long)(d * 2) * NW + q) * G.nl + line] = pw(pL, M, q);
@@ -329,9 +368,11 @@ __device__ double thinc_exp(double x) { return tjm_exp(x); }
 // ---------------------------------------------------------------------------
 // Per cell along d: stencil gradient of each THINC candidate the forward used.
 // ---------------------------------------------------------------------------
-__global__ void k_adj_thinc(AG G, int d, const double* X, const int* code, const double* lface, const double* limg,
+template <int MC>
+__global__ void __launch_bounds__(NT, 8) k_adj_thinc(AG G0, int d, const double* X, const int* code, const double* lface, const double* limg,
                             double* tcon, double* sur)
 {
+    const AGM<MC> G(G0);
     const int M = G.M, NW = G.NW;
     const long long N = G.N;
     const int n = d == 0 ? G.nx : G.ny;
@@ -339,6 +380,7 @@ __global__ void k_adj_thinc(AG G, int d, const double* X, const int* code, const
         const int cd = code[(long long)d * N + g];
         const int i = (int)(g % G.nx), j = (int)(g / G.nx);
         const int pos = d == 0 ? i : j, line = d == 0 ? j : i;
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             double* tc = tcon + (long long)((d * M + m) * 9) * N + g;
             double s[3][3], ls[3][3];
@@ -391,6 +433,7 @@ __global__ void k_adj_scratch(AG G, int d, const int* code, const double* lface,
         if (!cd) continue;
         const int i = (int)(g % G.nx), j = (int)(g / G.nx);
         const int pos = d == 0 ? i : j, line = d == 0 ? j : i;
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             if (((cd >> (2 * m)) & 3) != 2) continue;
             double lL = lface[((long long)(d * 2) * NW + m) * N + g];
@@ -406,16 +449,19 @@ __global__ void k_adj_scratch(AG G, int d, const int* code, const double* lface,
 // ---------------------------------------------------------------------------
 // Per cell: adjoint of the stage input (written, or added to lamX).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const int* code, const double* lface,
+template <int MC>
+__global__ void __launch_bounds__(NT, 8) k_adj_gather(AG G0, const double* X, const int* code, const double* lface,
                                                    const double* limg, const double* mu, const double* sstar0,
                                                    const double* sstar1, const double* tcon, double* lamX, double dt,
                                                    int accumulate)
 {
+    const AGM<MC> G(G0);
     const int M = G.M, NW = G.NW;
     const long long N = G.N;
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(g % G.nx), j = (int)(g / G.nx);
         double acc[2 * tja::MM + 3];  // reconstructed variables: alpha, rho_k, u0, u1, p
+#pragma unroll
         for (int q = 0; q < NW; ++q) acc[q] = 0.0;
         // non-conservative alpha term: -dt/dx alpha (S*_{i-1/2} - S*_{i+1/2})
         double dS = 0.0;
@@ -425,6 +471,7 @@ __global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const 
             const long long h0 = i + (long long)G.nx * j;
             dS += quot(dt, G.dx[1]) * (sstar1[h0] - sstar1[h0 + G.nx]);
         }
+#pragma unroll
         for (int m = 0; m < M; ++m) acc[m] -= dS * mu[(long long)m * N + g];
         // MUSCL: cells ip = pos-1..pos+1 along d read this cell
         for (int d = 0; d < 2; ++d) {
@@ -438,6 +485,7 @@ __global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const 
                 const int cd = G.thinc ? code[(long long)d * N + gi] : 0;
                 bool rm, rp;
                 const int mm = mapi(ip - 1, n, lo, hi, rm), mp = mapi(ip + 1, n, lo, hi, rp);
+#pragma unroll
                 for (int q = 0; q < NW; ++q) {
                     if (q < M && ((cd >> (2 * q)) & 3)) continue;  // alpha from THINC
                     double lul = lface[((long long)(d * 2) * NW + q) * N + gi];
@@ -465,6 +513,7 @@ __global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const 
                         const int ci = i + a, cj = j + c;
                         if (ci < 0 || ci >= G.nx || cj < 0 || cj >= G.ny) continue;
                         const long long gi = ci + (long long)G.nx * cj;
+#pragma unroll
                         for (int m = 0; m < M; ++m) {
                             // k_adj_thinc wrote every cell's slots (zero where
                             // no candidate of this pass carries an adjoint)
@@ -479,22 +528,26 @@ __global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const 
                     }
         }
         // write: identity on the conserved words, acc on the reconstructed ones
-        double out[64];
-        for (int w = 0; w < G.ns; ++w) out[w] = 0.0;
+        const auto put = [&](int w, double v) {
+            double& o = lamX[(long long)w * N + g];
+            o = accumulate ? o + v : v;
+        };
+#pragma unroll
         for (int m = 0; m < M; ++m) {
-            out[G.sa + m] = mu[(long long)m * N + g] + acc[m];
-            out[G.sar + m] = mu[(long long)(M + m) * N + g];
-            out[G.srk + m] = acc[M + m];
+            put(G.sa + m, mu[(long long)m * N + g] + acc[m]);
+            put(G.sar + m, mu[(long long)(M + m) * N + g]);
+            put(G.srk + m, acc[M + m]);
         }
         for (int r = 0; r < 2; ++r) {
-            out[G.sru + r] = mu[(long long)(2 * M + r) * N + g];
-            out[G.su + r] = acc[2 * M + r];
+            put(G.sru + r, mu[(long long)(2 * M + r) * N + g]);
+            put(G.su + r, acc[2 * M + r]);
         }
-        out[G.sE] = mu[(long long)(2 * M + 2) * N + g];
-        out[G.sp] = acc[2 * M + 2];
-        for (int w = 0; w < G.ns; ++w) {
-            if (accumulate) lamX[w * N + g] += out[w];
-            else lamX[w * N + g] = out[w];
+        put(G.sE, mu[(long long)(2 * M + 2) * N + g]);
+        put(G.sp, acc[2 * M + 2]);
+        if (!accumulate) {
+            put(G.srho, 0.0);
+            put(G.sru + 2, 0.0);
+            put(G.su + 2, 0.0);
         }
     }
 }
@@ -503,8 +556,10 @@ __global__ void __launch_bounds__(NT) k_adj_gather(AG G, const double* X, const 
 // Reverse of the initial primitiveToConservative: the adjoint of the
 // primitives in the layout of tj_set_primitive (alpha[M], rho_k[M], u[3], p).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(NT) k_adj_p2c0(AG G, const double* lam, const double* S0, double* gprim, double* gpart)
+template <int MC>
+__global__ void __launch_bounds__(NT, 8) k_adj_p2c0(AG G0, const double* lam, const double* S0, double* gprim, double* gpart)
 {
+    const AGM<MC> G(G0);
     const long long N = G.N;
     const int M = G.M;
     tja::GradEos gr;
@@ -514,6 +569,7 @@ __global__ void __launch_bounds__(NT) k_adj_p2c0(AG G, const double* lam, const 
         tja::Carried l;
         tja::zero(x);
         tja::zero(l);
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             x.a[m] = S0[(G.sa + m) * N + g];
             x.rk[m] = S0[(G.srk + m) * N + g];
@@ -533,7 +589,9 @@ __global__ void __launch_bounds__(NT) k_adj_p2c0(AG G, const double* lam, const 
         tja::Prim lx;
         tja::p2c_state_rev(G.E, x, l, lx, gr);
         int w = 0;
+#pragma unroll
         for (int m = 0; m < M; ++m) gprim[(long long)(w++) * N + g] = lx.a[m];
+#pragma unroll
         for (int m = 0; m < M; ++m) gprim[(long long)(w++) * N + g] = lx.rk[m];
         gprim[(long long)(w++) * N + g] = lx.u[0];
         gprim[(long long)(w++) * N + g] = lx.u[1];
@@ -543,16 +601,24 @@ __global__ void __launch_bounds__(NT) k_adj_p2c0(AG G, const double* lam, const 
     block_add_grad(gr, M, gpart);
 }
 
+// One warp per parameter: a fixed stride per lane, a fixed tree.
 __global__ void k_adj_gsum(const double* gpart, int nblk, double* out)
 {
-    const int k = threadIdx.x;
-    if (k >= NG) return;
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += gpart[(long long)b * NG + k];
-    out[k] = s;
+    for (int b = lane; b < nblk; b += 32) s += gpart[(long long)b * NG + k];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) out[k] = s;
 }
 
-inline int nb(long long n) { return (int)std::min<long long>((n + NT - 1) / NT, 152 * 16); }
+inline int nb(long long n) { return (int)std::min<long long>((n + NT - 1) / NT, NBLK); }
+// the instance of a templated kernel for M materials
+#define ADJ_M(M, kernel, ...)                        \
+    do {                                             \
+        if ((M) == 1) kernel<1><<<__VA_ARGS__;       \
+        else if ((M) == 2) kernel<2><<<__VA_ARGS__;  \
+        else kernel<0><<<__VA_ARGS__;                \
+    } while (0)
 
 AG make_ag(const DevParams& P, const DevDomain& D)
 {
@@ -783,7 +849,7 @@ long long adj_backward(AdjState* a, const DevParams& P, const Fp64Bufs& b, const
         // reverse it
         for (int k = K - 1; k >= 0; --k) {
             const double dtn = a->dt[n0 + k];
-            k_adj_finish<<<nb(N), NT, 0, st>>>(G, a->lam, a->lamA, S(k, 0), S(k, 2));
+            ADJ_M(M, k_adj_finish, nb(N), NT, 0, st>>>(G, a->lam, a->lamA, S(k, 0), S(k, 2)));
             launches += 1;
             for (int stage = 1; stage >= 0; --stage) {
                 const double* X = S(k, stage);
@@ -792,33 +858,40 @@ long long adj_backward(AdjState* a, const DevParams& P, const Fp64Bufs& b, const
                 double* lamX = stage == 1 ? a->lamB : a->lam;
                 const double* rec = a->rec + (size_t)(2 * k + stage) * recw;
                 const int* code = a->code + (size_t)(2 * k + stage) * 2 * N;
-                k_adj_c2p<<<NBLK, NT, 0, st>>>(G, lamY, Y, a->mu, a->gpart);
+                ADJ_M(M, k_adj_c2p, nb(N), NT, 0, st>>>(G, lamY, Y, a->mu, a->gpart));
                 launches += 1;
                 // the stage's passes in reverse order (d = 1, then d = 0): each
                 // pass's scratch writes are reversed before its reads
                 for (int d = 1; d >= 0; --d) {
-                    k_adj_face<<<NBLK, NT, 0, st>>>(G, d, X, rec, a->mu, a->lface, a->limg, a->sstar + (d ? nf0 : 0),
-                                                    dtn, a->gpart, P.thinc ? a->sul : nullptr);
+                    const int fb = nb(d ? (long long)G.nx * (G.ny + 1) : (long long)(G.nx + 1) * G.ny);
+#define ADJ_FACE(MC, D)                                                                                         \
+    k_adj_face<MC, D><<<fb, NT, 0, st>>>(G, X, rec, a->mu, a->lface, a->limg, a->sstar + (D ? nf0 : 0), dtn,    \
+                                         a->gpart, P.thinc ? a->sul : nullptr)
+                    if (M == 1) d ? ADJ_FACE(1, 1) : ADJ_FACE(1, 0);
+                    else if (M == 2) d ? ADJ_FACE(2, 1) : ADJ_FACE(2, 0);
+                    else d ? ADJ_FACE(0, 1) : ADJ_FACE(0, 0);
+#undef ADJ_FACE
                     launches += 1;
                     if (P.thinc) {
-                        k_adj_thinc<<<nb(N), NT, 0, st>>>(G, d, X, code, a->lface, a->limg, a->tcon, a->sur);
+                        ADJ_M(M, k_adj_thinc, nb(N), NT, 0, st>>>(G, d, X, code, a->lface, a->limg, a->tcon, a->sur));
                         k_adj_scratch<<<nb(N), NT, 0, st>>>(G, d, code, a->lface, a->limg, a->sul, a->sur);
                         launches += 2;
                     }
                 }
-                k_adj_gather<<<nb(N), NT, 0, st>>>(G, X, code, a->lface, a->limg, a->mu, a->sstar, a->sstar + nf0,
-                                                   a->tcon, lamX, dtn, stage == 0 ? 1 : 0);
+                ADJ_M(M, k_adj_gather, nb(N), NT, 0, st>>>(G, X, code, a->lface, a->limg, a->mu, a->sstar,
+                       a->sstar + nf0, a->tcon, lamX, dtn, stage == 0 ? 1 : 0));
                 launches += 1;
             }
         }
     }
     // the first interval's S(0, 0) is the initial state
-    k_adj_p2c0<<<NBLK, NT, 0, st>>>(G, a->lam, a->seg, grad_prim, a->gpart);
-    k_adj_gsum<<<1, 32, 0, st>>>(a->gpart, NBLK, a->gsum);
+    ADJ_M(M, k_adj_p2c0, nb(N), NT, 0, st>>>(G, a->lam, a->seg, grad_prim, a->gpart));
+    k_adj_gsum<<<1, 32 * NG, 0, st>>>(a->gpart, NBLK, a->gsum);
     launches += 2;
     double g[NG];
     cudaMemcpyAsync(g, a->gsum, sizeof g, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
+#pragma unroll
     for (int m = 0; m < M; ++m) {
         for (int k = 0; k < TJ_MAX_EOS_PARAMS; ++k) grad_eos[m * TJ_MAX_EOS_PARAMS + k] = 0.0;
         grad_eos[m * TJ_MAX_EOS_PARAMS + 0] = g[m];                // params[0]: G = params[0] - 1

@@ -29,10 +29,12 @@
 #include "tj_quot.h"
 
 #ifdef __CUDACC__
-#define TJA_HD __host__ __device__ inline
+#define TJA_HD __host__ __device__ __forceinline__
+#define TJA_UNROLL _Pragma("unroll")  // with a constant material count nothing is indexed by a variable
 #define TJA_NOTFINITE(x) (isinf(x) || isnan(x))
 #else
 #define TJA_HD inline
+#define TJA_UNROLL
 #define TJA_NOTFINITE(x) (std::isinf(x) || std::isnan(x))
 #endif
 
@@ -46,6 +48,17 @@ constexpr int MM = 4;  // materials
 struct Eos {
     int M;
     double G[MM], pr[MM], er[MM];  // G = params[0] - 1, p_ref = params[1], e_ref = params[2]
+};
+
+// The same with the material count known at compile time (it hides Eos::M).
+template <int MC>
+struct EosM : Eos {
+    static constexpr int M = MC;
+    EosM() = default;
+#ifdef __CUDACC__
+    __host__ __device__
+#endif
+    explicit EosM(const Eos& e) : Eos(e) {}
 };
 
 struct GradEos {
@@ -74,27 +87,53 @@ struct Carried {
 
 TJA_HD void zero(GradEos& g)
 {
+    TJA_UNROLL
     for (int m = 0; m < MM; ++m) g.G[m] = g.pr[m] = g.er[m] = 0.0;
 }
 TJA_HD void zero(Prim& x)
 {
+    TJA_UNROLL
     for (int m = 0; m < MM; ++m) x.a[m] = x.rk[m] = 0.0;
     x.u[0] = x.u[1] = x.p = 0.0;
 }
 TJA_HD void zero(FS& x)
 {
+    TJA_UNROLL
     for (int m = 0; m < MM; ++m) x.a[m] = x.ar[m] = 0.0;
     x.rho = x.ru[0] = x.ru[1] = x.u[0] = x.u[1] = x.E = x.p = x.c = 0.0;
 }
 TJA_HD void zero(Cons& x)
 {
+    TJA_UNROLL
     for (int m = 0; m < MM; ++m) x.a[m] = x.ar[m] = 0.0;
     x.ru[0] = x.ru[1] = x.E = 0.0;
 }
 TJA_HD void zero(Carried& x)
 {
+    TJA_UNROLL
     for (int m = 0; m < MM; ++m) x.a[m] = x.ar[m] = x.rk[m] = 0.0;
     x.rho = x.ru[0] = x.ru[1] = x.u[0] = x.u[1] = x.E = x.p = 0.0;
+}
+
+// c ? a : b word by word (a reference to one of two states would put both
+// into local memory)
+TJA_HD FS pick(bool c, const FS& a, const FS& b)
+{
+    FS x;
+    TJA_UNROLL
+    for (int m = 0; m < MM; ++m) {
+        x.a[m] = c ? a.a[m] : b.a[m];
+        x.ar[m] = c ? a.ar[m] : b.ar[m];
+    }
+    x.rho = c ? a.rho : b.rho;
+    for (int r = 0; r < 2; ++r) {
+        x.ru[r] = c ? a.ru[r] : b.ru[r];
+        x.u[r] = c ? a.u[r] : b.u[r];
+    }
+    x.E = c ? a.E : b.E;
+    x.p = c ? a.p : b.p;
+    x.c = c ? a.c : b.c;
+    return x;
 }
 
 // ---------------------------------------------------------------------------
@@ -103,6 +142,7 @@ TJA_HD void zero(Carried& x)
 TJA_HD void cleanup_fwd(int M, const double* a, double* out)
 {
     double tot = 0.0, c[MM];
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         double v = a[m];
         if (v < 0.0) v = 1E-6;
@@ -110,6 +150,7 @@ TJA_HD void cleanup_fwd(int M, const double* a, double* out)
         c[m] = v;
         tot += v;
     }
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) out[m] = c[m] * (quot(1.0, tot));
 }
 
@@ -117,6 +158,7 @@ TJA_HD void cleanup_fwd(int M, const double* a, double* out)
 TJA_HD void cleanup_rev(int M, const double* a, const double* lam_out, double* lam_in)
 {
     double tot = 0.0, c[MM];
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         double v = a[m];
         if (v < 0.0) v = 1E-6;
@@ -125,8 +167,10 @@ TJA_HD void cleanup_rev(int M, const double* a, const double* lam_out, double* l
         tot += v;
     }
     double s = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) s += lam_out[m] * c[m];
     const double it = quot(1.0, tot);
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         const bool in = !(a[m] < 0.0) && !(a[m] > 1.0);
         lam_in[m] = in ? (lam_out[m] * it - s * it * it) : 0.0;
@@ -136,13 +180,16 @@ TJA_HD void cleanup_rev(int M, const double* a, const double* lam_out, double* l
 // ---------------------------------------------------------------------------
 // Face state: [cleanUpAlpha], primitiveToConservative, getSoundSpeed.
 // ---------------------------------------------------------------------------
-TJA_HD void face_state_fwd(const Eos& E, const Prim& x, bool clean, FS& s)
+template <class EosT>
+TJA_HD void face_state_fwd(const EosT& E, const Prim& x, bool clean, FS& s)
 {
     const int M = E.M;
     if (clean) cleanup_fwd(M, x.a, s.a);
     else
+        TJA_UNROLL
         for (int m = 0; m < M; ++m) s.a[m] = x.a[m];
     s.rho = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         s.ar[m] = s.a[m] * x.rk[m];
         s.rho += s.ar[m];
@@ -155,6 +202,7 @@ TJA_HD void face_state_fwd(const Eos& E, const Prim& x, bool clean, FS& s)
     }
     s.p = x.p;
     double invG = 0.0, ent = 0.0, pnt = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         invG += quot(s.a[m], E.G[m]);
         ent += E.er[m] * s.ar[m];
@@ -162,6 +210,7 @@ TJA_HD void face_state_fwd(const Eos& E, const Prim& x, bool clean, FS& s)
     }
     s.E = x.p * invG + ent - pnt + ke;
     double A = 0.0, xit = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         const double xi = quot(1.0, E.G[m]);
         const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
@@ -173,12 +222,14 @@ TJA_HD void face_state_fwd(const Eos& E, const Prim& x, bool clean, FS& s)
     s.c = root(quot(A, xit));
 }
 
-TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l, Prim& lx, GradEos& g)
+template <class EosT>
+TJA_HD void face_state_rev(const EosT& E, const Prim& x, bool clean, const FS& l, Prim& lx, GradEos& g)
 {
     const int M = E.M;
     FS s;
     face_state_fwd(E, x, clean, s);
     double la[MM], lar[MM], lrk[MM];
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         la[m] = l.a[m];
         lar[m] = l.ar[m];
@@ -188,6 +239,7 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
     // getSoundSpeed: c = sqrt(A / xit)
     {
         double A = 0.0, xit = 0.0;
+        TJA_UNROLL
         for (int m = 0; m < M; ++m) {
             const double xi = quot(1.0, E.G[m]);
             const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
@@ -198,6 +250,7 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
         const bool floored = A <= 0.0;
         const double lA = floored ? 0.0 : quot(l.c, 2.0 * s.c * xit);
         const double lxit = quot(-l.c * s.c, 2.0 * xit);
+        TJA_UNROLL
         for (int m = 0; m < M; ++m) {
             const double xi = quot(1.0, E.G[m]);
             const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
@@ -221,8 +274,10 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
     {
         const double lE = l.E;
         double invG = 0.0;
+        TJA_UNROLL
         for (int m = 0; m < M; ++m) invG += quot(s.a[m], E.G[m]);
         lp += lE * invG;
+        TJA_UNROLL
         for (int m = 0; m < M; ++m) {
             la[m] += quot(lE * (x.p - E.pr[m]), E.G[m]);
             g.G[m] += -quot(lE * (x.p - E.pr[m]) * s.a[m], E.G[m] * E.G[m]);
@@ -235,6 +290,7 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
             lu[r] += lE * s.rho * x.u[r] + l.ru[r] * s.rho;
         }
     }
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         lar[m] += lrho;
         la[m] += lar[m] * x.rk[m];
@@ -242,7 +298,9 @@ TJA_HD void face_state_rev(const Eos& E, const Prim& x, bool clean, const FS& l,
     }
     if (clean) cleanup_rev(M, x.a, la, lx.a);
     else
+        TJA_UNROLL
         for (int m = 0; m < M; ++m) lx.a[m] = la[m];
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) lx.rk[m] = lrk[m];
     lx.u[0] = lu[0];
     lx.u[1] = lu[1];
@@ -276,6 +334,7 @@ TJA_HD void hllc_fwd(int M, const FS& L, const FS& R, int d, HllcOut& o)
     const double SK = side ? SR : SL, uK = K.u[d];
     const double mult = (Ss - uK == 0.0 && Ss != 0.0) ? 1.0 : quot(SK - uK, SK - Ss);
     double ars[MM], rs = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         ars[m] = mult * K.ar[m];
         rs += ars[m];
@@ -286,6 +345,7 @@ TJA_HD void hllc_fwd(int M, const FS& L, const FS& R, int d, HllcOut& o)
     const double vsd = quot(rus[d], rs);
     const double Es = mult * K.rho * (quot(K.E, K.rho) + (Ss - uK) * (Ss + quot(K.p, K.rho * (SK - uK))));
     const double w = hllc ? SK : 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         o.Fa[m] = K.a[m] * vsd;
         o.Far[m] = K.ar[m] * uK + w * (ars[m] - K.ar[m]);
@@ -311,12 +371,13 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     else if (Ss >= 0.0) { side = 0; hllc = true; }
     else if (SR >= 0.0) { side = 1; hllc = true; }
     else { side = 1; hllc = false; }
-    const FS& K = side ? R : L;
-    FS& lK = side ? lR : lL;
+    const FS K = pick(side != 0, R, L);
+    FS lK = pick(side != 0, lR, lL);
     const double SK = side ? SR : SL, uK = K.u[d];
     const bool guard = Ss - uK == 0.0 && Ss != 0.0;
     const double mult = guard ? 1.0 : quot(SK - uK, SK - Ss);
     double ars[MM], rs = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         ars[m] = mult * K.ar[m];
         rs += ars[m];
@@ -333,11 +394,13 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     double lSs = lF.Ss, lSK = 0.0, luK = 0.0, lmult = 0.0, lvsd = 0.0;
     double lars[MM], lrus[2] = {0.0, 0.0}, lEs = 0.0;
     // alpha flux: Fa = K.a vsd
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         lK.a[m] += lF.Fa[m] * vsd;
         lvsd += lF.Fa[m] * K.a[m];
     }
     // Far = K.ar uK + w (ars - K.ar)
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         lK.ar[m] += lF.Far[m] * (uK - w);
         luK += lF.Far[m] * K.ar[m];
@@ -361,8 +424,10 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     // vsd = rus_d / rs
     lrus[d] += quot(lvsd, rs);
     const double lrs = quot(-lvsd * vsd, rs);
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) lars[m] += lrs;
     // ars = mult K.ar; rus_d = mult K.rho Ss; rus_o = mult K.ru_o
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         lmult += lars[m] * K.ar[m];
         lK.ar[m] += lars[m] * mult;
@@ -395,6 +460,8 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     if (side) lSR += lSK;
     else lSL += lSK;
     lK.u[d] += luK;
+    lL = pick(side == 0, lK, lL);
+    lR = pick(side != 0, lK, lR);
     // Ss = Num / Den
     const double lNum = quot(lSs, Den), lDen = quot(-lSs * Ss, Den);
     lR.p += lNum;
@@ -428,10 +495,12 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
 // carried words rho_k, rho, u, p. lam is the adjoint of all carried words;
 // mu (out) the adjoint of the conserved words.
 // ---------------------------------------------------------------------------
-TJA_HD void c2p_fwd(const Eos& E, const Cons& c, Carried& o)
+template <class EosT>
+TJA_HD void c2p_fwd(const EosT& E, const Cons& c, Carried& o)
 {
     const int M = E.M;
     o.rho = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         o.a[m] = c.a[m];
         o.ar[m] = c.ar[m];
@@ -446,6 +515,7 @@ TJA_HD void c2p_fwd(const Eos& E, const Cons& c, Carried& o)
     }
     o.E = c.E;
     double invG = 0.0, ent = 0.0, pnt = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         invG += quot(c.a[m], E.G[m]);
         ent += E.er[m] * c.ar[m];
@@ -454,14 +524,17 @@ TJA_HD void c2p_fwd(const Eos& E, const Cons& c, Carried& o)
     o.p = quot(c.E - ke - ent + pnt, invG);
 }
 
-TJA_HD void c2p_rev(const Eos& E, const Cons& c, const Carried& lam, Cons& mu, GradEos& g)
+template <class EosT>
+TJA_HD void c2p_rev(const EosT& E, const Cons& c, const Carried& lam, Cons& mu, GradEos& g)
 {
     const int M = E.M;
     Carried o;
     c2p_fwd(E, c, o);
     double D = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) D += quot(c.a[m], E.G[m]);
     const double lN = quot(lam.p, D), lD = quot(-lam.p * o.p, D);
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         mu.a[m] = lam.a[m] - quot(lam.rk[m] * o.rk[m], c.a[m]) + quot(lN * E.pr[m], E.G[m]) + quot(lD, E.G[m]);
         mu.ar[m] = lam.ar[m] + quot(lam.rk[m], c.a[m]) - lN * E.er[m];
@@ -478,6 +551,7 @@ TJA_HD void c2p_rev(const Eos& E, const Cons& c, const Carried& lam, Cons& mu, G
         mu.ru[r] = lam.ru[r] + quot(lu, o.rho);
         lrho += -quot(lu * o.u[r], o.rho);
     }
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) mu.ar[m] += lrho;
 }
 
@@ -486,10 +560,12 @@ TJA_HD void c2p_rev(const Eos& E, const Cons& c, const Carried& lam, Cons& mu, G
 // from alpha, rho_k, u, p. lam: adjoint of the carried words; lx: adjoint of
 // the primitives.
 // ---------------------------------------------------------------------------
-TJA_HD void p2c_state_fwd(const Eos& E, const Prim& x, Carried& o)
+template <class EosT>
+TJA_HD void p2c_state_fwd(const EosT& E, const Prim& x, Carried& o)
 {
     const int M = E.M;
     o.rho = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         o.a[m] = x.a[m];
         o.rk[m] = x.rk[m];
@@ -504,6 +580,7 @@ TJA_HD void p2c_state_fwd(const Eos& E, const Prim& x, Carried& o)
     }
     o.p = x.p;
     double invG = 0.0, ent = 0.0, pnt = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         invG += quot(x.a[m], E.G[m]);
         ent += E.er[m] * o.ar[m];
@@ -512,12 +589,14 @@ TJA_HD void p2c_state_fwd(const Eos& E, const Prim& x, Carried& o)
     o.E = x.p * invG + ent - pnt + ke;
 }
 
-TJA_HD void p2c_state_rev(const Eos& E, const Prim& x, const Carried& lam, Prim& lx, GradEos& g)
+template <class EosT>
+TJA_HD void p2c_state_rev(const EosT& E, const Prim& x, const Carried& lam, Prim& lx, GradEos& g)
 {
     const int M = E.M;
     Carried o;
     p2c_state_fwd(E, x, o);
     double invG = 0.0;
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) invG += quot(x.a[m], E.G[m]);
     const double lE = lam.E;
     double lar[MM];
@@ -527,6 +606,7 @@ TJA_HD void p2c_state_rev(const Eos& E, const Prim& x, const Carried& lam, Prim&
         lrho += lE * 0.5 * x.u[r] * x.u[r] + lam.ru[r] * x.u[r];
         lx.u[r] = lam.u[r] + lE * o.rho * x.u[r] + lam.ru[r] * o.rho;
     }
+    TJA_UNROLL
     for (int m = 0; m < M; ++m) {
         lar[m] = lam.ar[m] + lE * E.er[m] + lrho;
         lx.a[m] = lam.a[m] + quot(lE * (x.p - E.pr[m]), E.G[m]) + lar[m] * x.rk[m];
@@ -661,21 +741,34 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
 // ---------------------------------------------------------------------------
 TJA_HD void muscl_fwd(double um, double u0, double up, double& l, double& r)
 {
-    double rr = quot(u0 - um, up - u0);
-    if (TJA_NOTFINITE(rr)) rr = 0.0;
-    double phi = 0.0;
-    if (rr > 0.0) {
-        const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);
-        phi = (b < a) ? b : a;
+    const double num = u0 - um, den = up - u0;
+    const tj::tjq_u64 bn = tj::tjq_bits(num), bd = tj::tjq_bits(den);
+    double half = 0.0;  // of the limiter
+    if (!((bn ^ bd) >> 63) && (bn << 1) != 0 && (bd << 1) != 0) {
+        const double rr = quot(num, den);
+        if (!TJA_NOTFINITE(rr)) half = quot(rr < 1.0 ? rr : 1.0, 1.0 + rr);
     }
-    const double grad = phi * 0.5 * (up - um);
-    l = u0 - 0.5 * grad;
-    r = u0 + 0.5 * grad;
+    const double grad = half * (up - um);
+    l = fma(-0.5, grad, u0);
+    r = fma(0.5, grad, u0);
 }
 
 TJA_HD int muscl_branch(double um, double u0, double up)
 {
-    double rr = quot(u0 - um, up - u0);
+    const double num = u0 - um, den = up - u0;
+    const tj::tjq_u64 bn = tj::tjq_bits(num), bd = tj::tjq_bits(den);
+    // a ratio that is not positive: no slope
+    if (((bn ^ bd) >> 63) || (bn << 1) == 0 || (bd << 1) == 0) return 0;
+    // r >= 1 takes 2 / (1 + r), and r < 1 - 2^-49 takes 2 r / (1 + r), whose
+    // rounded value is then the smaller one: no division. In between, and
+    // where r may overflow or underflow (or is not a number), as the forward.
+    const int ed = (int)((bn >> 52) & 0x7ff) - (int)((bd >> 52) & 0x7ff);
+    if (ed > -900 && ed < 900) {
+        const double n = fabs(num), m = fabs(den);
+        if (n >= m) return 2;
+        if (n < m * (1.0 - 1.7763568394002505e-15)) return 1;
+    }
+    double rr = quot(num, den);
     if (TJA_NOTFINITE(rr)) rr = 0.0;
     if (rr <= 0.0) return 0;
     const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);

@@ -27,7 +27,10 @@ struct Dual {
 // (an infinite or undefined quotient the value side discards, such as the
 // limiter ratio of a uniform state): every product with a direction is
 // taken only when that direction is nonzero.
-__device__ __forceinline__ double dmul(double t, double x) { return t != 0.0 ? t * x : 0.0; }
+// (The test is made on the bits: a binary64 comparison costs as much as the
+// product.)
+__device__ __forceinline__ bool nonzero(double t) { return ((__double2hiint(t) << 1) | __double2loint(t)) != 0; }
+__device__ __forceinline__ double dmul(double t, double x) { return nonzero(t) ? t * x : 0.0; }
 
 __device__ __forceinline__ Dual operator+(Dual a, Dual b) { return Dual(a.v + b.v, a.d + b.d); }
 __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return Dual(a.v - b.v, a.d - b.d); }
@@ -36,7 +39,7 @@ __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return Dual(a.v * b.
 __device__ __forceinline__ Dual operator/(Dual a, Dual b)
 {
     const double q = quot(a.v, b.v);
-    return Dual(q, (b.d != 0.0 ? quot(a.d - q * b.d, b.v) : (a.d != 0.0 ? quot(a.d, b.v) : 0.0)));
+    return Dual(q, (nonzero(b.d) ? quot(a.d - q * b.d, b.v) : (nonzero(a.d) ? quot(a.d, b.v) : 0.0)));
 }
 __device__ __forceinline__ Dual operator+(Dual a, double b) { return Dual(a.v + b, a.d); }
 __device__ __forceinline__ Dual operator+(double a, Dual b) { return Dual(a + b.v, b.d); }
@@ -44,11 +47,11 @@ __device__ __forceinline__ Dual operator-(Dual a, double b) { return Dual(a.v - 
 __device__ __forceinline__ Dual operator-(double a, Dual b) { return Dual(a - b.v, -b.d); }
 __device__ __forceinline__ Dual operator*(Dual a, double b) { return Dual(a.v * b, dmul(a.d, b)); }
 __device__ __forceinline__ Dual operator*(double a, Dual b) { return Dual(a * b.v, dmul(b.d, a)); }
-__device__ __forceinline__ Dual operator/(Dual a, double b) { return Dual(quot(a.v, b), a.d != 0.0 ? quot(a.d, b) : 0.0); }
+__device__ __forceinline__ Dual operator/(Dual a, double b) { return Dual(quot(a.v, b), nonzero(a.d) ? quot(a.d, b) : 0.0); }
 __device__ __forceinline__ Dual operator/(double a, Dual b)
 {
     const double q = quot(a, b.v);
-    return Dual(q, b.d != 0.0 ? quot(-q * b.d, b.v) : 0.0);
+    return Dual(q, nonzero(b.d) ? quot(-q * b.d, b.v) : 0.0);
 }
 __device__ __forceinline__ Dual& operator+=(Dual& a, Dual b) { return a = a + b; }
 __device__ __forceinline__ Dual& operator-=(Dual& a, Dual b) { return a = a - b; }
@@ -81,7 +84,7 @@ __device__ __forceinline__ Dual fabs(Dual a) { return a.v < 0.0 ? -a : a; }
 __device__ __forceinline__ Dual root(Dual a)
 {
     const double s = root(a.v);
-    return Dual(s, a.d == 0.0 ? 0.0 : quot(a.d, 2.0 * s));
+    return Dual(s, nonzero(a.d) ? quot(a.d, 2.0 * s) : 0.0);
 }
 __device__ __forceinline__ Dual quot(Dual a, Dual b) { return a / b; }
 // a constant argument
@@ -91,13 +94,13 @@ __device__ __forceinline__ Dual tjm_exp(Dual a)
     const double e = tjm_exp(a.v);
     return Dual(e, dmul(a.d, e));
 }
-__device__ __forceinline__ Dual tjm_log(Dual a) { return Dual(tjm_log(a.v), a.d != 0.0 ? quot(a.d, a.v) : 0.0); }
+__device__ __forceinline__ Dual tjm_log(Dual a) { return Dual(tjm_log(a.v), nonzero(a.d) ? quot(a.d, a.v) : 0.0); }
 __device__ __forceinline__ Dual tjm_pow(Dual x, Dual y)
 {
     const double p = tjm_pow(x.v, y.v);
     double d = 0.0;
-    if (x.d != 0.0) d += quot(p * y.v * x.d, x.v);
-    if (y.d != 0.0) d += p * ::log(x.v) * y.d;
+    if (nonzero(x.d)) d += quot(p * y.v * x.d, x.v);
+    if (nonzero(y.d)) d += p * ::log(x.v) * y.d;
     return Dual(p, d);
 }
 __device__ __forceinline__ Dual tjm_cosh(Dual a) { return Dual(tjm_cosh(a.v), dmul(a.d, ::sinh(a.v))); }
@@ -127,7 +130,7 @@ __device__ inline void sqrtm3(const Dual* A, Dual* Rm)
     for (int i = 0; i < 9; ++i) {
         a[i] = A[i].v;
         da[i] = A[i].d;
-        any |= da[i] != 0.0;
+        any |= nonzero(da[i]);
     }
     sqrtm3(a, r);
     if (!any) {
