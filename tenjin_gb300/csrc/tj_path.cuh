@@ -60,6 +60,21 @@ __device__ __forceinline__ void avg_pair32(float ah, float al, float& bh, float&
     bh = t;
 }
 
+// a / 2 + b / 2, the RK2 average of one word (hllc.cpp:705). The products are
+// exact, so in binary64 one is left to the fused multiply-add and the other to
+// the exponent: one operation of that pipe instead of three, the same bits.
+template <typename R>
+__device__ __forceinline__ R mean(R a, R b)
+{
+    return (a * (R(1.0) / R(2.0))) + (b * (R(1.0) / R(2.0)));
+}
+__device__ __forceinline__ double mean(double a, double b)
+{
+    const int h = __double2hiint(b), e = (h >> 20) & 0x7ff;
+    const double hb = e > 1 && e < 0x7ff ? __hiloint2double(h - 0x100000, __double2loint(b)) : 0.5 * b;
+    return fma(0.5, a, hb);
+}
+
 __device__ __forceinline__ int find_dom(const DevDomain* doms, int ndom, long long g)
 {
     int lo = 0, hi = ndom - 1;
@@ -447,15 +462,8 @@ __device__ __forceinline__ R gv(const PT& P, const DevDomain& D, const R* X, lon
 }
 
 // ---------------------------------------------------------------------------
-// BVD-THINC candidate of one cell (thinc.cpp:67-147).
+// BVD-THINC candidate of one material in one cell (thinc.cpp:67-147).
 // ---------------------------------------------------------------------------
-template <typename R>
-struct ThincCand {
-    int mixed[TJ_MAX_MAT];
-    R L[TJ_MAX_MAT], Rv[TJ_MAX_MAT];
-    int flag;
-};
-
 template <typename PT, typename R = typename PT::real>
 TJ_DEV R youngs(const PT& P, const DevDomain& D, const R* X, long long nt, int m, int i,
                                 int j, int k, int d)  // thinc.cpp:28-53
@@ -471,37 +479,62 @@ TJ_DEV R youngs(const PT& P, const DevDomain& D, const R* X, long long nt, int m
 }
 
 template <typename PT, typename R = typename PT::real>
-TJ_DEV void thinc_cand(const PT& P, const DevDomain& D, const R* X, long long nt, int i, int j,
-                                  int k, int d, ThincCand<R>& t)
+TJ_DEV bool thinc_cand(const PT& P, const DevDomain& D, const R* X, long long nt, int m, int i, int j, int k, int d,
+                       R& L, R& Rv)
 {
     const R eps = R(1E-20), beta0 = P.beta;
     int o[3] = {0, 0, 0};
     o[d] = 1;
-    t.flag = 0;
-    #pragma unroll UnrollM<PT>::n
-    for (int m = 0; m < P.M; ++m) {
-        int a = P.S_ALPHA + m;
-        R aL = gv(P, D, X, nt, a, i - o[0], j - o[1], k - o[2]);
-        R aR = gv(P, D, X, nt, a, i + o[0], j + o[1], k + o[2]);
-        R a0 = gv(P, D, X, nt, a, i, j, k);
-        R mn = (aR < aL) ? aR : aL;
-        R mx = ((aL < aR) ? aR : aL) - mn;
-        R theta = (R)((R(0.0) < aR - aL) - (aR - aL < R(0.0)));
-        R C = (mx < eps) ? R(0.0) : quot(a0 - mn + eps, mx + eps);
-        R delta = R(1E-4);
-        int mixed = (C > delta) && (C < (R(0.999999) - delta)) && ((aR - a0) * (a0 - aL) >= R(0.0));
-        t.mixed[m] = mixed;
-        t.flag = mixed;  // the last material wins (thinc.cpp:110-114)
-        t.L[m] = R(0.0);
-        t.Rv[m] = R(0.0);
-        if (mixed) {
-            R nvc = (P.dim == 2) ? youngs(P, D, X, nt, m, i, j, k, d) : R(1.0);
-            R beta = nvc * beta0 + R(0.01);
-            R coshB = tjm_cosh(beta), tanhB = tjm_tanh(beta);
-            R B = tjm_exp(theta * beta * ((R(2.0) * C) - R(1.0)));
-            R A = quot((quot(B, coshB)) - R(1.0), tanhB);
-            t.Rv[m] = mn + (mx * R(0.5)) * (R(1.0) + theta * (quot(tanhB + A, R(1.0) + A * tanhB)));
-            t.L[m] = mn + (mx * R(0.5)) * (R(1.0) + theta * A);
+    int a = P.S_ALPHA + m;
+    R aL = gv(P, D, X, nt, a, i - o[0], j - o[1], k - o[2]);
+    R aR = gv(P, D, X, nt, a, i + o[0], j + o[1], k + o[2]);
+    R a0 = gv(P, D, X, nt, a, i, j, k);
+    R mn = (aR < aL) ? aR : aL;
+    R mx = ((aL < aR) ? aR : aL) - mn;
+    R theta = (R)((R(0.0) < aR - aL) - (aR - aL < R(0.0)));
+    R C = (mx < eps) ? R(0.0) : quot(a0 - mn + eps, mx + eps);
+    R delta = R(1E-4);
+    if (!((C > delta) && (C < (R(0.999999) - delta)) && ((aR - a0) * (a0 - aL) >= R(0.0)))) return false;
+    R nvc = (P.dim == 2) ? youngs(P, D, X, nt, m, i, j, k, d) : R(1.0);
+    R beta = nvc * beta0 + R(0.01);
+    R coshB = tjm_cosh(beta), tanhB = tjm_tanh(beta);
+    R B = tjm_exp(theta * beta * ((R(2.0) * C) - R(1.0)));
+    R A = quot((quot(B, coshB)) - R(1.0), tanhB);
+    Rv = mn + (mx * R(0.5)) * (R(1.0) + theta * (quot(tanhB + A, R(1.0) + A * tanhB)));
+    L = mn + (mx * R(0.5)) * (R(1.0) + theta * A);
+    return true;
+}
+
+// The candidates of every cell and material (thinc.cpp:67-147, the first
+// pass), one thread each: those of mixed cells into the persistent scratch
+// (the reference's ULStar / URStar), and which they are into mixed[m nt + g]
+// (the flux array's memory, which the reconstruction of a direction does not
+// use otherwise). The scratch of a mixed cell is read in this pass as its
+// candidate and never as the older value, so writing it before the
+// reconstruction reads any changes nothing. A cell's reconstruction needs its
+// own and both neighbours' candidates: formed there, each was formed three
+// times, in one thread's serial chain (adjoint 96^2, every cell mixed: k_recon
+// 205 us a direction).
+template <typename PT, int DC = -1, typename R = typename PT::real>
+__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
+    k_thinc(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int* __restrict__ mixed, int dyn_d)
+{
+    const int d = DC >= 0 ? DC : dyn_d;
+    if (b.scal->done) return;
+    const long long nt = b.ntot, all = nt * P.M;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
+        int m = 0;
+        long long g = e;
+        for (; g >= nt; g -= nt) ++m;
+        const DevDomain D = b.doms[find_dom(b.doms, b.ndom, g)];
+        int i, j, k;
+        split3(g - D.off, D.n[0], D.n[1], i, j, k);
+        R L, Rv;
+        const bool mix = thinc_cand(P, D, X, nt, m, i, j, k, d, L, Rv);
+        mixed[e] = mix;
+        if (mix) {
+            b.ulstar[e] = L;
+            b.urstar[e] = Rv;
         }
     }
 }
@@ -557,52 +590,53 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
             int idx[3] = {i, j, k};
             const int in_m = idx[d] - 1 >= bx[d], in_p = idx[d] + 1 <= bx[3 + d];
             reps = D.nbox - b.cell_box[g];
-            ThincCand<R> tc, tm, tp;
-            thinc_cand(P, D, X, nt, i, j, k, d, tc);
-            if (in_m) thinc_cand(P, D, X, nt, i - o[0], j - o[1], k - o[2], d, tm);
-            if (in_p) thinc_cand(P, D, X, nt, i + o[0], j + o[1], k + o[2], d, tp);
             const long long gmm = D.off + (i - o[0]) + (long long)D.n[0] * ((j - o[1]) + (long long)D.n[1] * (k - o[2]));
             const long long gpp = D.off + (i + o[0]) + (long long)D.n[0] * ((j + o[1]) + (long long)D.n[1] * (k + o[2]));
+            // the candidates of mixed cells are in the scratch (k_thinc)
+            const int* mixed = reinterpret_cast<const int*>(b.FX);
+            const bool flag = mixed[(long long)(P.M - 1) * nt + g] != 0;  // the last material wins (thinc.cpp:110-114)
             int code = 0;
-            #pragma unroll UnrollM<PT>::n
-            for (int m = 0; m < P.M; ++m) {
-                const int a = P.S_ALPHA + m;
-                R urm, ulp, trm, tlp;
-                // UR.left / UL.right: MUSCL value inside the box, stage input in a ghost.
-                if (in_m) {
-                    R l_, r_;
-                    muscl1(gv(P, D, X, nt, a, i - 2 * o[0], j - 2 * o[1], k - 2 * o[2]), um.alpha[m], u0.alpha[m], l_, r_);
-                    urm = r_;
-                    trm = tm.mixed[m] ? tm.Rv[m] : b.urstar[(long long)m * nt + gmm];
-                } else {
-                    urm = um.alpha[m];
-                    trm = R(0.0);  // URStar ghosts are never written
-                }
-                if (in_p) {
-                    R l_, r_;
-                    muscl1(u0.alpha[m], up.alpha[m], gv(P, D, X, nt, a, i + 2 * o[0], j + 2 * o[1], k + 2 * o[2]), l_, r_);
-                    ulp = l_;
-                    tlp = tp.mixed[m] ? tp.L[m] : b.ulstar[(long long)m * nt + gpp];
-                } else {
-                    ulp = up.alpha[m];
-                    // ULStar's ghost at the box's hi+1 face: star alpha of the last flux pass along d
-                    tlp = b.gstar[d][(long long)m * b.nftot[d] + face_index(D, d, i + o[0], j + o[1], k + o[2])];
-                }
-                R tpl = tc.mixed[m] ? tc.L[m] : b.ulstar[(long long)m * nt + g];
-                R tpr = tc.mixed[m] ? tc.Rv[m] : b.urstar[(long long)m * nt + g];
-                R upl = L.alpha[m], upr = Rc.alpha[m];
+            if (flag) {
+                #pragma unroll UnrollM<PT>::n
+                for (int m = 0; m < P.M; ++m) {
+                    const int a = P.S_ALPHA + m;
+                    R urm, ulp, trm, tlp;
+                    // UR.left / UL.right: MUSCL value inside the box, stage input in a ghost.
+                    if (in_m) {
+                        R l_, r_;
+                        muscl1(gv(P, D, X, nt, a, i - 2 * o[0], j - 2 * o[1], k - 2 * o[2]), um.alpha[m], u0.alpha[m], l_, r_);
+                        urm = r_;
+                        trm = b.urstar[(long long)m * nt + gmm];
+                    } else {
+                        urm = um.alpha[m];
+                        trm = R(0.0);  // URStar ghosts are never written
+                    }
+                    if (in_p) {
+                        R l_, r_;
+                        muscl1(u0.alpha[m], up.alpha[m], gv(P, D, X, nt, a, i + 2 * o[0], j + 2 * o[1], k + 2 * o[2]), l_, r_);
+                        ulp = l_;
+                        tlp = b.ulstar[(long long)m * nt + gpp];
+                    } else {
+                        ulp = up.alpha[m];
+                        // ULStar's ghost at the box's hi+1 face: star alpha of the last flux pass along d
+                        tlp = b.gstar[d][(long long)m * b.nftot[d] + face_index(D, d, i + o[0], j + o[1], k + o[2])];
+                    }
+                    R tpl = b.ulstar[(long long)m * nt + g];
+                    R tpr = b.urstar[(long long)m * nt + g];
+                    R upl = L.alpha[m], upr = Rc.alpha[m];
 #define MN(x, y) (((y) < (x)) ? (y) : (x))
 #define TBV(PL, PR)                                                                                          \
-    MN(MN(fabs(urm - (PL)) + fabs((PR)-ulp), fabs(trm - (PL)) + fabs((PR)-tlp)),                            \
-       MN(fabs(urm - (PL)) + fabs((PR)-tlp), fabs(trm - (PL)) + fabs((PR)-ulp)))
-                R tbvm = TBV(upl, upr);
-                R tbvt = TBV(tpl, tpr);
+        MN(MN(fabs(urm - (PL)) + fabs((PR)-ulp), fabs(trm - (PL)) + fabs((PR)-tlp)),                            \
+           MN(fabs(urm - (PL)) + fabs((PR)-tlp), fabs(trm - (PL)) + fabs((PR)-ulp)))
+                    R tbvm = TBV(upl, upr);
+                    R tbvt = TBV(tpl, tpr);
 #undef TBV
 #undef MN
-                if (tc.flag && tbvt < tbvm) {
-                    L.alpha[m] = tpl;
-                    Rc.alpha[m] = tpr;
-                    code |= (tc.mixed[m] ? 1 : 2) << (2 * m);
+                    if (tbvt < tbvm) {
+                        L.alpha[m] = tpl;
+                        Rc.alpha[m] = tpr;
+                        code |= (mixed[(long long)m * nt + g] ? 1 : 2) << (2 * m);
+                    }
                 }
             }
             if (b.rec) {
@@ -613,13 +647,6 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
                 }
                 b.rec_code[(long long)d * nt + g] = code;
             }
-            // THINC pass 1 writes its candidates into the persistent scratch.
-            #pragma unroll UnrollM<PT>::n
-            for (int m = 0; m < P.M; ++m)
-                if (tc.mixed[m]) {
-                    b.ulstar[(long long)m * nt + g] = tc.L[m];
-                    b.urstar[(long long)m * nt + g] = tc.Rv[m];
-                }
         }
         if (compact_faces(P)) {  // closed by the flux kernel
             store_prim_face(P, b.UL, nt, g, L);
@@ -811,6 +838,33 @@ TJ_DEV void store_flux(const PT& P, R* FX, long long nf, long long f, const Flux
 #undef FXS
 }
 
+// K = first ? A : B over the words the Riemann solvers read.
+template <typename PT, typename R = typename PT::real>
+TJ_DEV void select_cell(const PT& P, bool first, const CellT<R>& A, const CellT<R>& B, CellT<R>& K)
+{
+#define TJ_PICK(w) K.w = first ? A.w : B.w
+    #pragma unroll UnrollM<PT>::n
+    for (int m = 0; m < P.M; ++m) {
+        TJ_PICK(alpha[m]);
+        TJ_PICK(arho[m]);
+        if (P.plastic) TJ_PICK(are[m]);
+    }
+    TJ_PICK(rho);
+    TJ_PICK(E);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        TJ_PICK(rhou[r]);
+        TJ_PICK(vel[r]);
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        TJ_PICK(sigma[q]);
+        if (P.solid) TJ_PICK(V[q]);
+    }
+    if (P.nmix) TJ_PICK(arl);
+#undef TJ_PICK
+}
+
 // HLLC (hllc.cpp:384-487) or the 5-wave solver (133-380) at one face. F gets
 // the conservative fluxes, Ss the contact speed, vstar the VSTAR(d, col)
 // values (solids). Returns the side whose star alpha the face carries: 0
@@ -823,119 +877,79 @@ TJ_DEV int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& Rc, int d, 
     R SR = (x1 < x2) ? x2 : x1;
     R SL = -SR;
     Ss = quot(-Rc.sigma[4 * d] + L.sigma[4 * d] + L.rhou[d] * (SL - L.vel[d]) - Rc.rhou[d] * (SR - Rc.vel[d]), L.rho * (SL - L.vel[d]) - Rc.rho * (SR - Rc.vel[d]));  // getSstar, hllc.cpp:5-8
-    if (!P.solid) {
-        // the state K of the upwind side and its star state (no pointer or
-        // reference selects between L and Rc: both stay in registers)
-        auto hllc_side = [&](const CellT<R>& K, R SK, bool hllc) {
-            CellT<R> Ks;
-            star_state(P, K, Ks, SK, Ss, d);
-            FluxV<R> FK, FS, QK, QS;
-            phys_flux(P, K, d, FK);
-            phys_flux(P, Ks, d, FS);
-            if (hllc) {
-                cons_vals(P, K, QK);
-                cons_vals(P, Ks, QS);
-                flux_combine<1>(P, F, FS, FK, QK, QS, QS, SK, R(0.0));
-            } else {
-                flux_combine<0>(P, F, FS, FK, FK, FK, FK, R(0.0), R(0.0));
-            }
-        };
-        if (SL >= R(0.0) || Ss >= R(0.0)) {
-            hllc_side(L, SL, !(SL >= R(0.0)));
-            return 0;
-        }
-        hllc_side(Rc, SR, SR >= R(0.0));
-        return 1;
-    }
-    CellT<R> Ls, Rs;
-
-    // 5-wave solver for solids (hllc.cpp:133-380).
-    if (isnan(SL) || isnan(SR) || isnan(Ss)) { set_status(scal, TJ_ERR_WAVESPEED); return 0; }
-    R SLT = R(0.0), SRT = R(0.0);
-    CellT<R> Uss;
-    FluxV<R> QK, QKs, QSS, FK, FAs;
-    int side;
+    // 5-wave solver for solids (hllc.cpp:133-380)
+    if (P.solid && (isnan(SL) || isnan(SR) || isnan(Ss))) { set_status(scal, TJ_ERR_WAVESPEED); return 0; }
+    // The two sides run one code path on the upwind state K (and, for the inner
+    // wave, the other state O), picked word by word: a warp whose faces blow
+    // both ways would run a path of each side, one after the other (copper
+    // plate with 1 % noise: 21 of 32 threads active).
+    const bool left = SL >= R(0.0) || Ss >= R(0.0);
+    const bool plain = left ? SL >= R(0.0) : !(SR >= R(0.0));  // supersonic: the flux of K itself
+    CellT<R> K, Ks;
+    select_cell(P, left, L, Rc, K);
+    const R SK = left ? SL : SR;
+    star_state(P, K, Ks, SK, Ss, d);
+    FluxV<R> FK, FAs, QK, QKs;
+    phys_flux(P, K, d, FK);
+    phys_flux(P, Ks, d, FAs);
     auto vstar_of = [&](const CellT<R>& U) {  // VSTAR(d, col), read by update
+        if (P.solid)
 #pragma unroll
-        for (int col = 0; col < 3; ++col) vstar[col] = U.V[3 * d + col];
+            for (int col = 0; col < 3; ++col) vstar[col] = U.V[3 * d + col];
     };
-    auto starstar = [&](const CellT<R>& UK, CellT<R>& UKs, R SKT) {  // getStarStarState, hllc.cpp:87-129
-        Uss = UKs;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)  // getSigmaStar, hllc.cpp:75-83
-            UKs.sigma[3 * i + d] =
-                quot(Ls.rho * (Ss - SLT) * Rs.rho * (Ss - SRT) * (L.vel[i] - Rc.vel[i]) + Ls.rho * (Ss - SLT) * Rc.sigma[3 * i + d] -
-                 Rs.rho * (Ss - SRT) * L.sigma[3 * i + d], Ls.rho * (Ss - SLT) - Rs.rho * (Ss - SRT));
-#pragma unroll
-        for (int row = 0; row < 3; ++row) {
-            if (row == d) continue;
-            Uss.rhou[row] += quot(UKs.sigma[3 * row + d] - UK.sigma[3 * row + d], Ss - SKT);
-            Uss.vel[row] = quot(Uss.rhou[row], Uss.rho);
-        }
-#pragma unroll
-        for (int row = 0; row < 3; ++row) {
-            if (row == d) continue;
-            Uss.E += quot(Uss.vel[row] * UKs.sigma[3 * row + d] - UK.vel[row] * UK.sigma[3 * row + d], Ss - SKT);
-#pragma unroll
-            for (int col = 0; col < 3; ++col)
-                Uss.V[3 * row + col] += quot(Uss.V[3 * d + col] * (Uss.vel[row] - UK.vel[row]), Ss - SKT);
-        }
-    };
-    if (SL >= R(0.0)) {
-        star_state(P, L, Ls, SL, Ss, d);
-        phys_flux(P, Ls, d, FAs);
-        phys_flux(P, L, d, FK);
+    if (plain) {
         flux_combine<0>(P, F, FAs, FK, FK, FK, FK, R(0.0), R(0.0));
-        vstar_of(L);
-        side = 0;
-    } else if (Ss >= R(0.0)) {
-        star_state(P, L, Ls, SL, Ss, d);
-        SLT = Ss - transverse_speed(P, Ls);
-        phys_flux(P, Ls, d, FAs);
-        phys_flux(P, L, d, FK);
-        cons_vals(P, L, QK);
-        cons_vals(P, Ls, QKs);
-        if (SLT >= R(0.0)) {
-            flux_combine<1>(P, F, FAs, FK, QK, QKs, QKs, SL, R(0.0));
-            vstar_of(Ls);
-        } else {
-            star_state(P, Rc, Rs, SR, Ss, d);
-            SRT = Ss + transverse_speed(P, Rs);
-            starstar(L, Ls, SLT);
-            cons_vals(P, Uss, QSS);
-            flux_combine<2>(P, F, FAs, FK, QK, QKs, QSS, SL, SLT);
-            vstar_of(Uss);
-        }
-        side = 0;
-    } else if (SR >= R(0.0)) {
-        star_state(P, Rc, Rs, SR, Ss, d);
-        SRT = Ss + transverse_speed(P, Rs);
-        phys_flux(P, Rs, d, FAs);
-        phys_flux(P, Rc, d, FK);
-        cons_vals(P, Rc, QK);
-        cons_vals(P, Rs, QKs);
-        if (SRT >= R(0.0)) {
-            star_state(P, L, Ls, SL, Ss, d);
-            SLT = Ss - transverse_speed(P, Ls);
-            starstar(Rc, Rs, SRT);
-            cons_vals(P, Uss, QSS);
-            flux_combine<2>(P, F, FAs, FK, QK, QKs, QSS, SR, SRT);
-            vstar_of(Uss);
-        } else {
-            flux_combine<1>(P, F, FAs, FK, QK, QKs, QKs, SR, R(0.0));
-            vstar_of(Rs);
-        }
-        side = 1;
-    } else {
-        star_state(P, Rc, Rs, SR, Ss, d);
-        phys_flux(P, Rs, d, FAs);
-        phys_flux(P, Rc, d, FK);
-        flux_combine<0>(P, F, FAs, FK, FK, FK, FK, R(0.0), R(0.0));
-        vstar_of(Rc);
-        side = 1;
+        vstar_of(K);
+        return left ? 0 : 1;
     }
-    if (isnan(SL) || isnan(SR) || isnan(Ss) || isnan(SLT) || isnan(SRT)) set_status(scal, TJ_ERR_WAVESPEED);
-    return side;
+    cons_vals(P, K, QK);
+    cons_vals(P, Ks, QKs);
+    if (!P.solid) {
+        flux_combine<1>(P, F, FAs, FK, QK, QKs, QKs, SK, R(0.0));
+        return left ? 0 : 1;
+    }
+    const R cK = transverse_speed(P, Ks);
+    const R SKT = left ? Ss - cK : Ss + cK;
+    if (left ? SKT >= R(0.0) : !(SKT >= R(0.0))) {
+        flux_combine<1>(P, F, FAs, FK, QK, QKs, QKs, SK, R(0.0));
+        vstar_of(Ks);
+        if (isnan(SKT)) set_status(scal, TJ_ERR_WAVESPEED);
+        return left ? 0 : 1;
+    }
+    CellT<R> O, Os;
+    select_cell(P, left, Rc, L, O);
+    star_state(P, O, Os, left ? SR : SL, Ss, d);
+    const R cO = transverse_speed(P, Os);
+    const R SOT = left ? Ss + cO : Ss - cO;
+    const R lr = left ? Ks.rho : Os.rho, rr = left ? Os.rho : Ks.rho;
+    const R SLT = left ? SKT : SOT, SRT = left ? SOT : SKT;
+    // getStarStarState, hllc.cpp:87-129
+    CellT<R> Uss = Ks;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)  // getSigmaStar, hllc.cpp:75-83
+        Ks.sigma[3 * i + d] = quot(lr * (Ss - SLT) * rr * (Ss - SRT) * (L.vel[i] - Rc.vel[i]) +
+                                       lr * (Ss - SLT) * Rc.sigma[3 * i + d] - rr * (Ss - SRT) * L.sigma[3 * i + d],
+                                   lr * (Ss - SLT) - rr * (Ss - SRT));
+#pragma unroll
+    for (int row = 0; row < 3; ++row) {
+        if (row == d) continue;
+        Uss.rhou[row] += quot(Ks.sigma[3 * row + d] - K.sigma[3 * row + d], Ss - SKT);
+        Uss.vel[row] = quot(Uss.rhou[row], Uss.rho);
+    }
+#pragma unroll
+    for (int row = 0; row < 3; ++row) {
+        if (row == d) continue;
+        Uss.E += quot(Uss.vel[row] * Ks.sigma[3 * row + d] - K.vel[row] * K.sigma[3 * row + d], Ss - SKT);
+#pragma unroll
+        for (int col = 0; col < 3; ++col)
+            Uss.V[3 * row + col] += quot(Uss.V[3 * d + col] * (Uss.vel[row] - K.vel[row]), Ss - SKT);
+    }
+    FluxV<R> QSS;
+    cons_vals(P, Uss, QSS);
+    flux_combine<2>(P, F, FAs, FK, QK, QKs, QSS, SK, SKT);
+    vstar_of(Uss);
+    if (isnan(SKT) || isnan(SOT)) set_status(scal, TJ_ERR_WAVESPEED);
+    return left ? 0 : 1;
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
@@ -1232,20 +1246,12 @@ struct FacePairGlobal {
     __device__ __forceinline__ R operator()(int w, int s) const { return FX[(long long)w * nf + (s ? f1 : f0)]; }
 };
 
-// Update of cell g along d from the fluxes of its two faces (FXW(w, side));
-// the last direction: c2p; second stage: the average and the post-advance
-// operators of main.cpp:145-187.
+// Adds the update along d of one cell from the fluxes of its two faces
+// (FXW(w, side)) to its accumulator Yc (hllc.cpp:493-523); U is the cell's
+// stage input.
 template <typename PT, typename FA, typename R = typename PT::real>
-__device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, const R* __restrict__ X, R* Y,
-                                            long long g, const DevDomain& D, int i, int d, int first, int last,
-                                            int finish, R dtdx_num, const FA& FXW)
+__device__ __forceinline__ void add_fluxes(const PT& P, const CellT<R>& U, CellT<R>& Yc, R dtdx, const FA& FXW)
 {
-    const long long nt = b.ntot;
-    CellT<R> U, Yc;
-    load_state(P, X, nt, g, nullptr, U);
-    if (first) Yc = U;
-    else load_state(P, Y, nt, g, nullptr, Yc);
-    const R dtdx = quot(dtdx_num, (R)D.dx[d]);
     #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         Yc.alpha[m] += dtdx * (FXW(P.X_ALPHA + m, 0) - FXW(P.X_ALPHA + m, 1) - U.alpha[m] * (FXW(P.X_SSTAR, 0) - FXW(P.X_SSTAR, 1)));
@@ -1267,88 +1273,113 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
         #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) Yc.are[m] += dtdx * (FXW(P.X_ARE + m, 0) - FXW(P.X_ARE + m, 1));
     if (P.nmix) Yc.arl += dtdx * (FXW(P.X_ARL, 0) - FXW(P.X_ARL, 1));
-    if (last) {
-        const int ce = c2p(P, Yc);
-        if (ce) set_status(b.scal, ce);
-        if (finish) {
-            const R p_stage = Yc.p;  // U2's pressure, before the average
-            // U1 = U*0.5 + U2*0.5 over every carried component (hllc.cpp:705)
-            CellT<R> A0;
-            load_state(P, b.A, nt, g, nullptr, A0);
-            #pragma unroll UnrollM<PT>::n
-            for (int m = 0; m < P.M; ++m) {
-                Yc.alpha[m] = (A0.alpha[m] * (R(1.0) / R(2.0))) + (Yc.alpha[m] * (R(1.0) / R(2.0)));
-                Yc.arho[m] = (A0.arho[m] * (R(1.0) / R(2.0))) + (Yc.arho[m] * (R(1.0) / R(2.0)));
-                Yc.rhok[m] = (A0.rhok[m] * (R(1.0) / R(2.0))) + (Yc.rhok[m] * (R(1.0) / R(2.0)));
-                if (P.plastic) {
-                    Yc.eps[m] = (A0.eps[m] * (R(1.0) / R(2.0))) + (Yc.eps[m] * (R(1.0) / R(2.0)));
-                    Yc.are[m] = (A0.are[m] * (R(1.0) / R(2.0))) + (Yc.are[m] * (R(1.0) / R(2.0)));
-                }
-            }
-            Yc.rho = (A0.rho * (R(1.0) / R(2.0))) + (Yc.rho * (R(1.0) / R(2.0)));
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                Yc.rhou[r] = (A0.rhou[r] * (R(1.0) / R(2.0))) + (Yc.rhou[r] * (R(1.0) / R(2.0)));
-                Yc.vel[r] = (A0.vel[r] * (R(1.0) / R(2.0))) + (Yc.vel[r] * (R(1.0) / R(2.0)));
-            }
-            if constexpr (sizeof(R) == 4) avg_pair32(A0.E, A0.Elo, Yc.E, Yc.Elo);
-            else Yc.E = (A0.E * (R(1.0) / R(2.0))) + (Yc.E * (R(1.0) / R(2.0)));
-            Yc.p = (A0.p * (R(1.0) / R(2.0))) + (Yc.p * (R(1.0) / R(2.0)));
-            if (P.solid) {
-#pragma unroll
-                for (int qq = 0; qq < 9; ++qq) Yc.V[qq] = (A0.V[qq] * (R(1.0) / R(2.0))) + (Yc.V[qq] * (R(1.0) / R(2.0)));
-                Yc.hj2 = (A0.hj2 * (R(1.0) / R(2.0))) + (Yc.hj2 * (R(1.0) / R(2.0)));
-            }
-            if (P.nmix) {
-                Yc.rm0 = (A0.rm0 * (R(1.0) / R(2.0))) + (Yc.rm0 * (R(1.0) / R(2.0)));
-                Yc.rm1 = (A0.rm1 * (R(1.0) / R(2.0))) + (Yc.rm1 * (R(1.0) / R(2.0)));
-                Yc.lam = (A0.lam * (R(1.0) / R(2.0))) + (Yc.lam * (R(1.0) / R(2.0)));
-                Yc.arl = (A0.arl * (R(1.0) / R(2.0))) + (Yc.arl * (R(1.0) / R(2.0)));
-            }
-            if (finish == 2) {  // advance() alone: the average only
-                store_state(P, b.A, nt, g, Yc);
-                return;
-            }
-            if (P.reactive && P.nmix) {  // main.cpp:149-152
-                const int re = reactive_cell(P, Yc, dtdx_num);
-                if (re) set_status(b.scal, re);
-            }
+}
+
+// The end of a stage of one cell whose accumulator holds every direction's
+// update: conservativeToPrimitive; second stage: the average and the
+// post-advance operators of main.cpp:145-187.
+template <typename PT, typename R = typename PT::real>
+__device__ __forceinline__ void finish_cell(const PT& P, const PathBufs<R>& b, CellT<R>& Yc, R* Y, long long g,
+                                            const DevDomain& D, int i, int finish, R dtdx_num)
+{
+    const long long nt = b.ntot;
+    const int ce = c2p(P, Yc);
+    if (ce) set_status(b.scal, ce);
+    if (finish) {
+        const R p_stage = Yc.p;  // U2's pressure, before the average
+        // U1 = U*0.5 + U2*0.5 over every carried component (hllc.cpp:705)
+        CellT<R> A0;
+        load_state(P, b.A, nt, g, nullptr, A0);
+        #pragma unroll UnrollM<PT>::n
+        for (int m = 0; m < P.M; ++m) {
+            Yc.alpha[m] = mean(A0.alpha[m], Yc.alpha[m]);
+            Yc.arho[m] = mean(A0.arho[m], Yc.arho[m]);
+            Yc.rhok[m] = mean(A0.rhok[m], Yc.rhok[m]);
             if (P.plastic) {
-                int e;
-                if constexpr (sizeof(R) == 4) e = plastic_cell_proj64(P, Yc);
-                else e = plastic_cell(P, Yc);
-                c2p(P, Yc);
-                if (e) set_status(b.scal, e);
+                Yc.eps[m] = mean(A0.eps[m], Yc.eps[m]);
+                Yc.are[m] = mean(A0.are[m], Yc.are[m]);
             }
-            if (P.radial) {
-                // the stress the reference's U1 holds here: fresh from the
-                // c2p of the plastic or the reactive update, else the
-                // average of U's and U2's (fluids only: -p I each,
-                // boxaccesscellarray.cpp:204-212)
-                const bool fresh = P.plastic || (P.reactive && P.nmix);
-                R sg[9];
+        }
+        Yc.rho = mean(A0.rho, Yc.rho);
 #pragma unroll
-                for (int r = 0; r < 3; ++r)
+        for (int r = 0; r < 3; ++r) {
+            Yc.rhou[r] = mean(A0.rhou[r], Yc.rhou[r]);
+            Yc.vel[r] = mean(A0.vel[r], Yc.vel[r]);
+        }
+        if constexpr (sizeof(R) == 4) avg_pair32(A0.E, A0.Elo, Yc.E, Yc.Elo);
+        else Yc.E = mean(A0.E, Yc.E);
+        Yc.p = mean(A0.p, Yc.p);
+        if (P.solid) {
 #pragma unroll
-                    for (int qq = 0; qq < 3; ++qq) {
-                        const R dl = (R)(r == qq);
-                        sg[3 * r + qq] = fresh ? Yc.sigma[3 * r + qq]
-                                                   : ((-A0.p * dl) * (R(1.0) / R(2.0))) +
-                                                         ((-p_stage * dl) * (R(1.0) / R(2.0)));
-                    }
-                radial_source(P, Yc, sg, i, D.dx[0], dtdx_num);
-                const int rc = c2p(P, Yc);  // geometricSourceTerm (radial.cpp:50)
-                if (rc) set_status(b.scal, rc);
-            }
-            if (P.solid) cleanup_v_cell(P, Yc);
-            int e = cleanup_alpha(P, Yc.alpha);
-            if (e) set_status(b.scal, e);
-            if (b.cell_box[g] == D.nbox - 1 && cell_has_nan(P, Yc)) atomicOr(&b.scal->nan_flag, 1);
+            for (int qq = 0; qq < 9; ++qq) Yc.V[qq] = mean(A0.V[qq], Yc.V[qq]);
+            Yc.hj2 = mean(A0.hj2, Yc.hj2);
+        }
+        if (P.nmix) {
+            Yc.rm0 = mean(A0.rm0, Yc.rm0);
+            Yc.rm1 = mean(A0.rm1, Yc.rm1);
+            Yc.lam = mean(A0.lam, Yc.lam);
+            Yc.arl = mean(A0.arl, Yc.arl);
+        }
+        if (finish == 2) {  // advance() alone: the average only
             store_state(P, b.A, nt, g, Yc);
             return;
         }
+        if (P.reactive && P.nmix) {  // main.cpp:149-152
+            const int re = reactive_cell(P, Yc, dtdx_num);
+            if (re) set_status(b.scal, re);
+        }
+        if (P.plastic) {
+            int e;
+            if constexpr (sizeof(R) == 4) e = plastic_cell_proj64(P, Yc);
+            else e = plastic_cell(P, Yc);
+            c2p(P, Yc);
+            if (e) set_status(b.scal, e);
+        }
+        if (P.radial) {
+            // the stress the reference's U1 holds here: fresh from the
+            // c2p of the plastic or the reactive update, else the
+            // average of U's and U2's (fluids only: -p I each,
+            // boxaccesscellarray.cpp:204-212)
+            const bool fresh = P.plastic || (P.reactive && P.nmix);
+            R sg[9];
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int qq = 0; qq < 3; ++qq) {
+                    const R dl = (R)(r == qq);
+                    sg[3 * r + qq] = fresh ? Yc.sigma[3 * r + qq]
+                                               : ((-A0.p * dl) * (R(1.0) / R(2.0))) +
+                                                     ((-p_stage * dl) * (R(1.0) / R(2.0)));
+                }
+            radial_source(P, Yc, sg, i, D.dx[0], dtdx_num);
+            const int rc = c2p(P, Yc);  // geometricSourceTerm (radial.cpp:50)
+            if (rc) set_status(b.scal, rc);
+        }
+        if (P.solid) cleanup_v_cell(P, Yc);
+        int e = cleanup_alpha(P, Yc.alpha);
+        if (e) set_status(b.scal, e);
+        if (b.cell_box[g] == D.nbox - 1 && cell_has_nan(P, Yc)) atomicOr(&b.scal->nan_flag, 1);
+        store_state(P, b.A, nt, g, Yc);
+        return;
     }
     store_state(P, Y, nt, g, Yc);
+}
+
+// Update of cell g along d alone, from the accumulator in Y (the stage input
+// for the first direction), with the stage's end after the last direction.
+template <typename PT, typename FA, typename R = typename PT::real>
+__device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, const R* __restrict__ X, R* Y,
+                                            long long g, const DevDomain& D, int i, int d, int first, int last,
+                                            int finish, R dtdx_num, const FA& FXW)
+{
+    const long long nt = b.ntot;
+    CellT<R> U, Yc;
+    load_state(P, X, nt, g, nullptr, U);
+    if (first) Yc = U;
+    else load_state(P, Y, nt, g, nullptr, Yc);
+    add_fluxes(P, U, Yc, quot(dtdx_num, (R)D.dx[d]), FXW);
+    if (last) finish_cell(P, b, Yc, Y, g, D, i, finish, dtdx_num);
+    else store_state(P, Y, nt, g, Yc);
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
@@ -1411,7 +1442,6 @@ __global__ void k_cfl(PT P, PathBufs<typename PT::real> b, const R* __restrict__
         }
         if (lane == 0) atomicMin(&b.scal->dtmin_bits, (unsigned long long)__double_as_longlong((double)mn));
     }
-
 }
 
 }  // namespace tj

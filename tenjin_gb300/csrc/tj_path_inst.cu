@@ -42,6 +42,10 @@ int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     const char* nu = f64 ? "tj_update_fp64" : "tj_update_fp32";
     const LaunchShape cells = path_shape<PT>(b.ntot), faces = path_shape<PT>(b.nftot[d]);
     if (pr) pr->begin(nr, st);
+    if (P.thinc) {
+        const LaunchShape sh = path_shape<PT>(b.ntot * P.M);
+        k_thinc<PT, DC><<<sh.blocks, sh.threads, 0, st>>>(P, b, X, reinterpret_cast<int*>(b.FX), d);
+    }
     k_recon<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, d);
     if (pr) pr->end(nr, st);
     if (pr) pr->begin(nf, st);
@@ -50,7 +54,7 @@ int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     if (pr) pr->begin(nu, st);
     k_update<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, d, first, last, finish);
     if (pr) pr->end(nu, st);
-    return 3;
+    return P.thinc ? 4 : 3;
 }
 
 template <class PT>
