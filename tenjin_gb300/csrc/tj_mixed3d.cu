@@ -44,7 +44,11 @@ namespace tj {
 
 namespace {
 
-constexpr int NT3 = 512;
+// Threads per CTA. One CTA's tiles fill an SM's shared memory; 20 warps of 96
+// registers deal a 16x8x4 tile's 1760 faces in three rounds where 16 warps
+// take four, and hide more of each other's waits (128 boxes, 30 steps, with the
+// changes to the index arithmetic: 36.7 / 36.3 / 39.9 ms with 512 / 640 / 896).
+constexpr int NT3 = 640;
 
 struct M3P {
     int M;
@@ -53,12 +57,30 @@ struct M3P {
     float cEh[TJ_MAX_MAT], cEl[TJ_MAX_MAT], eEh[TJ_MAX_MAT], eEl[TJ_MAX_MAT];
 };
 
+// Factors of the divisions that turn an entry of a tile's lists into its
+// coordinates: t / d = (t * div3(d)) >> 20 for t < 2048 and d <= 240 (the error
+// of the factor, below d, times t stays below 2^20), one multiplication where
+// the compiler's division by a variable takes about twenty instructions; three
+// per staged cell, face and output cell were a quarter of the kernel.
+__host__ __device__ constexpr unsigned div3(unsigned d) { return ((1u << 20) + d - 1) / d; }
+
 // one tile of one domain
 struct Work3 {
     int dom;
     short i0, j0, k0;
     unsigned char ex, ey, ez, pad;
+    // div3 of: the staged row and plane, the output row and plane, and the
+    // rows and planes of the x faces and (planes) of the y faces
+    unsigned m_sx, m_sxy, m_ex, m_exy, m_fx, m_fxy, m_exfy;
 };
+
+__device__ __forceinline__ void split_t(int t, unsigned m_row, unsigned m_plane, int row, int rows, int& x, int& y, int& z)
+{
+    const int r = (int)(((unsigned)t * m_row) >> 20);
+    z = (int)(((unsigned)t * m_plane) >> 20);
+    x = t - r * row;
+    y = r - z * rows;
+}
 
 // per-domain data the kernels need
 struct Dom3 {
@@ -270,8 +292,11 @@ __device__ __forceinline__ void cleanup3(float* a)
         tot += v;
     }
     if (nan > 0) {
-        a[nan] = 1.0f - tot;
-        tot += a[nan];
+        const float v = 1.0f - tot;
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            if (m == nan) a[m] = v;
+        tot += v;
     }
     const float it = 1.0f / tot;
 #pragma unroll
@@ -319,7 +344,8 @@ __device__ void stage_issue(const M3P& P, const Work3& w, const Dom3& D, const f
     const long long off = D.off;
     const int sx = ex + 4, sy = ey + 4, sz = ez + 4;
     for (int t = threadIdx.x; t < sx * sy * sz; t += NT3) {
-        const int x = t % sx, y = (t / sx) % sy, z = t / (sx * sy);
+        int x, y, z;
+        split_t(t, w.m_sx, w.m_sxy, sx, sy, x, y, z);
         bool rx, ry, rz;
         const int gi = map3(i0 - 2 + x, nx, P.lo_bc[0], P.hi_bc[0], rx);
         const int gj = map3(j0 - 2 + y, ny, P.lo_bc[1], P.hi_bc[1], ry);
@@ -336,7 +362,8 @@ __device__ void stage_issue(const M3P& P, const Work3& w, const Dom3& D, const f
         cp_async4(sp + SM::P_OFF + (2 * M + 3) * SM::SV + s, Xin + S3_P<M>() * N + g);
     }
     for (int t = threadIdx.x; t < ex * ey * ez; t += NT3) {
-        const int x = t % ex, y = (t / ex) % ey, z = t / (ex * ey);
+        int x, y, z;
+        split_t(t, w.m_ex, w.m_exy, ex, ey, x, y, z);
         const long long g = off + (i0 + x) + (long long)nx * ((j0 + y) + (long long)ny * (k0 + z));
         const int c = x + TX * (y + TY * z);
 #pragma unroll
@@ -384,7 +411,8 @@ __device__ bool stage_fix(const M3P& P, const Work3& w, const Dom3& D, float* sp
     if (!near) return false;
     const int sx = w.ex + 4, sy = w.ey + 4, sz = w.ez + 4;
     for (int t = threadIdx.x; t < sx * sy * sz; t += NT3) {
-        const int x = t % sx, y = (t / sx) % sy, z = t / (sx * sy);
+        int x, y, z;
+        split_t(t, w.m_sx, w.m_sxy, sx, sy, x, y, z);
         bool r3[3];
         map3(w.i0 - 2 + x, D.n[0], P.lo_bc[0], P.hi_bc[0], r3[0]);
         map3(w.j0 - 2 + y, D.n[1], P.lo_bc[1], P.hi_bc[1], r3[1]);
@@ -466,17 +494,21 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fo
                 int u0 = ((int)threadIdx.x - base) % NT3;
                 if (u0 < 0) u0 += NT3;
                 for (int t = u0; t < nfd; t += NT3) {
-                    const int x = t % fx, y = (t / fx) % fy, z = t / (fx * fy);
+                    int x, y, z;
+                    split_t(t, d == 0 ? w.m_fx : w.m_ex, d == 0 ? w.m_fxy : (d == 1 ? w.m_exfy : w.m_exy), fx, fy, x, y, z);
                     const int f_d = d == 0 ? x : (d == 1 ? y : z);
                     const int posR = p0 + f_d;  // the face's right cell along d
                     // staged index of the right cell and the left cell
                     const int sR = (x + 2) + SM::SX * ((y + 2) + SM::SY * (z + 2));
                     const int sL = sR - stride;
+                    // a boundary face's outer state is the image of the inner
+                    // cell's (UR(0), UL(n-1)): another cell for the same code,
+                    // not another branch of it (a warp of x faces nearly always
+                    // holds one)
+                    const bool lo_face = posR == 0, hi_face = posR == n_d;
                     FS3<M> L, R;
-                    if (posR == 0) recon3<M, TX, TY, TZ>(P, sp, sR, stride, 1, d, lo_refl, L);  // image of UR(0)
-                    else recon3<M, TX, TY, TZ>(P, sp, sL, stride, 1, d, false, L);
-                    if (posR == n_d) recon3<M, TX, TY, TZ>(P, sp, sL, stride, 0, d, hi_refl, R);  // image of UL(n-1)
-                    else recon3<M, TX, TY, TZ>(P, sp, sR, stride, 0, d, false, R);
+                    recon3<M, TX, TY, TZ>(P, sp, lo_face ? sR : sL, stride, 1, d, lo_face && lo_refl, L);
+                    recon3<M, TX, TY, TZ>(P, sp, hi_face ? sL : sR, stride, 0, d, hi_face && hi_refl, R);
                     float F[2 * M + 5];
                     hllc3<M>(L, R, d, F);
                     const int fidx = x + fx * (y + fy * z);
@@ -492,7 +524,8 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fo
         //      (hllc.cpp:493-523), then the finish; a cell's words are touched
         //      by its own thread only, so no barrier separates the two ----
         for (int t = threadIdx.x; t < ex * ey * ez; t += NT3) {
-            const int x = t % ex, y = (t / ex) % ey, z = t / (ex * ey);
+            int x, y, z;
+            split_t(t, w.m_ex, w.m_exy, ex, ey, x, y, z);
             const int c = x + TX * (y + TY * z);
             const int s = (x + 2) + SM::SX * ((y + 2) + SM::SY * (z + 2));
             float* C = sp + SM::C_OFF;
@@ -921,6 +954,14 @@ struct Mixed3D : MixedBase {
                         w.ey = (unsigned char)y.second;
                         w.ez = (unsigned char)z.second;
                         w.pad = 0;
+                        const unsigned ex = w.ex, ey = w.ey;
+                        w.m_sx = div3(ex + 4);
+                        w.m_sxy = div3((ex + 4) * (ey + 4));
+                        w.m_ex = div3(ex);
+                        w.m_exy = div3(ex * ey);
+                        w.m_fx = div3(ex + 1);
+                        w.m_fxy = div3((ex + 1) * ey);
+                        w.m_exfy = div3(ex * (ey + 1));
                         work.push_back(w);
                     }
         }
