@@ -44,8 +44,15 @@ constexpr int MH = 3;            // staged halo
 constexpr int MS = MT + 2 * MH;  // staged cells per axis (34)
 constexpr int MP = MS + 1;       // shared-memory pitch (odd: conflict-free columns)
 constexpr int CP = MT + 1;       // pitch of the output-cell arrays (odd)
-constexpr int NTH = 256;         // threads per CTA
-constexpr int NWARP = NTH / 32;
+// Threads per CTA: ten warps, three CTAs an SM, where there are tiles for it
+// (1024^2, 40 steps: 7.12 / 7.25 / 7.02 / 7.43 ms with 256 / 288 / 320 / 352);
+// a grid of fewer tiles leaves SMs with one or two CTAs whose warps walk 28 rows
+// in three rounds or four, so up to two tiles an SM take 14 warps a CTA (two
+// rounds) and up to one takes 28 (one round): 28 warps an SM all the same
+// (333^2 MUSCL, 144 tiles, 40 steps: 1.48 ms with 256, 1.35 with 896).
+// Three and four materials need more registers and binary64 more shared memory:
+// 256 for them.
+constexpr int NTH = 320, NTH_2 = 448, NTH_1 = 896, NTH_WIDE = 256;
 constexpr int XR0 = -2;          // first row (relative to y0) of the x sweep with THINC
 constexpr int XRN = 32;          // rows of the x sweep with THINC: y0-2 .. y0+29
 
@@ -186,8 +193,11 @@ __device__ __forceinline__ void cleanup_f(R* a)
         tot += v;
     }
     if (nan > 0) {
-        a[nan] = R(1) - tot;
-        tot += a[nan];
+        const R v = R(1) - tot;
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            if (m == nan) a[m] = v;
+        tot += v;
     }
     const R it = R(1) / tot;
 #pragma unroll
@@ -271,8 +281,16 @@ __device__ __forceinline__ void cleanup_pair(float2* a)
         a[m] = f2(vx, vy);
         tot = add2(tot, a[m]);
     }
-    if (nanx > 0) { a[nanx].x = 1.0f - tot.x; tot.x += a[nanx].x; }
-    if (nany > 0) { a[nany].y = 1.0f - tot.y; tot.y += a[nany].y; }
+    if (nanx > 0 || nany > 0) {
+        const float2 v = f2(1.0f - tot.x, 1.0f - tot.y);
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            if (nanx > 0 && m == nanx) a[m].x = v.x;
+            if (nany > 0 && m == nany) a[m].y = v.y;
+        }
+        if (nanx > 0) tot.x += v.x;
+        if (nany > 0) tot.y += v.y;
+    }
     const float2 it = rcp2(tot);
 #pragma unroll
     for (int m = 0; m < M; ++m) a[m] = mul2(a[m], it);
@@ -777,9 +795,11 @@ __device__ void sweep_line(const MixP<R>& P, const MixB<R>& b, R* sm, int x0, in
     C[(2 * M + 3) * MTT + oc] = el;
 }
 
-template <typename R, int M, bool THINC>
-__global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R> P, MixB<R> b, int stage)
+template <typename R, int M, bool THINC, int NT>
+__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / NT) : 1)
+    k_stage2d(MixP<R> P, MixB<R> b, int stage)
 {
+    constexpr int NWARP = NT / 32;
     if (b.scal->done) return;
     using SM = Smem<R, M, THINC>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -789,6 +809,7 @@ __global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R>
     const R* __restrict__ Xin = b.X[stage];
     R* __restrict__ Xout = b.X[stage == 0 ? 1 : 0];
     const long long N = b.N;
+
     // binary32: dt/dx as a product with 1/dx (no binary64 division per thread)
     const R dtdx = sizeof(R) == 8 ? (R)(b.scal->dt / P.dxd[0]) : (R)b.scal->dt * P.idx[0];
     const R dtdy = sizeof(R) == 8 ? (R)(b.scal->dt / P.dxd[1]) : (R)b.scal->dt * P.idx[1];
@@ -796,7 +817,7 @@ __global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R>
     // ---- stage the primitives of tile + halo and the output cells' conserved
     //      words (U1 = U, hllc.cpp:583) with asynchronous copies: every copy is
     //      in flight at once, none holds a register ----
-    for (int t = threadIdx.x; t < MS * MS; t += NTH) {
+    for (int t = threadIdx.x; t < MS * MS; t += NT) {
         const int tx = t % MS, ty = t / MS;
         bool rx, ry;
         const int gx = reflect_map(x0 - MH + tx, P.nx, P.lo_bc[0], P.hi_bc[0], rx);
@@ -812,7 +833,7 @@ __global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R>
         cp_async_r(Su + (2 * M + 1) * MS * MP, Xin + W_U<M>(1) * N + g);
         cp_async_r(Su + (2 * M + 2) * MS * MP, Xin + W_P<M>() * N + g);
     }
-    for (int t = threadIdx.x; t < MT * MT; t += NTH) {
+    for (int t = threadIdx.x; t < MT * MT; t += NT) {
         const int ci = t % MT, cj = t / MT;
         const int gx = x0 + ci, gy = y0 + cj;
         if (gx >= P.nx || gy >= P.ny) continue;
@@ -836,7 +857,7 @@ __global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R>
         // while the sweeps run (both ends of each 28-cell row, which may
         // span two 128-byte lines).
         constexpr int NW = NWORDS<M>();
-        for (int t = threadIdx.x; t < NW * MT * 2; t += NTH) {
+        for (int t = threadIdx.x; t < NW * MT * 2; t += NT) {
             const int w = t / (2 * MT), r = (t >> 1) % MT, e = t & 1;
             const int gx = min(x0 + e * (MT - 1), P.nx - 1), gy = y0 + r;
             if (gy < P.ny) {
@@ -851,7 +872,7 @@ __global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R>
     // staged cells that mirror across a reflective face
     if ((P.lo_bc[0] == TJ_BC_REFLECTIVE && x0 < MH) || (P.hi_bc[0] == TJ_BC_REFLECTIVE && x0 - MH + MS > P.nx) ||
         (P.lo_bc[1] == TJ_BC_REFLECTIVE && y0 < MH) || (P.hi_bc[1] == TJ_BC_REFLECTIVE && y0 - MH + MS > P.ny)) {
-        for (int t = threadIdx.x; t < MS * MS; t += NTH) {
+        for (int t = threadIdx.x; t < MS * MS; t += NT) {
             const int tx = t % MS, ty = t / MS;
             bool rx, ry;
             reflect_map(x0 - MH + tx, P.nx, P.lo_bc[0], P.hi_bc[0], rx);
@@ -886,7 +907,7 @@ __global__ void __launch_bounds__(NTH, sizeof(R) == 4 ? 3 : 1) k_stage2d(MixP<R>
     // ---- finish: c2p; stage 2: average, cleanUpAlpha, CFL, NaN check ----
     R dtmin = RT<R>::big();
     bool nan_seen = false;
-    for (int t = threadIdx.x; t < MT * MT; t += NTH) {
+    for (int t = threadIdx.x; t < MT * MT; t += NT) {
         const int ci = t % MT, cj = t / MT;
         const int gx = x0 + ci, gy = y0 + cj;
         if (gx >= P.nx || gy >= P.ny) continue;
@@ -1387,17 +1408,30 @@ struct MixedImpl : MixedBase {
         return 2;
     }
 
-    template <int MM, bool TH>
-    void launch_stage(int stage, cudaStream_t st)
+    template <int MM, bool TH, int NT>
+    void launch_stage_n(int stage, dim3 grid, cudaStream_t st)
     {
         static bool attr = false;
         const size_t smb = Smem<R, MM, TH>::BYTES;
         if (!attr) {
-            cudaFuncSetAttribute(k_stage2d<R, MM, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+            cudaFuncSetAttribute(k_stage2d<R, MM, TH, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
             attr = true;
         }
-        dim3 grid((P.nx + MT - 1) / MT, (P.ny + MT - 1) / MT);
-        k_stage2d<R, MM, TH><<<grid, NTH, smb, st>>>(P, b, stage);
+        k_stage2d<R, MM, TH, NT><<<grid, NT, smb, st>>>(P, b, stage);
+    }
+
+    template <int MM, bool TH>
+    void launch_stage(int stage, cudaStream_t st)
+    {
+        constexpr int kSMs = 152;
+        const dim3 grid((P.nx + MT - 1) / MT, (P.ny + MT - 1) / MT);
+        const long long tiles = (long long)grid.x * grid.y;
+        if constexpr (sizeof(R) == 4 && MM <= 2) {
+            if (tiles <= kSMs) return launch_stage_n<MM, TH, NTH_1>(stage, grid, st);
+            if (tiles <= 2 * kSMs) return launch_stage_n<MM, TH, NTH_2>(stage, grid, st);
+            return launch_stage_n<MM, TH, NTH>(stage, grid, st);
+        }
+        launch_stage_n<MM, TH, NTH_WIDE>(stage, grid, st);
     }
 
     void stage_dispatch(int stage, cudaStream_t st)
