@@ -461,13 +461,12 @@ int tj_set_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim_l)
         TJ_CUDA(c, cudaMalloc(&c->A, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->A, 0, sizeof(double) * P.NS * nt));
     } else {
-        size_t fmax = (size_t)std::max(c->nftot[0], std::max(c->nftot[1], c->nftot[2]));
         TJ_CUDA(c, cudaMalloc(&c->A, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMalloc(&c->B, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMalloc(&c->C, sizeof(double) * P.NS * nt));
-        TJ_CUDA(c, cudaMalloc(&c->UL, sizeof(double) * P.NF * nt));
-        TJ_CUDA(c, cudaMalloc(&c->UR, sizeof(double) * P.NF * nt));
-        TJ_CUDA(c, cudaMalloc(&c->FX, sizeof(double) * P.NX * fmax));
+        TJ_CUDA(c, cudaMalloc(&c->UL, sizeof(double) * face_words(P) * nt));
+        TJ_CUDA(c, cudaMalloc(&c->UR, sizeof(double) * face_words(P) * nt));
+        TJ_CUDA(c, cudaMalloc(&c->FX, sizeof(double) * flux_words(P, c->nftot)));
         TJ_CUDA(c, cudaMemset(c->A, 0, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->B, 0, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->C, 0, sizeof(double) * P.NS * nt));

@@ -90,14 +90,13 @@ struct General32 : MixedBase {
         P = make_params32(DP);
         ns32 = DP.NS + 1;
         const size_t nt = (size_t)ntot;
-        size_t fmax = (size_t)std::max(nftot[0], std::max(nftot[1], nftot[2]));
         auto al = [&](float** p, size_t n) {
             if (cudaMalloc(p, sizeof(float) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
             cudaMemsetAsync(*p, 0, sizeof(float) * std::max<size_t>(n, 1), st);
             return true;
         };
-        bool ok = al(&A, ns32 * nt) && al(&B, ns32 * nt) && al(&C, ns32 * nt) && al(&UL, DP.NF * nt) &&
-                  al(&UR, DP.NF * nt) && al(&FX, DP.NX * fmax);
+        bool ok = al(&A, ns32 * nt) && al(&B, ns32 * nt) && al(&C, ns32 * nt) &&
+                  al(&UL, face_words(DP) * nt) && al(&UR, face_words(DP) * nt) && al(&FX, flux_words(DP, nftot));
         if (ok && DP.thinc) {
             ok = al(&uls, DP.M * nt) && al(&urs, DP.M * nt);
             for (int d = 0; ok && d < DP.dim; ++d) ok = al(&gs[d], DP.M * (size_t)nftot[d]);
@@ -157,21 +156,13 @@ struct General32 : MixedBase {
         return 1 + path_cfl_any(P, b, (const float*)A, st, nullptr);
     }
 
-    int stage(const float* X, float* Y, int finish, cudaStream_t st, Prof* pr)
-    {
-        int n = 0;
-        for (int d = 0; d < P.dim; ++d) n += path_dir_any(P, b, X, Y, d, d == 0, d == P.dim - 1, finish, st, pr);
-        return n;
-    }
-
     int step(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr) override
     {
         sync_geometry(fb);
-        int n = 0;
-        n += path_cfl_any(P, b, (const float*)A, st, pr);
+        int n = path_cfl_any(P, b, (const float*)A, st, pr);
         n += fp64_dt_finalize(DP, fb, 1, st);
-        n += stage(A, B, 0, st, pr);
-        n += stage(B, C, 1, st, pr);
+        n += path_stage_any(P, b, (const float*)A, B, 0, st, pr);
+        n += path_stage_any(P, b, (const float*)B, C, 1, st, pr);
         n += fp64_step_end(fb, st);
         return n;
     }

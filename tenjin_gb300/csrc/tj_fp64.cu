@@ -370,9 +370,7 @@ int fp64_dt_finalize(const DevParams& P, const Fp64Bufs& b, int clamp, cudaStrea
 
 int fp64_stage(const DevParams& P, const Fp64Bufs& b, const double* X, double* Y, int finish, cudaStream_t st, Prof* pr)
 {
-    int n = 0;
-    for (int d = 0; d < P.dim; ++d) n += path_dir_any(P, b, X, Y, d, d == 0, d == P.dim - 1, finish, st, pr);
-    return n;
+    return path_stage_any(P, b, X, Y, finish, st, pr);
 }
 
 int fp64_step_end(const Fp64Bufs& b, cudaStream_t st)

@@ -48,6 +48,21 @@ inline LaunchShape launch_shape(long long n, int most)
     return {(int)b, t};
 }
 
+// Words per cell of a face-state array (UL, UR): the primitives alone where the
+// flux kernel closes them (tj_path.cuh compact_faces), else the closed state.
+inline size_t face_words(const DevParams& P)
+{
+    if (P.thinc || P.nmix) return (size_t)P.NF;
+    return 2 * (size_t)P.M + 4 + (P.solid ? 9 + (P.any_solid ? 0 : 1) : 0) + (P.plastic ? (size_t)P.M : 0);
+}
+// Words of the flux array: every direction's faces.
+inline size_t flux_words(const DevParams& P, const long long* nftot)
+{
+    size_t n = 0;
+    for (int d = 0; d < P.dim; ++d) n += (size_t)P.NX * (size_t)nftot[d];
+    return n;
+}
+
 // The binary32 parameter block of a binary64 one (tj_fp32.cu).
 DevParams32 make_params32(const DevParams& P);
 

@@ -4,7 +4,8 @@
 // TJ_INST_K = its ParamKind (0 if not given);
 // TJ_INST_D = direction, -1 for the generic instance; TJ_INST_R = 128 is the
 // tangent instance (DevParamsT, tj_dual.cuh), which has no CFL pass. The CFL
-// pass is instantiated with the first direction of each material count.
+// pass and the whole-stage update are instantiated with the first direction of
+// each material count.
 #if defined(TJ_INST_R) && TJ_INST_R == 128
 #include "tj_dual.cuh"
 #elif defined(TJ_INST_K) && TJ_INST_K > 0
@@ -33,13 +34,12 @@ inline LaunchShape path_shape(long long n)
 }  // namespace
 
 template <class PT, int DC>
-int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, typename PT::real* Y,
-             int d, int first, int last, int finish, cudaStream_t st, Prof* pr)
+int path_faces(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, int d, cudaStream_t st,
+               Prof* pr)
 {
     constexpr bool f64 = sizeof(typename PT::real) == 8;
     const char* nr = f64 ? "tj_recon_fp64" : "tj_recon_fp32";
     const char* nf = f64 ? "tj_flux_fp64" : "tj_flux_fp32";
-    const char* nu = f64 ? "tj_update_fp64" : "tj_update_fp32";
     const LaunchShape cells = path_shape<PT>(b.ntot), faces = path_shape<PT>(b.nftot[d]);
     if (pr) pr->begin(nr, st);
     if (P.thinc) {
@@ -51,10 +51,32 @@ int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     if (pr) pr->begin(nf, st);
     k_flux<PT, DC><<<faces.blocks, faces.threads, 0, st>>>(P, b, d);
     if (pr) pr->end(nf, st);
+    return P.thinc ? 3 : 2;
+}
+
+template <class PT, int DC>
+int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, typename PT::real* Y,
+             int d, int first, int last, int finish, cudaStream_t st, Prof* pr)
+{
+    const char* nu = sizeof(typename PT::real) == 8 ? "tj_update_fp64" : "tj_update_fp32";
+    const LaunchShape cells = path_shape<PT>(b.ntot);
+    const int n = path_faces<PT, DC>(P, b, X, d, st, pr);
     if (pr) pr->begin(nu, st);
     k_update<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, d, first, last, finish);
     if (pr) pr->end(nu, st);
-    return P.thinc ? 4 : 3;
+    return n + 1;
+}
+
+template <class PT>
+int path_update(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, typename PT::real* Y,
+                int finish, cudaStream_t st, Prof* pr)
+{
+    const char* nu = sizeof(typename PT::real) == 8 ? "tj_update_fp64" : "tj_update_fp32";
+    const LaunchShape cells = path_shape<PT>(b.ntot);
+    if (pr) pr->begin(nu, st);
+    k_update_all<PT><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, finish);
+    if (pr) pr->end(nu, st);
+    return 1;
 }
 
 template <class PT>
@@ -63,7 +85,7 @@ int path_cfl(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     const char* nc = sizeof(typename PT::real) == 8 ? "tj_cfl_fp64" : "tj_cfl_fp32";
     if (pr) pr->begin(nc, st);
     const LaunchShape s = path_shape<PT>(b.ntot);
-    k_cfl<<<s.blocks, s.threads, 0, st>>>(P, b, X);
+    k_cfl<PT><<<s.blocks, s.threads, 0, st>>>(P, b, X);
     if (pr) pr->end(nc, st);
     return 1;
 }
@@ -86,7 +108,13 @@ using InstPT = InstBase;
 
 template int path_dir<InstPT, TJ_INST_D>(const InstPT&, const PathBufs<InstPT::real>&, const InstPT::real*,
                                          InstPT::real*, int, int, int, int, cudaStream_t, Prof*);
+#if TJ_INST_R != 128
+template int path_faces<InstPT, TJ_INST_D>(const InstPT&, const PathBufs<InstPT::real>&, const InstPT::real*, int,
+                                           cudaStream_t, Prof*);
+#endif
 #if TJ_INST_D <= 0 && TJ_INST_R != 128
+template int path_update<InstPT>(const InstPT&, const PathBufs<InstPT::real>&, const InstPT::real*, InstPT::real*, int,
+                                 cudaStream_t, Prof*);
 template int path_cfl<InstPT>(const InstPT&, const PathBufs<InstPT::real>&, const InstPT::real*, cudaStream_t, Prof*);
 #endif
 

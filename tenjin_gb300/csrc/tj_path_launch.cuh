@@ -23,6 +23,15 @@ namespace tj {
 template <class PT, int DC>
 int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, typename PT::real* Y,
              int d, int first, int last, int finish, cudaStream_t st, Prof* pr);
+// The fluxes of one direction alone (k_thinc, k_recon, k_flux), into b.FX.
+template <class PT, int DC>
+int path_faces(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, int d, cudaStream_t st,
+               Prof* pr);
+// The update of a stage from the fluxes of every direction (k_update_all):
+// direction d's follow those of d - 1 in b.FX.
+template <class PT>
+int path_update(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, typename PT::real* Y,
+                int finish, cudaStream_t st, Prof* pr);
 // The CFL pass (k_cfl) over the state X.
 template <class PT>
 int path_cfl(const PT& P, const PathBufs<typename PT::real>& b, const typename PT::real* X, cudaStream_t st,
@@ -62,6 +71,45 @@ inline int path_dir_any(const Base& P, const PathBufs<typename Base::real>& b, c
     if constexpr (kHasKind<Base, KIND_PLASTIC>)
         if (param_kind(P) == KIND_PLASTIC) return path_dir_kind<Base, KIND_PLASTIC>(P, b, X, Y, d, first, last, finish, st, pr);
     return path_dir_kind<Base, KIND_ANY>(P, b, X, Y, d, first, last, finish, st, pr);
+}
+
+template <class Base, int K>
+inline int path_stage_kind(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
+                           typename Base::real* Y, int finish, cudaStream_t st, Prof* pr)
+{
+    int n = 0;
+    PathBufs<typename Base::real> bd = b;
+    for (int d = 0; d < P.dim; ++d) {
+#define TJ_FACES(MC, DC) path_faces<WithM<Base, MC, K>, DC>(WithM<Base, MC, K>(P), bd, X, d, st, pr)
+        switch (P.M * 4 + d) {
+            case 4: n += TJ_FACES(1, 0); break;
+            case 5: n += TJ_FACES(1, 1); break;
+            case 6: n += TJ_FACES(1, 2); break;
+            case 8: n += TJ_FACES(2, 0); break;
+            case 9: n += TJ_FACES(2, 1); break;
+            case 10: n += TJ_FACES(2, 2); break;
+            default: n += path_faces<Base, -1>(P, bd, X, d, st, pr);
+        }
+#undef TJ_FACES
+        bd.FX += P.NX * b.nftot[d];
+    }
+    if (P.M == 1) return n + path_update(WithM<Base, 1, K>(P), b, X, Y, finish, st, pr);
+    if (P.M == 2) return n + path_update(WithM<Base, 2, K>(P), b, X, Y, finish, st, pr);
+    return n + path_update(P, b, X, Y, finish, st, pr);
+}
+
+// One RK stage: every direction's fluxes from the stage input X, then one
+// update into Y, or with finish into b.A. b.FX holds every direction's fluxes
+// (flux_words).
+template <class Base>
+inline int path_stage_any(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
+                          typename Base::real* Y, int finish, cudaStream_t st, Prof* pr)
+{
+    if constexpr (kHasKind<Base, KIND_FLUID>)
+        if (param_kind(P) == KIND_FLUID) return path_stage_kind<Base, KIND_FLUID>(P, b, X, Y, finish, st, pr);
+    if constexpr (kHasKind<Base, KIND_PLASTIC>)
+        if (param_kind(P) == KIND_PLASTIC) return path_stage_kind<Base, KIND_PLASTIC>(P, b, X, Y, finish, st, pr);
+    return path_stage_kind<Base, KIND_ANY>(P, b, X, Y, finish, st, pr);
 }
 
 template <class Base, int K>
