@@ -17,6 +17,7 @@
 // hllc.cpp:642-646,690-691).
 #include <cuda_runtime.h>
 
+#include "tj_launch.cuh"
 #include "tj_path.cuh"
 #include "tj_path_launch.cuh"
 
@@ -28,29 +29,12 @@ static constexpr int kThreads = 256;
 
 __global__ void k_dt_finalize(DevParams P, DevScalars* s, int clamp)
 {
-    if (threadIdx.x != 0) return;
-    double raw = __longlong_as_double((long long)s->dtmin_bits);
-    s->dtmin_raw = raw;
-    s->dtmin_bits = 0x7FEFFFFFFFFFFFFFull;
-    if (!clamp) return;
-    if (s->done) return;
-    if (!(s->t < s->t_end)) { s->done = 1; return; }
-    double dt = P.cfl * raw;
-    if (s->t + dt > s->t_end) dt = s->t_end - s->t;
-    if (s->n < 5) dt *= 0.2;
-    s->dt = dt;
+    if (threadIdx.x == 0) finalize_dt(s, P.cfl, clamp);
 }
 
 __global__ void k_step_end(DevScalars* s)
 {
-    if (threadIdx.x != 0 || s->done) return;
-    if (s->nan_flag) {
-        s->done = 1;
-        atomicCAS(&s->status, 0, TJ_ERR_NAN);
-        return;
-    }
-    s->t += s->dt;
-    s->n += 1;
+    if (threadIdx.x == 0 && !s->done) end_step(s);
 }
 
 __global__ void k_set_dt(DevScalars* s, double dt)

@@ -32,6 +32,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tj_launch.cuh"
 #include "tj_math.cuh"
 #include "tj_mixed.cuh"
 
@@ -93,7 +94,7 @@ struct MixP {
     R g[TJ_MAX_MAT], ig[TJ_MAX_MAT], pref[TJ_MAX_MAT], eref[TJ_MAX_MAT];
     // pref/Gamma and eref as pairs (hi + lo) for the pressure closure
     R cEh[TJ_MAX_MAT], cEl[TJ_MAX_MAT], eEh[TJ_MAX_MAT], eEl[TJ_MAX_MAT];
-    double dxd[2];
+    double dxd[2], cfl;
     int last_box[4];  // lo x, lo y, hi x, hi y of the last box in MFIter order
 };
 
@@ -800,7 +801,20 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
     k_stage2d(MixP<R> P, MixB<R> b, int stage)
 {
     constexpr int NWARP = NT / 32;
+    grid_wait();
+    grid_go();
     if (b.scal->done) return;
+    // the first stage takes the step's dt from the CFL minimum that the step
+    // before left: every block's first thread forms it while the tile is
+    // staged, the last block to end stores it
+    __shared__ R dt_over_dx[2];
+    __shared__ int run_over;
+    if (threadIdx.x == 0) {
+        double dt = b.scal->dt;
+        run_over = stage == 0 && step_dt(b.scal, P.cfl, __longlong_as_double((long long)b.scal->dtmin_bits), dt);
+        // binary32: a product with 1/dx (no binary64 division)
+        for (int d = 0; d < 2; ++d) dt_over_dx[d] = sizeof(R) == 8 ? (R)(dt / P.dxd[d]) : (R)dt * P.idx[d];
+    }
     using SM = Smem<R, M, THINC>;
     extern __shared__ __align__(16) unsigned char smraw[];
     R* sm = reinterpret_cast<R*>(smraw);
@@ -809,10 +823,6 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
     const R* __restrict__ Xin = b.X[stage];
     R* __restrict__ Xout = b.X[stage == 0 ? 1 : 0];
     const long long N = b.N;
-
-    // binary32: dt/dx as a product with 1/dx (no binary64 division per thread)
-    const R dtdx = sizeof(R) == 8 ? (R)(b.scal->dt / P.dxd[0]) : (R)b.scal->dt * P.idx[0];
-    const R dtdy = sizeof(R) == 8 ? (R)(b.scal->dt / P.dxd[1]) : (R)b.scal->dt * P.idx[1];
 
     // ---- stage the primitives of tile + halo and the output cells' conserved
     //      words (U1 = U, hllc.cpp:583) with asynchronous copies: every copy is
@@ -868,6 +878,11 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
+    const R dtdx = dt_over_dx[0], dtdy = dt_over_dx[1];
+    if (run_over) {
+        if (last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
+        return;
+    }
     // reflect_odd ghosts (FillDomainBoundary): negate the normal velocity of
     // staged cells that mirror across a reflective face
     if ((P.lo_bc[0] == TJ_BC_REFLECTIVE && x0 < MH) || (P.hi_bc[0] == TJ_BC_REFLECTIVE && x0 - MH + MS > P.nx) ||
@@ -1035,6 +1050,14 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
             atomicMin(&b.scal->dtmin_bits, (unsigned long long)__double_as_longlong((double)mn));
         }
     }
+    if (last_block(b.scal)) {
+        if (stage == 0) {
+            finalize_dt(b.scal, P.cfl, 1);
+        } else {
+            *b.stage_ctr += 2;  // the THINC stage stamp
+            end_step(b.scal);
+        }
+    }
 }
 
 // CFL of the current state (used after the state is set from outside).
@@ -1182,20 +1205,6 @@ __global__ void k_to_fp64(DevParams DP, MixB<R> b, double* A)
     }
 }
 
-// End of a step (main.cpp:121 t += dt; NaN stop) and the THINC stage stamp.
-__global__ void k_step_end_mixed(DevScalars* s, int* ctr)
-{
-    if (threadIdx.x != 0 || s->done) return;
-    *ctr += 2;
-    if (s->nan_flag) {
-        s->done = 1;
-        atomicCAS(&s->status, 0, TJ_ERR_NAN);
-        return;
-    }
-    s->t += s->dt;
-    s->n += 1;
-}
-
 __global__ void k_reset_dtmin(DevScalars* s)
 {
     if (threadIdx.x == 0) s->dtmin_bits = 0x7FEFFFFFFFFFFFFFull;
@@ -1249,6 +1258,7 @@ struct MixedImpl : MixedBase {
             P.dxd[d] = D.dx[d];
         }
         P.beta = (R)DP.beta;
+        P.cfl = DP.cfl;
         P.mxfloor = (R)1e-20;
         for (int k = 0; k < DP.M; ++k) {
             const double G = DP.prm[k][0] - 1.0;
@@ -1409,7 +1419,7 @@ struct MixedImpl : MixedBase {
     }
 
     template <int MM, bool TH, int NT>
-    void launch_stage_n(int stage, dim3 grid, cudaStream_t st)
+    void launch_stage_n(int stage, dim3 grid, cudaStream_t st, bool overlap)
     {
         static bool attr = false;
         const size_t smb = Smem<R, MM, TH>::BYTES;
@@ -1417,50 +1427,49 @@ struct MixedImpl : MixedBase {
             cudaFuncSetAttribute(k_stage2d<R, MM, TH, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
             attr = true;
         }
-        k_stage2d<R, MM, TH, NT><<<grid, NT, smb, st>>>(P, b, stage);
+        launch(k_stage2d<R, MM, TH, NT>, grid, NT, smb, st, overlap, P, b, stage);
     }
 
     template <int MM, bool TH>
-    void launch_stage(int stage, cudaStream_t st)
+    void launch_stage(int stage, cudaStream_t st, bool overlap)
     {
         constexpr int kSMs = 152;
         const dim3 grid((P.nx + MT - 1) / MT, (P.ny + MT - 1) / MT);
         const long long tiles = (long long)grid.x * grid.y;
         if constexpr (sizeof(R) == 4 && MM <= 2) {
-            if (tiles <= kSMs) return launch_stage_n<MM, TH, NTH_1>(stage, grid, st);
-            if (tiles <= 2 * kSMs) return launch_stage_n<MM, TH, NTH_2>(stage, grid, st);
-            return launch_stage_n<MM, TH, NTH>(stage, grid, st);
+            if (tiles <= kSMs) return launch_stage_n<MM, TH, NTH_1>(stage, grid, st, overlap);
+            if (tiles <= 2 * kSMs) return launch_stage_n<MM, TH, NTH_2>(stage, grid, st, overlap);
+            return launch_stage_n<MM, TH, NTH>(stage, grid, st, overlap);
         }
-        launch_stage_n<MM, TH, NTH_WIDE>(stage, grid, st);
+        launch_stage_n<MM, TH, NTH_WIDE>(stage, grid, st, overlap);
     }
 
-    void stage_dispatch(int stage, cudaStream_t st)
+    void stage_dispatch(int stage, cudaStream_t st, bool overlap)
     {
         switch (M * 2 + (thinc ? 1 : 0)) {
-            case 2: launch_stage<1, false>(stage, st); break;
-            case 3: launch_stage<1, true>(stage, st); break;
-            case 4: launch_stage<2, false>(stage, st); break;
-            case 5: launch_stage<2, true>(stage, st); break;
-            case 6: launch_stage<3, false>(stage, st); break;
-            case 7: launch_stage<3, true>(stage, st); break;
-            case 8: launch_stage<4, false>(stage, st); break;
-            default: launch_stage<4, true>(stage, st); break;
+            case 2: launch_stage<1, false>(stage, st, overlap); break;
+            case 3: launch_stage<1, true>(stage, st, overlap); break;
+            case 4: launch_stage<2, false>(stage, st, overlap); break;
+            case 5: launch_stage<2, true>(stage, st, overlap); break;
+            case 6: launch_stage<3, false>(stage, st, overlap); break;
+            case 7: launch_stage<3, true>(stage, st, overlap); break;
+            case 8: launch_stage<4, false>(stage, st, overlap); break;
+            default: launch_stage<4, true>(stage, st, overlap); break;
         }
     }
 
     int step(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr) override
     {
+        (void)DP;
         b.scal = fb.scal;
         int n = 0;
-        n += fp64_dt_finalize(DP, fb, 1, st);
         for (int stage = 0; stage < 2; ++stage) {
             if (pr) pr->begin(sizeof(R) == 4 ? "tj_stage_mixed" : "tj_stage_fused64", st);
-            stage_dispatch(stage, st);
+            stage_dispatch(stage, st, !pr);
             if (pr) pr->end(sizeof(R) == 4 ? "tj_stage_mixed" : "tj_stage_fused64", st);
             n += 1;
         }
-        k_step_end_mixed<<<1, 32, 0, st>>>(fb.scal, ctr);
-        return n + 1;
+        return n;
     }
 };
 
@@ -1577,7 +1586,7 @@ int mixed_step(MixedState& ms, const DevParams& DP, const Fp64Bufs& fb, cudaStre
 int mixed_launches_per_step(const DevParams& DP)
 {
     (void)DP;
-    return 4;
+    return 2;
 }
 
 }  // namespace tj

@@ -37,6 +37,7 @@
 #include <string>
 #include <vector>
 
+#include "tj_launch.cuh"
 #include "tj_math.cuh"
 #include "tj_mixed.cuh"
 
@@ -50,7 +51,12 @@ namespace {
 // changes to the index arithmetic: 36.7 / 36.3 / 39.9 ms with 512 / 640 / 896).
 constexpr int NT3 = 640;
 
+// k_stage3d's flags: a trial launch of the tuner; the last launch of a stage
+// (the classes of boxes are launched one after the other).
+constexpr int kForce = 1, kLastClass = 2;
+
 struct M3P {
+    double cfl;
     int M;
     int lo_bc[3], hi_bc[3];
     float g[TJ_MAX_MAT], ig[TJ_MAX_MAT], pref[TJ_MAX_MAT], eref[TJ_MAX_MAT];
@@ -110,8 +116,6 @@ template <int M> __host__ __device__ constexpr int S3_EH() { return 3 * M + 6; }
 template <int M> __host__ __device__ constexpr int S3_EL() { return 3 * M + 7; }
 template <int M> __host__ __device__ constexpr int S3_P() { return 3 * M + 8; }
 template <int M> __host__ __device__ constexpr int S3_N() { return 3 * M + 9; }
-
-__host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 
 template <int M, int TX, int TY, int TZ>
 struct Sm3 {
@@ -426,16 +430,35 @@ __device__ bool stage_fix(const M3P& P, const Work3& w, const Dom3& D, float* sp
 }
 
 template <int M, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int force)
+__global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int flags)
 {
+    const bool force = flags & kForce;
+    grid_wait();
+    grid_go();
     if (!force && b.scal->done) return;
+    // the first stage takes the step's dt from the CFL minimum that the step
+    // before left: every block of every class forms it, the last block of the
+    // last class stores it
+    __shared__ float dt_step;
+    __shared__ int run_over;
+    if (threadIdx.x == 0) {
+        double dt = b.scal->dt;
+        run_over = !force && stage == 0 &&
+                   step_dt(b.scal, P.cfl, __longlong_as_double((long long)b.scal->dtmin_bits), dt);
+        dt_step = (float)dt;
+    }
+    __syncthreads();
+    const float dtf = dt_step;
+    if (run_over) {
+        if ((flags & kLastClass) && last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
+        return;
+    }
     using SM = Sm3<M, TX, TY, TZ>;
     extern __shared__ __align__(16) unsigned char smraw3[];
     float* sm = reinterpret_cast<float*>(smraw3);
     const float* __restrict__ Xin = b.X[stage];
     float* __restrict__ Xout = b.X[stage == 0 ? 1 : 0];
     const long long N = b.N;
-    const float dtf = (float)b.scal->dt;
     float dtmin = 3.0e38f;
     bool nan_seen = false;
     __shared__ Work3 wsh[2];
@@ -673,6 +696,10 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fo
             atomicMin(&b.scal->dtmin_bits, (unsigned long long)__double_as_longlong((double)mn));
         }
     }
+    if ((flags & kLastClass) && last_block(b.scal)) {
+        if (stage == 0) finalize_dt(b.scal, P.cfl, 1);
+        else end_step(b.scal);
+    }
 }
 
 // CFL of the current state, per tile of the work list.
@@ -788,14 +815,15 @@ void split_axis(int L, int T, std::vector<std::pair<int, int>>& out)
 struct Shape {
     int tx, ty, tz;
     size_t smem;
-    void (*stage)(const M3P&, const M3B&, int, int, int, size_t, cudaStream_t);
+    void (*stage)(const M3P&, const M3B&, int, int, int, size_t, cudaStream_t, bool);
     int (*occupancy)(size_t);
 };
 
 template <int M, int TX, int TY, int TZ>
-void stage_launch(const M3P& P, const M3B& b, int stage, int force, int grid, size_t smem, cudaStream_t st)
+void stage_launch(const M3P& P, const M3B& b, int stage, int flags, int grid, size_t smem, cudaStream_t st,
+                  bool overlap)
 {
-    k_stage3d<M, TX, TY, TZ><<<grid, NT3, smem, st>>>(P, b, stage, force);
+    launch(k_stage3d<M, TX, TY, TZ>, dim3(grid), NT3, smem, st, overlap, P, b, stage, flags);
 }
 
 template <int M, int TX, int TY, int TZ>
@@ -889,6 +917,7 @@ struct Mixed3D : MixedBase {
         N = ntot;
         std::memset(&P, 0, sizeof P);
         P.M = M;
+        P.cfl = DP.cfl;
         for (int d = 0; d < 3; ++d) {
             P.lo_bc[d] = DP.lo_bc[d];
             P.hi_bc[d] = DP.hi_bc[d];
@@ -1095,9 +1124,9 @@ struct Mixed3D : MixedBase {
             for (size_t s = 0; s < cand.size(); ++s) {
                 if (plan_class(c, (int)s, st) != TJ_OK) continue;
                 const M3B bc = class_bufs(c);
-                cand[s].stage(P, bc, 0, 1, C.grid, cand[s].smem, st);  // warm-up
+                cand[s].stage(P, bc, 0, kForce, C.grid, cand[s].smem, st, false);  // warm-up
                 cudaEventRecord(e0, st);
-                for (int r = 0; r < 3; ++r) cand[s].stage(P, bc, 0, 1, C.grid, cand[s].smem, st);
+                for (int r = 0; r < 3; ++r) cand[s].stage(P, bc, 0, kForce, C.grid, cand[s].smem, st, false);
                 cudaEventRecord(e1, st);
                 cudaEventSynchronize(e1);
                 float ms = 0.0f;
@@ -1157,19 +1186,20 @@ struct Mixed3D : MixedBase {
 
     int step(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr) override
     {
+        (void)DP;
         b.scal = fb.scal;
-        int n = fp64_dt_finalize(DP, fb, 1, st);
+        int n = 0, last = kClasses - 1;
+        while (last > 0 && cls[last].doms.empty()) --last;
         for (int stage = 0; stage < 2; ++stage)
             for (int c = 0; c < kClasses; ++c) {
                 const ClassPlan& C = cls[c];
                 if (C.doms.empty()) continue;
                 const Shape& S = cand[C.best < 0 ? 0 : C.best];
                 if (pr) pr->begin("tj_stage3d_mixed", st);
-                S.stage(P, class_bufs(c), stage, 0, C.grid, S.smem, st);
+                S.stage(P, class_bufs(c), stage, c == last ? kLastClass : 0, C.grid, S.smem, st, !pr);
                 if (pr) pr->end("tj_stage3d_mixed", st);
                 n += 1;
             }
-        n += fp64_step_end(fb, st);
         return n;
     }
 

@@ -134,6 +134,7 @@ struct DevScalars {
     double t, dt, t_end, dtmin_raw;
     unsigned long long dtmin_bits;  // atomicMin over positive doubles as bits
     int n, status, done, nan_flag;
+    unsigned ticket;  // blocks of the running kernel that have ended (last_block)
 };
 
 // Launch-timing hook: begin/end bracket one kernel launch on a stream.
