@@ -711,7 +711,7 @@ int tj_set_primitive(tj_ctx* c, int q, const double* prim)
     TJ_CUDA(c, cudaMemcpyAsync(c->staging, prim, bytes, cudaMemcpyDefault, c->stream));
     a_sync(c);
     Fp64Bufs b = bufs(c);
-    c->launches += fp64_prim_to_state(c->P, b, q, c->staging, c->A, c->stream);
+    c->launches += fp64_prim_to_state(c->P, b, q, (long long)D.n[0] * D.n[1] * D.n[2], c->staging, c->A, c->stream);
     a_written(c);
     TJ_CUDA(c, cudaStreamSynchronize(c->stream));
     TJ_CUDA(c, cudaGetLastError());
@@ -1065,7 +1065,7 @@ int tj_forward(tj_ctx* c, int q, const double* prim0, const double* eos, int nst
                 TJ_CUDA(c, cudaMemsetAsync(c->gstar[d], 0, sizeof(double) * c->P.M * c->nftot[d], c->stream));
     }
     Fp64Bufs b = bufs(c);
-    c->launches += fp64_prim_to_state(c->P, b, 0, c->staging, c->A, c->stream);
+    c->launches += fp64_prim_to_state(c->P, b, 0, c->ntot, c->staging, c->A, c->stream);
     c->adj_general = general;
     long long n;
     if (general) {

@@ -32,20 +32,20 @@ inline int nb32(long long n, int cap = 152 * 16)
 }
 
 // binary64 carried state (+ THINC scratch) -> binary32, the energy split into (hi, lo)
-__global__ void k_to32(DevParams32 P, PathBufs<float> b, const double* A, const double* uls, const double* urs,
-                       const double* gs0, const double* gs1, const double* gs2)
+__global__ void k_to32(DevParams32 P, PathBufs<float> b, const double* __restrict__ A, const double* uls,
+                       const double* urs, const double* gs0, const double* gs1, const double* gs2)
 {
     const long long nt = b.ntot;
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nt; g += (long long)gridDim.x * blockDim.x) {
-        for (int w = 0; w < P.d.NS; ++w) b.A[w * nt + g] = (float)A[w * nt + g];
+        float* __restrict__ X = b.A;
+#pragma unroll 8
+        for (int w = 0; w < P.d.NS; ++w) X[w * nt + g] = narrow(A[w * nt + g]);
         const double E = A[P.S_E * nt + g];
-        const float eh = (float)E;
-        b.A[P.S_E * nt + g] = eh;
-        b.A[P.S_ELO * nt + g] = (float)(E - (double)eh);
+        X[P.S_ELO * nt + g] = narrow(E - widen(narrow(E)));
         if (uls)
             for (int m = 0; m < P.M; ++m) {
-                b.ulstar[(long long)m * nt + g] = (float)uls[(long long)m * nt + g];
-                b.urstar[(long long)m * nt + g] = (float)urs[(long long)m * nt + g];
+                b.ulstar[(long long)m * nt + g] = narrow(uls[(long long)m * nt + g]);
+                b.urstar[(long long)m * nt + g] = narrow(urs[(long long)m * nt + g]);
             }
     }
     const double* gsrc[3] = {gs0, gs1, gs2};
@@ -53,16 +53,18 @@ __global__ void k_to32(DevParams32 P, PathBufs<float> b, const double* A, const 
         if (!gsrc[d]) continue;
         const long long nf = (long long)P.M * b.nftot[d];
         for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < nf; f += (long long)gridDim.x * blockDim.x)
-            b.gstar[d][f] = (float)gsrc[d][f];
+            b.gstar[d][f] = narrow(gsrc[d][f]);
     }
 }
 
-__global__ void k_to64(DevParams32 P, PathBufs<float> b, double* A)
+__global__ void k_to64(DevParams32 P, PathBufs<float> b, double* __restrict__ A)
 {
     const long long nt = b.ntot;
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nt; g += (long long)gridDim.x * blockDim.x) {
-        for (int w = 0; w < P.d.NS; ++w) A[w * nt + g] = b.A[w * nt + g];
-        A[P.S_E * nt + g] = (double)b.A[P.S_E * nt + g] + (double)b.A[P.S_ELO * nt + g];
+        const float* __restrict__ X = b.A;
+#pragma unroll 8
+        for (int w = 0; w < P.d.NS; ++w) A[w * nt + g] = widen(X[w * nt + g]);
+        A[P.S_E * nt + g] = widen(X[P.S_E * nt + g]) + widen(X[P.S_ELO * nt + g]);
     }
 }
 

@@ -113,7 +113,8 @@ __global__ void k_ap_to_state(DevParams P, Fp64Bufs b, int dom, int lx, int ly, 
     const long long nt = b.ntot, nb = (long long)nx * ny * nz;
     const DevDomain D = b.doms[dom];
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nb; t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / ((long long)nx * ny));
+        int i, j, k;
+        split3(t, nx, ny, i, j, k);
         long long src = (i + go) + (long long)ld_i * ((j + (P.dim > 1 ? go : 0)) + (long long)ld_j * (k + (P.dim > 2 ? go : 0)));
         long long g = D.off + (lx + i) + (long long)D.n[0] * ((ly + j) + (long long)D.n[1] * (lz + k));
 #define APV(comp) ap[(long long)(comp)*cs + src]
@@ -148,14 +149,16 @@ __global__ void k_ap_to_state(DevParams P, Fp64Bufs b, int dom, int lx, int ly, 
     }
 }
 
-__global__ void k_state_to_ap(DevParams P, Fp64Bufs b, int dom, int lx, int ly, int lz, int nx, int ny, int nz,
-                              const double* X, double* ap, int ld_i, int ld_j, long long cs, int go, long long t0,
-                              long long t1)
+template <class PT>
+__global__ void __launch_bounds__(128, 4)
+    k_state_to_ap(PT P, Fp64Bufs b, int dom, int lx, int ly, int lz, int nx, int ny, int nz, const double* X, double* ap,
+                  int ld_i, int ld_j, long long cs, int go, long long t0, long long t1)
 {
     const long long nt = b.ntot;
     const DevDomain D = b.doms[dom];
     for (long long t = t0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; t < t1; t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / ((long long)nx * ny));
+        int i, j, k;
+        split3(t, nx, ny, i, j, k);
         long long dst = (i + go) + (long long)ld_i * ((j + (P.dim > 1 ? go : 0)) + (long long)ld_j * (k + (P.dim > 2 ? go : 0)));
         long long g = D.off + (lx + i) + (long long)D.n[0] * ((ly + j) + (long long)D.n[1] * (lz + k));
         CellS c;
@@ -168,12 +171,14 @@ __global__ void k_state_to_ap(DevParams P, Fp64Bufs b, int dom, int lx, int ly, 
         stress(P, c);
         c.a = sound_speed(P, c);
 #define APV(comp) ap[(long long)(comp)*cs + dst]
+#pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             APV(P.A_ALPHA + m) = c.alpha[m];
             APV(P.A_ARHO + m) = c.arho[m];
             APV(P.A_RHOK + m) = c.rhok[m];
         }
         APV(P.A_RHO) = c.rho;
+#pragma unroll
         for (int r = 0; r < 3; ++r) {
             APV(P.A_RHOU + r) = c.rhou[r];
             APV(P.A_VEL + r) = c.vel[r];
@@ -182,8 +187,10 @@ __global__ void k_state_to_ap(DevParams P, Fp64Bufs b, int dom, int lx, int ly, 
         APV(P.A_P) = c.p;
         APV(P.A_A) = c.a;
         APV(P.A_USTAR) = 0.0;
+#pragma unroll
         for (int qq = 0; qq < 9; ++qq) APV(P.A_SIGMA + qq) = c.sigma[qq];
         if (P.solid) {
+#pragma unroll
             for (int qq = 0; qq < 9; ++qq) {
                 APV(P.A_V + qq) = c.V[qq];
                 APV(P.A_VSTAR + qq) = 0.0;
@@ -192,6 +199,7 @@ __global__ void k_state_to_ap(DevParams P, Fp64Bufs b, int dom, int lx, int ly, 
             APV(P.A_HJ2) = c.hj2;
         }
         if (P.plastic)
+#pragma unroll UnrollM<PT>::n
             for (int m = 0; m < P.M; ++m) {
                 APV(P.A_EPS + m) = c.eps[m];
                 APV(P.A_ARE + m) = c.are[m];
@@ -206,7 +214,9 @@ __global__ void k_state_to_ap(DevParams P, Fp64Bufs b, int dom, int lx, int ly, 
     }
 }
 
-__global__ void k_prim_to_state(DevParams P, Fp64Bufs b, int dom, const double* prim, double* X)
+template <class PT>
+__global__ void __launch_bounds__(128, 4)
+    k_prim_to_state(PT P, Fp64Bufs b, int dom, const double* prim, double* X)
 {
     const long long nt = b.ntot;
     const DevDomain D = b.doms[dom];
@@ -214,15 +224,23 @@ __global__ void k_prim_to_state(DevParams P, Fp64Bufs b, int dom, const double* 
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nd; t += (long long)gridDim.x * blockDim.x) {
         CellS c;
         int w = 0;
+#pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) c.alpha[m] = prim[(w++) * nd + t];
+#pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) c.rhok[m] = prim[(w++) * nd + t];
+#pragma unroll
         for (int r = 0; r < 3; ++r) c.vel[r] = prim[(w++) * nd + t];
         c.p = prim[(w++) * nd + t];
         c.hj2 = 0.0;
         if (P.solid)
+#pragma unroll
             for (int qq = 0; qq < 9; ++qq) c.V[qq] = prim[(w++) * nd + t];
         if (P.plastic)
-            for (int m = 0; m < P.M; ++m) c.eps[m] = prim[(w++) * nd + t];
+#pragma unroll UnrollM<PT>::n
+            for (int m = 0; m < P.M; ++m) {
+                c.eps[m] = prim[(w++) * nd + t];
+                c.are[m] = 0.0;  // a fluid's: not set by the closure
+            }
         if (P.nmix) {  // initialise.cpp:66-71
             c.lam = prim[(w++) * nd + t];
             c.rm0 = c.rhok[0];
@@ -341,6 +359,21 @@ __global__ void k_state_component(DevParams P, Fp64Bufs b, int dom, const double
 #define PROF_END(name) \
     if (pr) pr->end(name, st)
 
+// kernel<instance>(instance(P), ...) for the kind and the material count of P:
+// one or two stiffened gases, one or two materials with a plastic solid, or
+// anything.
+#define TJ_BY_KIND(P, kernel, sh, st, ...)                                                                     \
+    do {                                                                                                       \
+        const int kind_ = param_kind(P);                                                                       \
+        if (kind_ == KIND_FLUID && (P).M == 1) TJ_WITH(1, KIND_FLUID, P, kernel, sh, st, __VA_ARGS__);         \
+        else if (kind_ == KIND_FLUID && (P).M == 2) TJ_WITH(2, KIND_FLUID, P, kernel, sh, st, __VA_ARGS__);    \
+        else if (kind_ == KIND_PLASTIC && (P).M == 1) TJ_WITH(1, KIND_PLASTIC, P, kernel, sh, st, __VA_ARGS__);\
+        else if (kind_ == KIND_PLASTIC && (P).M == 2) TJ_WITH(2, KIND_PLASTIC, P, kernel, sh, st, __VA_ARGS__);\
+        else kernel<DevParams><<<(sh).blocks, (sh).threads, 0, st>>>(P, __VA_ARGS__);                          \
+    } while (0)
+#define TJ_WITH(MC, K, P, kernel, sh, st, ...) \
+    kernel<WithM<DevParams, MC, K>><<<(sh).blocks, (sh).threads, 0, st>>>(WithM<DevParams, MC, K>(P), __VA_ARGS__)
+
 int fp64_cfl(const DevParams& P, const Fp64Bufs& b, const double* X, cudaStream_t st, Prof* pr)
 {
     return path_cfl_any(P, b, X, st, pr);
@@ -394,16 +427,16 @@ int fp64_state_to_ap(const DevParams& P, const Fp64Bufs& b, int dom, const int* 
     int nx = bx[3] - bx[0] + 1, ny = bx[4] - bx[1] + 1, nz = bx[5] - bx[2] + 1;
     if (t1 < 0) t1 = (long long)nx * ny * nz;
     if (t1 <= t0) return 0;
-    const LaunchShape sh = launch_shape(t1 - t0, 64);
-    k_state_to_ap<<<sh.blocks, sh.threads, 0, st>>>(P, b, dom, bx[0], bx[1], bx[2], nx, ny, nz, X, ap, ld_i, ld_j,
-                                                         cs, go, t0, t1);
+    const LaunchShape sh = launch_shape(t1 - t0, 128);
+    TJ_BY_KIND(P, k_state_to_ap, sh, st, b, dom, bx[0], bx[1], bx[2], nx, ny, nz, X, ap, ld_i, ld_j, cs, go, t0, t1);
     return 1;
 }
 
-int fp64_prim_to_state(const DevParams& P, const Fp64Bufs& b, int dom, const double* prim, double* X, cudaStream_t st)
+int fp64_prim_to_state(const DevParams& P, const Fp64Bufs& b, int dom, long long cells, const double* prim, double* X,
+                       cudaStream_t st)
 {
-    const LaunchShape sh = launch_shape(b.ntot, 64);
-    k_prim_to_state<<<sh.blocks, sh.threads, 0, st>>>(P, b, dom, prim, X);
+    const LaunchShape sh = launch_shape(cells, 128);
+    TJ_BY_KIND(P, k_prim_to_state, sh, st, b, dom, prim, X);
     return 1;
 }
 

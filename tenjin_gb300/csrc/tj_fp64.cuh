@@ -88,7 +88,9 @@ int fp64_ap_to_state(const DevParams& P, const Fp64Bufs& b, int dom, const int* 
 int fp64_state_to_ap(const DevParams& P, const Fp64Bufs& b, int dom, const int* box_lohi, const double* X, double* ap,
                      int ld_i, int ld_j, int ld_k, long long cstride, int ghost_off, cudaStream_t st,
                      long long t0 = 0, long long t1 = -1);
-int fp64_prim_to_state(const DevParams& P, const Fp64Bufs& b, int dom, const double* prim, double* X, cudaStream_t st);
+// cells: of domain dom.
+int fp64_prim_to_state(const DevParams& P, const Fp64Bufs& b, int dom, long long cells, const double* prim, double* X,
+                       cudaStream_t st);
 
 // Deterministic binary64 sums over all valid cells of alphaRho_k (M), rhoU
 // (3) and E, each times the cell volume: out[M + 4] (device), part: scratch of

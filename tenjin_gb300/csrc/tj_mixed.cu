@@ -1098,29 +1098,40 @@ __global__ void k_cfl_mixed(MixP<R> P, MixB<R> b)
     if ((threadIdx.x & 31) == 0) atomicMin(&b.scal->dtmin_bits, (unsigned long long)__double_as_longlong((double)dtmin));
 }
 
+// Binary64 to the working type and back (tj_quot.h narrow / widen).
+template <typename R>
+__device__ __forceinline__ R to_r(double x)
+{
+    if constexpr (sizeof(R) == 4) return narrow(x);
+    else return x;
+}
+__device__ __forceinline__ double to_d(float x) { return widen(x); }
+__device__ __forceinline__ double to_d(double x) { return x; }
+__device__ __forceinline__ bool zero_bits(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
 // FP64 carried state (the layout of tj_fp64) <-> fused state.
 template <typename R, int M>
-__global__ void k_from_fp64(DevParams DP, MixB<R> b, const double* A, int* bad)
+__global__ void __launch_bounds__(256, 4) k_from_fp64(DevParams DP, MixB<R> b, const double* __restrict__ A, int* bad)
 {
     const long long N = b.N;
-    R* X = b.X[0];
+    R* __restrict__ X = b.X[0];
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            X[W_A(m) * N + g] = (R)A[(DP.S_ALPHA + m) * N + g];
-            X[W_AR<M>(m) * N + g] = (R)A[(DP.S_ARHO + m) * N + g];
-            X[W_RK<M>(m) * N + g] = (R)A[(DP.S_RHOK + m) * N + g];
+            X[W_A(m) * N + g] = to_r<R>(A[(DP.S_ALPHA + m) * N + g]);
+            X[W_AR<M>(m) * N + g] = to_r<R>(A[(DP.S_ARHO + m) * N + g]);
+            X[W_RK<M>(m) * N + g] = to_r<R>(A[(DP.S_RHOK + m) * N + g]);
         }
         for (int r = 0; r < 2; ++r) {
-            X[W_RU<M>(r) * N + g] = (R)A[(DP.S_RHOU + r) * N + g];
-            X[W_U<M>(r) * N + g] = (R)A[(DP.S_VEL + r) * N + g];
+            X[W_RU<M>(r) * N + g] = to_r<R>(A[(DP.S_RHOU + r) * N + g]);
+            X[W_U<M>(r) * N + g] = to_r<R>(A[(DP.S_VEL + r) * N + g]);
         }
         const double E = A[DP.S_E * N + g];
-        const R eh = (R)E;
+        const R eh = to_r<R>(E);
         X[W_EH<M>() * N + g] = eh;
-        X[W_EL<M>() * N + g] = (R)(E - (double)eh);
-        X[W_P<M>() * N + g] = (R)A[DP.S_P * N + g];
-        if (A[(DP.S_VEL + 2) * N + g] != 0.0 || A[(DP.S_RHOU + 2) * N + g] != 0.0) atomicOr(bad, 1);
+        X[W_EL<M>() * N + g] = to_r<R>(E - to_d(eh));
+        X[W_P<M>() * N + g] = to_r<R>(A[DP.S_P * N + g]);
+        if (!zero_bits(A[(DP.S_VEL + 2) * N + g]) || !zero_bits(A[(DP.S_RHOU + 2) * N + g])) atomicOr(bad, 1);
     }
 }
 
@@ -1131,7 +1142,7 @@ __global__ void k_from_fp64(DevParams DP, MixB<R> b, const double* A, int* bad)
 // over the host link. The values written are those of k_ap_to_state followed
 // by k_from_fp64.
 template <typename R, int M>
-__global__ void k_from_ap(DevParams DP, MixB<R> b, const double* __restrict__ ap, double* __restrict__ A, int* bad)
+__global__ void __launch_bounds__(256, 4) k_from_ap(DevParams DP, MixB<R> b, const double* __restrict__ ap, double* __restrict__ A, int* bad)
 {
     const long long N = b.N;
     R* __restrict__ X = b.X[0];
@@ -1154,9 +1165,9 @@ __global__ void k_from_ap(DevParams DP, MixB<R> b, const double* __restrict__ ap
             A[(DP.S_ALPHA + m) * N + g] = al[m];
             A[(DP.S_ARHO + m) * N + g] = ar[m];
             A[(DP.S_RHOK + m) * N + g] = rk[m];
-            X[W_A(m) * N + g] = (R)al[m];
-            X[W_AR<M>(m) * N + g] = (R)ar[m];
-            X[W_RK<M>(m) * N + g] = (R)rk[m];
+            X[W_A(m) * N + g] = to_r<R>(al[m]);
+            X[W_AR<M>(m) * N + g] = to_r<R>(ar[m]);
+            X[W_RK<M>(m) * N + g] = to_r<R>(rk[m]);
         }
         A[DP.S_RHO * N + g] = rho;
 #pragma unroll
@@ -1166,42 +1177,42 @@ __global__ void k_from_ap(DevParams DP, MixB<R> b, const double* __restrict__ ap
         }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            X[W_RU<M>(r) * N + g] = (R)ru[r];
-            X[W_U<M>(r) * N + g] = (R)u[r];
+            X[W_RU<M>(r) * N + g] = to_r<R>(ru[r]);
+            X[W_U<M>(r) * N + g] = to_r<R>(u[r]);
         }
         A[DP.S_E * N + g] = E;
-        const R eh = (R)E;
+        const R eh = to_r<R>(E);
         X[W_EH<M>() * N + g] = eh;
-        X[W_EL<M>() * N + g] = (R)(E - (double)eh);
+        X[W_EL<M>() * N + g] = to_r<R>(E - to_d(eh));
         A[DP.S_P * N + g] = p;
-        X[W_P<M>() * N + g] = (R)p;
-        if (u[2] != 0.0 || ru[2] != 0.0) atomicOr(bad, 1);
+        X[W_P<M>() * N + g] = to_r<R>(p);
+        if (!zero_bits(u[2]) || !zero_bits(ru[2])) atomicOr(bad, 1);
     }
 }
 
 template <typename R, int M>
-__global__ void k_to_fp64(DevParams DP, MixB<R> b, double* A)
+__global__ void __launch_bounds__(256, 4) k_to_fp64(DevParams DP, MixB<R> b, double* __restrict__ A)
 {
     const long long N = b.N;
-    const R* X = b.X[0];
+    const R* __restrict__ X = b.X[0];
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
         double rho = 0.0;
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            A[(DP.S_ALPHA + m) * N + g] = X[W_A(m) * N + g];
-            A[(DP.S_ARHO + m) * N + g] = X[W_AR<M>(m) * N + g];
-            A[(DP.S_RHOK + m) * N + g] = X[W_RK<M>(m) * N + g];
-            rho += (double)X[W_AR<M>(m) * N + g];
+            A[(DP.S_ALPHA + m) * N + g] = to_d(X[W_A(m) * N + g]);
+            A[(DP.S_ARHO + m) * N + g] = to_d(X[W_AR<M>(m) * N + g]);
+            A[(DP.S_RHOK + m) * N + g] = to_d(X[W_RK<M>(m) * N + g]);
+            rho += to_d(X[W_AR<M>(m) * N + g]);
         }
         A[DP.S_RHO * N + g] = rho;
         for (int r = 0; r < 2; ++r) {
-            A[(DP.S_RHOU + r) * N + g] = X[W_RU<M>(r) * N + g];
-            A[(DP.S_VEL + r) * N + g] = X[W_U<M>(r) * N + g];
+            A[(DP.S_RHOU + r) * N + g] = to_d(X[W_RU<M>(r) * N + g]);
+            A[(DP.S_VEL + r) * N + g] = to_d(X[W_U<M>(r) * N + g]);
         }
         A[(DP.S_RHOU + 2) * N + g] = 0.0;
         A[(DP.S_VEL + 2) * N + g] = 0.0;
-        A[DP.S_E * N + g] = (double)X[W_EH<M>() * N + g] + (double)X[W_EL<M>() * N + g];
-        A[DP.S_P * N + g] = X[W_P<M>() * N + g];
+        A[DP.S_E * N + g] = to_d(X[W_EH<M>() * N + g]) + to_d(X[W_EL<M>() * N + g]);
+        A[DP.S_P * N + g] = to_d(X[W_P<M>() * N + g]);
     }
 }
 

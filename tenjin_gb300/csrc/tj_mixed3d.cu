@@ -742,35 +742,35 @@ __global__ void k_cfl3d(M3P P, M3B b)
 }
 
 template <int M>
-__global__ void k_from_fp64_3d(DevParams DP, M3B b, const double* A)
+__global__ void __launch_bounds__(256, 4) k_from_fp64_3d(DevParams DP, M3B b, const double* __restrict__ A)
 {
     const long long N = b.N;
-    float* X = b.X[0];
+    float* __restrict__ X = b.X[0];
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            X[S3_A<M>(m) * N + g] = (float)A[(DP.S_ALPHA + m) * N + g];
-            X[S3_AR<M>(m) * N + g] = (float)A[(DP.S_ARHO + m) * N + g];
-            X[S3_RK<M>(m) * N + g] = (float)A[(DP.S_RHOK + m) * N + g];
+            X[S3_A<M>(m) * N + g] = narrow(A[(DP.S_ALPHA + m) * N + g]);
+            X[S3_AR<M>(m) * N + g] = narrow(A[(DP.S_ARHO + m) * N + g]);
+            X[S3_RK<M>(m) * N + g] = narrow(A[(DP.S_RHOK + m) * N + g]);
         }
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            X[S3_RU<M>(r) * N + g] = (float)A[(DP.S_RHOU + r) * N + g];
-            X[S3_U<M>(r) * N + g] = (float)A[(DP.S_VEL + r) * N + g];
+            X[S3_RU<M>(r) * N + g] = narrow(A[(DP.S_RHOU + r) * N + g]);
+            X[S3_U<M>(r) * N + g] = narrow(A[(DP.S_VEL + r) * N + g]);
         }
         const double E = A[DP.S_E * N + g];
-        const float eh = (float)E;
+        const float eh = narrow(E);
         X[S3_EH<M>() * N + g] = eh;
-        X[S3_EL<M>() * N + g] = (float)(E - (double)eh);
-        X[S3_P<M>() * N + g] = (float)A[DP.S_P * N + g];
+        X[S3_EL<M>() * N + g] = narrow(E - widen(eh));
+        X[S3_P<M>() * N + g] = narrow(A[DP.S_P * N + g]);
     }
 }
 
 template <int M>
-__global__ void k_to_fp64_3d(DevParams DP, M3B b, double* A)
+__global__ void __launch_bounds__(256, 4) k_to_fp64_3d(DevParams DP, M3B b, double* __restrict__ A)
 {
     const long long N = b.N;
-    const float* X = b.X[0];
+    const float* __restrict__ X = b.X[0];
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
         double rho = 0.0;
 #pragma unroll
@@ -778,7 +778,7 @@ __global__ void k_to_fp64_3d(DevParams DP, M3B b, double* A)
             A[(DP.S_ALPHA + m) * N + g] = X[S3_A<M>(m) * N + g];
             A[(DP.S_ARHO + m) * N + g] = X[S3_AR<M>(m) * N + g];
             A[(DP.S_RHOK + m) * N + g] = X[S3_RK<M>(m) * N + g];
-            rho += (double)X[S3_AR<M>(m) * N + g];
+            rho += widen(X[S3_AR<M>(m) * N + g]);
         }
         A[DP.S_RHO * N + g] = rho;
 #pragma unroll
@@ -786,7 +786,7 @@ __global__ void k_to_fp64_3d(DevParams DP, M3B b, double* A)
             A[(DP.S_RHOU + r) * N + g] = X[S3_RU<M>(r) * N + g];
             A[(DP.S_VEL + r) * N + g] = X[S3_U<M>(r) * N + g];
         }
-        A[DP.S_E * N + g] = (double)X[S3_EH<M>() * N + g] + (double)X[S3_EL<M>() * N + g];
+        A[DP.S_E * N + g] = widen(X[S3_EH<M>() * N + g]) + widen(X[S3_EL<M>() * N + g]);
         A[DP.S_P * N + g] = X[S3_P<M>() * N + g];
     }
 }

@@ -208,6 +208,29 @@ TJQ_HD double tjq_sqrt(double a)
     return tjq_double(s + ((tjq_u64)((ea + 1021 - odd) / 2) << 52));
 }
 
+// Conversions between binary64 and binary32 on the integer units (the
+// conversion instruction takes the binary64 pipe's 16 cycles a warp as well):
+// the bits of the cast, which is left what is not a normal number or zero in
+// both types.
+TJQ_HD float narrow(double x)
+{
+    const tjq_u64 u = tjq_bits(x);
+    const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u, sign = hi & 0x80000000u;
+    const unsigned e = (hi >> 20) & 0x7ffu;
+    if ((u << 1) == 0) return tjq_float(sign);
+    if (e - 897u > 253u) return (float)x;
+    const unsigned f = ((e - 896u) << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29), rest = lo << 3;
+    // to nearest, ties to even; a carry goes into the exponent
+    return tjq_float(sign | (f + (rest > 0x80000000u || (rest == 0x80000000u && (f & 1u)) ? 1u : 0u)));
+}
+TJQ_HD double widen(float x)
+{
+    const unsigned b = tjq_fbits(x), e = (b >> 23) & 0xffu, sign = b & 0x80000000u;
+    if ((b << 1) == 0) return tjq_double((tjq_u64)sign << 32);
+    if (e - 1u > 253u) return (double)x;
+    return tjq_double(((tjq_u64)(sign | ((e + 896u) << 20) | ((b & 0x7FFFFFu) >> 3)) << 32) | ((tjq_u64)(b << 29) & 0xFFFFFFFFull));
+}
+
 // Division and square root of the templated device code, by working type.
 TJQ_HD double quot(double a, double b)
 {

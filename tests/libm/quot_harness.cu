@@ -22,7 +22,44 @@ extern "C" int tjq_eval(const double* a, const double* b, int n, int ulps, doubl
     }
     return 0;
 }
+extern "C" int tjq_convert(const double* a, int n, float* f, float* f0, double* w, double* w0)
+{
+    for (int i = 0; i < n; ++i) {
+        f[i] = tj::narrow(a[i]);
+        f0[i] = (float)a[i];
+        w[i] = tj::widen(f0[i]);
+        w0[i] = (double)f0[i];
+    }
+    return 0;
+}
 #else
+__global__ void k_convert(const double* a, int n, float* f, double* w)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    f[i] = tj::narrow(a[i]);
+    f[n + i] = (float)a[i];
+    w[i] = tj::widen(f[n + i]);
+    w[n + i] = (double)f[n + i];
+}
+
+extern "C" int tjq_convert(const double* a, int n, float* f, float* f0, double* w, double* w0)
+{
+    double* d = nullptr;
+    const size_t m = (size_t)n;
+    if (cudaMalloc(&d, sizeof(double) * 4 * m) != cudaSuccess) return -1;
+    float* df = reinterpret_cast<float*>(d + 3 * m);
+    cudaMemcpy(d, a, sizeof(double) * m, cudaMemcpyHostToDevice);
+    k_convert<<<(n + 255) / 256, 256>>>(d, n, df, d + m);
+    cudaMemcpy(f, df, sizeof(float) * m, cudaMemcpyDeviceToHost);
+    cudaMemcpy(f0, df + m, sizeof(float) * m, cudaMemcpyDeviceToHost);
+    cudaMemcpy(w, d + m, sizeof(double) * m, cudaMemcpyDeviceToHost);
+    cudaMemcpy(w0, d + 2 * m, sizeof(double) * m, cudaMemcpyDeviceToHost);
+    const cudaError_t e = cudaDeviceSynchronize();
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : -2;
+}
+
 __global__ void k_eval(const double* a, const double* b, int n, double* o)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -4,7 +4,8 @@ all bit patterns, significands at both ends of their range, quotients next to
 one and to a power of two, small integers, zeros, infinities, NaN, subnormal
 numbers and results. On the host every step runs with the binary32 seed moved
 by up to three units in the last place; on the GPU with the hardware's seed.
-The tolerance is none: IEEE division and square root are correctly rounded."""
+The tolerance is none: IEEE division and square root are correctly rounded. The
+conversions to and from binary32 against the casts, in the same way."""
 import ctypes
 import os
 import shutil
@@ -61,6 +62,22 @@ def _check(lib, kind, ulps):
         assert same.all(), f"{name}: {(~same).sum()} differ, first a={a[k].hex()} b={b[k].hex()}: {got[k].hex()} for {want[k].hex()}"
 
 
+def _check_convert(lib, kind):
+    a, b = _args(kind)
+    # the same significands over the binary32 exponents, their ends and the ties between binary32 neighbours
+    e = np.uint64(890) + b.view(np.uint64) % np.uint64(270)
+    c = (a.view(np.uint64) & (FRAC | np.uint64(1 << 63))) | (e << np.uint64(52))
+    tie = (c & ~np.uint64(0x1FFFFFFF)) | np.uint64(0x10000000)
+    a = np.concatenate([a, c.view(np.float64), tie.view(np.float64)])
+    f, f0 = np.empty(len(a), np.float32), np.empty(len(a), np.float32)
+    w, w0 = np.empty_like(a), np.empty_like(a)
+    D, F = ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_float)
+    assert lib.tjq_convert(a.ctypes.data_as(D), len(a), f.ctypes.data_as(F), f0.ctypes.data_as(F), w.ctypes.data_as(D),
+                           w0.ctypes.data_as(D)) == 0
+    assert np.array_equal(f.view(np.int32)[~np.isnan(f0)], f0.view(np.int32)[~np.isnan(f0)]) and np.isnan(f[np.isnan(f0)]).all()
+    assert np.array_equal(w.view(np.int64)[~np.isnan(w0)], w0.view(np.int64)[~np.isnan(w0)]) and np.isnan(w[np.isnan(w0)]).all()
+
+
 @pytest.fixture(scope="module")
 def host_lib(tmp_path_factory):
     cxx = shutil.which("g++") or shutil.which("c++")
@@ -94,3 +111,16 @@ def test_host_build_gives_the_ieee_bits(host_lib, kind, ulps):
 def test_gpu_build_gives_the_ieee_bits(gpu_lib, kind):
     with np.errstate(all="ignore"):
         _check(gpu_lib, kind, 0)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_host_conversions_are_the_casts(host_lib, kind):
+    with np.errstate(all="ignore"):
+        _check_convert(host_lib, kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_gpu_conversions_are_the_casts(gpu_lib, kind):
+    with np.errstate(all="ignore"):
+        _check_convert(gpu_lib, kind)
