@@ -33,6 +33,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tj_adjoint_local.h"
 #include "tj_dual.cuh"
 #include "tj_dual_path.cuh"
 #include "tj_path.cuh"
@@ -328,10 +329,11 @@ __device__ __forceinline__ int face_src(const DevParams& P, int w, bool& rec)
 }
 
 // ---------------------------------------------------------------------------
-// MUSCL reconstruction, reversed per cell h: the adjoints of UL / UR of the
-// cells whose stencil holds h (h - 1, h, h + 1 along d, boundary images
-// included) times the active branch's coefficients, added to h's carried
-// words of the stage input.
+// MUSCL reconstruction, reversed per cell h and word of the face state: the
+// adjoints of UL / UR of the cells whose stencil holds h (h - 1, h, h + 1 along
+// d, boundary images included) times the active branch's coefficients, added
+// to h's carried word of the stage input. One thread per cell and word (they
+// are independent), cells fastest.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kGT) k_gen_recon_rev(DevParams P, Fp64Bufs fb, const double* X,
                                                        const double* lamLf, const double* lamRf, double* lamU, int d,
@@ -339,21 +341,26 @@ __global__ void __launch_bounds__(kGT) k_gen_recon_rev(DevParams P, Fp64Bufs fb,
 {
     const long long nt = fb.ntot, nf = fb.nftot[d];
     const DevDomain D = fb.doms[0];
-    for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < nt; h += (long long)gridDim.x * blockDim.x) {
+    const long long all = nt * nfw;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
+        const int w = (int)(e / nt);
+        const long long h = e - (long long)w * nt;
         int c[3];
         split3(h - D.off, D.n[0], D.n[1], c[0], c[1], c[2]);
         const int n = D.n[d];
-        double acc[kNF];
-        for (int w = 0; w < nfw; ++w) acc[w] = 0.0;
+        bool rec;
+        const int src = face_src(P, w, rec);
+        const bool vd = (src == P.S_VEL + d);
+        double acc = 0.0;
         for (int kq = -1; kq <= 1; ++kq) {
             int kc[3] = {c[0], c[1], c[2]};
             kc[d] += kq;
             if (kc[d] < 0 || kc[d] >= n) continue;
             // adjoints of UL / UR of cell kc (faces below and above, and the
             // boundary face whose ghost side is this cell's state)
-            int lo[3] = {kc[0], kc[1], kc[2]}, hi[3] = {kc[0], kc[1], kc[2]};
+            int hi[3] = {kc[0], kc[1], kc[2]};
             hi[d] += 1;
-            const long long fl = face_index(D, d, lo[0], lo[1], lo[2]), fh = face_index(D, d, hi[0], hi[1], hi[2]);
+            const long long fl = face_index(D, d, kc[0], kc[1], kc[2]), fh = face_index(D, d, hi[0], hi[1], hi[2]);
             int e0[3] = {kc[0], kc[1], kc[2]}, en[3] = {kc[0], kc[1], kc[2]};
             e0[d] = 0;
             en[d] = n;
@@ -366,44 +373,29 @@ __global__ void __launch_bounds__(kGT) k_gen_recon_rev(DevParams P, Fp64Bufs fb,
                 s[d] += q - 1;
                 gs[q] = map_cell(P, D, s[0], s[1], s[2], rf[q]);
             }
-            for (int w = 0; w < nfw; ++w) {
-                const double lR = lamLf[w * nf + fh] + (kc[d] == 0 ? lamLf[w * nf + fz] : 0.0);
-                const double lL = lamRf[w * nf + fl] + (kc[d] == n - 1 ? lamRf[w * nf + fn] : 0.0);
-                bool rec;
-                const int src = face_src(P, w, rec);
-                if (!rec || !P.muscl) {
-                    if (gs[1] == h) acc[w] += lL + lR;
-                    continue;
-                }
-                const bool vd = (src == P.S_VEL + d);
-                double u[3];
-                for (int q = 0; q < 3; ++q) {
-                    const double v = X[src * nt + gs[q]];
-                    u[q] = (vd && rf[q][d]) ? -v : v;
-                }
-                double rr = quot(u[1] - u[0], u[2] - u[1]);
-                if (isinf(rr) || isnan(rr)) rr = 0.0;
-                double b1 = 0.0, b2 = 0.0;
-                if (rr > 0.0) {
-                    const double a = quot(2.0, 1.0 + rr), b = quot(2.0 * rr, 1.0 + rr);
-                    if (b < a) b1 = 1.0;
-                    else b2 = 1.0;
-                }
-                // L = u0 - g / 2, R = u0 + g / 2 with g = b1 (u0 - um) + b2 (up - u0)
-                const double cL[3] = {0.5 * b1, 1.0 - 0.5 * (b1 - b2), -0.5 * b2};
-                const double cR[3] = {-0.5 * b1, 1.0 + 0.5 * (b1 - b2), 0.5 * b2};
-                for (int q = 0; q < 3; ++q)
-                    if (gs[q] == h) {
-                        const double sg = (vd && rf[q][d]) ? -1.0 : 1.0;
-                        acc[w] += sg * (cL[q] * lL + cR[q] * lR);
-                    }
+            const double lR = lamLf[w * nf + fh] + (kc[d] == 0 ? lamLf[w * nf + fz] : 0.0);
+            const double lL = lamRf[w * nf + fl] + (kc[d] == n - 1 ? lamRf[w * nf + fn] : 0.0);
+            if (!rec || !P.muscl) {
+                if (gs[1] == h) acc += lL + lR;
+                continue;
             }
+            double u[3];
+            for (int q = 0; q < 3; ++q) {
+                const double v = X[src * nt + gs[q]];
+                u[q] = (vd && rf[q][d]) ? -v : v;
+            }
+            const int branch = tja::muscl_branch(u[0], u[1], u[2]);
+            const double b1 = branch == 1 ? 1.0 : 0.0, b2 = branch == 2 ? 1.0 : 0.0;
+            // L = u0 - g / 2, R = u0 + g / 2 with g = b1 (u0 - um) + b2 (up - u0)
+            const double cL[3] = {0.5 * b1, 1.0 - 0.5 * (b1 - b2), -0.5 * b2};
+            const double cR[3] = {-0.5 * b1, 1.0 + 0.5 * (b1 - b2), 0.5 * b2};
+            for (int q = 0; q < 3; ++q)
+                if (gs[q] == h) {
+                    const double sg = (vd && rf[q][d]) ? -1.0 : 1.0;
+                    acc += sg * (cL[q] * lL + cR[q] * lR);
+                }
         }
-        for (int w = 0; w < nfw; ++w) {
-            bool rec;
-            const int src = face_src(P, w, rec);
-            lamU[src * nt + h] += acc[w];
-        }
+        lamU[src * nt + h] += acc;
     }
 }
 
@@ -429,33 +421,29 @@ __device__ __noinline__ double p2c_pass(const DevParamsT& P, const Dual* pr, Dua
     return s;
 }
 
-// primitiveToConservative of the initial state, reversed per cell: the
-// adjoints of the primitives (tj_set_primitive layout) and each EOS
-// parameter's part.
-__global__ void __launch_bounds__(kGT) k_gen_p2c_rev(DevParamsT P, Fp64Bufs fb, const double* prim,
-                                                     const double* lamA, double* gprim, double* geos, int npar,
-                                                     int nprim)
+// primitiveToConservative of the initial state, reversed: the adjoints of the
+// primitives (tj_set_primitive layout) and each EOS parameter's part, one
+// thread per cell and pass.
+__global__ void __launch_bounds__(kGT) k_gen_p2c_rev(const __grid_constant__ DevParamsT P, Fp64Bufs fb,
+                                                     const double* prim, const double* lamA, double* gprim,
+                                                     double* geos, int npar, int nprim)
 {
-    const long long nt = fb.ntot;
+    const long long nt = fb.ntot, all = nt * (nprim + P.M * npar);
     const int NS = P.NS;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nt; t += (long long)gridDim.x * blockDim.x) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
+        const int pass = (int)(e / nt);
+        const long long t = e - (long long)pass * nt;
         Dual pr[kNF], out[kNS];
         double lo[kNS];
-        for (int w = 0; w < nprim; ++w) pr[w] = Dual(prim[w * nt + t]);
+        for (int w = 0; w < nprim; ++w) pr[w] = Dual(prim[w * nt + t], w == pass ? 1.0 : 0.0);
         for (int w = 0; w < NS; ++w) lo[w] = lamA[w * nt + t];
-        for (int w = 0; w < nprim; ++w) {
-            pr[w].d = 1.0;
-            gprim[w * nt + t] = p2c_pass(P, pr, out, lo);
-            pr[w].d = 0.0;
-        }
-        if (geos && npar > 0) {
+        if (pass < nprim) {
+            gprim[pass * nt + t] = p2c_pass(P, pr, out, lo);
+        } else {
+            const int q = pass - nprim;
             DevParamsT Q = P;
-            for (int m = 0; m < P.M; ++m)
-                for (int q = 0; q < npar; ++q) {
-                    Q.prm[m][q].d = 1.0;
-                    geos[(long long)(m * npar + q) * nt + t] += p2c_pass(Q, pr, out, lo);
-                    Q.prm[m][q].d = 0.0;
-                }
+            Q.prm[q / npar][q % npar].d = 1.0;
+            geos[(long long)q * nt + t] += p2c_pass(Q, pr, out, lo);
         }
     }
 }
@@ -753,7 +741,8 @@ long long gen_backward(GenAdj* a, const DevParams& P, const Fp64Bufs& b, const d
         const LaunchShape sf = launch_shape(b.nftot[d] * lists[PL_FACE].n, kGT);
         k_gen_flux_rev<<<sf.blocks, sf.threads, 0, st>>>(PT, fb, a->passes + PL_FACE, a->lamF0, a->lamF1, a->lamLf,
                                                          a->lamRf, a->geosf, d, npar, nfw);
-        k_gen_recon_rev<<<gblocks(N), kGT, 0, st>>>(P, fb, U, a->lamLf, a->lamRf, lamU, d, nfw);
+        const LaunchShape sr = launch_shape(N * nfw, kGT);
+        k_gen_recon_rev<<<sr.blocks, sr.threads, 0, st>>>(P, fb, U, a->lamLf, a->lamRf, lamU, d, nfw);
         launches += 3;
         fold_faces(d);
     };
@@ -814,8 +803,8 @@ long long gen_backward(GenAdj* a, const DevParams& P, const Fp64Bufs& b, const d
         }
     }
     // the initial primitiveToConservative
-    k_gen_p2c_rev<<<gblocks(N), kGT, 0, st>>>(PT, fb, a->prim0, a->lamA, grad_prim, mp > 0 ? a->geos : nullptr, npar,
-                                              a->nprim);
+    const LaunchShape sp = launch_shape(N * (a->nprim + P.M * npar), kGT);
+    k_gen_p2c_rev<<<sp.blocks, sp.threads, 0, st>>>(PT, fb, a->prim0, a->lamA, grad_prim, a->geos, npar, a->nprim);
     ++launches;
     if (mp > 0) {
         k_gen_sum<<<mp, 256, 0, st>>>(a->geos, N, a->gsum);
