@@ -130,6 +130,7 @@ __device__ __forceinline__ void face_prim(const GT& G, const double* X, const do
     const long long g = i + (long long)G.nx * j;
 #pragma unroll
     for (int q = 0; q < G.NW; ++q) {
+        if (q < G.M && G.thinc) continue;  // alpha is the recorded one
         const double u0 = qat(G, X, i, j, d, 0, q);
         double v = u0;
         if (G.muscl) {
@@ -296,8 +297,9 @@ __global__ void __launch_bounds__(NT, 8) k_adj_face(AG G0, const double* X, cons
         if (reflL) xl.u[d] = -xl.u[d];
         if (reflR) xr.u[d] = -xr.u[d];
         tja::FS L, R;
-        tja::face_state_fwd(G.E, xl, G.thinc != 0, L);
-        tja::face_state_fwd(G.E, xr, G.thinc != 0, R);
+        tja::FaceParts fl, fr;
+        tja::face_state_parts(G.E, xl, G.thinc != 0, L, fl);
+        tja::face_state_parts(G.E, xr, G.thinc != 0, R, fr);
         // flux adjoint: the face adds F to its right cell and subtracts it
         // from its left cell; S* enters as -alpha_right S* + alpha_left S*
         tja::HllcOut lF;
@@ -345,8 +347,8 @@ __global__ void __launch_bounds__(NT, 8) k_adj_face(AG G0, const double* X, cons
         tja::Prim pL, pR;
         tja::zero(pL);
         tja::zero(pR);
-        tja::face_state_rev(G.E, xl, G.thinc != 0, lL, pL, gr);
-        tja::face_state_rev(G.E, xr, G.thinc != 0, lR, pR, gr);
+        tja::face_state_rev(G.E, xl, G.thinc != 0, L, fl, lL, pL, gr);
+        tja::face_state_rev(G.E, xr, G.thinc != 0, R, fr, lR, pR, gr);
         if (reflL) pL.u[d] = -pL.u[d];
         if (reflR) pR.u[d] = -pR.u[d];
 #pragma unroll
@@ -366,7 +368,8 @@ __device__ double thinc_tanh(double x) { return tjm_tanh(x); }
 __device__ double thinc_exp(double x) { return tjm_exp(x); }
 
 // ---------------------------------------------------------------------------
-// Per cell along d: stencil gradient of each THINC candidate the forward used.
+// Per cell and material along d (one thread each): stencil gradient of each
+// THINC candidate the forward used.
 // ---------------------------------------------------------------------------
 template <int MC>
 __global__ void __launch_bounds__(NT, 8) k_adj_thinc(AG G0, int d, const double* X, const int* code, const double* lface, const double* limg,
@@ -376,43 +379,41 @@ __global__ void __launch_bounds__(NT, 8) k_adj_thinc(AG G0, int d, const double*
     const int M = G.M, NW = G.NW;
     const long long N = G.N;
     const int n = d == 0 ? G.nx : G.ny;
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < N * M; e += (long long)gridDim.x * blockDim.x) {
+        int m = 0;
+        long long g = e;
+        for (; g >= N; g -= N) ++m;
         const int cd = code[(long long)d * N + g];
         const int i = (int)(g % G.nx), j = (int)(g / G.nx);
         const int pos = d == 0 ? i : j, line = d == 0 ? j : i;
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-            double* tc = tcon + (long long)((d * M + m) * 9) * N + g;
-            double s[3][3], ls[3][3];
-            for (int a = 0; a < 3; ++a)
-                for (int c = 0; c < 3; ++c) {
-                    bool r0, r1;
-                    const int ii = mapi(i + a - 1, G.nx, G.lo_bc[0], G.hi_bc[0], r0);
-                    const int jj = mapi(j + c - 1, G.ny, G.lo_bc[1], G.hi_bc[1], r1);
-                    s[a][c] = X[(G.sa + m) * N + ii + (long long)G.nx * jj];
-                    ls[a][c] = 0.0;
-                }
-            double cL = 0.0, cR = 0.0;
-            const bool mixed = tja::thinc_cand_fwd(s, d, G.beta, G.dx[0], G.dx[1], thinc_cosh, thinc_tanh, thinc_exp,
-                                                   cL, cR);
-            double lL = 0.0, lR = 0.0;
-            if (((cd >> (2 * m)) & 3) == 1) {  // the cell's own candidate, used in this pass
-                lL = lface[((long long)(d * 2) * NW + m) * N + g];
-                lR = lface[((long long)(d * 2 + 1) * NW + m) * N + g];
-                if (pos == n - 1) lL += limg[((long long)(d * 2 + 1) * NW + m) * G.nl + line];
-                if (pos == 0) lR += limg[((long long)(d * 2) * NW + m) * G.nl + line];
+        double* tc = tcon + (long long)((d * M + m) * 9) * N + g;
+        double s[3][3], ls[3][3];
+        for (int a = 0; a < 3; ++a)
+            for (int c = 0; c < 3; ++c) {
+                bool r0, r1;
+                const int ii = mapi(i + a - 1, G.nx, G.lo_bc[0], G.hi_bc[0], r0);
+                const int jj = mapi(j + c - 1, G.ny, G.lo_bc[1], G.hi_bc[1], r1);
+                s[a][c] = X[(G.sa + m) * N + ii + (long long)G.nx * jj];
+                ls[a][c] = 0.0;
             }
-            if (mixed && sur) {
-                // this pass wrote the right candidate into URStar
-                // (thinc.cpp:138-147): the adjoint of its later reads
-                lR += sur[(long long)m * N + g];
-                sur[(long long)m * N + g] = 0.0;
-            }
-            if (mixed && (lL != 0.0 || lR != 0.0))
-                tja::thinc_cand_rev(s, d, G.beta, G.dx[0], G.dx[1], thinc_cosh, thinc_tanh, thinc_exp, lL, lR, ls);
-            for (int a = 0; a < 3; ++a)
-                for (int c = 0; c < 3; ++c) tc[(long long)(a * 3 + c) * N] = ls[a][c];
+        const bool mixed = tja::thinc_mixed(s, d);
+        double lL = 0.0, lR = 0.0;
+        if (((cd >> (2 * m)) & 3) == 1) {  // the cell's own candidate, used in this pass
+            lL = lface[((long long)(d * 2) * NW + m) * N + g];
+            lR = lface[((long long)(d * 2 + 1) * NW + m) * N + g];
+            if (pos == n - 1) lL += limg[((long long)(d * 2 + 1) * NW + m) * G.nl + line];
+            if (pos == 0) lR += limg[((long long)(d * 2) * NW + m) * G.nl + line];
         }
+        if (mixed && sur) {
+            // this pass wrote the right candidate into URStar
+            // (thinc.cpp:138-147): the adjoint of its later reads
+            lR += sur[e];
+            sur[e] = 0.0;
+        }
+        if (mixed && (lL != 0.0 || lR != 0.0))
+            tja::thinc_cand_rev(s, d, G.beta, G.dx[0], G.dx[1], thinc_cosh, thinc_tanh, thinc_exp, lL, lR, ls);
+        for (int a = 0; a < 3; ++a)
+            for (int c = 0; c < 3; ++c) tc[(long long)(a * 3 + c) * N] = ls[a][c];
     }
 }
 
@@ -505,8 +506,20 @@ __global__ void __launch_bounds__(NT, 8) k_adj_gather(AG G0, const double* X, co
                 }
             }
         }
-        // THINC candidates of the 3x3 neighbours that read this cell
-        if (G.thinc) {
+        // THINC candidates of the 3x3 neighbours that read this cell. Two cells
+        // or more from the edge a neighbour reads it in one place of its
+        // stencil; near the edge boundary images read it in others as well.
+        const bool inner = i >= 2 && i < G.nx - 2 && j >= 2 && j < G.ny - 2;
+        if (G.thinc && inner) {
+            for (int d = 0; d < 2; ++d)
+                for (int a = -1; a <= 1; ++a)
+                    for (int c = -1; c <= 1; ++c) {
+                        const long long gi = (i + a) + (long long)G.nx * (j + c);
+#pragma unroll
+                        for (int m = 0; m < M; ++m)
+                            acc[m] += tcon[((long long)((d * M + m) * 9) + (1 - a) * 3 + (1 - c)) * N + gi];
+                    }
+        } else if (G.thinc) {
             for (int d = 0; d < 2; ++d)
                 for (int a = -1; a <= 1; ++a)
                     for (int c = -1; c <= 1; ++c) {
@@ -873,7 +886,7 @@ long long adj_backward(AdjState* a, const DevParams& P, const Fp64Bufs& b, const
 #undef ADJ_FACE
                     launches += 1;
                     if (P.thinc) {
-                        ADJ_M(M, k_adj_thinc, nb(N), NT, 0, st>>>(G, d, X, code, a->lface, a->limg, a->tcon, a->sur));
+                        ADJ_M(M, k_adj_thinc, nb(N * M), NT, 0, st>>>(G, d, X, code, a->lface, a->limg, a->tcon, a->sur));
                         k_adj_scratch<<<nb(N), NT, 0, st>>>(G, d, code, a->lface, a->limg, a->sul, a->sur);
                         launches += 2;
                     }

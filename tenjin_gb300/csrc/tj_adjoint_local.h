@@ -180,8 +180,14 @@ TJA_HD void cleanup_rev(int M, const double* a, const double* lam_out, double* l
 // ---------------------------------------------------------------------------
 // Face state: [cleanUpAlpha], primitiveToConservative, getSoundSpeed.
 // ---------------------------------------------------------------------------
+// The intermediates of a face state that its reverse uses.
+struct FaceParts {
+    double xi[MM], c2[MM], v[MM];  // 1 / G, the material's c^2, its part of A
+    double A, xit, invG;           // c = sqrt(max(A, floor) / xit)
+};
+
 template <class EosT>
-TJA_HD void face_state_fwd(const EosT& E, const Prim& x, bool clean, FS& s)
+TJA_HD void face_state_parts(const EosT& E, const Prim& x, bool clean, FS& s, FaceParts& f)
 {
     const int M = E.M;
     if (clean) cleanup_fwd(M, x.a, s.a);
@@ -201,33 +207,43 @@ TJA_HD void face_state_fwd(const EosT& E, const Prim& x, bool clean, FS& s)
         ke += 0.5 * s.rho * x.u[r] * x.u[r];
     }
     s.p = x.p;
-    double invG = 0.0, ent = 0.0, pnt = 0.0;
+    double ent = 0.0, pnt = 0.0;
+    f.invG = 0.0;
     TJA_UNROLL
     for (int m = 0; m < M; ++m) {
-        invG += quot(s.a[m], E.G[m]);
+        f.invG += quot(s.a[m], E.G[m]);
         ent += E.er[m] * s.ar[m];
         pnt += quot(E.pr[m] * s.a[m], E.G[m]);
     }
-    s.E = x.p * invG + ent - pnt + ke;
-    double A = 0.0, xit = 0.0;
+    s.E = x.p * f.invG + ent - pnt + ke;
+    f.A = f.xit = 0.0;
     TJA_UNROLL
     for (int m = 0; m < M; ++m) {
-        const double xi = quot(1.0, E.G[m]);
-        const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
-        const double v = quot(xi * c2 * s.ar[m], s.rho);
-        A += (0.0 < v) ? v : 0.0;
-        xit += xi * s.a[m];
+        f.xi[m] = quot(1.0, E.G[m]);
+        f.c2[m] = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
+        f.v[m] = quot(f.xi[m] * f.c2[m] * s.ar[m], s.rho);
+        f.A += (0.0 < f.v[m]) ? f.v[m] : 0.0;
+        f.xit += f.xi[m] * s.a[m];
     }
-    if (A <= 0.0) A = 1E-6;
-    s.c = root(quot(A, xit));
+    s.c = root(quot(f.A <= 0.0 ? 1E-6 : f.A, f.xit));
 }
 
 template <class EosT>
-TJA_HD void face_state_rev(const EosT& E, const Prim& x, bool clean, const FS& l, Prim& lx, GradEos& g)
+TJA_HD void face_state_fwd(const EosT& E, const Prim& x, bool clean, FS& s)
+{
+    FaceParts f;
+    face_state_parts(E, x, clean, s, f);
+}
+
+// s and f: face_state_parts of the same state. The quotients that share a
+// divisor are products with its reciprocal (the branches come from the
+// forward's own values): four quotients instead of about forty, each a serial
+// chain of some 150 cycles.
+template <class EosT>
+TJA_HD void face_state_rev(const EosT& E, const Prim& x, bool clean, const FS& s, const FaceParts& f, const FS& l,
+                           Prim& lx, GradEos& g)
 {
     const int M = E.M;
-    FS s;
-    face_state_fwd(E, x, clean, s);
     double la[MM], lar[MM], lrk[MM];
     TJA_UNROLL
     for (int m = 0; m < M; ++m) {
@@ -236,52 +252,39 @@ TJA_HD void face_state_rev(const EosT& E, const Prim& x, bool clean, const FS& l
         lrk[m] = 0.0;
     }
     double lrho = l.rho, lp = l.p, lu[2] = {l.u[0], l.u[1]};
+    const double irho = quot(1.0, s.rho);
     // getSoundSpeed: c = sqrt(A / xit)
     {
-        double A = 0.0, xit = 0.0;
+        const double h = quot(l.c, 2.0 * s.c * f.xit);
+        const double lA = f.A <= 0.0 ? 0.0 : h, lxit = -h * (s.c * s.c);
         TJA_UNROLL
         for (int m = 0; m < M; ++m) {
-            const double xi = quot(1.0, E.G[m]);
-            const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
-            const double v = quot(xi * c2 * s.ar[m], s.rho);
-            A += (0.0 < v) ? v : 0.0;
-            xit += xi * s.a[m];
-        }
-        const bool floored = A <= 0.0;
-        const double lA = floored ? 0.0 : quot(l.c, 2.0 * s.c * xit);
-        const double lxit = quot(-l.c * s.c, 2.0 * xit);
-        TJA_UNROLL
-        for (int m = 0; m < M; ++m) {
-            const double xi = quot(1.0, E.G[m]);
-            const double c2 = quot(x.p * (E.G[m] + 1.0), x.rk[m]) - quot(E.pr[m], x.rk[m]);
-            const double v = quot(xi * c2 * s.ar[m], s.rho);
             double lxi = lxit * s.a[m];
-            la[m] += lxit * xi;
-            if (0.0 < v) {
-                const double lc2 = quot(lA * xi * s.ar[m], s.rho);
-                lar[m] += quot(lA * xi * c2, s.rho);
-                lrho += -quot(lA * v, s.rho);
-                lxi += quot(lA * c2 * s.ar[m], s.rho);
-                lp += quot(lc2 * (E.G[m] + 1.0), x.rk[m]);
-                lrk[m] += -quot(lc2 * c2, x.rk[m]);
-                g.G[m] += quot(lc2 * x.p, x.rk[m]);
-                g.pr[m] += -quot(lc2, x.rk[m]);
+            la[m] += lxit * f.xi[m];
+            if (0.0 < f.v[m]) {
+                const double irk = quot(1.0, x.rk[m]), t = lA * irho;
+                const double lc2 = t * f.xi[m] * s.ar[m], lq = lc2 * irk;
+                lar[m] += t * f.xi[m] * f.c2[m];
+                lrho -= t * f.v[m];
+                lxi += t * f.c2[m] * s.ar[m];
+                lp += lq * (E.G[m] + 1.0);
+                lrk[m] -= lq * f.c2[m];
+                g.G[m] += lq * x.p;
+                g.pr[m] -= lq;
             }
-            g.G[m] += -lxi * xi * xi;
+            g.G[m] += -lxi * f.xi[m] * f.xi[m];
         }
     }
     // primitiveToConservative: E = p invG + sum e_ref ar - sum p_ref a / G + ke
     {
         const double lE = l.E;
-        double invG = 0.0;
-        TJA_UNROLL
-        for (int m = 0; m < M; ++m) invG += quot(s.a[m], E.G[m]);
-        lp += lE * invG;
+        lp += lE * f.invG;
         TJA_UNROLL
         for (int m = 0; m < M; ++m) {
-            la[m] += quot(lE * (x.p - E.pr[m]), E.G[m]);
-            g.G[m] += -quot(lE * (x.p - E.pr[m]) * s.a[m], E.G[m] * E.G[m]);
-            g.pr[m] += -quot(lE * s.a[m], E.G[m]);
+            const double q = lE * (x.p - E.pr[m]) * f.xi[m];
+            la[m] += q;
+            g.G[m] -= q * s.a[m] * f.xi[m];
+            g.pr[m] -= lE * s.a[m] * f.xi[m];
             g.er[m] += lE * s.ar[m];
             lar[m] += lE * E.er[m];
         }
@@ -305,6 +308,15 @@ TJA_HD void face_state_rev(const EosT& E, const Prim& x, bool clean, const FS& l
     lx.u[0] = lu[0];
     lx.u[1] = lu[1];
     lx.p = lp;
+}
+
+template <class EosT>
+TJA_HD void face_state_rev(const EosT& E, const Prim& x, bool clean, const FS& l, Prim& lx, GradEos& g)
+{
+    FS s;
+    FaceParts f;
+    face_state_parts(E, x, clean, s, f);
+    face_state_rev(E, x, clean, s, f, l, lx, g);
 }
 
 // ---------------------------------------------------------------------------
@@ -375,6 +387,7 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     FS lK = pick(side != 0, lR, lL);
     const double SK = side ? SR : SL, uK = K.u[d];
     const bool guard = Ss - uK == 0.0 && Ss != 0.0;
+    const double iden = quot(1.0, SK - Ss), iSK = quot(1.0, SK - uK);
     const double mult = guard ? 1.0 : quot(SK - uK, SK - Ss);
     double ars[MM], rs = 0.0;
     TJA_UNROLL
@@ -385,8 +398,9 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     double rus[2];
     rus[d] = mult * K.rho * Ss;
     rus[1 - d] = mult * K.ru[1 - d];
+    const double irs = quot(1.0, rs);
     const double vsd = quot(rus[d], rs);
-    const double D1 = Ss - uK, D2 = K.rho * Ss + quot(K.p, SK - uK);
+    const double D1 = Ss - uK, D2 = K.rho * Ss + K.p * iSK;
     const double W = K.E + D1 * D2;
     const double Es = mult * W;
     const double w = hllc ? SK : 0.0;
@@ -422,8 +436,8 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     lEs = lF.FE * w;
     if (hllc) lSK += lF.FE * (Es - K.E);
     // vsd = rus_d / rs
-    lrus[d] += quot(lvsd, rs);
-    const double lrs = quot(-lvsd * vsd, rs);
+    lrus[d] += lvsd * irs;
+    const double lrs = -lvsd * vsd * irs;
     TJA_UNROLL
     for (int m = 0; m < M; ++m) lars[m] += lrs;
     // ars = mult K.ar; rus_d = mult K.rho Ss; rus_o = mult K.ru_o
@@ -446,15 +460,16 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     luK -= lD1;
     lK.rho += lD2 * Ss;
     lSs += lD2 * K.rho;
-    lK.p += quot(lD2, SK - uK);
-    lSK += -quot(lD2 * K.p, (SK - uK) * (SK - uK));
-    luK += quot(lD2 * K.p, (SK - uK) * (SK - uK));
+    const double lq = lD2 * iSK, lqp = lq * K.p * iSK;
+    lK.p += lq;
+    lSK -= lqp;
+    luK += lqp;
     // mult = (SK - uK) / (SK - Ss)
     if (!guard) {
-        const double den = SK - Ss;
-        lSK += quot(lmult * (uK - Ss), den * den);
-        luK += -quot(lmult, den);
-        lSs += quot(lmult * mult, den);
+        const double lm = lmult * iden;
+        lSK += lm * (uK - Ss) * iden;
+        luK -= lm;
+        lSs += lm * mult;
     }
     double lSL = 0.0, lSR = 0.0;
     if (side) lSR += lSK;
@@ -463,7 +478,7 @@ TJA_HD double hllc_rev(int M, const FS& L, const FS& R, int d, const HllcOut& lF
     lL = pick(side == 0, lK, lL);
     lR = pick(side != 0, lK, lR);
     // Ss = Num / Den
-    const double lNum = quot(lSs, Den), lDen = quot(-lSs * Ss, Den);
+    const double lNum = quot(lSs, Den), lDen = -lNum * Ss;
     lR.p += lNum;
     lL.p -= lNum;
     lL.ru[d] += lNum * (SL - uL);
@@ -530,16 +545,20 @@ TJA_HD void c2p_rev(const EosT& E, const Cons& c, const Carried& lam, Cons& mu, 
     const int M = E.M;
     Carried o;
     c2p_fwd(E, c, o);
-    double D = 0.0;
-    TJA_UNROLL
-    for (int m = 0; m < M; ++m) D += quot(c.a[m], E.G[m]);
-    const double lN = quot(lam.p, D), lD = quot(-lam.p * o.p, D);
+    double D = 0.0, iG[MM];
     TJA_UNROLL
     for (int m = 0; m < M; ++m) {
-        mu.a[m] = lam.a[m] - quot(lam.rk[m] * o.rk[m], c.a[m]) + quot(lN * E.pr[m], E.G[m]) + quot(lD, E.G[m]);
-        mu.ar[m] = lam.ar[m] + quot(lam.rk[m], c.a[m]) - lN * E.er[m];
-        g.G[m] += -quot((lN * E.pr[m] + lD) * c.a[m], E.G[m] * E.G[m]);
-        g.pr[m] += quot(lN * c.a[m], E.G[m]);
+        iG[m] = quot(1.0, E.G[m]);
+        D += quot(c.a[m], E.G[m]);
+    }
+    const double lN = quot(lam.p, D), lD = -lN * o.p, irho = quot(1.0, o.rho);
+    TJA_UNROLL
+    for (int m = 0; m < M; ++m) {
+        const double lk = quot(lam.rk[m], c.a[m]);
+        mu.a[m] = lam.a[m] - lk * o.rk[m] + lN * E.pr[m] * iG[m] + lD * iG[m];
+        mu.ar[m] = lam.ar[m] + lk - lN * E.er[m];
+        g.G[m] -= (lN * E.pr[m] + lD) * c.a[m] * iG[m] * iG[m];
+        g.pr[m] += lN * c.a[m] * iG[m];
         g.er[m] += -lN * c.ar[m];
     }
     mu.E = lam.E + lN;
@@ -548,8 +567,9 @@ TJA_HD void c2p_rev(const EosT& E, const Cons& c, const Carried& lam, Cons& mu, 
         // ke = 0.5 rho u^2 with u = ru / rho
         const double lu = lam.u[r] - lN * o.rho * o.u[r];
         lrho += -lN * 0.5 * o.u[r] * o.u[r];
-        mu.ru[r] = lam.ru[r] + quot(lu, o.rho);
-        lrho += -quot(lu * o.u[r], o.rho);
+        const double lr = lu * irho;
+        mu.ru[r] = lam.ru[r] + lr;
+        lrho -= lr * o.u[r];
     }
     TJA_UNROLL
     for (int m = 0; m < M; ++m) mu.ar[m] += lrho;
@@ -629,6 +649,18 @@ struct ThincMath {
     double (*exp_)(double);
 };
 
+// Whether the cell is mixed (thinc.cpp:67-114).
+TJA_HD bool thinc_mixed(const double s[3][3], int d)
+{
+    const double eps = 1E-20;
+    const double aL = d == 0 ? s[0][1] : s[1][0], aR = d == 0 ? s[2][1] : s[1][2], a0 = s[1][1];
+    const double mn = (aR < aL) ? aR : aL;
+    const double mx = ((aL < aR) ? aR : aL) - mn;
+    const double C = (mx < eps) ? 0.0 : quot(a0 - mn + eps, mx + eps);
+    const double delta = 1E-4;
+    return (C > delta) && (C < (0.999999 - delta)) && ((aR - a0) * (a0 - aL) >= 0.0);
+}
+
 template <typename CoshF, typename TanhF, typename ExpF>
 TJA_HD bool thinc_cand_fwd(const double s[3][3], int d, double beta0, double dx, double dy, CoshF ch, TanhF th, ExpF ex,
                            double& L, double& R)
@@ -672,7 +704,7 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
     const double norm = root(nx * nx + ny * ny);
     const bool flat = norm < 1E-20;
     const double nd = d == 0 ? nx : ny;
-    const double nvc = flat ? 0.0 : fabs(nd / norm);
+    const double nvc = flat ? 0.0 : fabs(quot(nd, norm));
     const double beta = nvc * beta0 + 0.01;
     const double coshB = ch(beta), tanhB = th(beta);
     const double B = ex(theta * beta * ((2.0 * C) - 1.0));
@@ -684,20 +716,21 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
     double lmx = lL * 0.5 * (1.0 + theta * A) + lR * 0.5 * (1.0 + theta * T);
     double lA = lL * (0.5 * mx) * theta;
     const double lT = lR * (0.5 * mx) * theta;
-    double lt = quot(lT * (1.0 - A * A), q * q);
-    lA += quot(lT * (1.0 - tanhB * tanhB), q * q);
+    const double lTq = quot(lT, q * q);
+    double lt = lTq * (1.0 - A * A);
+    lA += lTq * (1.0 - tanhB * tanhB);
     const double lB = quot(lA, coshB * tanhB);
-    const double lch = quot(-lA * B, coshB * coshB * tanhB);
-    lt += -quot(lA * A, tanhB);
+    const double lch = quot(-lB * B, coshB);
+    lt -= lB * coshB * A;
     double lbeta = lB * B * theta * (2.0 * C - 1.0);
     const double lC = lB * B * theta * beta * 2.0;
     lbeta += lch * tanhB * coshB;  // d cosh = sinh = tanh cosh
     lbeta += lt * (1.0 - tanhB * tanhB);
     const double lnvc = lbeta * beta0;
     // C = (a0 - mn + eps) / (mx + eps)
-    double la0 = quot(lC, mx + eps);
-    lmn -= quot(lC, mx + eps);
-    lmx -= quot(lC * C, mx + eps);
+    const double la0 = quot(lC, mx + eps);
+    lmn -= la0;
+    lmx -= la0 * C;
     // mx = max - mn
     const double lmax = lmx;
     lmn -= lmx;
@@ -719,9 +752,9 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
     ls[1][1] += la0;
     if (!flat) {
         const double sg = (double)((nd > 0.0) - (nd < 0.0));
-        const double n3 = norm * norm * norm;
-        const double lnx = lnvc * sg * (quot(d == 0 ? 1.0 : 0.0, norm) - quot(nd * nx, n3));
-        const double lny = lnvc * sg * (quot(d == 1 ? 1.0 : 0.0, norm) - quot(nd * ny, n3));
+        const double in = quot(1.0, norm), ns = nd * in * in * in;
+        const double lnx = lnvc * sg * ((d == 0 ? in : 0.0) - ns * nx);
+        const double lny = lnvc * sg * ((d == 1 ? in : 0.0) - ns * ny);
         const double cx = quot(-1.0, 8.0 * dx) * lnx, cy = quot(-1.0, 8.0 * dy) * lny;
         ls[2][2] += cx + cy;
         ls[2][1] += 2.0 * cx;
