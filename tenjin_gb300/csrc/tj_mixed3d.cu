@@ -24,8 +24,9 @@
 // The tile shape (TX, TY, TZ) is a template parameter. The boxes fall into
 // size classes (up to 16^3 cells, up to 32^3, larger); a host-side autotuner
 // times each candidate shape on each class's tiles once and keeps the fastest
-// per class, and each class runs as its own persistent launch per stage (the
-// environment variable TJ_TILE3D=AxBxC pins one candidate for all classes).
+// per class, and the classes of one shape run as one persistent launch per
+// stage (the environment variable TJ_TILE3D=AxBxC pins one candidate for all
+// classes).
 // Results do not depend on the tile shape (every face and cell is computed
 // by the same arithmetic whichever tile owns it).
 #include <cuda_runtime.h>
@@ -50,10 +51,14 @@ namespace {
 // take four, and hide more of each other's waits (128 boxes, 30 steps, with the
 // changes to the index arithmetic: 36.7 / 36.3 / 39.9 ms with 512 / 640 / 896).
 constexpr int NT3 = 640;
+// A pair of smaller CTAs an SM, each with one staging buffer: the one computes
+// while the other stages or waits at a barrier (two of the candidate shapes;
+// with the classes' launches merged, 128 boxes, 30 steps 34.7 -> 31.2 ms).
+constexpr int NT3_PAIR = 320;
 
 // k_stage3d's flags: a trial launch of the tuner; the last launch of a stage
-// (the classes of boxes are launched one after the other).
-constexpr int kForce = 1, kLastClass = 2;
+// (classes of boxes with different tile shapes are launched one after the other).
+constexpr int kForce = 1, kLastRun = 2;
 
 struct M3P {
     double cfl;
@@ -338,7 +343,7 @@ __device__ __forceinline__ void recon3(const M3P& P, const float* sm, int s, int
 // ghosts at their boundary images) and of its output cells' conserved words
 // into the staging buffer at sp. Values arrive unmodified: stage_fix negates
 // the reflected velocities once they have landed.
-template <int M, int TX, int TY, int TZ>
+template <int M, int TX, int TY, int TZ, int NT>
 __device__ void stage_issue(const M3P& P, const Work3& w, const Dom3& D, const float* __restrict__ Xin, long long N,
                             float* sp)
 {
@@ -347,7 +352,7 @@ __device__ void stage_issue(const M3P& P, const Work3& w, const Dom3& D, const f
     const int nx = D.n[0], ny = D.n[1], nz = D.n[2];
     const long long off = D.off;
     const int sx = ex + 4, sy = ey + 4, sz = ez + 4;
-    for (int t = threadIdx.x; t < sx * sy * sz; t += NT3) {
+    for (int t = threadIdx.x; t < sx * sy * sz; t += NT) {
         int x, y, z;
         split_t(t, w.m_sx, w.m_sxy, sx, sy, x, y, z);
         bool rx, ry, rz;
@@ -365,7 +370,7 @@ __device__ void stage_issue(const M3P& P, const Work3& w, const Dom3& D, const f
         for (int r = 0; r < 3; ++r) cp_async4(sp + SM::P_OFF + (2 * M + r) * SM::SV + s, Xin + S3_U<M>(r) * N + g);
         cp_async4(sp + SM::P_OFF + (2 * M + 3) * SM::SV + s, Xin + S3_P<M>() * N + g);
     }
-    for (int t = threadIdx.x; t < ex * ey * ez; t += NT3) {
+    for (int t = threadIdx.x; t < ex * ey * ez; t += NT) {
         int x, y, z;
         split_t(t, w.m_ex, w.m_exy, ex, ey, x, y, z);
         const long long g = off + (i0 + x) + (long long)nx * ((j0 + y) + (long long)ny * (k0 + z));
@@ -385,12 +390,12 @@ __device__ void stage_issue(const M3P& P, const Work3& w, const Dom3& D, const f
 // The second stage's finish averages with U^n (hllc.cpp:705): ask L2 for the
 // rows of a tile's output cells in every U^n word when the tile's staging is
 // queued, so that they arrive while the tile before it computes.
-template <int M>
+template <int M, int NT>
 __device__ __forceinline__ void prefetch_un(const Work3& w, const Dom3& D, const float* __restrict__ Xun, long long N)
 {
     const int ey = w.ey, ez = w.ez, ex = w.ex;
     const int nrow = ey * ez;
-    for (int t = threadIdx.x; t < S3_N<M>() * nrow * 2; t += NT3) {
+    for (int t = threadIdx.x; t < S3_N<M>() * nrow * 2; t += NT) {
         const int q = t / (2 * nrow), r = (t >> 1) % nrow, e = t & 1;
         const int y = r % ey, z = r / ey;
         const long long g = D.off + (w.i0 + e * (ex - 1)) + (long long)D.n[0] * ((w.j0 + y) + (long long)D.n[1] * (w.k0 + z));
@@ -402,7 +407,7 @@ __device__ __forceinline__ void prefetch_un(const Work3& w, const Dom3& D, const
 // negate the velocity normal to each reflective face the ghost crosses.
 // Returns whether the tile reaches a reflective face (the same answer in
 // every thread of the block).
-template <int M, int TX, int TY, int TZ>
+template <int M, int TX, int TY, int TZ, int NT>
 __device__ bool stage_fix(const M3P& P, const Work3& w, const Dom3& D, float* sp)
 {
     using SM = Sm3<M, TX, TY, TZ>;
@@ -414,7 +419,7 @@ __device__ bool stage_fix(const M3P& P, const Work3& w, const Dom3& D, float* sp
                 (P.hi_bc[d] == TJ_BC_REFLECTIVE && lo[d] + ext[d] + 2 > D.n[d]);
     if (!near) return false;
     const int sx = w.ex + 4, sy = w.ey + 4, sz = w.ez + 4;
-    for (int t = threadIdx.x; t < sx * sy * sz; t += NT3) {
+    for (int t = threadIdx.x; t < sx * sy * sz; t += NT) {
         int x, y, z;
         split_t(t, w.m_sx, w.m_sxy, sx, sy, x, y, z);
         bool r3[3];
@@ -429,16 +434,17 @@ __device__ bool stage_fix(const M3P& P, const Work3& w, const Dom3& D, float* sp
     return true;
 }
 
-template <int M, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int flags)
+template <int M, int TX, int TY, int TZ, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? NT3_PAIR : NT3, PAIR ? 2 : 1) k_stage3d(M3P P, M3B b, int stage, int flags)
 {
+    constexpr int NT = PAIR ? NT3_PAIR : NT3;
     const bool force = flags & kForce;
     grid_wait();
     grid_go();
     if (!force && b.scal->done) return;
     // the first stage takes the step's dt from the CFL minimum that the step
-    // before left: every block of every class forms it, the last block of the
-    // last class stores it
+    // before left: every block forms it, the last block of the last launch
+    // stores it
     __shared__ float dt_step;
     __shared__ int run_over;
     if (threadIdx.x == 0) {
@@ -450,7 +456,7 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fl
     __syncthreads();
     const float dtf = dt_step;
     if (run_over) {
-        if ((flags & kLastClass) && last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
+        if ((flags & kLastRun) && last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
         return;
     }
     using SM = Sm3<M, TX, TY, TZ>;
@@ -465,34 +471,36 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fl
     __shared__ Dom3 Dsh[2];
 
     int wi = blockIdx.x;
-    if (wi < b.nwork) {
+    if (!PAIR && wi < b.nwork) {
         if (threadIdx.x == 0) {
             wsh[0] = b.work[wi];
             Dsh[0] = b.doms[wsh[0].dom];
         }
         __syncthreads();
-        stage_issue<M, TX, TY, TZ>(P, wsh[0], Dsh[0], Xin, N, sm);
-        if (stage == 1) prefetch_un<M>(wsh[0], Dsh[0], Xout, N);
+        stage_issue<M, TX, TY, TZ, NT>(P, wsh[0], Dsh[0], Xin, N, sm);
+        if (stage == 1) prefetch_un<M, NT>(wsh[0], Dsh[0], Xout, N);
     }
     cp_async_commit();
     for (int it = 0; wi < b.nwork; wi += gridDim.x, ++it) {
-        const int cur = it & 1, nxt = cur ^ 1;
-        float* const sp = sm + (cur ? SM::TOTAL : 0);  // this tile's staging buffer
-        const int wn = wi + gridDim.x;
-        __syncthreads();  // the previous tile is done with the other buffer and its slot
+        // the slot and the staging buffer of this tile, and of the one whose
+        // copies are issued now: the next tile's, of a pair this tile's own
+        const int cur = PAIR ? 0 : it & 1, nxt = PAIR ? 0 : cur ^ 1;
+        float* const sp = sm + (cur ? SM::TOTAL : 0);
+        const int wn = PAIR ? wi : wi + gridDim.x;
+        __syncthreads();  // the previous tile is done with that buffer and slot
         if (threadIdx.x == 0 && wn < b.nwork) {
             wsh[nxt] = b.work[wn];
             Dsh[nxt] = b.doms[wsh[nxt].dom];
         }
         __syncthreads();
         if (wn < b.nwork) {
-            stage_issue<M, TX, TY, TZ>(P, wsh[nxt], Dsh[nxt], Xin, N, sm + (nxt ? SM::TOTAL : 0));
-            if (stage == 1) prefetch_un<M>(wsh[nxt], Dsh[nxt], Xout, N);
+            stage_issue<M, TX, TY, TZ, NT>(P, wsh[nxt], Dsh[nxt], Xin, N, sm + (nxt ? SM::TOTAL : 0));
+            if (stage == 1) prefetch_un<M, NT>(wsh[nxt], Dsh[nxt], Xout, N);
         }
         cp_async_commit();
-        cp_async_wait<1>();  // this tile's copies have landed
+        cp_async_wait<PAIR ? 0 : 1>();  // this tile's copies have landed
         __syncthreads();
-        if (stage_fix<M, TX, TY, TZ>(P, wsh[cur], Dsh[cur], sp)) __syncthreads();
+        if (stage_fix<M, TX, TY, TZ, NT>(P, wsh[cur], Dsh[cur], sp)) __syncthreads();
         const Work3& w = wsh[cur];
         const Dom3& D = Dsh[cur];
         const int ex = w.ex, ey = w.ey, ez = w.ez;
@@ -514,9 +522,9 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fl
                 const int n_d = d == 0 ? nx : (d == 1 ? ny : nz);
                 const int p0 = d == 0 ? i0 : (d == 1 ? j0 : k0);
                 const bool lo_refl = P.lo_bc[d] == TJ_BC_REFLECTIVE, hi_refl = P.hi_bc[d] == TJ_BC_REFLECTIVE;
-                int u0 = ((int)threadIdx.x - base) % NT3;
-                if (u0 < 0) u0 += NT3;
-                for (int t = u0; t < nfd; t += NT3) {
+                int u0 = ((int)threadIdx.x - base) % NT;
+                if (u0 < 0) u0 += NT;
+                for (int t = u0; t < nfd; t += NT) {
                     int x, y, z;
                     split_t(t, d == 0 ? w.m_fx : w.m_ex, d == 0 ? w.m_fxy : (d == 1 ? w.m_exfy : w.m_exy), fx, fy, x, y, z);
                     const int f_d = d == 0 ? x : (d == 1 ? y : z);
@@ -546,7 +554,7 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fl
         // ---- per cell: the update of the three directions in order x, y, z
         //      (hllc.cpp:493-523), then the finish; a cell's words are touched
         //      by its own thread only, so no barrier separates the two ----
-        for (int t = threadIdx.x; t < ex * ey * ez; t += NT3) {
+        for (int t = threadIdx.x; t < ex * ey * ez; t += NT) {
             int x, y, z;
             split_t(t, w.m_ex, w.m_exy, ex, ey, x, y, z);
             const int c = x + TX * (y + TY * z);
@@ -692,11 +700,11 @@ __global__ void __launch_bounds__(NT3) k_stage3d(M3P P, M3B b, int stage, int fl
         __syncthreads();
         if (threadIdx.x == 0) {
             float mn = red[0];
-            for (int k = 1; k < NT3 / 32; ++k) mn = fminf(mn, red[k]);
+            for (int k = 1; k < NT / 32; ++k) mn = fminf(mn, red[k]);
             atomicMin(&b.scal->dtmin_bits, (unsigned long long)__double_as_longlong((double)mn));
         }
     }
-    if ((flags & kLastClass) && last_block(b.scal)) {
+    if ((flags & kLastRun) && last_block(b.scal)) {
         if (stage == 0) finalize_dt(b.scal, P.cfl, 1);
         else end_step(b.scal);
     }
@@ -819,49 +827,52 @@ struct Shape {
     int (*occupancy)(size_t);
 };
 
-template <int M, int TX, int TY, int TZ>
+template <int M, int TX, int TY, int TZ, bool PAIR>
 void stage_launch(const M3P& P, const M3B& b, int stage, int flags, int grid, size_t smem, cudaStream_t st,
                   bool overlap)
 {
-    launch(k_stage3d<M, TX, TY, TZ>, dim3(grid), NT3, smem, st, overlap, P, b, stage, flags);
+    launch(k_stage3d<M, TX, TY, TZ, PAIR>, dim3(grid), PAIR ? NT3_PAIR : NT3, smem, st, overlap, P, b, stage, flags);
 }
 
-template <int M, int TX, int TY, int TZ>
+template <int M, int TX, int TY, int TZ, bool PAIR>
 int stage_occupancy(size_t smem)
 {
     // a shape whose shared memory exceeds the opt-in maximum cannot run here:
     // 0, with the error the attribute call raised cleared
-    if (cudaFuncSetAttribute(k_stage3d<M, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(k_stage3d<M, TX, TY, TZ, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_stage3d<M, TX, TY, TZ>, NT3, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_stage3d<M, TX, TY, TZ, PAIR>,
+                                                      PAIR ? NT3_PAIR : NT3, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return nb;
 }
 
-template <int M, int TX, int TY, int TZ>
+template <int M, int TX, int TY, int TZ, bool PAIR = false>
 Shape make_shape()
 {
-    return Shape{TX, TY, TZ, Sm3<M, TX, TY, TZ>::BYTES, stage_launch<M, TX, TY, TZ>, stage_occupancy<M, TX, TY, TZ>};
+    using SM = Sm3<M, TX, TY, TZ>;
+    return Shape{TX, TY, TZ, PAIR ? sizeof(float) * SM::TOTAL : SM::BYTES, stage_launch<M, TX, TY, TZ, PAIR>,
+                 stage_occupancy<M, TX, TY, TZ, PAIR>};
 }
 
 template <int M>
 std::vector<Shape> shapes()
 {
     return {make_shape<M, 8, 8, 8>(), make_shape<M, 8, 8, 4>(), make_shape<M, 16, 8, 4>(), make_shape<M, 16, 4, 4>(),
-            make_shape<M, 4, 4, 4>()};
+            make_shape<M, 4, 4, 4>(), make_shape<M, 8, 8, 4, true>(), make_shape<M, 16, 4, 4, true>()};
 }
 
 // Box-size classes of the autotuner, by valid-cell count: small boxes up to
 // 16^3 cells, medium up to 32^3, large above. Each class gets its own tile
-// shape, chosen by timing, and its own persistent launch per RK stage: the
-// boxes are independent domains, so the classes' launches need no ordering
-// among themselves beyond the stream's.
+// shape, chosen by timing; the classes of one shape share a persistent launch
+// per RK stage (the boxes are independent domains), which has one tail in place
+// of one per class.
 constexpr int kClasses = 3;
 constexpr long long kClassMaxCells[kClasses - 1] = {16LL * 16 * 16, 32LL * 32 * 32};
 constexpr const char* kClassName[kClasses] = {"small", "medium", "large"};
@@ -885,6 +896,12 @@ struct ClassPlan {
     std::vector<double> tune_ms;
 };
 
+// One launch of a stage: the tiles of the classes of one shape.
+struct Run {
+    int shape = 0, grid = 0, nwork = 0;
+    Work3* d_work = nullptr;
+};
+
 struct Mixed3D : MixedBase {
     M3P P;
     M3B b;
@@ -895,6 +912,8 @@ struct Mixed3D : MixedBase {
     std::vector<Shape> cand;
     std::vector<int> occ;  // resident CTAs per SM of each candidate (0: does not fit)
     ClassPlan cls[kClasses];
+    Run runs[kClasses];
+    int nruns = 0;
     bool tuned = false;
     int sms = 0;
     long long N = 0;
@@ -909,6 +928,8 @@ struct Mixed3D : MixedBase {
         if (d_work) cudaFree(d_work);
         for (auto& c : cls)
             if (c.d_work) cudaFree(c.d_work);
+        for (auto& r : runs)
+            if (r.d_work) cudaFree(r.d_work);
     }
 
     int alloc(const DevParams& DP, const std::vector<DevDomain>& doms, long long ntot, cudaStream_t st)
@@ -1034,13 +1055,24 @@ struct Mixed3D : MixedBase {
         return TJ_OK;
     }
 
-    // The CFL pass's work list: every tile of every class under its shape.
+    // The launches of a stage, and the CFL pass's work list: every tile of every
+    // class under its shape.
     int plan_all(cudaStream_t st)
     {
         std::vector<Work3> all;
-        for (int c = 0; c < kClasses; ++c) {
-            if (cls[c].doms.empty()) continue;
-            const std::vector<Work3> w = tiles(cls[c].doms, cls[c].best >= 0 ? cls[c].best : std::max(0, first_fit()));
+        nruns = 0;
+        for (size_t s = 0; s < cand.size(); ++s) {
+            std::vector<int> doms;
+            for (const ClassPlan& C : cls)
+                if (!C.doms.empty() && C.best == (int)s) doms.insert(doms.end(), C.doms.begin(), C.doms.end());
+            if (doms.empty()) continue;
+            const std::vector<Work3> w = tiles(doms, (int)s);
+            Run& r = runs[nruns];
+            if (int e = upload(r.d_work, w, st)) return e;
+            r.shape = (int)s;
+            r.nwork = (int)w.size();
+            r.grid = std::max(1, std::min(r.nwork, sms * occ[s]));
+            ++nruns;
             all.insert(all.end(), w.begin(), w.end());
         }
         if (int e = upload(d_work, all, st)) return e;
@@ -1188,15 +1220,15 @@ struct Mixed3D : MixedBase {
     {
         (void)DP;
         b.scal = fb.scal;
-        int n = 0, last = kClasses - 1;
-        while (last > 0 && cls[last].doms.empty()) --last;
+        int n = 0;
         for (int stage = 0; stage < 2; ++stage)
-            for (int c = 0; c < kClasses; ++c) {
-                const ClassPlan& C = cls[c];
-                if (C.doms.empty()) continue;
-                const Shape& S = cand[C.best < 0 ? 0 : C.best];
+            for (int r = 0; r < nruns; ++r) {
+                const Shape& S = cand[runs[r].shape];
+                M3B br = b;
+                br.work = runs[r].d_work;
+                br.nwork = runs[r].nwork;
                 if (pr) pr->begin("tj_stage3d_mixed", st);
-                S.stage(P, class_bufs(c), stage, c == last ? kLastClass : 0, C.grid, S.smem, st, !pr);
+                S.stage(P, br, stage, r == nruns - 1 ? kLastRun : 0, runs[r].grid, S.smem, st, !pr);
                 if (pr) pr->end("tj_stage3d_mixed", st);
                 n += 1;
             }
