@@ -63,6 +63,13 @@ INSTANCES.update({
         ("tj_path_inst.cu", ["-DTJ_INST_R=128", f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", "-fmad=false"])
     for m, d in [(2, 0), (2, 1), (0, -1)]
 })
+# the general reverse mode's kernels: the update (u) and the faces (of each
+# direction), for plastic solids and (m0) for every configuration
+INSTANCES.update({
+    f"tj_gen_m{m}_d{'u' if d < 0 else d}.o":
+        ("tj_gen_inst.cu", [f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", "-fmad=false"])
+    for m, dirs in ((1, (-1, 0, 1, 2)), (2, (-1, 0, 1, 2)), (0, (-1, 0))) for d in dirs
+})
 
 
 def nvcc() -> str:

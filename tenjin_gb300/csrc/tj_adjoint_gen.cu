@@ -24,9 +24,8 @@
 //
 // Cost: a local Jacobian takes as many passes as the operator has inputs
 // (about 100 for a copper cell's last-direction update, 34 for a copper
-// face), so a backward step costs tens of forward steps: the general reverse
-// mode is exact and deterministic; the 2-D fluid adjoint is the fast one
-// (backward about 3 forward steps).
+// face), one thread each (tj_gen_rev.cuh): the general reverse mode is exact
+// and deterministic; the 2-D fluid adjoint is the fast one.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,125 +35,37 @@
 #include "tj_adjoint_local.h"
 #include "tj_dual.cuh"
 #include "tj_dual_path.cuh"
+#include "tj_gen_rev.cuh"
 #include "tj_path.cuh"
 #include "tj_path_launch.cuh"
 #include "tj_adjoint_gen.cuh"
 
 namespace tj {
 
-namespace {
+template <int MC>
+using Plastic = WithM<DevParamsT, MC, KIND_PLASTIC>;
+// compiled in tj_gen_inst.cu
+#define TJ_GEN_FLUX(PT, D) \
+    extern template void gen_flux_rev<PT, D>(const PT&, const Fp64Bufs&, const UpdPasses*, int, const GenFlux&, cudaStream_t)
+#define TJ_GEN_UPD(PT) \
+    extern template void gen_upd_rev<PT>(const PT&, const Fp64Bufs&, const UpdPasses*, int, const GenUpd&, cudaStream_t)
+TJ_GEN_FLUX(DevParamsT, -1);
+TJ_GEN_FLUX(Plastic<1>, 0);
+TJ_GEN_FLUX(Plastic<1>, 1);
+TJ_GEN_FLUX(Plastic<1>, 2);
+TJ_GEN_FLUX(Plastic<2>, 0);
+TJ_GEN_FLUX(Plastic<2>, 1);
+TJ_GEN_FLUX(Plastic<2>, 2);
+TJ_GEN_UPD(DevParamsT);
+TJ_GEN_UPD(Plastic<1>);
+TJ_GEN_UPD(Plastic<2>);
 
-constexpr int kGT = 128;  // threads per block of the reverse kernels
-constexpr int kNS = 48;   // carried words (39 at most: 4 solid plastic materials)
-constexpr int kNX = 32;   // flux words (29 at most)
-constexpr int kNF = 32;   // face-state words (31 at most)
+namespace {
 
 inline int gblocks(long long n)
 {
     long long b = (n + kGT - 1) / kGT;
     return (int)std::max(1LL, std::min(b, 152LL * 32));
-}
-
-// Flux words of a cell's two faces, read in place; the word `seed` carries
-// direction 1 on face 0.
-struct FacePairSeed {
-    const double* FX;
-    long long nf, f0, f1;
-    int seed;
-    __device__ __forceinline__ Dual operator()(int w, int s) const
-    {
-        return Dual(FX[(long long)w * nf + (s ? f1 : f0)], (!s && w == seed) ? 1.0 : 0.0);
-    }
-};
-
-// The inputs of a cell's update whose derivatives are formed, one pass each
-// (the others have none: conservativeToPrimitive and the radial return
-// overwrite the words they would come from, and a face flux enters as the
-// difference of the two faces, so face 1's adjoint is the negative of face
-// 0's). kind 0: accumulator, 1: stage input, 2: flux of face 0, 3: U^n,
-// 4: EOS parameter (word = material * npar + parameter).
-struct UpdPass {
-    short kind, word;
-};
-constexpr int kMaxPass = 3 * kNS + kNX + TJ_MAX_MAT * TJ_MAX_EOS_PARAMS;
-struct UpdPasses {
-    int n;
-    UpdPass p[kMaxPass];
-};
-
-// ---------------------------------------------------------------------------
-// Update of one direction, reversed per cell. Inputs: the accumulator Yin
-// (not read by the first direction, whose accumulator is U), the stage input
-// U, the two face fluxes F0 / F1 and, with the finish, U^n (A0). The output
-// adjoint lamOut is that of the direction's output (the next accumulator, or
-// U^{n+1} for the finish). Writes the adjoints of Yin and of the two fluxes
-// (per cell: F0 of the face below, F1 of the face above; the words without a
-// pass are zeroed by the host), adds those of U and A0, and adds each EOS
-// parameter's part into geos (per cell).
-//
-// One thread per cell and pass, cells fastest: the passes are independent
-// forward-mode evaluations of the cell's update whose values are the same and
-// whose direction is one input's. (One thread per cell running its ~110
-// passes in turn left 32 blocks for the 16^3 copper plate and spent its time in
-// the latency of one serial chain: backward 580 ms for 4 steps.) A warp's
-// lanes share the pass, so zero directions are skipped together.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kGT) k_gen_upd_rev(const __grid_constant__ DevParamsT P, Fp64Bufs fb,
-                                                     const UpdPasses* __restrict__ passes,
-                                                     const double* Yin, const double* U, const double* A0,
-                                                     const double* lamOut, double* lamYin, double* lamU, double* lamA0,
-                                                     double* lamF0, double* lamF1, double* geos, int d, int first,
-                                                     int last, int finish, int npar)
-{
-    const long long nt = fb.ntot, all = nt * passes->n;
-    const int NS = P.NS;
-    const DevDomain D = fb.doms[0];
-    const Dual dtv(fb.scal->dt);
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
-        const int pass = (int)(e / nt);
-        const long long g = e - (long long)pass * nt;
-        const int kind = passes->p[pass].kind, word = passes->p[pass].word;
-        int i, j, k;
-        split3(g - D.off, D.n[0], D.n[1], i, j, k);
-        int o[3] = {0, 0, 0};
-        o[d] = 1;
-        const FacePairSeed fx{fb.FX, fb.nftot[d], face_index(D, d, i, j, k),
-                              face_index(D, d, i + o[0], j + o[1], k + o[2]), kind == 2 ? word : -1};
-        Dual X[kNS], Y[kNS], A[kNS];
-        for (int w = 0; w < NS; ++w) {
-            X[w] = Dual(U[w * nt + g], (kind == 1 && w == word) ? 1.0 : 0.0);
-            Y[w] = first ? Dual(0.0) : Dual(Yin[w * nt + g], (kind == 0 && w == word) ? 1.0 : 0.0);
-            A[w] = finish ? Dual(A0[w * nt + g], (kind == 3 && w == word) ? 1.0 : 0.0) : Dual(0.0);
-        }
-        int cb = fb.cell_box[g];
-        PathBufs<Dual> lb{};
-        lb.ntot = 1;
-        lb.A = A;
-        lb.cell_box = &cb;
-        lb.scal = fb.scal;
-        DevParamsT Q;
-        const DevParamsT* par = &P;
-        if (kind == 4) {  // an EOS parameter's direction: a copy of the block with it
-            Q = P;
-            Q.prm[word / npar][word % npar].d = 1.0;
-            par = &Q;
-        }
-        update_cell(*par, lb, X, Y, 0LL, D, i, d, first, last, finish, dtv, fx);
-        const Dual* out = finish ? A : Y;
-        double s = 0.0;
-        for (int w = 0; w < NS; ++w) {
-            const double lo = lamOut[w * nt + g];
-            if (lo != 0.0) s += lo * out[w].d;  // a zero adjoint takes no part
-        }
-        const long long at = (long long)word * nt + g;
-        if (kind == 0) lamYin[at] = s;
-        else if (kind == 1) lamU[at] += s;
-        else if (kind == 2) {
-            lamF0[at] = s;
-            lamF1[at] = -s;
-        } else if (kind == 3) lamA0[at] += s;
-        else geos[at] += s;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -231,70 +142,6 @@ __global__ void __launch_bounds__(kGT) k_gen_upd_rev_lin(DevParams P, Fp64Bufs f
             if (first) lamU[(long long)w * nt + g] += lo(w);
             else lamYin[(long long)w * nt + g] = lo(w);
         }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Riemann problem of one face, reversed: the face's flux adjoint is gathered
-// from the cell above (its F0) and the cell below (its F1); one pass per
-// word of the two stored face states (UR of the cell below, UL of the cell
-// above, boundary images as k_flux maps them) gives their adjoints, per face,
-// one per EOS parameter in use those of the parameters: one thread per face
-// and pass, faces fastest, as in k_gen_upd_rev.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kGT) k_gen_flux_rev(const __grid_constant__ DevParamsT P, Fp64Bufs fb,
-                                                      const UpdPasses* __restrict__ passes,
-                                                      const double* lamF0, const double* lamF1, double* lamLf,
-                                                      double* lamRf, double* geos_f, int d, int npar, int nfw)
-{
-    const long long nt = fb.ntot, nf = fb.nftot[d];
-    const int NX = P.NX;
-    const DevDomain D = fb.doms[0];
-    const long long all = nf * passes->n;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
-        const int pass = (int)(e / nf);
-        const long long f = e - (long long)pass * nf;
-        const int kind = passes->p[pass].kind, word = passes->p[pass].word;
-        int nfv[3] = {D.n[0], D.n[1], D.n[2]};
-        nfv[d] += 1;
-        int i, j, k;
-        split3(f - D.foff[d], nfv[0], nfv[1], i, j, k);
-        int o[3] = {0, 0, 0};
-        o[d] = 1;
-        int idx[3] = {i, j, k};
-        int rl[3], rr[3];
-        const long long gl = map_cell(P, D, i - o[0], j - o[1], k - o[2], rl);
-        const long long gr = map_cell(P, D, i, j, k, rr);
-        Dual Lp[kNF], Rp[kNF], Fo[kNX];
-        for (int w = 0; w < nfw; ++w) {
-            Lp[w] = Dual(fb.UR[w * nt + gl], (kind == 0 && w == word) ? 1.0 : 0.0);
-            Rp[w] = Dual(fb.UL[w * nt + gr], (kind == 1 && w == word) ? 1.0 : 0.0);
-        }
-        CellT<Dual> L, R;
-        FluxV<Dual> F;
-        Dual Ss, vstar[3] = {Dual(0.0), Dual(0.0), Dual(0.0)};
-        DevParamsT Q;
-        const DevParamsT* par = &P;
-        if (kind == 4) {
-            Q = P;
-            Q.prm[word / npar][word % npar].d = 1.0;
-            par = &Q;
-        }
-        load_prim_face(*par, Lp, 1LL, 0LL, rl[d] ? d : -1, L);
-        load_prim_face(*par, Rp, 1LL, 0LL, rr[d] ? d : -1, R);
-        face_flux(*par, L, R, d, F, Ss, vstar, fb.scal);
-        for (int w = 0; w < NX; ++w) Fo[w] = Dual(0.0);
-        store_flux(P, Fo, 1LL, 0LL, F, Ss, vstar);
-        double s = 0.0;
-        for (int w = 0; w < NX; ++w) {
-            double lF = 0.0;
-            if (idx[d] >= 1) lF += lamF1[w * nt + D.off + (i - o[0]) + (long long)D.n[0] * ((j - o[1]) + (long long)D.n[1] * (k - o[2]))];
-            if (idx[d] < D.n[d]) lF += lamF0[w * nt + D.off + i + (long long)D.n[0] * (j + (long long)D.n[1] * k)];
-            if (lF != 0.0) s += lF * Fo[w].d;
-        }
-        if (kind == 0) lamLf[word * nf + f] = s;
-        else if (kind == 1) lamRf[word * nf + f] = s;
-        else geos_f[(long long)word * nf + f] += s;
     }
 }
 
@@ -505,6 +352,30 @@ DevParamsT params_t(const DevParams& D)
 }
 
 }  // namespace
+
+// The reverse of an update / of the faces of direction d: an instance of its own
+// for plastic solids of one and two materials (compile-time material count and
+// direction, no code for the rest), else the generic one.
+static void upd_rev(const DevParamsT& P, const Fp64Bufs& fb, const UpdPasses* pl, int n, const GenUpd& a,
+                    cudaStream_t st)
+{
+    if (param_kind(P) == KIND_PLASTIC && P.M == 1) gen_upd_rev(Plastic<1>(P), fb, pl, n, a, st);
+    else if (param_kind(P) == KIND_PLASTIC && P.M == 2) gen_upd_rev(Plastic<2>(P), fb, pl, n, a, st);
+    else gen_upd_rev(P, fb, pl, n, a, st);
+}
+static void flux_rev(const DevParamsT& P, const Fp64Bufs& fb, const UpdPasses* pl, int n, const GenFlux& a,
+                     cudaStream_t st)
+{
+    switch (param_kind(P) == KIND_PLASTIC ? P.M * 4 + a.d : 0) {
+        case 4: return gen_flux_rev<Plastic<1>, 0>(Plastic<1>(P), fb, pl, n, a, st);
+        case 5: return gen_flux_rev<Plastic<1>, 1>(Plastic<1>(P), fb, pl, n, a, st);
+        case 6: return gen_flux_rev<Plastic<1>, 2>(Plastic<1>(P), fb, pl, n, a, st);
+        case 8: return gen_flux_rev<Plastic<2>, 0>(Plastic<2>(P), fb, pl, n, a, st);
+        case 9: return gen_flux_rev<Plastic<2>, 1>(Plastic<2>(P), fb, pl, n, a, st);
+        case 10: return gen_flux_rev<Plastic<2>, 2>(Plastic<2>(P), fb, pl, n, a, st);
+        default: gen_flux_rev<DevParamsT, -1>(P, fb, pl, n, a, st);
+    }
+}
 
 struct GenAdj {
     int nsteps = 0, stride = 0, nck = 0, npar = 0, nprim = 0;
@@ -725,22 +596,19 @@ long long gen_backward(GenAdj* a, const DevParams& P, const Fp64Bufs& b, const d
                        double* lamU, double* lamA0, int d, int first, int last, int finish) {
         // the forward reconstruction and fluxes of this direction
         Fp64Bufs f2 = fb;
-        launches += path_dir_any(P, f2, U, a->yscr2, d, 1, 0, 0, st, nullptr);
+        launches += path_faces_any(P, f2, U, d, st, nullptr);
         if (mp > 0) cudaMemsetAsync(a->geosf, 0, sizeof(double) * mp * b.nftot[d], st);
         const int pl = finish ? (first ? PL_FINISH_FIRST : PL_FINISH) : (first ? PL_LAST_FIRST : PL_LAST);
-        if (!last && !finish)
+        if (!last && !finish) {
             k_gen_upd_rev_lin<<<gblocks(N), kGT, 0, st>>>(P, fb, U, lamOut, lamYin, lamU, a->lamF0, a->lamF1, d, first);
-        else {
+        } else {
             // the accumulator words without a pass
             if (!first) cudaMemsetAsync(lamYin, 0, sizeof(double) * S, st);
-            const LaunchShape sh = launch_shape(N * lists[pl].n, kGT);
-            k_gen_upd_rev<<<sh.blocks, sh.threads, 0, st>>>(PT, fb, a->passes + pl, Yin, U, A0, lamOut, lamYin, lamU,
-                                                            lamA0, a->lamF0, a->lamF1, a->geos, d, first, last, finish,
-                                                            npar);
+            const GenUpd u{Yin, U, A0, lamOut, lamYin, lamU, lamA0, a->lamF0, a->lamF1, a->geos, d, first, finish, npar};
+            upd_rev(PT, fb, a->passes + pl, lists[pl].n, u, st);
         }
-        const LaunchShape sf = launch_shape(b.nftot[d] * lists[PL_FACE].n, kGT);
-        k_gen_flux_rev<<<sf.blocks, sf.threads, 0, st>>>(PT, fb, a->passes + PL_FACE, a->lamF0, a->lamF1, a->lamLf,
-                                                         a->lamRf, a->geosf, d, npar, nfw);
+        const GenFlux f{a->lamF0, a->lamF1, a->lamLf, a->lamRf, a->geosf, d, npar};
+        flux_rev(PT, fb, a->passes + PL_FACE, lists[PL_FACE].n, f, st);
         const LaunchShape sr = launch_shape(N * nfw, kGT);
         k_gen_recon_rev<<<sr.blocks, sr.threads, 0, st>>>(P, fb, U, a->lamLf, a->lamRf, lamU, d, nfw);
         launches += 3;

@@ -149,9 +149,11 @@ __device__ __forceinline__ long long face_index(const DevDomain& D, int d, int i
     return D.foff[d] + i + (long long)nf0 * (j + (long long)nf1 * k);
 }
 
-// Carried-state load with the reflect_odd sign applied.
-template <typename PT, typename R = typename PT::real>
-TJ_DEV void load_state(const PT& P, const R* X, long long nt, long long g, const int* refl,
+// Carried-state load with the reflect_odd sign applied. X here and the arrays of
+// the other accessors below are pointers to the state's words, or what reads
+// (takes) a word by its index in place of one.
+template <typename PT, typename XP, typename R = typename PT::real>
+TJ_DEV void load_state(const PT& P, const XP& X, long long nt, long long g, const int* refl,
                                   CellT<R>& c)
 {
     #pragma unroll UnrollM<PT>::n
@@ -225,8 +227,8 @@ TJ_DEV void load_prims(const PT& P, const R* X, long long nt, long long g, const
     if (P.nmix) c.lam = X[P.S_LAM * nt + g];
 }
 
-template <typename PT, typename R = typename PT::real>
-TJ_DEV void store_state(const PT& P, R* X, long long nt, long long g, const CellT<R>& c)
+template <typename PT, typename XP, typename R = typename PT::real>
+TJ_DEV void store_state(const PT& P, const XP& X, long long nt, long long g, const CellT<R>& c)
 {
     #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
@@ -368,8 +370,8 @@ TJ_DEV void store_prim_face(const PT& P, R* F, long long nt, long long g, const 
 // The closed face state of load_face from stored primitives: the closures
 // of the reconstruction, then the fields load_face leaves at zero, then the
 // reflect_odd sign of a boundary image.
-template <typename PT, typename R = typename PT::real>
-TJ_DEV void load_prim_face(const PT& P, const R* F, long long nt, long long g, int oddir, CellT<R>& c)
+template <typename PT, typename FP, typename R = typename PT::real>
+TJ_DEV void load_prim_face(const PT& P, const FP& F, long long nt, long long g, int oddir, CellT<R>& c)
 {
     int w = 0;
     #pragma unroll UnrollM<PT>::n
@@ -811,8 +813,8 @@ TJ_DEV void flux_combine(const PT& P, FluxV<R>& F, const FluxV<R>& FA, const Flu
 }
 
 // One face into the flux-word layout (nf faces per word).
-template <typename PT, typename R = typename PT::real>
-TJ_DEV void store_flux(const PT& P, R* FX, long long nf, long long f, const FluxV<R>& F, R Ss,
+template <typename PT, typename FP, typename R = typename PT::real>
+TJ_DEV void store_flux(const PT& P, const FP& FX, long long nf, long long f, const FluxV<R>& F, R Ss,
                                   const R* vstar)
 {
 #define FXS(w) FX[(long long)(w) * nf + f]
@@ -1279,18 +1281,18 @@ __device__ __forceinline__ void add_fluxes(const PT& P, const CellT<R>& U, CellT
 // The end of a stage of one cell whose accumulator holds every direction's
 // update: conservativeToPrimitive; second stage: the average and the
 // post-advance operators of main.cpp:145-187.
-template <typename PT, typename R = typename PT::real>
-__device__ __forceinline__ void finish_cell(const PT& P, const PathBufs<R>& b, CellT<R>& Yc, R* Y, long long g,
-                                            const DevDomain& D, int i, int finish, R dtdx_num)
+template <typename PT, typename YP, typename AP, typename R = typename PT::real>
+__device__ __forceinline__ void finish_cell(const PT& P, DevScalars* scal, bool last_box, CellT<R>& Yc, const YP& Y,
+                                            const AP& A, long long nt, long long g, const DevDomain& D, int i,
+                                            int finish, R dtdx_num)
 {
-    const long long nt = b.ntot;
     const int ce = c2p(P, Yc);
-    if (ce) set_status(b.scal, ce);
+    if (ce) set_status(scal, ce);
     if (finish) {
         const R p_stage = Yc.p;  // U2's pressure, before the average
         // U1 = U*0.5 + U2*0.5 over every carried component (hllc.cpp:705)
         CellT<R> A0;
-        load_state(P, b.A, nt, g, nullptr, A0);
+        load_state(P, A, nt, g, nullptr, A0);
         #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
             Yc.alpha[m] = mean(A0.alpha[m], Yc.alpha[m]);
@@ -1322,19 +1324,19 @@ __device__ __forceinline__ void finish_cell(const PT& P, const PathBufs<R>& b, C
             Yc.arl = mean(A0.arl, Yc.arl);
         }
         if (finish == 2) {  // advance() alone: the average only
-            store_state(P, b.A, nt, g, Yc);
+            store_state(P, A, nt, g, Yc);
             return;
         }
         if (P.reactive && P.nmix) {  // main.cpp:149-152
             const int re = reactive_cell(P, Yc, dtdx_num);
-            if (re) set_status(b.scal, re);
+            if (re) set_status(scal, re);
         }
         if (P.plastic) {
             int e;
             if constexpr (sizeof(R) == 4) e = plastic_cell_proj64(P, Yc);
             else e = plastic_cell(P, Yc);
             c2p(P, Yc);
-            if (e) set_status(b.scal, e);
+            if (e) set_status(scal, e);
         }
         if (P.radial) {
             // the stress the reference's U1 holds here: fresh from the
@@ -1354,13 +1356,13 @@ __device__ __forceinline__ void finish_cell(const PT& P, const PathBufs<R>& b, C
                 }
             radial_source(P, Yc, sg, i, D.dx[0], dtdx_num);
             const int rc = c2p(P, Yc);  // geometricSourceTerm (radial.cpp:50)
-            if (rc) set_status(b.scal, rc);
+            if (rc) set_status(scal, rc);
         }
         if (P.solid) cleanup_v_cell(P, Yc);
         int e = cleanup_alpha(P, Yc.alpha);
-        if (e) set_status(b.scal, e);
-        if (b.cell_box[g] == D.nbox - 1 && cell_has_nan(P, Yc)) atomicOr(&b.scal->nan_flag, 1);
-        store_state(P, b.A, nt, g, Yc);
+        if (e) set_status(scal, e);
+        if (last_box && cell_has_nan(P, Yc)) atomicOr(&scal->nan_flag, 1);
+        store_state(P, A, nt, g, Yc);
         return;
     }
     store_state(P, Y, nt, g, Yc);
@@ -1368,18 +1370,17 @@ __device__ __forceinline__ void finish_cell(const PT& P, const PathBufs<R>& b, C
 
 // Update of cell g along d alone, from the accumulator in Y (the stage input
 // for the first direction), with the stage's end after the last direction.
-template <typename PT, typename FA, typename R = typename PT::real>
-__device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, const R* __restrict__ X, R* Y,
-                                            long long g, const DevDomain& D, int i, int d, int first, int last,
-                                            int finish, R dtdx_num, const FA& FXW)
+template <typename PT, typename XP, typename YP, typename AP, typename FA, typename R = typename PT::real>
+__device__ __forceinline__ void update_cell(const PT& P, DevScalars* scal, bool last_box, const XP& X, const YP& Y,
+                                            const AP& A, long long nt, long long g, const DevDomain& D, int i, int d,
+                                            int first, int last, int finish, R dtdx_num, const FA& FXW)
 {
-    const long long nt = b.ntot;
     CellT<R> U, Yc;
     load_state(P, X, nt, g, nullptr, U);
     if (first) Yc = U;
     else load_state(P, Y, nt, g, nullptr, Yc);
     add_fluxes(P, U, Yc, quot(dtdx_num, (R)D.dx[d]), FXW);
-    if (last) finish_cell(P, b, Yc, Y, g, D, i, finish, dtdx_num);
+    if (last) finish_cell(P, scal, last_box, Yc, Y, A, nt, g, D, i, finish, dtdx_num);
     else store_state(P, Y, nt, g, Yc);
 }
 
@@ -1412,7 +1413,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
                 add_fluxes(P, U, Yc, quot(dtdx_num, (R)D.dx[d]), fx);
                 FX += P.NX * b.nftot[d];
             }
-        finish_cell(P, b, Yc, Y, g, D, i, finish, dtdx_num);
+        finish_cell(P, b.scal, b.cell_box[g] == D.nbox - 1, Yc, Y, b.A, nt, g, D, i, finish, dtdx_num);
     }
 }
 
@@ -1434,7 +1435,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
         int o[3] = {0, 0, 0};
         o[d] = 1;
         const FacePairGlobal<R> fx{b.FX, nf, face_index(D, d, i, j, k), face_index(D, d, i + o[0], j + o[1], k + o[2])};
-        update_cell(P, b, X, Y, g, D, i, d, first, last, finish, dtdx_num, fx);
+        update_cell(P, b.scal, b.cell_box[g] == D.nbox - 1, X, Y, b.A, nt, g, D, i, d, first, last, finish, dtdx_num, fx);
     }
 }
 

@@ -74,23 +74,41 @@ inline int path_dir_any(const Base& P, const PathBufs<typename Base::real>& b, c
 }
 
 template <class Base, int K>
+inline int path_faces_kind(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X, int d,
+                           cudaStream_t st, Prof* pr)
+{
+#define TJ_FACES(MC, DC) path_faces<WithM<Base, MC, K>, DC>(WithM<Base, MC, K>(P), b, X, d, st, pr)
+    switch (P.M * 4 + d) {
+        case 4: return TJ_FACES(1, 0);
+        case 5: return TJ_FACES(1, 1);
+        case 6: return TJ_FACES(1, 2);
+        case 8: return TJ_FACES(2, 0);
+        case 9: return TJ_FACES(2, 1);
+        case 10: return TJ_FACES(2, 2);
+        default: return path_faces<Base, -1>(P, b, X, d, st, pr);
+    }
+#undef TJ_FACES
+}
+
+template <class Base>
+inline int path_faces_any(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X, int d,
+                          cudaStream_t st, Prof* pr)
+{
+    if constexpr (kHasKind<Base, KIND_FLUID>)
+        if (param_kind(P) == KIND_FLUID) return path_faces_kind<Base, KIND_FLUID>(P, b, X, d, st, pr);
+    if constexpr (kHasKind<Base, KIND_PLASTIC>)
+        if (param_kind(P) == KIND_PLASTIC) return path_faces_kind<Base, KIND_PLASTIC>(P, b, X, d, st, pr);
+    return path_faces_kind<Base, KIND_ANY>(P, b, X, d, st, pr);
+}
+
+template <class Base, int K>
 inline int path_stage_kind(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
                            typename Base::real* Y, int finish, cudaStream_t st, Prof* pr)
 {
     int n = 0;
     PathBufs<typename Base::real> bd = b;
     for (int d = 0; d < P.dim; ++d) {
-#define TJ_FACES(MC, DC) path_faces<WithM<Base, MC, K>, DC>(WithM<Base, MC, K>(P), bd, X, d, st, pr)
-        switch (P.M * 4 + d) {
-            case 4: n += TJ_FACES(1, 0); break;
-            case 5: n += TJ_FACES(1, 1); break;
-            case 6: n += TJ_FACES(1, 2); break;
-            case 8: n += TJ_FACES(2, 0); break;
-            case 9: n += TJ_FACES(2, 1); break;
-            case 10: n += TJ_FACES(2, 2); break;
-            default: n += path_faces<Base, -1>(P, bd, X, d, st, pr);
-        }
-#undef TJ_FACES
+        n += path_faces_kind<Base, K>(P, bd, X, d, st, pr);
         bd.FX += P.NX * b.nftot[d];
     }
     if (P.M == 1) return n + path_update(WithM<Base, 1, K>(P), b, X, Y, finish, st, pr);
