@@ -1,15 +1,18 @@
 // FP64 reference-faithful kernels of Tenjin's per-timestep update.
 //
 // One RK stage (HLLCadvance, hllc.cpp:579-695) is, per direction d:
-//   k_recon   per cell : MUSCL (hllc.cpp:541-575), BVD-THINC (thinc.cpp:67-208),
+//   k_thinc   per cell and material: the cell's THINC candidates (thinc.cpp:67-147)
+//   k_recon   per cell : MUSCL (hllc.cpp:541-575), the BVD choice (thinc.cpp:148-208),
 //                        cleanUpAlpha of the reconstructed states (hllc.cpp:628-629),
 //                        primitiveToConservative + getSoundSpeed (634-638)
 //   k_flux    per face : HLLC (hllc.cpp:384-487) or 5-wave (133-380)
-//   k_update  per cell : update (hllc.cpp:493-523); after the last direction
+// and, with every direction's fluxes, once:
+//   k_update_all per cell : update (hllc.cpp:493-523) in the order x, y, z;
 //                        conservativeToPrimitive (689), and at the end of the
 //                        second stage the RK2 average (705), plasticUpdate,
 //                        cleanUpV, cleanUpAlpha and the NaN check
 //                        (main.cpp:145-187).
+// The adjoint's and the tangent's runs update direction by direction (k_update).
 // Ghost cells are never stored: a read outside a domain maps the index back
 // (foextrap: nearest cell; reflect: mirror, negating the normal velocity and
 // momentum), which is what the reference's FillDomainBoundary and
@@ -24,8 +27,6 @@
 namespace tj {
 
 static constexpr int kThreads = 256;
-
-
 
 __global__ void k_dt_finalize(DevParams P, DevScalars* s, int clamp)
 {

@@ -9,7 +9,7 @@ template <typename R>
 struct PathBufs {
     R *A, *B, *C;        // state: U^n (and result), stage-1 output, stage-2 partial
     R *UL, *UR;          // reconstructed face states, one per cell
-    R* FX;               // face fluxes of the current direction
+    R* FX;               // face fluxes, one direction after the other
     R *ulstar, *urstar;  // THINC scratch (alpha of the reference's ULStar / URStar)
     R* gstar[3];         // ULStar ghost alpha at box hi+1 faces, per direction
     int* cell_box;            // domain-local box index of each cell

@@ -26,6 +26,7 @@ struct SeedWords {
     const double* X;
     long long n, at;
     int seed;
+    __device__ __forceinline__ SeedWords operator+(long long) const { return *this; }  // at the cell already
     __device__ __forceinline__ Dual operator[](long long w) const
     {
         return Dual(X[w * n + at], w == seed ? 1.0 : 0.0);
@@ -45,6 +46,7 @@ struct DotWords {
             if (lo != 0.0) sum += lo * x.d;
         }
     };
+    __device__ __forceinline__ DotWords operator+(long long) const { return *this; }
     __device__ __forceinline__ Word operator[](long long w) const { return {lam((int)w), sum}; }
 };
 // The second stage's end reads U^n from the words it then replaces.
@@ -63,6 +65,7 @@ struct SeedDotWords {
             if (lo != 0.0) sum += lo * y.d;
         }
     };
+    __device__ __forceinline__ SeedDotWords operator+(long long) const { return *this; }
     __device__ __forceinline__ Word operator[](long long w) const { return {in[w], lam((int)w), sum}; }
 };
 // Flux words of a cell's two faces; the seed is on face 0.

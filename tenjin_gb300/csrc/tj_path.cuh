@@ -7,15 +7,18 @@
 // binary64 (plastic_cell_proj64); everything else is the same code.
 //
 // One RK stage (HLLCadvance, hllc.cpp:579-695) is, per direction d:
-//   k_recon   per cell : MUSCL (hllc.cpp:541-575), BVD-THINC (thinc.cpp:67-208),
+//   k_thinc   per cell and material: the cell's THINC candidates (thinc.cpp:67-147)
+//   k_recon   per cell : MUSCL (hllc.cpp:541-575), the BVD choice (thinc.cpp:148-208),
 //                        cleanUpAlpha of the reconstructed states (hllc.cpp:628-629),
 //                        primitiveToConservative + getSoundSpeed (634-638)
 //   k_flux    per face : HLLC (hllc.cpp:384-487) or 5-wave (133-380)
-//   k_update  per cell : update (hllc.cpp:493-523); after the last direction
+// and, with every direction's fluxes, once:
+//   k_update_all per cell : update (hllc.cpp:493-523) in the order x, y, z;
 //                        conservativeToPrimitive (689), and at the end of the
 //                        second stage the RK2 average (705), plasticUpdate,
 //                        cleanUpV, cleanUpAlpha and the NaN check
 //                        (main.cpp:145-187).
+// The adjoint's and the tangent's runs update direction by direction (k_update).
 // Ghost cells are never stored: a read outside a domain maps the index back
 // (foextrap: nearest cell; reflect: mirror, negating the normal velocity and
 // momentum), which is what the reference's FillDomainBoundary and
@@ -36,6 +39,22 @@ namespace tj {
 // than four, spills included: bubble 256^2, 20 steps 21.6 / 17.2 / 18.0 ms and
 // copper 40^3, 10 steps 24.6 / 19.5 / 20.3 ms with 4 / 8 / 12 blocks of 64.
 constexpr int kBlocks64 = 8;
+
+// Blocks of the per-direction kernels and how many an SM is to hold. binary32:
+// blocks of 128 (finer waves than 256) with 128 registers; the one-material
+// solids' reconstruction and fluxes fit in 102, a fifth block (copper 128^3,
+// 5 steps: 15.46 ms with two blocks of 256, 14.97 with three and 80 registers,
+// 14.83 so).
+template <class PT>
+constexpr bool kPath32 = sizeof(typename PT::real) == 4;
+template <class PT>
+constexpr int kPathThreads = kPath32<PT> ? 128 : 64;
+template <class PT>
+constexpr int kUpdateBlocks = kPath32<PT> ? 4 : kBlocks64;
+template <class PT>
+constexpr int kFaceBlocks = kPath32<PT> ? 4 : kBlocks64;
+template <int K>
+constexpr int kFaceBlocks<WithM<DevParams32, 1, K>> = 5;
 
 // Error-free accumulation of b into the pair (hi, lo) (binary32 energy).
 __device__ __forceinline__ void dd_add32(float& hi, float& lo, float b)
@@ -149,6 +168,10 @@ __device__ __forceinline__ long long face_index(const DevDomain& D, int d, int i
     return D.foff[d] + i + (long long)nf0 * (j + (long long)nf1 * k);
 }
 
+// The words of a cell are addressed from a pointer to its first one: a word's
+// offset from there is the same for every thread, so less is computed and held
+// per thread (spills of the binary32 stage's end 300 -> 4 bytes; copper 128^3,
+// 5 steps 14.9 -> 13.5 ms).
 // Carried-state load with the reflect_odd sign applied. X here and the arrays of
 // the other accessors below are pointers to the state's words, or what reads
 // (takes) a word by its index in place of one.
@@ -156,40 +179,41 @@ template <typename PT, typename XP, typename R = typename PT::real>
 TJ_DEV void load_state(const PT& P, const XP& X, long long nt, long long g, const int* refl,
                                   CellT<R>& c)
 {
+    const auto Xg = X + g;
     #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
-        c.alpha[m] = X[(P.S_ALPHA + m) * nt + g];
-        c.arho[m] = X[(P.S_ARHO + m) * nt + g];
-        c.rhok[m] = X[(P.S_RHOK + m) * nt + g];
+        c.alpha[m] = Xg[(P.S_ALPHA + m) * nt];
+        c.arho[m] = Xg[(P.S_ARHO + m) * nt];
+        c.rhok[m] = Xg[(P.S_RHOK + m) * nt];
     }
-    c.rho = X[P.S_RHO * nt + g];
+    c.rho = Xg[P.S_RHO * nt];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        R u = X[(P.S_VEL + r) * nt + g], ru = X[(P.S_RHOU + r) * nt + g];
+        R u = Xg[(P.S_VEL + r) * nt], ru = Xg[(P.S_RHOU + r) * nt];
         if (refl && refl[r]) { u = -u; ru = -ru; }
         c.vel[r] = u;
         c.rhou[r] = ru;
     }
-    c.E = X[P.S_E * nt + g];
-    if constexpr (sizeof(R) == 4) c.Elo = X[P.S_ELO * nt + g];
-    c.p = X[P.S_P * nt + g];
+    c.E = Xg[P.S_E * nt];
+    if constexpr (sizeof(R) == 4) c.Elo = Xg[P.S_ELO * nt];
+    c.p = Xg[P.S_P * nt];
     c.hj2 = R(0.0);
     if (P.solid) {
 #pragma unroll
-        for (int q = 0; q < 9; ++q) c.V[q] = X[(P.S_V + q) * nt + g];
-        c.hj2 = X[P.S_HJ2 * nt + g];
+        for (int q = 0; q < 9; ++q) c.V[q] = Xg[(P.S_V + q) * nt];
+        c.hj2 = Xg[P.S_HJ2 * nt];
     }
     if (P.plastic)
         #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
-            c.eps[m] = X[(P.S_EPS + m) * nt + g];
-            c.are[m] = X[(P.S_ARE + m) * nt + g];
+            c.eps[m] = Xg[(P.S_EPS + m) * nt];
+            c.are[m] = Xg[(P.S_ARE + m) * nt];
         }
     if (P.nmix) {
-        c.rm0 = X[P.S_RMIX * nt + g];
-        c.rm1 = X[(P.S_RMIX + 1) * nt + g];
-        c.lam = X[P.S_LAM * nt + g];
-        c.arl = X[P.S_ARL * nt + g];
+        c.rm0 = Xg[P.S_RMIX * nt];
+        c.rm1 = Xg[(P.S_RMIX + 1) * nt];
+        c.lam = Xg[P.S_LAM * nt];
+        c.arl = Xg[P.S_ARL * nt];
     }
 }
 
@@ -200,67 +224,69 @@ TJ_DEV void load_state(const PT& P, const XP& X, long long nt, long long g, cons
 template <typename PT, typename R = typename PT::real>
 TJ_DEV void load_prims(const PT& P, const R* X, long long nt, long long g, const int* refl, CellT<R>& c)
 {
+    const auto Xg = X + g;
     #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
-        c.alpha[m] = X[(P.S_ALPHA + m) * nt + g];
-        c.rhok[m] = X[(P.S_RHOK + m) * nt + g];
+        c.alpha[m] = Xg[(P.S_ALPHA + m) * nt];
+        c.rhok[m] = Xg[(P.S_RHOK + m) * nt];
     }
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        R u = X[(P.S_VEL + r) * nt + g];
+        R u = Xg[(P.S_VEL + r) * nt];
         if (refl && refl[r]) u = -u;
         c.vel[r] = u;
     }
-    c.p = X[P.S_P * nt + g];
+    c.p = Xg[P.S_P * nt];
     c.hj2 = R(0.0);
     if (P.solid) {
 #pragma unroll
-        for (int q = 0; q < 9; ++q) c.V[q] = X[(P.S_V + q) * nt + g];
-        c.hj2 = X[P.S_HJ2 * nt + g];
+        for (int q = 0; q < 9; ++q) c.V[q] = Xg[(P.S_V + q) * nt];
+        c.hj2 = Xg[P.S_HJ2 * nt];
     }
     if (P.plastic)
         #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
-            c.eps[m] = X[(P.S_EPS + m) * nt + g];
-            c.are[m] = X[(P.S_ARE + m) * nt + g];
+            c.eps[m] = Xg[(P.S_EPS + m) * nt];
+            c.are[m] = Xg[(P.S_ARE + m) * nt];
         }
-    if (P.nmix) c.lam = X[P.S_LAM * nt + g];
+    if (P.nmix) c.lam = Xg[P.S_LAM * nt];
 }
 
 template <typename PT, typename XP, typename R = typename PT::real>
 TJ_DEV void store_state(const PT& P, const XP& X, long long nt, long long g, const CellT<R>& c)
 {
+    const auto Xg = X + g;
     #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
-        X[(P.S_ALPHA + m) * nt + g] = c.alpha[m];
-        X[(P.S_ARHO + m) * nt + g] = c.arho[m];
-        X[(P.S_RHOK + m) * nt + g] = c.rhok[m];
+        Xg[(P.S_ALPHA + m) * nt] = c.alpha[m];
+        Xg[(P.S_ARHO + m) * nt] = c.arho[m];
+        Xg[(P.S_RHOK + m) * nt] = c.rhok[m];
     }
-    X[P.S_RHO * nt + g] = c.rho;
+    Xg[P.S_RHO * nt] = c.rho;
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        X[(P.S_VEL + r) * nt + g] = c.vel[r];
-        X[(P.S_RHOU + r) * nt + g] = c.rhou[r];
+        Xg[(P.S_VEL + r) * nt] = c.vel[r];
+        Xg[(P.S_RHOU + r) * nt] = c.rhou[r];
     }
-    X[P.S_E * nt + g] = c.E;
-    if constexpr (sizeof(R) == 4) X[P.S_ELO * nt + g] = c.Elo;
-    X[P.S_P * nt + g] = c.p;
+    Xg[P.S_E * nt] = c.E;
+    if constexpr (sizeof(R) == 4) Xg[P.S_ELO * nt] = c.Elo;
+    Xg[P.S_P * nt] = c.p;
     if (P.solid) {
 #pragma unroll
-        for (int q = 0; q < 9; ++q) X[(P.S_V + q) * nt + g] = c.V[q];
-        X[P.S_HJ2 * nt + g] = c.hj2;
+        for (int q = 0; q < 9; ++q) Xg[(P.S_V + q) * nt] = c.V[q];
+        Xg[P.S_HJ2 * nt] = c.hj2;
     }
     if (P.plastic)
         #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
-            X[(P.S_EPS + m) * nt + g] = c.eps[m];
-            X[(P.S_ARE + m) * nt + g] = c.are[m];
+            Xg[(P.S_EPS + m) * nt] = c.eps[m];
+            Xg[(P.S_ARE + m) * nt] = c.are[m];
         }
     if (P.nmix) {
-        X[P.S_RMIX * nt + g] = c.rm0;
-        X[(P.S_RMIX + 1) * nt + g] = c.rm1;
-        X[P.S_LAM * nt + g] = c.lam;
-        X[P.S_ARL * nt + g] = c.arl;
+        Xg[P.S_RMIX * nt] = c.rm0;
+        Xg[(P.S_RMIX + 1) * nt] = c.rm1;
+        Xg[P.S_LAM * nt] = c.lam;
+        Xg[P.S_ARL * nt] = c.arl;
     }
 }
 
@@ -349,22 +375,23 @@ __device__ __forceinline__ bool compact_faces(const PT& P)
 template <typename PT, typename R = typename PT::real>
 TJ_DEV void store_prim_face(const PT& P, R* F, long long nt, long long g, const CellT<R>& c)
 {
+    const auto Fg = F + g;
     int w = 0;
     #pragma unroll UnrollM<PT>::n
-    for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = c.alpha[m];
+    for (int m = 0; m < P.M; ++m) Fg[(long long)(w++) * nt] = c.alpha[m];
     #pragma unroll UnrollM<PT>::n
-    for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = c.rhok[m];
+    for (int m = 0; m < P.M; ++m) Fg[(long long)(w++) * nt] = c.rhok[m];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) F[(long long)(w++) * nt + g] = c.vel[r];
-    F[(long long)(w++) * nt + g] = c.p;
+    for (int r = 0; r < 3; ++r) Fg[(long long)(w++) * nt] = c.vel[r];
+    Fg[(long long)(w++) * nt] = c.p;
     if (P.solid) {
 #pragma unroll
-        for (int q = 0; q < 9; ++q) F[(long long)(w++) * nt + g] = c.V[q];
-        if (!P.any_solid) F[(long long)(w++) * nt + g] = c.hj2;  // getHenckyJ2 does not run: the cell's own
+        for (int q = 0; q < 9; ++q) Fg[(long long)(w++) * nt] = c.V[q];
+        if (!P.any_solid) Fg[(long long)(w++) * nt] = c.hj2;  // getHenckyJ2 does not run: the cell's own
     }
     if (P.plastic)  // epsilon of a solid closes alphaRhoEps; a fluid's alphaRhoEps is the cell's own
         #pragma unroll UnrollM<PT>::n
-        for (int m = 0; m < P.M; ++m) F[(long long)(w++) * nt + g] = phase_of(P, m) == TJ_PHASE_SOLID ? c.eps[m] : c.are[m];
+        for (int m = 0; m < P.M; ++m) Fg[(long long)(w++) * nt] = phase_of(P, m) == TJ_PHASE_SOLID ? c.eps[m] : c.are[m];
 }
 
 // The closed face state of load_face from stored primitives: the closures
@@ -373,24 +400,25 @@ TJ_DEV void store_prim_face(const PT& P, R* F, long long nt, long long g, const 
 template <typename PT, typename FP, typename R = typename PT::real>
 TJ_DEV void load_prim_face(const PT& P, const FP& F, long long nt, long long g, int oddir, CellT<R>& c)
 {
+    const auto Fg = F + g;
     int w = 0;
     #pragma unroll UnrollM<PT>::n
-    for (int m = 0; m < P.M; ++m) c.alpha[m] = F[(long long)(w++) * nt + g];
+    for (int m = 0; m < P.M; ++m) c.alpha[m] = Fg[(long long)(w++) * nt];
     #pragma unroll UnrollM<PT>::n
-    for (int m = 0; m < P.M; ++m) c.rhok[m] = F[(long long)(w++) * nt + g];
+    for (int m = 0; m < P.M; ++m) c.rhok[m] = Fg[(long long)(w++) * nt];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) c.vel[r] = F[(long long)(w++) * nt + g];
-    c.p = F[(long long)(w++) * nt + g];
+    for (int r = 0; r < 3; ++r) c.vel[r] = Fg[(long long)(w++) * nt];
+    c.p = Fg[(long long)(w++) * nt];
     c.hj2 = R(0.0);
     if (P.solid) {
 #pragma unroll
-        for (int q = 0; q < 9; ++q) c.V[q] = F[(long long)(w++) * nt + g];
-        if (!P.any_solid) c.hj2 = F[(long long)(w++) * nt + g];
+        for (int q = 0; q < 9; ++q) c.V[q] = Fg[(long long)(w++) * nt];
+        if (!P.any_solid) c.hj2 = Fg[(long long)(w++) * nt];
     }
     if (P.plastic)
         #pragma unroll UnrollM<PT>::n
         for (int m = 0; m < P.M; ++m) {
-            const R v = F[(long long)(w++) * nt + g];
+            const R v = Fg[(long long)(w++) * nt];
             if (phase_of(P, m) == TJ_PHASE_SOLID) c.eps[m] = v;
             else c.are[m] = v;
         }
@@ -518,7 +546,7 @@ TJ_DEV bool thinc_cand(const PT& P, const DevDomain& D, const R* X, long long nt
 // times, in one thread's serial chain (adjoint 96^2, every cell mixed: k_recon
 // 205 us a direction).
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
+__global__ void __launch_bounds__(kPathThreads<PT>, kFaceBlocks<PT>)
     k_thinc(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int* __restrict__ mixed, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
@@ -546,7 +574,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
 // ---------------------------------------------------------------------------
 // DC >= 0: the direction as a compile-time constant (d is then ignored).
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
+__global__ void __launch_bounds__(kPathThreads<PT>, kFaceBlocks<PT>)
     k_recon(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
@@ -817,7 +845,8 @@ template <typename PT, typename FP, typename R = typename PT::real>
 TJ_DEV void store_flux(const PT& P, const FP& FX, long long nf, long long f, const FluxV<R>& F, R Ss,
                                   const R* vstar)
 {
-#define FXS(w) FX[(long long)(w) * nf + f]
+    const auto FXf = FX + f;
+#define FXS(w) FXf[(long long)(w) * nf]
     #pragma unroll UnrollM<PT>::n
     for (int m = 0; m < P.M; ++m) {
         FXS(P.X_ALPHA + m) = F.alpha[m];
@@ -955,7 +984,7 @@ TJ_DEV int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& Rc, int d, 
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
+__global__ void __launch_bounds__(kPathThreads<PT>, kFaceBlocks<PT>)
     k_flux(PT P, PathBufs<typename PT::real> b, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
@@ -1244,9 +1273,9 @@ TJ_DEV void radial_source(const PT& P, CellT<R>& c, const R* sg, int i, double d
 // face below the cell along d, 1: the face above).
 template <typename R>
 struct FacePairGlobal {
-    const R* FX;
-    long long nf, f0, f1;
-    __device__ __forceinline__ R operator()(int w, int s) const { return FX[(long long)w * nf + (s ? f1 : f0)]; }
+    const R *F0, *F1;  // at the faces
+    long long nf;
+    __device__ __forceinline__ R operator()(int w, int s) const { return (s ? F1 : F0)[(long long)w * nf]; }
 };
 
 // Adds the update along d of one cell from the fluxes of its two faces
@@ -1389,8 +1418,9 @@ __device__ __forceinline__ void update_cell(const PT& P, DevScalars* scal, bool 
 // stage's end. One pass over the state instead of one per direction that
 // carries the accumulator through memory: the words a copper cell moves a
 // stage fall from about 200 to 103, the same arithmetic in the same order.
-template <typename PT, typename R = typename PT::real>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
+// Two instances: the first stage's has no code for the second's end (FIN).
+template <typename PT, bool FIN, typename R = typename PT::real>
+__global__ void __launch_bounds__(kPathThreads<PT>, kUpdateBlocks<PT>)
     k_update_all(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, R* Y, int finish)
 {
     if (b.scal->done) return;
@@ -1408,17 +1438,17 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
 #pragma unroll
         for (int d = 0; d < 3; ++d)
             if (d < P.dim) {
-                const FacePairGlobal<R> fx{FX, b.nftot[d], face_index(D, d, i, j, k),
-                                           face_index(D, d, i + (d == 0), j + (d == 1), k + (d == 2))};
+                const FacePairGlobal<R> fx{FX + face_index(D, d, i, j, k),
+                                           FX + face_index(D, d, i + (d == 0), j + (d == 1), k + (d == 2)), b.nftot[d]};
                 add_fluxes(P, U, Yc, quot(dtdx_num, (R)D.dx[d]), fx);
                 FX += P.NX * b.nftot[d];
             }
-        finish_cell(P, b.scal, b.cell_box[g] == D.nbox - 1, Yc, Y, b.A, nt, g, D, i, finish, dtdx_num);
+        finish_cell(P, b.scal, b.cell_box[g] == D.nbox - 1, Yc, Y, b.A, nt, g, D, i, FIN ? finish : 0, dtdx_num);
     }
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 : kBlocks64)
+__global__ void __launch_bounds__(kPathThreads<PT>, kUpdateBlocks<PT>)
     k_update(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, R* Y, int dyn_d, int first, int last,
              int finish)
 {
@@ -1434,7 +1464,7 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? 256 : 64, sizeof(R) == 4 ? 2 
         split3(l, D.n[0], D.n[1], i, j, k);
         int o[3] = {0, 0, 0};
         o[d] = 1;
-        const FacePairGlobal<R> fx{b.FX, nf, face_index(D, d, i, j, k), face_index(D, d, i + o[0], j + o[1], k + o[2])};
+        const FacePairGlobal<R> fx{b.FX + face_index(D, d, i, j, k), b.FX + face_index(D, d, i + o[0], j + o[1], k + o[2]), nf};
         update_cell(P, b.scal, b.cell_box[g] == D.nbox - 1, X, Y, b.A, nt, g, D, i, d, first, last, finish, dtdx_num, fx);
     }
 }

@@ -24,12 +24,10 @@
 namespace tj {
 
 namespace {
-// binary64 kernels keep eight warps an SM (up to 255 registers): blocks of two
-// warps balance best; binary32 ones hold two blocks of eight.
 template <class PT>
 inline LaunchShape path_shape(long long n)
 {
-    return launch_shape(n, sizeof(typename PT::real) == 4 ? 256 : 64);
+    return launch_shape(n, kPathThreads<PT>);
 }
 }  // namespace
 
@@ -74,7 +72,8 @@ int path_update(const PT& P, const PathBufs<typename PT::real>& b, const typenam
     const char* nu = sizeof(typename PT::real) == 8 ? "tj_update_fp64" : "tj_update_fp32";
     const LaunchShape cells = path_shape<PT>(b.ntot);
     if (pr) pr->begin(nu, st);
-    k_update_all<PT><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, finish);
+    if (finish) k_update_all<PT, true><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, finish);
+    else k_update_all<PT, false><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, 0);
     if (pr) pr->end(nu, st);
     return 1;
 }
