@@ -25,6 +25,7 @@ struct PathBufs {
     // own THINC candidate, 2 a value of the THINC scratch
     R* rec = nullptr;
     int* rec_code = nullptr;
+    int overlap = 0;  // the kernel is launched to overlap the one before it (tj_path_inst.cu)
 };
 using Fp64Bufs = PathBufs<double>;
 

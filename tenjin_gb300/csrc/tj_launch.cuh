@@ -1,5 +1,5 @@
-// Launches of the fused kernels, each of which starts while the one before it
-// drains, and the scalars of a step, handled inside them.
+// Launches of kernels each of which starts while the one before it drains, and
+// the scalars of a step, handled inside the fused kernels.
 //
 // A step of a small grid is two kernels of a few microseconds; the gap between
 // two of them is mostly the next one's launch. Launched with programmatic stream
@@ -10,11 +10,6 @@
 // plain stream order. Measured, with the scalars' own launches folded in:
 // 333^2 cells in binary32, 40 steps in graphs 1.35 -> 1.26 ms, 1024^2 7.02 ->
 // 6.96 ms; 128 boxes in 3-D, 30 steps 36.3 -> 34.7 ms.
-//
-// Not for the per-direction kernels: their graphs lose by it (Sod, 1000 cells,
-// 100 steps: 6.8 -> 7.8 ms), and outside of graphs the two statements cost the
-// long kernels what they save the short ones (copper 40^3, 10 steps 14.05 ->
-// 14.5 ms; 64^2 cells driven operator by operator 1.70 -> 1.63 ms).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -30,6 +30,7 @@
 
 #include "tj_device.cuh"
 #include "tj_fp64.cuh"
+#include "tj_launch.cuh"
 
 namespace tj {
 
@@ -55,6 +56,16 @@ template <class PT>
 constexpr int kFaceBlocks = kPath32<PT> ? 4 : kBlocks64;
 template <int K>
 constexpr int kFaceBlocks<WithM<DevParams32, 1, K>> = 5;
+
+// The first statement of every per-direction kernel (tj_launch.cuh).
+template <typename R>
+__device__ __forceinline__ void overlap_start(const PathBufs<R>& b)
+{
+    if (b.overlap) {
+        grid_wait();
+        grid_go();
+    }
+}
 
 // Error-free accumulation of b into the pair (hi, lo) (binary32 energy).
 __device__ __forceinline__ void dd_add32(float& hi, float& lo, float b)
@@ -550,6 +561,7 @@ __global__ void __launch_bounds__(kPathThreads<PT>, kFaceBlocks<PT>)
     k_thinc(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int* __restrict__ mixed, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
+    overlap_start(b);
     if (b.scal->done) return;
     const long long nt = b.ntot, all = nt * P.M;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < all; e += (long long)gridDim.x * blockDim.x) {
@@ -578,6 +590,7 @@ __global__ void __launch_bounds__(kPathThreads<PT>, kFaceBlocks<PT>)
     k_recon(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
+    overlap_start(b);
     if (b.scal->done) return;
     const long long nt = b.ntot;
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nt; g += (long long)gridDim.x * blockDim.x) {
@@ -988,6 +1001,7 @@ __global__ void __launch_bounds__(kPathThreads<PT>, kFaceBlocks<PT>)
     k_flux(PT P, PathBufs<typename PT::real> b, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
+    overlap_start(b);
     if (b.scal->done) return;
     const long long nt = b.ntot, nf = b.nftot[d];
     for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < nf; f += (long long)gridDim.x * blockDim.x) {
@@ -1423,6 +1437,7 @@ template <typename PT, bool FIN, typename R = typename PT::real>
 __global__ void __launch_bounds__(kPathThreads<PT>, kUpdateBlocks<PT>)
     k_update_all(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, R* Y, int finish)
 {
+    overlap_start(b);
     if (b.scal->done) return;
     const long long nt = b.ntot;
     const R dtdx_num = b.scal->dt;
@@ -1453,6 +1468,7 @@ __global__ void __launch_bounds__(kPathThreads<PT>, kUpdateBlocks<PT>)
              int finish)
 {
     const int d = DC >= 0 ? DC : dyn_d;
+    overlap_start(b);
     if (b.scal->done) return;
     const long long nt = b.ntot, nf = b.nftot[d];
     const R dtdx_num = b.scal->dt;
@@ -1475,6 +1491,7 @@ __global__ void __launch_bounds__(kPathThreads<PT>, kUpdateBlocks<PT>)
 template <typename PT, typename R = typename PT::real>
 __global__ void k_cfl(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X)
 {
+    overlap_start(b);
     if (b.scal->done) return;
     const long long nt = b.ntot;
     R mn = R(sizeof(R) == 4 ? 3.0e38 : 1.79769313486231570815e+308);

@@ -29,6 +29,24 @@ inline LaunchShape path_shape(long long n)
 {
     return launch_shape(n, kPathThreads<PT>);
 }
+
+// kernel(P, b, args...), overlapping the launch before it (tj_launch.cuh) where
+// the grid leaves each SM room: up to the four blocks an SM that launch_shape
+// halves the blocks for (64^2 cells driven operator by operator 1.70 -> 1.62
+// ms). With more, the blocks of the next kernel take the SMs that drain first
+// and are dealt unevenly (copper 40^3 in binary64, 1000 blocks, 10 steps: 14.05
+// ms, overlapped 14.5). Not while the stream is captured, where plain edges are
+// the faster ones (Sod, 1000 cells, 100 steps in binary64: 6.8 ms, overlapped
+// 7.8), nor around single kernels' events (pr).
+template <class PT, class... Params, class... Args>
+inline void path_launch(void (*kernel)(PT, PathBufs<typename PT::real>, Params...), LaunchShape s, cudaStream_t st,
+                        Prof* pr, const PT& P, PathBufs<typename PT::real> b, const Args&... args)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    b.overlap = !pr && s.blocks <= 152 * 4 && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+                capture == cudaStreamCaptureStatusNone;
+    launch(kernel, dim3(s.blocks), s.threads, 0, st, b.overlap, P, b, args...);
+}
 }  // namespace
 
 template <class PT, int DC>
@@ -42,12 +60,12 @@ int path_faces(const PT& P, const PathBufs<typename PT::real>& b, const typename
     if (pr) pr->begin(nr, st);
     if (P.thinc) {
         const LaunchShape sh = path_shape<PT>(b.ntot * P.M);
-        k_thinc<PT, DC><<<sh.blocks, sh.threads, 0, st>>>(P, b, X, reinterpret_cast<int*>(b.FX), d);
+        path_launch(k_thinc<PT, DC>, sh, st, pr, P, b, X, reinterpret_cast<int*>(b.FX), d);
     }
-    k_recon<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, d);
+    path_launch(k_recon<PT, DC>, cells, st, pr, P, b, X, d);
     if (pr) pr->end(nr, st);
     if (pr) pr->begin(nf, st);
-    k_flux<PT, DC><<<faces.blocks, faces.threads, 0, st>>>(P, b, d);
+    path_launch(k_flux<PT, DC>, faces, st, pr, P, b, d);
     if (pr) pr->end(nf, st);
     return P.thinc ? 3 : 2;
 }
@@ -60,7 +78,7 @@ int path_dir(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     const LaunchShape cells = path_shape<PT>(b.ntot);
     const int n = path_faces<PT, DC>(P, b, X, d, st, pr);
     if (pr) pr->begin(nu, st);
-    k_update<PT, DC><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, d, first, last, finish);
+    path_launch(k_update<PT, DC>, cells, st, pr, P, b, X, Y, d, first, last, finish);
     if (pr) pr->end(nu, st);
     return n + 1;
 }
@@ -72,8 +90,8 @@ int path_update(const PT& P, const PathBufs<typename PT::real>& b, const typenam
     const char* nu = sizeof(typename PT::real) == 8 ? "tj_update_fp64" : "tj_update_fp32";
     const LaunchShape cells = path_shape<PT>(b.ntot);
     if (pr) pr->begin(nu, st);
-    if (finish) k_update_all<PT, true><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, finish);
-    else k_update_all<PT, false><<<cells.blocks, cells.threads, 0, st>>>(P, b, X, Y, 0);
+    if (finish) path_launch(k_update_all<PT, true>, cells, st, pr, P, b, X, Y, finish);
+    else path_launch(k_update_all<PT, false>, cells, st, pr, P, b, X, Y, 0);
     if (pr) pr->end(nu, st);
     return 1;
 }
@@ -84,7 +102,7 @@ int path_cfl(const PT& P, const PathBufs<typename PT::real>& b, const typename P
     const char* nc = sizeof(typename PT::real) == 8 ? "tj_cfl_fp64" : "tj_cfl_fp32";
     if (pr) pr->begin(nc, st);
     const LaunchShape s = path_shape<PT>(b.ntot);
-    k_cfl<PT><<<s.blocks, s.threads, 0, st>>>(P, b, X);
+    path_launch(k_cfl<PT>, s, st, pr, P, b, X);
     if (pr) pr->end(nc, st);
     return 1;
 }
