@@ -49,11 +49,18 @@ INSTANCES = {
                              "-fmad=false" if r == 64 else "-use_fast_math"])
     for r in (64, 32) for m, d in _INST
 }
+# The binary64 kernels of the plastic solids, and the general reverse mode's,
+# call their divisions (tj_quot.h): in line, a 5-wave flux is 12700 instructions
+# of straight-line code, and its warps mostly wait for instructions (copper
+# 40^3, 10 steps 14.05 -> 13.59 ms called; general adjoint 16^3 48.9 -> 46.6 ms).
+# The fluids' kernels fit and lose by the calls (Sod 6.80 -> 7.52 ms, bubble 256^2
+# 7.78 -> 8.09 ms).
+CALLED = ["-DTJ_QUOT_CALL"]
 # fluids (kind 1, binary64) and plastic solids (kind 2): ParamKind in tj_types.h
 INSTANCES.update({
     f"tj_path_{r}_m{m}_d{d}_k{k}.o":
         ("tj_path_inst.cu", [f"-DTJ_INST_R={r}", f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", f"-DTJ_INST_K={k}",
-                             "-fmad=false" if r == 64 else "-use_fast_math"])
+                             "-fmad=false" if r == 64 else "-use_fast_math"] + (CALLED if (r, k) == (64, 2) else []))
     for r, k in ((64, 1), (64, 2), (32, 2)) for m in (1, 2) for d in (0, 1, 2)
 })
 # the tangent instance (tj_dual.cuh): two materials along x and y, and the
@@ -67,7 +74,7 @@ INSTANCES.update({
 # direction), for plastic solids and (m0) for every configuration
 INSTANCES.update({
     f"tj_gen_m{m}_d{'u' if d < 0 else d}.o":
-        ("tj_gen_inst.cu", [f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", "-fmad=false"])
+        ("tj_gen_inst.cu", [f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", "-fmad=false"] + CALLED)
     for m, dirs in ((1, (-1, 0, 1, 2)), (2, (-1, 0, 1, 2)), (0, (-1, 0))) for d in dirs
 })
 

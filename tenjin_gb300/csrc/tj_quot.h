@@ -232,7 +232,14 @@ TJQ_HD double widen(float x)
 }
 
 // Division and square root of the templated device code, by working type.
-TJQ_HD double quot(double a, double b)
+// TJ_QUOT_CALL: called out of line (the kernels whose straight-line code does
+// not fit the instruction cache and whose warps are too few to hide its misses).
+#if defined(__CUDACC__) && defined(TJ_QUOT_CALL)
+#define TJQ_OP static __host__ __device__ __noinline__
+#else
+#define TJQ_OP TJQ_HD
+#endif
+TJQ_OP double quot(double a, double b)
 {
 #ifdef __CUDA_ARCH__
     return tjq_div(a, b);
@@ -241,7 +248,7 @@ TJQ_HD double quot(double a, double b)
 #endif
 }
 TJQ_HD float quot(float a, float b) { return a / b; }
-TJQ_HD double root(double a)
+TJQ_OP double root(double a)
 {
 #ifdef __CUDA_ARCH__
     return tjq_sqrt(a);
