@@ -6,6 +6,9 @@
 // tangent instance (DevParamsT, tj_dual.cuh), which has no CFL pass. The CFL
 // pass and the whole-stage update are instantiated with the first direction of
 // each material count.
+#if defined(TJ_INST_R) && TJ_INST_R == 32
+#define TJ_QUOT_EXPR
+#endif
 #if defined(TJ_INST_R) && TJ_INST_R == 128
 #include "tj_dual.cuh"
 #elif defined(TJ_INST_K) && TJ_INST_K > 0

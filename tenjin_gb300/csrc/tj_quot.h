@@ -258,4 +258,19 @@ TJQ_OP double root(double a)
 }
 TJQ_HD float root(float a) { return sqrtf(a); }
 
+// TJ_QUOT_EXPR: quot(a, b) stands for the expression a / b itself (the binary64
+// one by way of an overloaded operator). As an argument of a function the
+// divisor is evaluated before the dividend, and the compiler then contracts
+// other pairs of products and sums: with fast math the binary32 results of
+// stiff mixtures differ as much as two roundings of them do.
+#if defined(__CUDACC__) && defined(TJ_QUOT_EXPR)
+struct QuotBy {
+    double v;
+};
+TJQ_HD float quot_by(float b) { return b; }
+TJQ_HD QuotBy quot_by(double b) { return {b}; }
+TJQ_HD double operator/(double a, QuotBy b) { return quot(a, b.v); }
+#define quot(a, b) ((a) / quot_by(b))
+#endif
+
 }  // namespace tj
