@@ -47,7 +47,7 @@ INSTANCES = {
     f"tj_path_{r}_m{m}_d{'g' if d < 0 else d}.o":
         ("tj_path_inst.cu", [f"-DTJ_INST_R={r}", f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}",
                              "-fmad=false" if r == 64 else "-use_fast_math"])
-    for r in (64, 32) for m, d in _INST
+    for r in (64, 32) for m, d in _INST if r == 64 or m == 1
 }
 # The binary64 kernels of the plastic solids, and the general reverse mode's,
 # call their divisions (tj_quot.h): in line, a 5-wave flux is 12700 instructions
@@ -61,7 +61,13 @@ INSTANCES.update({
     f"tj_path_{r}_m{m}_d{d}_k{k}.o":
         ("tj_path_inst.cu", [f"-DTJ_INST_R={r}", f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", f"-DTJ_INST_K={k}",
                              "-fmad=false" if r == 64 else "-use_fast_math"] + (CALLED if (r, k) == (64, 2) else []))
-    for r, k in ((64, 1), (64, 2), (32, 2)) for m in (1, 2) for d in (0, 1, 2)
+    for r, k in ((64, 1), (64, 2), (32, 2)) for m in (1, 2) for d in (0, 1, 2) if r == 64 or m == 1
+})
+# binary32 with several materials: kernels of their own
+INSTANCES.update({
+    f"tj_multi32_m{m}_d{'g' if d < 0 else d}.o":
+        ("tj_multi32.cu", [f"-DTJ_INST_M={m}", f"-DTJ_INST_D={d}", "-use_fast_math"])
+    for m, d in ((2, 0), (2, 1), (2, 2), (0, -1))
 })
 # the tangent instance (tj_dual.cuh): two materials along x and y, and the
 # generic instance for every other material count and direction

@@ -15,6 +15,7 @@
 
 #include "tj_mixed.cuh"
 #include "tj_path.cuh"
+#include "tj_multi32.cuh"
 #include "tj_path_launch.cuh"
 
 namespace tj {
@@ -155,16 +156,26 @@ struct General32 : MixedBase {
     {
         sync_geometry(fb);
         k_reset_dtmin32<<<1, 32, 0, st>>>(fb.scal);
-        return 1 + path_cfl_any(P, b, (const float*)A, st, nullptr);
+        return 1 + cfl_pass(st, nullptr);
+    }
+
+    // One material: tj_path.cuh; several: tj_multi32_path.cuh.
+    int cfl_pass(cudaStream_t st, Prof* pr)
+    {
+        return P.M == 1 ? path_cfl_any(P, b, (const float*)A, st, pr) : multi32::cfl(P, b, A, st, pr);
+    }
+    int stage(const float* X, float* Y, int finish, cudaStream_t st, Prof* pr)
+    {
+        return P.M == 1 ? path_stage_any(P, b, X, Y, finish, st, pr) : multi32::stage(P, b, X, Y, finish, st, pr);
     }
 
     int step(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr) override
     {
         sync_geometry(fb);
-        int n = path_cfl_any(P, b, (const float*)A, st, pr);
+        int n = cfl_pass(st, pr);
         n += fp64_dt_finalize(DP, fb, 1, st);
-        n += path_stage_any(P, b, (const float*)A, B, 0, st, pr);
-        n += path_stage_any(P, b, (const float*)B, C, 1, st, pr);
+        n += stage(A, B, 0, st, pr);
+        n += stage(B, C, 1, st, pr);
         n += fp64_step_end(fb, st);
         return n;
     }

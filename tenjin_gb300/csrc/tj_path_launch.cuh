@@ -45,6 +45,11 @@ constexpr bool kHasKind = K == KIND_FLUID ? std::is_same<Base, DevParams>::value
                                           : std::is_same<Base, DevParams>::value ||
                                                 std::is_same<Base, DevParams32>::value;
 
+// Whether it serves several materials: those of binary32 have kernels of their
+// own (tj_multi32.cuh).
+template <class Base>
+constexpr bool kSeveral = !std::is_same<Base, DevParams32>::value;
+
 template <class Base, int K>
 inline int path_dir_kind(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
                          typename Base::real* Y, int d, int first, int last, int finish, cudaStream_t st, Prof* pr)
@@ -78,15 +83,12 @@ inline int path_faces_kind(const Base& P, const PathBufs<typename Base::real>& b
                            cudaStream_t st, Prof* pr)
 {
 #define TJ_FACES(MC, DC) path_faces<WithM<Base, MC, K>, DC>(WithM<Base, MC, K>(P), b, X, d, st, pr)
-    switch (P.M * 4 + d) {
-        case 4: return TJ_FACES(1, 0);
-        case 5: return TJ_FACES(1, 1);
-        case 6: return TJ_FACES(1, 2);
-        case 8: return TJ_FACES(2, 0);
-        case 9: return TJ_FACES(2, 1);
-        case 10: return TJ_FACES(2, 2);
-        default: return path_faces<Base, -1>(P, b, X, d, st, pr);
+    if (P.M == 1) return d == 0 ? TJ_FACES(1, 0) : d == 1 ? TJ_FACES(1, 1) : TJ_FACES(1, 2);
+    if constexpr (kSeveral<Base>) {
+        if (P.M == 2) return d == 0 ? TJ_FACES(2, 0) : d == 1 ? TJ_FACES(2, 1) : TJ_FACES(2, 2);
+        return path_faces<Base, -1>(P, b, X, d, st, pr);
     }
+    return 0;
 #undef TJ_FACES
 }
 
@@ -112,8 +114,11 @@ inline int path_stage_kind(const Base& P, const PathBufs<typename Base::real>& b
         bd.FX += P.NX * b.nftot[d];
     }
     if (P.M == 1) return n + path_update(WithM<Base, 1, K>(P), b, X, Y, finish, st, pr);
-    if (P.M == 2) return n + path_update(WithM<Base, 2, K>(P), b, X, Y, finish, st, pr);
-    return n + path_update(P, b, X, Y, finish, st, pr);
+    if constexpr (kSeveral<Base>) {
+        if (P.M == 2) return n + path_update(WithM<Base, 2, K>(P), b, X, Y, finish, st, pr);
+        return n + path_update(P, b, X, Y, finish, st, pr);
+    }
+    return n;
 }
 
 // One RK stage: every direction's fluxes from the stage input X, then one
@@ -135,8 +140,11 @@ inline int path_cfl_kind(const Base& P, const PathBufs<typename Base::real>& b, 
                          cudaStream_t st, Prof* pr)
 {
     if (P.M == 1) return path_cfl<WithM<Base, 1, K>>(WithM<Base, 1, K>(P), b, X, st, pr);
-    if (P.M == 2) return path_cfl<WithM<Base, 2, K>>(WithM<Base, 2, K>(P), b, X, st, pr);
-    return path_cfl<Base>(P, b, X, st, pr);
+    if constexpr (kSeveral<Base>) {
+        if (P.M == 2) return path_cfl<WithM<Base, 2, K>>(WithM<Base, 2, K>(P), b, X, st, pr);
+        return path_cfl<Base>(P, b, X, st, pr);
+    }
+    return 0;
 }
 
 template <class Base>
