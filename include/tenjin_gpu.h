@@ -227,7 +227,7 @@ int tj_kernel_config(const tj_ctx* ctx, char* buf, unsigned long len);
  * takes the general reverse mode, built from local Jacobians of the FP64
  * path's own device functions (forward-mode passes, one per input of each
  * cell's update and each face's Riemann problem): exact, deterministic, a
- * backward 50-110 times the forward's time.
+ * backward 7-53 times the forward's time.
  * tj_forward: initial state from the primitives prim0 (the tj_set_primitive
  * layout without mixture words) with the EOS parameters eos
  * ([n_materials][TJ_MAX_EOS_PARAMS] in the getMaterialParameters order,
