@@ -783,10 +783,11 @@ TJA_HD int muscl_branch(double um, double u0, double up)
     // a ratio that is not positive: no slope
     if (((bn ^ bd) >> 63) || (bn << 1) == 0 || (bd << 1) == 0) return 0;
     // r >= 1 takes 2 / (1 + r), and r < 1 - 2^-49 takes 2 r / (1 + r), whose
-    // rounded value is then the smaller one: no division. In between, and
-    // where r may overflow or underflow (or is not a number), as the forward.
-    const int ed = (int)((bn >> 52) & 0x7ff) - (int)((bd >> 52) & 0x7ff);
-    if (ed > -900 && ed < 900) {
+    // rounded value is then the smaller one: no division. In between, where r
+    // may overflow or underflow, and where a difference is infinite or not a
+    // number, as the forward.
+    const int en = (int)((bn >> 52) & 0x7ff), ed = (int)((bd >> 52) & 0x7ff);
+    if (en < 0x7ff && ed < 0x7ff && en - ed > -900 && en - ed < 900) {
         const double n = fabs(num), m = fabs(den);
         if (n >= m) return 2;
         if (n < m * (1.0 - 1.7763568394002505e-15)) return 1;

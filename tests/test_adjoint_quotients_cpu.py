@@ -1,6 +1,7 @@
 """The reverse-mode operators of the 2-D adjoint (tenjin_gb300/csrc/tj_adjoint_local.h)
 against the same derivatives written out in Python floats with one division per
-quotient, on seeded states: the same bits. A quotient formed as a product with a
+quotient, on seeded states: the same bits. The limiter's branch likewise, over zeros,
+subnormal and huge numbers, infinities and NaN. A quotient formed as a product with a
 reciprocal rounds twice, so an operator that does so is further from the exact
 derivative than this and differs here. No tolerance: both sides are IEEE binary64
 in one order of operations (compiled without contraction)."""
@@ -374,3 +375,30 @@ def test_thinc_candidate_rev(lib, d):
         lib.h_thinc_rev(p(s), d, 1.6, 1.0 / 512, 1.0 / 300, lL, lR, p(ls))
         assert ls.tolist() == _thinc_rev(s.tolist(), d, 1.6, 1.0 / 512, 1.0 / 300, float(lL), float(lR))
         done += 1
+
+
+def _muscl_branch(um, u0, up):
+    with np.errstate(all="ignore"):
+        um, u0, up, two = np.float64(um), np.float64(u0), np.float64(up), np.float64(2.0)
+        r = (u0 - um) / (up - u0)
+        if np.isinf(r) or np.isnan(r):
+            r = np.float64(0.0)
+        if r <= 0.0:
+            return 0
+        return 1 if two * r / (1.0 + r) < two / (1.0 + r) else 2
+
+
+def test_muscl_branch(lib):
+    """The active piece of the limiter (hllc.cpp:527-568): the reverse of L = R = u0 (0), of the
+    slope u0 - um (1) and of up - u0 (2), told apart by the adjoint of um and up."""
+    v = [0.0, -0.0, 1.0, -1.0, 1.0 + 2.0 ** -52, 1.0 - 2.0 ** -50, 2.0, 1.0 / 3.0, 5e-324, -5e-324, 2.2250738585072014e-308,
+         1e-200, 1e200, 1e300, -1e300, 1.7976931348623157e308, -1.7976931348623157e308, math.inf, -math.inf, math.nan]
+    rng = np.random.default_rng(5)
+    cases = [(a, b, c) for a in v for b in v for c in v]
+    cases += [tuple(x) for x in rng.standard_normal((2000, 3)) * 10.0 ** rng.integers(-300, 300, (2000, 1))]
+    cases += [(1.0 - k * 2.0 ** -53, 1.0, 1.0 + j * 2.0 ** -52) for k in range(9) for j in range(9)]
+    out = np.zeros(3)
+    for um, u0, up in cases:
+        lib.h_muscl_rev(um, u0, up, 0.0, 2.0, p(out))
+        got = 1 if out[0] != 0.0 else 2 if out[2] != 0.0 else 0
+        assert got == _muscl_branch(um, u0, up), (um, u0, up)
