@@ -769,11 +769,20 @@ TJA_HD void muscl_fwd(double um, double u0, double up, double& l, double& r)
     double half = 0.0;  // of the limiter
     if (!((bn ^ bd) >> 63) && (bn << 1) != 0 && (bd << 1) != 0) {
         const double rr = quot(num, den);
-        if (!TJA_NOTFINITE(rr)) half = quot(rr < 1.0 ? rr : 1.0, 1.0 + rr);
+        const int er = (int)(tj::tjq_bits(rr) >> 52) & 0x7ff;
+        if (er != 0x7ff) {  // finite
+            half = quot(er < 0x3ff ? rr : er < 0x7fd ? 1.0 : 2.0, 1.0 + rr);
+            if (er >= 0x7fd) half *= 0.5;  // a subnormal half: rounded twice, as the limiter's value is
+        }
     }
     const double grad = half * (up - um);
     l = fma(-0.5, grad, u0);
     r = fma(0.5, grad, u0);
+    const tj::tjq_u64 bg = tj::tjq_bits(grad) << 1;
+    if (bg != 0 && bg < 0x40000000000000ull) {  // half of it is subnormal: a product that rounds
+        l = u0 - 0.5 * grad;
+        r = u0 + 0.5 * grad;
+    }
 }
 
 TJA_HD int muscl_branch(double um, double u0, double up)

@@ -471,8 +471,9 @@ __device__ __forceinline__ void muscl1(R um, R u0, R up, R& l, R& r)  // hllc.cp
 // a ratio that is not positive and finite gives slope 0 without a division;
 // of the limiter's two quotients 2 / (1 + r) and 2 r / (1 + r) the smaller is
 // the one with the smaller numerator (rounding is monotonic), so one is formed;
-// and the factors of one half are exact, so they go into that quotient and
-// into the fused multiply-adds (7 binary64 operations instead of about 45).
+// and the factors of one half are exact (but next to the subnormal numbers), so
+// they go into that quotient and into the fused multiply-adds (7 binary64
+// operations instead of about 45).
 __device__ __forceinline__ void muscl1(double um, double u0, double up, double& l, double& r)
 {
     const double num = u0 - um, den = up - u0;
@@ -480,12 +481,20 @@ __device__ __forceinline__ void muscl1(double um, double u0, double up, double& 
     double half = 0.0;
     if ((hn ^ hd) >= 0 && ((hn << 1) | __double2loint(num)) != 0 && ((hd << 1) | __double2loint(den)) != 0) {
         const double rr = quot(num, den);
-        if ((__double2hiint(rr) & 0x7ff00000) != 0x7ff00000)  // finite
-            half = quot(__double2hiint(rr) < 0x3ff00000 ? rr : 1.0, 1.0 + rr);
+        const int er = __double2hiint(rr) & 0x7ff00000;
+        if (er != 0x7ff00000) {  // finite
+            half = quot(er < 0x3ff00000 ? rr : er < 0x7fd00000 ? 1.0 : 2.0, 1.0 + rr);
+            if (er >= 0x7fd00000) half *= 0.5;  // a subnormal half: rounded twice, as the limiter's value is
+        }
     }
     const double grad = half * (up - um);
     l = fma(-0.5, grad, u0);
     r = fma(0.5, grad, u0);
+    const unsigned hg = (unsigned)__double2hiint(grad) << 1;
+    if (hg < 0x400000u && (hg | __double2loint(grad)) != 0) {  // half of it is subnormal: a product that rounds
+        l = u0 - 0.5 * grad;
+        r = u0 + 0.5 * grad;
+    }
 }
 
 // One carried word at a possibly-ghost cell.

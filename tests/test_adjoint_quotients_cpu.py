@@ -1,7 +1,7 @@
 """The reverse-mode operators of the 2-D adjoint (tenjin_gb300/csrc/tj_adjoint_local.h)
 against the same derivatives written out in Python floats with one division per
-quotient, on seeded states: the same bits. The limiter's branch likewise, over zeros,
-subnormal and huge numbers, infinities and NaN. A quotient formed as a product with a
+quotient, on seeded states: the same bits. The limiter's branch and its extrapolation
+likewise, over zeros, subnormal and huge numbers, infinities and NaN. A quotient formed as a product with a
 reciprocal rounds twice, so an operator that does so is further from the exact
 derivative than this and differs here. No tolerance: both sides are IEEE binary64
 in one order of operations (compiled without contraction)."""
@@ -28,6 +28,7 @@ def lib(tmp_path_factory):
     d, i = ctypes.c_double, ctypes.c_int
     L.h_thinc.argtypes = [D, i, d, d, d, D]
     L.h_thinc_rev.argtypes = [D, i, d, d, d, d, d, D]
+    L.h_muscl.argtypes = [d, d, d, D]
     L.h_muscl_rev.argtypes = [d, d, d, d, d, D]
     return L
 
@@ -388,17 +389,44 @@ def _muscl_branch(um, u0, up):
         return 1 if two * r / (1.0 + r) < two / (1.0 + r) else 2
 
 
+def _limiter_inputs():
+    v = [0.0, -0.0, 1.0, -1.0, 1.0 + 2.0 ** -52, 1.0 - 2.0 ** -50, 2.0, 1.0 / 3.0, 5e-324, -5e-324, 1e-320,
+         2.2250738585072014e-308, 1e-200, 1e200, 1e300, -1e300, 1.7976931348623157e308, -1.7976931348623157e308, math.inf, -math.inf, math.nan]
+    rng = np.random.default_rng(5)
+    cases = [(a, b, c) for a in v for b in v for c in v]
+    cases += [tuple(x) for x in rng.standard_normal((4000, 3)) * 10.0 ** rng.integers(-323, 300, (4000, 1))]
+    cases += [(1.0 - k * 2.0 ** -53, 1.0, 1.0 + j * 2.0 ** -52) for k in range(9) for j in range(9)]
+    return cases
+
+
+def _same(a, b):
+    return (np.isnan(a) and np.isnan(b)) or np.float64(a).tobytes() == np.float64(b).tobytes()
+
+
+def test_muscl_extrapolation(lib):
+    """The limited extrapolation in the reference's order (hllc.cpp:527-568): two quotients, the
+    smaller one, and each factor of one half as a product of its own."""
+    f = np.float64
+    out = np.zeros(2)
+    for um, u0, up in _limiter_inputs():
+        lib.h_muscl(um, u0, up, p(out))
+        with np.errstate(all="ignore"):
+            a, b, c = f(um), f(u0), f(up)
+            r = (b - a) / (c - b)
+            phi = f(0.0)
+            if not (np.isinf(r) or np.isnan(r) or r <= 0.0):
+                x, y = f(2.0) / (f(1.0) + r), f(2.0) * r / (f(1.0) + r)
+                phi = y if y < x else x
+            g = phi * f(0.5) * (c - a)
+            want = b - f(0.5) * g, b + f(0.5) * g
+        assert _same(out[0], want[0]) and _same(out[1], want[1]), (um, u0, up)
+
+
 def test_muscl_branch(lib):
     """The active piece of the limiter (hllc.cpp:527-568): the reverse of L = R = u0 (0), of the
     slope u0 - um (1) and of up - u0 (2), told apart by the adjoint of um and up."""
-    v = [0.0, -0.0, 1.0, -1.0, 1.0 + 2.0 ** -52, 1.0 - 2.0 ** -50, 2.0, 1.0 / 3.0, 5e-324, -5e-324, 2.2250738585072014e-308,
-         1e-200, 1e200, 1e300, -1e300, 1.7976931348623157e308, -1.7976931348623157e308, math.inf, -math.inf, math.nan]
-    rng = np.random.default_rng(5)
-    cases = [(a, b, c) for a in v for b in v for c in v]
-    cases += [tuple(x) for x in rng.standard_normal((2000, 3)) * 10.0 ** rng.integers(-300, 300, (2000, 1))]
-    cases += [(1.0 - k * 2.0 ** -53, 1.0, 1.0 + j * 2.0 ** -52) for k in range(9) for j in range(9)]
     out = np.zeros(3)
-    for um, u0, up in cases:
+    for um, u0, up in _limiter_inputs():
         lib.h_muscl_rev(um, u0, up, 0.0, 2.0, p(out))
         got = 1 if out[0] != 0.0 else 2 if out[2] != 0.0 else 0
         assert got == _muscl_branch(um, u0, up), (um, u0, up)
