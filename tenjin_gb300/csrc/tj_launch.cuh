@@ -8,8 +8,8 @@
 // waits until that one is complete and its writes are visible. Every kernel
 // launched this way waits first, so each sees everything before it, as in
 // plain stream order. Measured, with the scalars' own launches folded in:
-// 333^2 cells in binary32, 40 steps in graphs 1.35 -> 1.26 ms, 1024^2 7.02 ->
-// 6.96 ms; 128 boxes in 3-D, 30 steps 36.3 -> 34.7 ms.
+// 333^2 cells in binary32, 40 steps in graphs 1.35 -> 1.26 ms; 128 boxes in 3-D,
+// 30 steps 36.3 -> 34.7 ms. (Large 2-D grids lose by the folding: tj_mixed.cu.)
 #pragma once
 
 #include <cuda_runtime.h>

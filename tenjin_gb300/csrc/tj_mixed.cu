@@ -45,15 +45,25 @@ constexpr int MH = 3;            // staged halo
 constexpr int MS = MT + 2 * MH;  // staged cells per axis (34)
 constexpr int MP = MS + 1;       // shared-memory pitch (odd: conflict-free columns)
 constexpr int CP = MT + 1;       // pitch of the output-cell arrays (odd)
-// Threads per CTA: ten warps, three CTAs an SM, where there are tiles for it
-// (1024^2, 40 steps: 7.12 / 7.25 / 7.02 / 7.43 ms with 256 / 288 / 320 / 352);
-// a grid of fewer tiles leaves SMs with one or two CTAs whose warps walk 28 rows
-// in three rounds or four, so up to two tiles an SM take 14 warps a CTA (two
-// rounds) and up to one takes 28 (one round): 28 warps an SM all the same
-// (333^2 MUSCL, 144 tiles, 40 steps: 1.48 ms with 256, 1.35 with 896).
-// Three and four materials need more registers and binary64 more shared memory:
-// 256 for them.
-constexpr int NTH = 320, NTH_2 = 448, NTH_1 = 896, NTH_WIDE = 256;
+// Threads per CTA: eight warps, three CTAs an SM, where there are tiles for it
+// (20 steps with 256 / 288 / 320: 1024^2 5.84 / 6.01 / 5.91 ms, 1500^2 11.44 /
+// 11.83 / 11.45 ms, 640^2 2.93 / 2.97 / 2.87 ms); a grid of fewer tiles leaves
+// SMs with one or two CTAs whose warps walk 28 rows in three rounds or four, so up
+// to two tiles an SM take 14 warps a CTA (two rounds) and up to one takes 28 (one
+// round): 28 warps an SM all the same (333^2 MUSCL, 144 tiles, 40 steps: 1.48 ms
+// with 256, 1.35 with 896). Three and four materials need more registers and
+// binary64 more shared memory: 256 for them at any size.
+constexpr int NTH = 256, NTH_2 = 448, NTH_1 = 896;
+
+// The step's scalars (dt from the CFL minimum, the step's end) are handled inside
+// the stage kernels on grids of up to kInside tiles, two an SM, and by launches
+// of one thread on larger ones: there a CTA's slot waits for its block's turn at
+// the counter (last_block) in every wave (2500^2, 20 steps: 30.35 ms inside,
+// 29.63 apart; 300^2: 0.91 ms inside, 1.42 apart). Their launches do not overlap
+// either: the next kernel's CTAs take the SMs that drain first and are dealt
+// unevenly (500^2, 324 tiles, 20 steps: 1.90 ms overlapped, 1.81 one after the
+// other).
+constexpr int kSMs = 152, kInside = 2 * kSMs;
 constexpr int XR0 = -2;          // first row (relative to y0) of the x sweep with THINC
 constexpr int XRN = 32;          // rows of the x sweep with THINC: y0-2 .. y0+29
 
@@ -796,22 +806,24 @@ __device__ void sweep_line(const MixP<R>& P, const MixB<R>& b, R* sm, int x0, in
     C[(2 * M + 3) * MTT + oc] = el;
 }
 
-template <typename R, int M, bool THINC, int NT>
+template <typename R, int M, bool THINC, int NT, bool INSIDE>
 __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / NT) : 1)
     k_stage2d(MixP<R> P, MixB<R> b, int stage)
 {
     constexpr int NWARP = NT / 32;
-    grid_wait();
-    grid_go();
+    if (INSIDE) {  // these overlap the launch before them (launch_stage)
+        grid_wait();
+        grid_go();
+    }
     if (b.scal->done) return;
-    // the first stage takes the step's dt from the CFL minimum that the step
-    // before left: every block's first thread forms it while the tile is
-    // staged, the last block to end stores it
+    // the step's dt: stored by the kernel before (scalars apart), or formed from
+    // the CFL minimum that the step before left, by every block's first thread while
+    // the tile is staged; the last block to end then stores it
     __shared__ R dt_over_dx[2];
     __shared__ int run_over;
     if (threadIdx.x == 0) {
         double dt = b.scal->dt;
-        run_over = stage == 0 && step_dt(b.scal, P.cfl, __longlong_as_double((long long)b.scal->dtmin_bits), dt);
+        run_over = INSIDE && stage == 0 && step_dt(b.scal, P.cfl, __longlong_as_double((long long)b.scal->dtmin_bits), dt);
         // binary32: a product with 1/dx (no binary64 division)
         for (int d = 0; d < 2; ++d) dt_over_dx[d] = sizeof(R) == 8 ? (R)(dt / P.dxd[d]) : (R)dt * P.idx[d];
     }
@@ -879,7 +891,7 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     const R dtdx = dt_over_dx[0], dtdy = dt_over_dx[1];
-    if (run_over) {
+    if (INSIDE && run_over) {
         if (last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
         return;
     }
@@ -1050,7 +1062,7 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
             atomicMin(&b.scal->dtmin_bits, (unsigned long long)__double_as_longlong((double)mn));
         }
     }
-    if (last_block(b.scal)) {
+    if (INSIDE && last_block(b.scal)) {
         if (stage == 0) {
             finalize_dt(b.scal, P.cfl, 1);
         } else {
@@ -1214,6 +1226,14 @@ __global__ void __launch_bounds__(256, 4) k_to_fp64(DevParams DP, MixB<R> b, dou
         A[DP.S_E * N + g] = to_d(X[W_EH<M>() * N + g]) + to_d(X[W_EL<M>() * N + g]);
         A[DP.S_P * N + g] = to_d(X[W_P<M>() * N + g]);
     }
+}
+
+// End of a step whose scalars are handled apart, and the THINC stage stamp.
+__global__ void k_step_end_mixed(DevScalars* s, int* ctr)
+{
+    if (threadIdx.x != 0 || s->done) return;
+    *ctr += 2;
+    end_step(s);
 }
 
 __global__ void k_reset_dtmin(DevScalars* s)
@@ -1429,30 +1449,33 @@ struct MixedImpl : MixedBase {
         return 2;
     }
 
-    template <int MM, bool TH, int NT>
+    template <int MM, bool TH, int NT, bool INSIDE>
     void launch_stage_n(int stage, dim3 grid, cudaStream_t st, bool overlap)
     {
         static bool attr = false;
         const size_t smb = Smem<R, MM, TH>::BYTES;
         if (!attr) {
-            cudaFuncSetAttribute(k_stage2d<R, MM, TH, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+            cudaFuncSetAttribute(k_stage2d<R, MM, TH, NT, INSIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
             attr = true;
         }
-        launch(k_stage2d<R, MM, TH, NT>, grid, NT, smb, st, overlap, P, b, stage);
+        launch(k_stage2d<R, MM, TH, NT, INSIDE>, grid, NT, smb, st, overlap, P, b, stage);
     }
+
+    dim3 tiles() const { return dim3((P.nx + MT - 1) / MT, (P.ny + MT - 1) / MT); }
+    bool apart() const { return (long long)tiles().x * tiles().y > kInside; }
 
     template <int MM, bool TH>
     void launch_stage(int stage, cudaStream_t st, bool overlap)
     {
-        constexpr int kSMs = 152;
-        const dim3 grid((P.nx + MT - 1) / MT, (P.ny + MT - 1) / MT);
-        const long long tiles = (long long)grid.x * grid.y;
+        const dim3 grid = tiles();
+        const long long n = (long long)grid.x * grid.y;
+        if (apart()) return launch_stage_n<MM, TH, NTH, false>(stage, grid, st, overlap);
         if constexpr (sizeof(R) == 4 && MM <= 2) {
-            if (tiles <= kSMs) return launch_stage_n<MM, TH, NTH_1>(stage, grid, st, overlap);
-            if (tiles <= 2 * kSMs) return launch_stage_n<MM, TH, NTH_2>(stage, grid, st, overlap);
-            return launch_stage_n<MM, TH, NTH>(stage, grid, st, overlap);
+            if (n <= kSMs) launch_stage_n<MM, TH, NTH_1, true>(stage, grid, st, overlap);
+            else launch_stage_n<MM, TH, NTH_2, true>(stage, grid, st, overlap);
+        } else {
+            launch_stage_n<MM, TH, NTH, true>(stage, grid, st, overlap);
         }
-        launch_stage_n<MM, TH, NTH_WIDE>(stage, grid, st, overlap);
     }
 
     void stage_dispatch(int stage, cudaStream_t st, bool overlap)
@@ -1471,13 +1494,16 @@ struct MixedImpl : MixedBase {
 
     int step(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr) override
     {
-        (void)DP;
         b.scal = fb.scal;
-        int n = 0;
+        int n = apart() ? fp64_dt_finalize(DP, fb, 1, st) : 0;
         for (int stage = 0; stage < 2; ++stage) {
             if (pr) pr->begin(sizeof(R) == 4 ? "tj_stage_mixed" : "tj_stage_fused64", st);
-            stage_dispatch(stage, st, !pr);
+            stage_dispatch(stage, st, !pr && !apart());
             if (pr) pr->end(sizeof(R) == 4 ? "tj_stage_mixed" : "tj_stage_fused64", st);
+            n += 1;
+        }
+        if (apart()) {
+            k_step_end_mixed<<<1, 32, 0, st>>>(fb.scal, ctr);
             n += 1;
         }
         return n;
@@ -1592,12 +1618,6 @@ int mixed_compute_dt(MixedState& ms, const DevParams& DP, const Fp64Bufs& fb, cu
 int mixed_step(MixedState& ms, const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr)
 {
     return ((MixedBase*)ms.impl)->step(DP, fb, st, pr);
-}
-
-int mixed_launches_per_step(const DevParams& DP)
-{
-    (void)DP;
-    return 2;
 }
 
 }  // namespace tj

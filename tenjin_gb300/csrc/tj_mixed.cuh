@@ -60,7 +60,6 @@ int mixed_from_ap(MixedState& m, const DevParams& P, const Fp64Bufs& b, const do
 // CFL minimum of the current mixed state into DevScalars::dtmin_bits.
 int mixed_compute_dt(MixedState& m, const DevParams& P, const Fp64Bufs& b, cudaStream_t st);
 int mixed_step(MixedState& m, const DevParams& P, const Fp64Bufs& b, cudaStream_t st, Prof* pr = nullptr);
-int mixed_launches_per_step(const DevParams& P);
 void mixed_describe(const MixedState& m, char* buf, size_t len);
 
 }  // namespace tj
