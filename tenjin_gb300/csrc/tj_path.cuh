@@ -43,9 +43,12 @@ constexpr int kBlocks64 = 8;
 
 // Blocks of the per-direction kernels and how many an SM is to hold. binary32:
 // blocks of 128 (finer waves than 256) with 128 registers; the one-material
-// solids' reconstruction and fluxes fit in 102, a fifth block (copper 128^3,
-// 5 steps: 15.46 ms with two blocks of 256, 14.97 with three and 80 registers,
-// 14.83 so).
+// plastic solids' reconstruction and fluxes fit in 102, a fifth block (copper
+// 128^3, 5 steps: 15.46 ms with two blocks of 256, 14.97 with three and 80
+// registers, 14.83 so). The instance for every other one-material configuration
+// does not (its flux spills 490 bytes there): 2 / 3 / 4 / 5 blocks take 1.27 / 1.28 /
+// 1.36 / 1.49 ms for a gas of 4000 cells in 1-D, 40 steps, and 8.01 / 5.59 / 5.48 /
+// 5.77 ms for 1000^2 with RADIAL, 10 steps.
 template <class PT>
 constexpr bool kPath32 = sizeof(typename PT::real) == 4;
 template <class PT>
@@ -53,9 +56,9 @@ constexpr int kPathThreads = kPath32<PT> ? 128 : 64;
 template <class PT>
 constexpr int kUpdateBlocks = kPath32<PT> ? 4 : kBlocks64;
 template <class PT>
-constexpr int kFaceBlocks = kPath32<PT> ? 4 : kBlocks64;
-template <int K>
-constexpr int kFaceBlocks<WithM<DevParams32, 1, K>> = 5;
+constexpr int kFaceBlocks = kPath32<PT> ? 3 : kBlocks64;
+template <>
+constexpr int kFaceBlocks<WithM<DevParams32, 1, KIND_PLASTIC>> = 5;
 
 // The first statement of every per-direction kernel (tj_launch.cuh).
 template <typename R>
