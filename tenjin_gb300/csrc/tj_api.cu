@@ -131,6 +131,7 @@ struct tj_ctx {
     // graph-captured step groups
     cudaGraphExec_t graph_exec = nullptr;
     int graph_steps = 0;
+    int graph_plan = 0;  // mixed_plan() of the captured steps
     long long launches = 0;
     EventProf* prof = nullptr;
     long long graph_launches = 0;
@@ -947,7 +948,8 @@ int tj_run(tj_ctx* c, int nsteps, double t_end, int* steps_done, double* t_out)
     if (is_mixed(c) && nsteps > 0) c->a_current = false;
     const int group = 20;
     long long per_group = 0;
-    if (!c->graph_exec || c->graph_steps != group) {
+    const int plan = mixed_plan(c->mixed);  // x_sync may have re-tuned the tiles
+    if (!c->graph_exec || c->graph_steps != group || c->graph_plan != plan) {
         if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
         cudaGraph_t g;
         long long before = c->launches;
@@ -969,6 +971,7 @@ int tj_run(tj_ctx* c, int nsteps, double t_end, int* steps_done, double* t_out)
         per_group = c->launches - before;
         c->launches = before;  // counted when launched
         c->graph_steps = group;
+        c->graph_plan = plan;
         c->graph_launches = per_group;
     }
     per_group = c->graph_launches;

@@ -1620,4 +1620,6 @@ int mixed_step(MixedState& ms, const DevParams& DP, const Fp64Bufs& fb, cudaStre
     return ((MixedBase*)ms.impl)->step(DP, fb, st, pr);
 }
 
+int mixed_plan(const MixedState& ms) { return ms.impl ? ((const MixedBase*)ms.impl)->plan() : 0; }
+
 }  // namespace tj

@@ -32,6 +32,9 @@ struct MixedBase {
     }
     virtual int cfl(const Fp64Bufs& fb, cudaStream_t st) = 0;
     virtual int step(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st, Prof* pr) = 0;
+    // Another number when the launches of step(), or the buffers that they read,
+    // are others than before: a captured graph of steps is stale then.
+    virtual int plan() const { return 0; }
     // a one-line description of the launch configuration in use
     virtual void describe(char* buf, size_t len) const
     {
@@ -60,6 +63,7 @@ int mixed_from_ap(MixedState& m, const DevParams& P, const Fp64Bufs& b, const do
 // CFL minimum of the current mixed state into DevScalars::dtmin_bits.
 int mixed_compute_dt(MixedState& m, const DevParams& P, const Fp64Bufs& b, cudaStream_t st);
 int mixed_step(MixedState& m, const DevParams& P, const Fp64Bufs& b, cudaStream_t st, Prof* pr = nullptr);
+int mixed_plan(const MixedState& m);
 void mixed_describe(const MixedState& m, char* buf, size_t len);
 
 }  // namespace tj

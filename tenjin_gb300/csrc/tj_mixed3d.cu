@@ -914,6 +914,7 @@ struct Mixed3D : MixedBase {
     ClassPlan cls[kClasses];
     Run runs[kClasses];
     int nruns = 0;
+    int nplans = 0;  // times the runs were made
     bool tuned = false;
     int sms = 0;
     long long N = 0;
@@ -1061,6 +1062,7 @@ struct Mixed3D : MixedBase {
     {
         std::vector<Work3> all;
         nruns = 0;
+        ++nplans;
         for (size_t s = 0; s < cand.size(); ++s) {
             std::vector<int> doms;
             for (const ClassPlan& C : cls)
@@ -1234,6 +1236,8 @@ struct Mixed3D : MixedBase {
             }
         return n;
     }
+
+    int plan() const override { return nplans; }
 
     void describe(char* buf, size_t len) const override
     {
