@@ -41,6 +41,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tj_alloc.h"
 #include "tj_adjoint.cuh"
 #include "tj_adjoint_local.h"
 #include "tj_device.cuh"
@@ -716,6 +717,7 @@ static void free_all(AdjState* a)
     a->gpart = a->gsum = nullptr;
     a->sul = a->sur = nullptr;
     a->code = nullptr;
+    a->nck = 0;  // nothing to reverse
     a->bytes = 0;
     a->cap_ck = a->cap_seg = 0;
     a->capN = -1;
@@ -733,7 +735,7 @@ size_t adj_bytes(const AdjState* a) { return a ? a->bytes : 0; }
 template <typename T>
 static bool dalloc(AdjState* a, T** p, size_t n)
 {
-    if (cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
+    if (dev_malloc(p, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
     a->bytes += sizeof(T) * n;
     return true;
 }

@@ -32,6 +32,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tj_alloc.h"
 #include "tj_adjoint_local.h"
 #include "tj_dual.cuh"
 #include "tj_dual_path.cuh"
@@ -402,6 +403,7 @@ static void gen_free(GenAdj* a)
     a->a_to_s = nullptr;
     if (a->passes) cudaFree(a->passes);
     a->passes = nullptr;
+    a->nck = 0;  // nothing to reverse
     for (long long& m : a->made) m = 0;
 }
 
@@ -485,7 +487,7 @@ static int gen_alloc(GenAdj* a, const DevParams& P, const Fp64Bufs& b, int nstep
     if (same) return TJ_OK;
     gen_free(a);
     auto al = [&](double** p, size_t n) {
-        if (cudaMalloc(p, sizeof(double) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
+        if (dev_malloc(p, sizeof(double) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
         a->bufs.push_back(*p);
         return true;
     };
@@ -497,8 +499,8 @@ static int gen_alloc(GenAdj* a, const DevParams& P, const Fp64Bufs& b, int nstep
               al(&a->lamF1, (size_t)P.NX * N) && al(&a->lamLf, (size_t)P.NF * nfmax) &&
               al(&a->lamRf, (size_t)P.NF * nfmax) && al(&a->geos, (size_t)mp * N) &&
               al(&a->geosf, (size_t)mp * nfmax) && al(&a->prim0, (size_t)P.NS * N) && al(&a->gsum, mp);
-    ok = ok && cudaMalloc(&a->a_to_s, sizeof(int) * 64) == cudaSuccess &&
-         cudaMalloc(&a->passes, sizeof(UpdPasses) * kPassLists) == cudaSuccess;
+    ok = ok && dev_malloc(&a->a_to_s, sizeof(int) * 64) == cudaSuccess &&
+         dev_malloc(&a->passes, sizeof(UpdPasses) * kPassLists) == cudaSuccess;
     if (!ok) {
         gen_free(a);
         return TJ_ERR_CUDA;

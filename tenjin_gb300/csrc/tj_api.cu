@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "tj_alloc.h"
 #include "tj_fp64.cuh"
 #include "tj_adjoint.cuh"
 #include "tj_tangent.cuh"
@@ -228,7 +229,7 @@ bool is_mixed(const tj_ctx* c)
 // Upload the box table and the cell -> box map (geometry changes only).
 int sync_boxes(tj_ctx* c)
 {
-    c->geometry_dirty = false;
+    c->geometry_dirty = true;  // until all of it is there
     std::vector<int> flat;
     std::vector<int> cell_box(c->ntot);
     for (size_t q = 0; q < c->doms.size(); ++q) {
@@ -245,12 +246,17 @@ int sync_boxes(tj_ctx* c)
         }
     }
     if (c->d_boxes) cudaFree(c->d_boxes);
-    TJ_CUDA(c, cudaMalloc(&c->d_boxes, sizeof(int) * std::max<size_t>(flat.size(), 6)));
+    c->d_boxes = nullptr;
+    TJ_CUDA(c, dev_malloc(&c->d_boxes, sizeof(int) * std::max<size_t>(flat.size(), 6)));
     TJ_CUDA(c, cudaMemcpy(c->d_boxes, flat.data(), sizeof(int) * flat.size(), cudaMemcpyHostToDevice));
     TJ_CUDA(c, cudaMemcpy(c->d_cell_box, cell_box.data(), sizeof(int) * c->ntot, cudaMemcpyHostToDevice));
     TJ_CUDA(c, cudaMemcpy(c->d_doms, c->doms.data(), sizeof(DevDomain) * c->doms.size(), cudaMemcpyHostToDevice));
     if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
-    if (is_mixed(c)) return mixed_set_boxes(c->mixed, c->P, c->doms, c->boxes, c->stream);
+    if (is_mixed(c)) {
+        const int e = mixed_set_boxes(c->mixed, c->P, c->doms, c->boxes, c->stream);
+        if (e) return fail(c, e, "no device memory for the launches of these boxes");
+    }
+    c->geometry_dirty = false;
     return TJ_OK;
 }
 
@@ -388,7 +394,7 @@ int tj_create(const tj_params* p, tj_ctx** out)
                    "in binary32 only");
     make_layouts(*p, c->P);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return bad("no CUDA device");
-    if (cudaMalloc(&c->d_scal, sizeof(DevScalars)) != cudaSuccess) return bad("cudaMalloc failed");
+    if (dev_malloc(&c->d_scal, sizeof(DevScalars)) != cudaSuccess) return bad("cudaMalloc failed");
     DevScalars s;
     std::memset(&s, 0, sizeof s);
     s.t_end = 1e300;
@@ -424,11 +430,26 @@ int tj_last_error(const tj_ctx* c, char* buf, unsigned long len)
 
 int tj_ncomp(const tj_ctx* c) { return c ? c->P.NCOMP : TJ_ERR_ARG; }
 
+static int make_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim_l);
+
 int tj_set_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim_l)
 {
-    if (!c || nd < 1 || !n_cells || !dim_l) return fail(c, TJ_ERR_ARG, "bad domain arguments");
+    if (!c) return TJ_ERR_ARG;
+    if (nd < 1 || !n_cells || !dim_l) return fail(c, TJ_ERR_ARG, "bad domain arguments");
     TJ_CUDA(c, cudaStreamSynchronize(c->stream));
     free_dev(c);
+    const int e = make_domains(c, nd, n_cells, dim_l);
+    if (e) {  // no domains rather than some of their buffers
+        free_dev(c);
+        c->doms.clear();
+        c->boxes.clear();
+        c->ntot = 0;
+    }
+    return e;
+}
+
+static int make_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim_l)
+{
     c->doms.assign(nd, DevDomain());
     c->boxes.assign(nd, std::vector<int>());
     long long off = 0, foff[3] = {0, 0, 0};
@@ -453,31 +474,31 @@ int tj_set_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim_l)
     for (int d = 0; d < 3; ++d) c->nftot[d] = foff[d];
     const DevParams& P = c->P;
     size_t nt = (size_t)c->ntot;
-    TJ_CUDA(c, cudaMalloc(&c->d_doms, sizeof(DevDomain) * nd));
-    TJ_CUDA(c, cudaMalloc(&c->d_cell_box, sizeof(int) * nt));
+    TJ_CUDA(c, dev_malloc(&c->d_doms, sizeof(DevDomain) * nd));
+    TJ_CUDA(c, dev_malloc(&c->d_cell_box, sizeof(int) * nt));
     if (is_mixed(c)) {
         int e = mixed_alloc(c->mixed, P, c->doms, c->ntot, c->nftot, c->stream);
         if (e) return fail(c, e, "mixed-precision allocation failed");
         // the FP64 buffers double as the mixed path's conversion staging
-        TJ_CUDA(c, cudaMalloc(&c->A, sizeof(double) * P.NS * nt));
+        TJ_CUDA(c, dev_malloc(&c->A, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->A, 0, sizeof(double) * P.NS * nt));
     } else {
-        TJ_CUDA(c, cudaMalloc(&c->A, sizeof(double) * P.NS * nt));
-        TJ_CUDA(c, cudaMalloc(&c->B, sizeof(double) * P.NS * nt));
-        TJ_CUDA(c, cudaMalloc(&c->C, sizeof(double) * P.NS * nt));
-        TJ_CUDA(c, cudaMalloc(&c->UL, sizeof(double) * face_words(P) * nt));
-        TJ_CUDA(c, cudaMalloc(&c->UR, sizeof(double) * face_words(P) * nt));
-        TJ_CUDA(c, cudaMalloc(&c->FX, sizeof(double) * flux_words(P, c->nftot)));
+        TJ_CUDA(c, dev_malloc(&c->A, sizeof(double) * P.NS * nt));
+        TJ_CUDA(c, dev_malloc(&c->B, sizeof(double) * P.NS * nt));
+        TJ_CUDA(c, dev_malloc(&c->C, sizeof(double) * P.NS * nt));
+        TJ_CUDA(c, dev_malloc(&c->UL, sizeof(double) * face_words(P) * nt));
+        TJ_CUDA(c, dev_malloc(&c->UR, sizeof(double) * face_words(P) * nt));
+        TJ_CUDA(c, dev_malloc(&c->FX, sizeof(double) * flux_words(P, c->nftot)));
         TJ_CUDA(c, cudaMemset(c->A, 0, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->B, 0, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->C, 0, sizeof(double) * P.NS * nt));
         if (P.thinc) {
-            TJ_CUDA(c, cudaMalloc(&c->ulstar, sizeof(double) * P.M * nt));
-            TJ_CUDA(c, cudaMalloc(&c->urstar, sizeof(double) * P.M * nt));
+            TJ_CUDA(c, dev_malloc(&c->ulstar, sizeof(double) * P.M * nt));
+            TJ_CUDA(c, dev_malloc(&c->urstar, sizeof(double) * P.M * nt));
             TJ_CUDA(c, cudaMemset(c->ulstar, 0, sizeof(double) * P.M * nt));
             TJ_CUDA(c, cudaMemset(c->urstar, 0, sizeof(double) * P.M * nt));
             for (int d = 0; d < P.dim; ++d) {
-                TJ_CUDA(c, cudaMalloc(&c->gstar[d], sizeof(double) * P.M * c->nftot[d]));
+                TJ_CUDA(c, dev_malloc(&c->gstar[d], sizeof(double) * P.M * c->nftot[d]));
                 TJ_CUDA(c, cudaMemset(c->gstar[d], 0, sizeof(double) * P.M * c->nftot[d]));
             }
         }
@@ -540,7 +561,8 @@ static int ensure_staging(tj_ctx* c, size_t bytes)
     if (c->staging_bytes >= bytes) return TJ_OK;
     if (c->staging) cudaFree(c->staging);
     c->staging = nullptr;
-    TJ_CUDA(c, cudaMalloc(&c->staging, bytes));
+    c->staging_bytes = 0;
+    TJ_CUDA(c, dev_malloc(&c->staging, bytes));
     c->staging_bytes = bytes;
     return TJ_OK;
 }
@@ -848,7 +870,7 @@ int tj_conservation_sums(tj_ctx* c, double* sums)
     int e = need_state(c);
     if (e) return e;
     const int nv = c->P.M + 4;
-    if (!c->cons) TJ_CUDA(c, cudaMalloc(&c->cons, sizeof(double) * (size_t)(kConsPartials + 1) * nv));
+    if (!c->cons) TJ_CUDA(c, dev_malloc(&c->cons, sizeof(double) * (size_t)(kConsPartials + 1) * nv));
     a_sync(c);
     Fp64Bufs b = bufs(c);
     double* out = c->cons + (size_t)kConsPartials * nv;

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tj_alloc.h"
 #include "tj_mixed.cuh"
 #include "tj_path.cuh"
 #include "tj_multi32.cuh"
@@ -94,7 +95,7 @@ struct General32 : MixedBase {
         ns32 = DP.NS + 1;
         const size_t nt = (size_t)ntot;
         auto al = [&](float** p, size_t n) {
-            if (cudaMalloc(p, sizeof(float) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
+            if (dev_malloc(p, sizeof(float) * std::max<size_t>(n, 1)) != cudaSuccess) return false;
             cudaMemsetAsync(*p, 0, sizeof(float) * std::max<size_t>(n, 1), st);
             return true;
         };

@@ -32,6 +32,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tj_alloc.h"
 #include "tj_launch.cuh"
 #include "tj_math.cuh"
 #include "tj_mixed.cuh"
@@ -1305,32 +1306,32 @@ struct MixedImpl : MixedBase {
         }
         const int NW = 3 * DP.M + 7;
         for (int q = 0; q < 2; ++q) {
-            if (cudaMalloc(&X[q], sizeof(R) * NW * N) != cudaSuccess) return TJ_ERR_CUDA;
+            if (dev_malloc(&X[q], sizeof(R) * NW * N) != cudaSuccess) return TJ_ERR_CUDA;
             cudaMemsetAsync(X[q], 0, sizeof(R) * NW * N, st);
         }
         if (DP.thinc) {
             const long long nf[2] = {(long long)(P.nx + 1) * P.ny, (long long)P.nx * (P.ny + 1)};
             for (int q = 0; q < 2; ++q) {
-                if (cudaMalloc(&starA[q], sizeof(R) * DP.M * N) != cudaSuccess) return TJ_ERR_CUDA;
+                if (dev_malloc(&starA[q], sizeof(R) * DP.M * N) != cudaSuccess) return TJ_ERR_CUDA;
                 cudaMemsetAsync(starA[q], 0, sizeof(R) * DP.M * N, st);
-                if (cudaMalloc(&urv[q], sizeof(R) * DP.M * N) != cudaSuccess) return TJ_ERR_CUDA;
+                if (dev_malloc(&urv[q], sizeof(R) * DP.M * N) != cudaSuccess) return TJ_ERR_CUDA;
                 cudaMemsetAsync(urv[q], 0, sizeof(R) * DP.M * N, st);
-                if (cudaMalloc(&urs[q], sizeof(int) * DP.M * N) != cudaSuccess) return TJ_ERR_CUDA;
+                if (dev_malloc(&urs[q], sizeof(int) * DP.M * N) != cudaSuccess) return TJ_ERR_CUDA;
                 cudaMemsetAsync(urs[q], 0xFF, sizeof(int) * DP.M * N, st);
                 for (int d = 0; d < 2; ++d) {
-                    if (cudaMalloc(&gstar[d][q], sizeof(R) * DP.M * nf[d]) != cudaSuccess) return TJ_ERR_CUDA;
+                    if (dev_malloc(&gstar[d][q], sizeof(R) * DP.M * nf[d]) != cudaSuccess) return TJ_ERR_CUDA;
                     cudaMemsetAsync(gstar[d][q], 0, sizeof(R) * DP.M * nf[d], st);
                 }
             }
         }
         for (int d = 0; d < 2; ++d) {
             const int n = d == 0 ? P.nx : P.ny;
-            if (cudaMalloc(&bx[2 * d], sizeof(int) * n) != cudaSuccess) return TJ_ERR_CUDA;
-            if (cudaMalloc(&bx[2 * d + 1], sizeof(int) * n) != cudaSuccess) return TJ_ERR_CUDA;
+            if (dev_malloc(&bx[2 * d], sizeof(int) * n) != cudaSuccess) return TJ_ERR_CUDA;
+            if (dev_malloc(&bx[2 * d + 1], sizeof(int) * n) != cudaSuccess) return TJ_ERR_CUDA;
         }
-        if (cudaMalloc(&ctr, sizeof(int)) != cudaSuccess) return TJ_ERR_CUDA;
+        if (dev_malloc(&ctr, sizeof(int)) != cudaSuccess) return TJ_ERR_CUDA;
         cudaMemsetAsync(ctr, 0, sizeof(int), st);
-        if (cudaMalloc(&bad, sizeof(int)) != cudaSuccess) return TJ_ERR_CUDA;
+        if (dev_malloc(&bad, sizeof(int)) != cudaSuccess) return TJ_ERR_CUDA;
         cudaMemsetAsync(bad, 0, sizeof(int), st);
         if (cudaMallocHost(&bad_h, sizeof(int)) != cudaSuccess) return TJ_ERR_CUDA;
         *bad_h = 0;

@@ -38,6 +38,7 @@
 #include <string>
 #include <vector>
 
+#include "tj_alloc.h"
 #include "tj_launch.cuh"
 #include "tj_math.cuh"
 #include "tj_mixed.cuh"
@@ -958,7 +959,7 @@ struct Mixed3D : MixedBase {
         }
         const int NW = S3_N<4>() - 3 * (4 - M);  // 3M + 9
         for (int q = 0; q < 2; ++q) {
-            if (cudaMalloc(&X[q], sizeof(float) * NW * N) != cudaSuccess) return TJ_ERR_CUDA;
+            if (dev_malloc(&X[q], sizeof(float) * NW * N) != cudaSuccess) return TJ_ERR_CUDA;
             cudaMemsetAsync(X[q], 0, sizeof(float) * NW * N, st);
         }
         switch (M) {
@@ -1026,7 +1027,7 @@ struct Mixed3D : MixedBase {
     {
         if (dst) cudaFree(dst);
         dst = nullptr;
-        if (cudaMalloc(&dst, sizeof(Work3) * std::max<size_t>(w.size(), 1)) != cudaSuccess) return TJ_ERR_CUDA;
+        if (dev_malloc(&dst, sizeof(Work3) * std::max<size_t>(w.size(), 1)) != cudaSuccess) return TJ_ERR_CUDA;
         if (!w.empty()) cudaMemcpyAsync(dst, w.data(), sizeof(Work3) * w.size(), cudaMemcpyHostToDevice, st);
         cudaStreamSynchronize(st);
         return TJ_OK;
@@ -1119,7 +1120,7 @@ struct Mixed3D : MixedBase {
         }
         if (d_doms) cudaFree(d_doms);
         d_doms = nullptr;
-        if (cudaMalloc(&d_doms, sizeof(Dom3) * d3.size()) != cudaSuccess) return TJ_ERR_CUDA;
+        if (dev_malloc(&d_doms, sizeof(Dom3) * d3.size()) != cudaSuccess) return TJ_ERR_CUDA;
         cudaMemcpyAsync(d_doms, d3.data(), sizeof(Dom3) * d3.size(), cudaMemcpyHostToDevice, st);
         b.doms = d_doms;
         tuned = false;  // re-tune on the next upload

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "tj_alloc.h"
 #include "tj_dual.cuh"
 #include "tj_dual_path.cuh"
 #include "tj_path.cuh"
@@ -137,7 +138,7 @@ bool grow(Dual** p, size_t& cap, size_t n)
     if (*p) cudaFree(*p);
     *p = nullptr;
     cap = 0;
-    if (cudaMalloc(p, sizeof(Dual) * n) != cudaSuccess) return false;
+    if (dev_malloc(p, sizeof(Dual) * n) != cudaSuccess) return false;
     cap = n;
     return true;
 }
@@ -189,8 +190,8 @@ long long tan_run(TanState* t, const DevParams& DP, const Fp64Bufs& fb, int dom,
         ok = grow(&t->uls, t->cap[6], DP.M * nt) && grow(&t->urs, t->cap[7], DP.M * nt);
         for (int d = 0; ok && d < DP.dim; ++d) ok = grow(&t->gs[d], t->cap[8 + d], DP.M * (size_t)fb.nftot[d]);
     }
-    if (ok && !t->scal) ok = cudaMalloc(&t->scal, sizeof(DevScalars)) == cudaSuccess;
-    if (ok && !t->a_to_s) ok = cudaMalloc(&t->a_to_s, sizeof(int) * 64) == cudaSuccess;
+    if (ok && !t->scal) ok = dev_malloc(&t->scal, sizeof(DevScalars)) == cudaSuccess;
+    if (ok && !t->a_to_s) ok = dev_malloc(&t->a_to_s, sizeof(int) * 64) == cudaSuccess;
     if (!ok) return TJ_ERR_CUDA;
     // AccessPattern component -> carried word (-1: derived)
     int a2s[64];
