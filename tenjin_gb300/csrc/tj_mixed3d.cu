@@ -890,17 +890,15 @@ inline int box_class(const DevDomain& D)
 struct ClassPlan {
     std::vector<int> doms;  // domains of the class
     int best = -1;          // chosen shape
-    int grid = 0;
-    Work3* d_work = nullptr;
-    int nwork = 0;
+    int nwork = 0;          // its tiles
     long long cells = 0;
     std::vector<double> tune_ms;
 };
 
-// One launch of a stage: the tiles of the classes of one shape.
+// One launch of a stage: the tiles of the classes of one shape, a range of the
+// plan's work list.
 struct Run {
-    int shape = 0, grid = 0, nwork = 0;
-    Work3* d_work = nullptr;
+    int shape = 0, grid = 0, first = 0, nwork = 0;
 };
 
 struct Mixed3D : MixedBase {
@@ -909,7 +907,7 @@ struct Mixed3D : MixedBase {
     int M = 0;
     float* X[2] = {nullptr, nullptr};
     Dom3* d_doms = nullptr;
-    Work3* d_work = nullptr;  // every tile of every class (the CFL pass)
+    Work3* d_work = nullptr;  // the plan: every tile of every class, run after run
     std::vector<Shape> cand;
     std::vector<int> occ;  // resident CTAs per SM of each candidate (0: does not fit)
     ClassPlan cls[kClasses];
@@ -928,10 +926,6 @@ struct Mixed3D : MixedBase {
         if (X[1]) cudaFree(X[1]);
         if (d_doms) cudaFree(d_doms);
         if (d_work) cudaFree(d_work);
-        for (auto& c : cls)
-            if (c.d_work) cudaFree(c.d_work);
-        for (auto& r : runs)
-            if (r.d_work) cudaFree(r.d_work);
     }
 
     int alloc(const DevParams& DP, const std::vector<DevDomain>& doms, long long ntot, cudaStream_t st)
@@ -1017,20 +1011,15 @@ struct Mixed3D : MixedBase {
                         work.push_back(w);
                     }
         }
-        // largest tiles first: the persistent CTAs balance the tail
-        std::stable_sort(work.begin(), work.end(),
-                         [](const Work3& a, const Work3& c) { return a.ex * a.ey * a.ez > c.ex * c.ey * c.ez; });
-        return work;
-    }
-
-    static int upload(Work3*& dst, const std::vector<Work3>& w, cudaStream_t st)
-    {
-        if (dst) cudaFree(dst);
-        dst = nullptr;
-        if (dev_malloc(&dst, sizeof(Work3) * std::max<size_t>(w.size(), 1)) != cudaSuccess) return TJ_ERR_CUDA;
-        if (!w.empty()) cudaMemcpyAsync(dst, w.data(), sizeof(Work3) * w.size(), cudaMemcpyHostToDevice, st);
-        cudaStreamSynchronize(st);
-        return TJ_OK;
+        // largest tiles first: the persistent CTAs balance the tail (a counting
+        // sort: a tile has at most S.tx S.ty S.tz cells)
+        std::vector<size_t> at(S.tx * S.ty * S.tz + 2, 0);
+        const auto key = [&](const Work3& w) { return S.tx * S.ty * S.tz - w.ex * w.ey * w.ez; };
+        for (const Work3& w : work) ++at[key(w) + 1];
+        for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+        std::vector<Work3> sorted(work.size());
+        for (const Work3& w : work) sorted[at[key(w)]++] = w;
+        return sorted;
     }
 
     // Whether shape s fits this GPU at this material count (its shared
@@ -1044,53 +1033,52 @@ struct Mixed3D : MixedBase {
         return -1;
     }
 
-    // Class c's work list under shape s, on the device, and its grid.
-    int plan_class(int c, int s, cudaStream_t st)
-    {
-        if (s < 0 || !fits(s)) return TJ_ERR_ARG;
-        ClassPlan& C = cls[c];
-        const std::vector<Work3> w = tiles(C.doms, s);
-        if (int e = upload(C.d_work, w, st)) return e;
-        C.nwork = (int)w.size();
-        C.best = s;
-        C.grid = std::max(1, std::min(C.nwork, sms * occ[s]));
-        return TJ_OK;
-    }
-
-    // The launches of a stage, and the CFL pass's work list: every tile of every
-    // class under its shape.
-    int plan_all(cudaStream_t st)
+    // The launches of a stage, and their work list, with shape best[c] for class
+    // c. All of it is made before any of it replaces the plan that was there: on
+    // an error that one stays, and covers every box.
+    int make_plan(const int* best, cudaStream_t st)
     {
         std::vector<Work3> all;
-        nruns = 0;
-        ++nplans;
+        Run made[kClasses];
+        int n = 0, nwork[kClasses] = {};
         for (size_t s = 0; s < cand.size(); ++s) {
+            const size_t first = all.size();
             std::vector<int> doms;
-            for (const ClassPlan& C : cls)
-                if (!C.doms.empty() && C.best == (int)s) doms.insert(doms.end(), C.doms.begin(), C.doms.end());
+            for (int c = 0; c < kClasses; ++c)
+                if (!cls[c].doms.empty() && best[c] == (int)s)
+                    doms.insert(doms.end(), cls[c].doms.begin(), cls[c].doms.end());
             if (doms.empty()) continue;
             const std::vector<Work3> w = tiles(doms, (int)s);
-            Run& r = runs[nruns];
-            if (int e = upload(r.d_work, w, st)) return e;
-            r.shape = (int)s;
-            r.nwork = (int)w.size();
-            r.grid = std::max(1, std::min(r.nwork, sms * occ[s]));
-            ++nruns;
+            for (const Work3& t : w) ++nwork[box_class(hdoms[t.dom])];
+            made[n].shape = (int)s;
+            made[n].first = (int)first;
+            made[n].nwork = (int)w.size();
+            made[n].grid = grid_of((int)s, made[n].nwork);
+            ++n;
             all.insert(all.end(), w.begin(), w.end());
         }
-        if (int e = upload(d_work, all, st)) return e;
+        Work3* dst = nullptr;
+        if (dev_malloc(&dst, sizeof(Work3) * std::max<size_t>(all.size(), 1)) != cudaSuccess) return TJ_ERR_CUDA;
+        if (cudaMemcpyAsync(dst, all.data(), sizeof(Work3) * all.size(), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            cudaFree(dst);
+            return TJ_ERR_CUDA;
+        }
+        if (d_work) cudaFree(d_work);
+        d_work = dst;
+        nruns = n;
+        std::copy(made, made + kClasses, runs);
+        for (int c = 0; c < kClasses; ++c) {
+            cls[c].best = best[c];
+            cls[c].nwork = nwork[c];
+        }
         b.work = d_work;
         b.nwork = (int)all.size();
+        ++nplans;
         return TJ_OK;
     }
 
-    M3B class_bufs(int c) const
-    {
-        M3B bc = b;
-        bc.work = cls[c].d_work;
-        bc.nwork = cls[c].nwork;
-        return bc;
-    }
+    int grid_of(int s, int nwork) const { return std::max(1, std::min(nwork, sms * occ[s])); }
 
     int set_boxes(const std::vector<DevDomain>& doms, const std::vector<std::vector<int>>& boxes,
                   cudaStream_t st) override
@@ -1118,67 +1106,101 @@ struct Mixed3D : MixedBase {
             C.doms.push_back((int)q);
             C.cells += (long long)D.n[0] * D.n[1] * D.n[2];
         }
-        if (d_doms) cudaFree(d_doms);
-        d_doms = nullptr;
-        if (dev_malloc(&d_doms, sizeof(Dom3) * d3.size()) != cudaSuccess) return TJ_ERR_CUDA;
-        cudaMemcpyAsync(d_doms, d3.data(), sizeof(Dom3) * d3.size(), cudaMemcpyHostToDevice, st);
+        if (!d_doms && dev_malloc(&d_doms, sizeof(Dom3) * d3.size()) != cudaSuccess) return TJ_ERR_CUDA;
+        if (cudaMemcpyAsync(d_doms, d3.data(), sizeof(Dom3) * d3.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
+            return TJ_ERR_CUDA;
         b.doms = d_doms;
         tuned = false;  // re-tune on the next upload
         const int s0 = first_fit();
         if (s0 < 0) return TJ_ERR_ARG;
-        for (int c = 0; c < kClasses; ++c)
-            if (!cls[c].doms.empty())
-                if (int e = plan_class(c, s0, st)) return e;
-        return plan_all(st);
+        int best[kClasses];
+        std::fill(best, best + kClasses, s0);
+        return make_plan(best, st);
     }
 
     // For each box-size class, times one stage launch per candidate shape
     // over that class's tiles on the current state and keeps the fastest
     // (the trial results are discarded: the stage-1 output buffer is scratch
     // until the next step). TJ_TILE3D=AxBxC pins one candidate for every
-    // class instead.
+    // class instead. Where the device has no room for the trials or for the
+    // plan that comes of them, the plan of set_boxes stays: the same results.
     void autotune(cudaStream_t st)
     {
-        int pinned = -1;
-        if (const char* env = std::getenv("TJ_TILE3D")) {
-            int a = 0, c = 0, d = 0;
-            if (std::sscanf(env, "%dx%dx%d", &a, &c, &d) == 3)
-                for (size_t s = 0; s < cand.size(); ++s)
-                    if (cand[s].tx == a && cand[s].ty == c && cand[s].tz == d) pinned = (int)s;
+        tuned = true;
+        int best[kClasses];
+        for (int c = 0; c < kClasses; ++c) best[c] = cls[c].best;
+        const int pinned = pinned_shape();
+        if (pinned >= 0) std::fill(best, best + kClasses, pinned);
+        else if (!time_shapes(best, st)) return;
+        make_plan(best, st);
+    }
+
+    // The candidate that TJ_TILE3D names, -1 without one that fits.
+    int pinned_shape() const
+    {
+        int a = 0, c = 0, d = 0, pinned = -1;
+        const char* env = std::getenv("TJ_TILE3D");
+        if (env && std::sscanf(env, "%dx%dx%d", &a, &c, &d) == 3)
+            for (size_t s = 0; s < cand.size(); ++s)
+                if (cand[s].tx == a && cand[s].ty == c && cand[s].tz == d && fits((int)s)) pinned = (int)s;
+        return pinned;
+    }
+
+    // The trials: every list in one buffer, in order on the stream, waited for
+    // once (a synchronisation, a copy and an allocation per trial, and a fourth
+    // launch of it, cost a fresh batch what the chosen shapes save in its first ten
+    // steps).
+    bool time_shapes(int* best, cudaStream_t st)
+    {
+        struct Trial {
+            int c, s, first, nwork;
+            cudaEvent_t e0, e1;
+        };
+        std::vector<Trial> trials;
+        std::vector<Work3> all;
+        for (int c = 0; c < kClasses; ++c)
+            for (size_t s = 0; s < cand.size() && !cls[c].doms.empty(); ++s) {
+                if (!fits((int)s)) continue;
+                const std::vector<Work3> w = tiles(cls[c].doms, (int)s);
+                trials.push_back({c, (int)s, (int)all.size(), (int)w.size(), nullptr, nullptr});
+                all.insert(all.end(), w.begin(), w.end());
+            }
+        Work3* list = nullptr;
+        bool ok = dev_malloc(&list, sizeof(Work3) * std::max<size_t>(all.size(), 1)) == cudaSuccess;
+        for (Trial& t : trials)
+            ok = ok && cudaEventCreate(&t.e0) == cudaSuccess && cudaEventCreate(&t.e1) == cudaSuccess;
+        ok = ok && cudaMemcpyAsync(list, all.data(), sizeof(Work3) * all.size(), cudaMemcpyHostToDevice, st) == cudaSuccess;
+        for (size_t k = 0; ok && k < trials.size(); ++k) {
+            const Trial& t = trials[k];
+            const Shape& S = cand[t.s];
+            M3B bc = b;
+            bc.work = list + t.first;
+            bc.nwork = t.nwork;
+            const int grid = grid_of(t.s, t.nwork);
+            S.stage(P, bc, 0, kForce, grid, S.smem, st, false);  // warm-up
+            cudaEventRecord(t.e0, st);
+            for (int r = 0; r < 2; ++r) S.stage(P, bc, 0, kForce, grid, S.smem, st, false);
+            cudaEventRecord(t.e1, st);
+            ok = cudaGetLastError() == cudaSuccess;
         }
-        cudaEvent_t e0, e1;
-        cudaEventCreate(&e0);
-        cudaEventCreate(&e1);
-        for (int c = 0; c < kClasses; ++c) {
-            ClassPlan& C = cls[c];
-            if (C.doms.empty()) continue;
-            if (pinned >= 0 && plan_class(c, pinned, st) == TJ_OK) continue;
-            C.tune_ms.assign(cand.size(), 0.0);
-            float bestms = 3e38f;
-            int bi = first_fit();
-            for (size_t s = 0; s < cand.size(); ++s) {
-                if (plan_class(c, (int)s, st) != TJ_OK) continue;
-                const M3B bc = class_bufs(c);
-                cand[s].stage(P, bc, 0, kForce, C.grid, cand[s].smem, st, false);  // warm-up
-                cudaEventRecord(e0, st);
-                for (int r = 0; r < 3; ++r) cand[s].stage(P, bc, 0, kForce, C.grid, cand[s].smem, st, false);
-                cudaEventRecord(e1, st);
-                cudaEventSynchronize(e1);
-                float ms = 0.0f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                C.tune_ms[s] = ms / 3.0;
-                if (ms < bestms) {
-                    bestms = ms;
-                    bi = (int)s;
+        ok = cudaStreamSynchronize(st) == cudaSuccess && ok;
+        float least[kClasses];
+        std::fill(least, least + kClasses, 3e38f);
+        for (int c = 0; c < kClasses; ++c) cls[c].tune_ms.assign(cand.size(), 0.0);
+        for (Trial& t : trials) {
+            float ms = 0.0f;
+            if (ok && cudaEventElapsedTime(&ms, t.e0, t.e1) == cudaSuccess) {
+                cls[t.c].tune_ms[t.s] = ms / 2.0;
+                if (ms < least[t.c]) {
+                    least[t.c] = ms;
+                    best[t.c] = t.s;
                 }
             }
-            plan_class(c, bi, st);
+            if (t.e0) cudaEventDestroy(t.e0);
+            if (t.e1) cudaEventDestroy(t.e1);
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        plan_all(st);
-        tuned = true;
-        cudaGetLastError();
+        if (list) cudaFree(list);
+        return ok;
     }
 
     int from_fp64(const DevParams& DP, const Fp64Bufs& fb, cudaStream_t st) override
@@ -1228,7 +1250,7 @@ struct Mixed3D : MixedBase {
             for (int r = 0; r < nruns; ++r) {
                 const Shape& S = cand[runs[r].shape];
                 M3B br = b;
-                br.work = runs[r].d_work;
+                br.work = d_work + runs[r].first;
                 br.nwork = runs[r].nwork;
                 if (pr) pr->begin("tj_stage3d_mixed", st);
                 S.stage(P, br, stage, r == nruns - 1 ? kLastRun : 0, runs[r].grid, S.smem, st, !pr);
@@ -1248,9 +1270,14 @@ struct Mixed3D : MixedBase {
             if (C.doms.empty()) continue;
             const Shape& S = cand[C.best < 0 ? 0 : C.best];
             char line[192];
-            std::snprintf(line, sizeof line, "%s%s boxes (%zu, %lld cells): tile %dx%dx%d, %d tiles, grid %d, smem %zu B",
-                          out.empty() ? "" : "; ", kClassName[c], C.doms.size(), C.cells, S.tx, S.ty, S.tz, C.nwork,
-                          C.grid, S.smem);
+            std::snprintf(line, sizeof line, "%s%s boxes (%zu, %lld cells): tile %dx%dx%d, %d tiles",
+                          out.empty() ? "" : "; ", kClassName[c], C.doms.size(), C.cells, S.tx, S.ty, S.tz, C.nwork);
+            out += line;
+        }
+        for (int r = 0; r < nruns; ++r) {
+            char line[96];
+            std::snprintf(line, sizeof line, "; launch: %d tiles, grid %d, smem %zu B", runs[r].nwork, runs[r].grid,
+                          cand[runs[r].shape].smem);
             out += line;
         }
         std::snprintf(buf, len, "%s", out.c_str());

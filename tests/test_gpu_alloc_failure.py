@@ -20,6 +20,7 @@ CASES = {
     "copper_fp64": (lambda: cases.copper_plate_3d(n=8, max_grid_size=4, max_steps=3), FP64),
     "bubble_mixed": (lambda: cases.shock_bubble_2d(n=24, max_grid_size=8, max_steps=22), MIXED),
     "bubble_fused64": (lambda: cases.shock_bubble_2d(n=24, max_grid_size=8, max_steps=3), FUSED64),
+    "boxes_mixed": (lambda: cases.uneven_boxes_3d(nbox=6, seed=4, lo=5, hi=36, max_steps=22), MIXED),
     "copper_mixed": (lambda: cases.copper_plate_3d(n=8, max_grid_size=4, max_steps=3), MIXED),
     "solid_gas_mixed": (lambda: cases.solid_mixture_2d(n=12, max_steps=3), MIXED),
 }
