@@ -26,7 +26,7 @@
 // times each candidate shape on each class's tiles once and keeps the fastest
 // per class, and the classes of one shape run as one persistent launch per
 // stage (the environment variable TJ_TILE3D=AxBxC pins one candidate for all
-// classes).
+// classes; AxBxCp the one with a pair of CTAs an SM, where there are both).
 // Results do not depend on the tile shape (every face and cell is computed
 // by the same arithmetic whichever tile owns it).
 #include <cuda_runtime.h>
@@ -823,6 +823,7 @@ void split_axis(int L, int T, std::vector<std::pair<int, int>>& out)
 // One tile shape: launch helpers of one template instance.
 struct Shape {
     int tx, ty, tz;
+    bool pair;
     size_t smem;
     void (*stage)(const M3P&, const M3B&, int, int, int, size_t, cudaStream_t, bool);
     int (*occupancy)(size_t);
@@ -858,7 +859,7 @@ template <int M, int TX, int TY, int TZ, bool PAIR = false>
 Shape make_shape()
 {
     using SM = Sm3<M, TX, TY, TZ>;
-    return Shape{TX, TY, TZ, PAIR ? sizeof(float) * SM::TOTAL : SM::BYTES, stage_launch<M, TX, TY, TZ, PAIR>,
+    return Shape{TX, TY, TZ, PAIR, PAIR ? sizeof(float) * SM::TOTAL : SM::BYTES, stage_launch<M, TX, TY, TZ, PAIR>,
                  stage_occupancy<M, TX, TY, TZ, PAIR>};
 }
 
@@ -1138,11 +1139,13 @@ struct Mixed3D : MixedBase {
     // The candidate that TJ_TILE3D names, -1 without one that fits.
     int pinned_shape() const
     {
-        int a = 0, c = 0, d = 0, pinned = -1;
+        int a = 0, c = 0, d = 0, end = 0, pinned = -1;
         const char* env = std::getenv("TJ_TILE3D");
-        if (env && std::sscanf(env, "%dx%dx%d", &a, &c, &d) == 3)
+        if (env && std::sscanf(env, "%dx%dx%d%n", &a, &c, &d, &end) == 3)
             for (size_t s = 0; s < cand.size(); ++s)
-                if (cand[s].tx == a && cand[s].ty == c && cand[s].tz == d && fits((int)s)) pinned = (int)s;
+                if (cand[s].tx == a && cand[s].ty == c && cand[s].tz == d && cand[s].pair == (env[end] == 'p') &&
+                    fits((int)s))
+                    pinned = (int)s;
         return pinned;
     }
 
@@ -1270,14 +1273,15 @@ struct Mixed3D : MixedBase {
             if (C.doms.empty()) continue;
             const Shape& S = cand[C.best < 0 ? 0 : C.best];
             char line[192];
-            std::snprintf(line, sizeof line, "%s%s boxes (%zu, %lld cells): tile %dx%dx%d, %d tiles",
-                          out.empty() ? "" : "; ", kClassName[c], C.doms.size(), C.cells, S.tx, S.ty, S.tz, C.nwork);
+            std::snprintf(line, sizeof line, "%s%s boxes (%zu, %lld cells): tile %dx%dx%d%s, %d tiles",
+                          out.empty() ? "" : "; ", kClassName[c], C.doms.size(), C.cells, S.tx, S.ty, S.tz,
+                          S.pair ? "p" : "", C.nwork);
             out += line;
         }
         for (int r = 0; r < nruns; ++r) {
             char line[96];
-            std::snprintf(line, sizeof line, "; launch: %d tiles, grid %d, smem %zu B", runs[r].nwork, runs[r].grid,
-                          cand[runs[r].shape].smem);
+            std::snprintf(line, sizeof line, "; launch: %d tiles, grid %d, %d threads, smem %zu B", runs[r].nwork,
+                          runs[r].grid, cand[runs[r].shape].pair ? NT3_PAIR : NT3, cand[runs[r].shape].smem);
             out += line;
         }
         std::snprintf(buf, len, "%s", out.c_str());
