@@ -132,6 +132,7 @@ struct tj_ctx {
     // graph-captured step groups
     cudaGraphExec_t graph_exec = nullptr;
     int graph_steps = 0;
+    bool flux_all = true;  // FX holds every direction's fluxes
     int graph_plan = 0;  // mixed_plan() of the captured steps
     long long launches = 0;
     EventProf* prof = nullptr;
@@ -216,14 +217,56 @@ Fp64Bufs bufs(tj_ctx* c)
     b.ulstar = c->ulstar; b.urstar = c->urstar;
     for (int d = 0; d < 3; ++d) { b.gstar[d] = c->gstar[d]; b.nftot[d] = c->nftot[d]; }
     b.cell_box = c->d_cell_box; b.boxes = c->d_boxes; b.doms = c->d_doms; b.scal = c->d_scal;
+    b.all_dirs = c->flux_all;
     b.ntot = c->ntot; b.ndom = (int)c->doms.size();
     return b;
+}
+
+// The flux array, with every direction's fluxes where the device has the room.
+cudaError_t alloc_flux(tj_ctx* c)
+{
+    cudaError_t e = cudaErrorMemoryAllocation;
+    for (int all = 1; all >= 0 && e != cudaSuccess; --all) {
+        c->flux_all = all != 0;
+        e = dev_malloc(&c->FX, sizeof(double) * flux_words(c->P, c->nftot, c->flux_all));
+    }
+    return e;
 }
 
 // both fused precisions run the fused kernels
 bool is_mixed(const tj_ctx* c)
 {
     return c->params.precision == TJ_PRECISION_MIXED || c->params.precision == TJ_PRECISION_FUSED64;
+}
+
+// Gives back the fluxes of all directions but one, which a later allocation may
+// need more; whether there were any. (The smaller array takes the larger one's
+// place: it cannot fail, and does not go through dev_malloc.)
+bool shrink(tj_ctx* c)
+{
+    cudaStreamSynchronize(c->stream);
+    if (is_mixed(c)) {
+        const int r = mixed_shrink(c->mixed);
+        if (r < 0) c->doms.clear();  // no domains rather than some of their buffers
+        return r > 0;
+    }
+    if (!c->flux_all || c->P.dim == 1 || !c->FX) return false;
+    cudaFree(c->FX);
+    c->FX = nullptr;
+    c->flux_all = false;
+    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
+    if (cudaMalloc(&c->FX, sizeof(double) * flux_words(c->P, c->nftot, false)) == cudaSuccess) return true;
+    cudaGetLastError();
+    c->FX = nullptr;
+    c->doms.clear();
+    return false;
+}
+
+template <class T>
+cudaError_t ctx_malloc(tj_ctx* c, T** p, size_t bytes)
+{
+    const cudaError_t e = dev_malloc(p, bytes);
+    return e != cudaSuccess && shrink(c) ? dev_malloc(p, bytes) : e;
 }
 
 // Upload the box table and the cell -> box map (geometry changes only).
@@ -247,7 +290,7 @@ int sync_boxes(tj_ctx* c)
     }
     if (c->d_boxes) cudaFree(c->d_boxes);
     c->d_boxes = nullptr;
-    TJ_CUDA(c, dev_malloc(&c->d_boxes, sizeof(int) * std::max<size_t>(flat.size(), 6)));
+    TJ_CUDA(c, ctx_malloc(c, &c->d_boxes, sizeof(int) * std::max<size_t>(flat.size(), 6)));
     TJ_CUDA(c, cudaMemcpy(c->d_boxes, flat.data(), sizeof(int) * flat.size(), cudaMemcpyHostToDevice));
     TJ_CUDA(c, cudaMemcpy(c->d_cell_box, cell_box.data(), sizeof(int) * c->ntot, cudaMemcpyHostToDevice));
     TJ_CUDA(c, cudaMemcpy(c->d_doms, c->doms.data(), sizeof(DevDomain) * c->doms.size(), cudaMemcpyHostToDevice));
@@ -488,7 +531,6 @@ static int make_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim
         TJ_CUDA(c, dev_malloc(&c->C, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, dev_malloc(&c->UL, sizeof(double) * face_words(P) * nt));
         TJ_CUDA(c, dev_malloc(&c->UR, sizeof(double) * face_words(P) * nt));
-        TJ_CUDA(c, dev_malloc(&c->FX, sizeof(double) * flux_words(P, c->nftot)));
         TJ_CUDA(c, cudaMemset(c->A, 0, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->B, 0, sizeof(double) * P.NS * nt));
         TJ_CUDA(c, cudaMemset(c->C, 0, sizeof(double) * P.NS * nt));
@@ -502,6 +544,7 @@ static int make_domains(tj_ctx* c, int nd, const int* n_cells, const double* dim
                 TJ_CUDA(c, cudaMemset(c->gstar[d], 0, sizeof(double) * P.M * c->nftot[d]));
             }
         }
+        TJ_CUDA(c, alloc_flux(c));
     }
     c->a_current = c->x_current = true;  // both copies start zero
     int e = sync_boxes(c);
@@ -562,7 +605,7 @@ static int ensure_staging(tj_ctx* c, size_t bytes)
     if (c->staging) cudaFree(c->staging);
     c->staging = nullptr;
     c->staging_bytes = 0;
-    TJ_CUDA(c, dev_malloc(&c->staging, bytes));
+    TJ_CUDA(c, ctx_malloc(c, &c->staging, bytes));
     c->staging_bytes = bytes;
     return TJ_OK;
 }
@@ -643,6 +686,7 @@ static int exchange(tj_ctx* c, int q, const int* bx, double* host, int ncomp, in
     }
     e = ensure_staging(c, bytes);
     if (e) return e;
+    b = bufs(c);
     if (up) {
         if (!whole) a_sync(c);
         // only the component planes the carried state is built from cross the
@@ -870,7 +914,7 @@ int tj_conservation_sums(tj_ctx* c, double* sums)
     int e = need_state(c);
     if (e) return e;
     const int nv = c->P.M + 4;
-    if (!c->cons) TJ_CUDA(c, dev_malloc(&c->cons, sizeof(double) * (size_t)(kConsPartials + 1) * nv));
+    if (!c->cons) TJ_CUDA(c, ctx_malloc(c, &c->cons, sizeof(double) * (size_t)(kConsPartials + 1) * nv));
     a_sync(c);
     Fp64Bufs b = bufs(c);
     double* out = c->cons + (size_t)kConsPartials * nv;
@@ -1092,13 +1136,16 @@ int tj_forward(tj_ctx* c, int q, const double* prim0, const double* eos, int nst
     Fp64Bufs b = bufs(c);
     c->launches += fp64_prim_to_state(c->P, b, 0, c->ntot, c->staging, c->A, c->stream);
     c->adj_general = general;
-    long long n;
-    if (general) {
-        if (!c->gen) c->gen = gen_create();
-        n = gen_forward(c->gen, c->P, b, c->staging, (int)nprim, dt, nsteps, stride, c->stream);
-    } else {
-        if (!c->adj) c->adj = adj_create();
-        n = adj_forward(c->adj, c->P, b, D, dt, nsteps, stride, c->stream);
+    if (general && !c->gen) c->gen = gen_create();
+    if (!general && !c->adj) c->adj = adj_create();
+    const auto forward = [&] {  // allocates before it does anything else
+        return general ? gen_forward(c->gen, c->P, b, c->staging, (int)nprim, dt, nsteps, stride, c->stream)
+                       : adj_forward(c->adj, c->P, b, D, dt, nsteps, stride, c->stream);
+    };
+    long long n = forward();
+    if (n == TJ_ERR_CUDA && shrink(c)) {
+        b = bufs(c);
+        n = forward();
     }
     if (n < 0) return fail(c, (int)n, "tj_forward: device allocation failed");
     c->launches += n;
@@ -1189,8 +1236,15 @@ int tj_tangent(tj_ctx* c, int q, const double* prim0, const double* dprim0, cons
     if (dprim0) TJ_CUDA(c, cudaMemcpyAsync(dir_dev, dprim0, sizeof(double) * pw, cudaMemcpyDefault, c->stream));
     if (!c->tan) c->tan = tan_create();
     Fp64Bufs b = bufs(c);
-    long long n = tan_run(c->tan, c->P, b, 0, prim_dev, dprim0 ? dir_dev : nullptr, deos, nsteps, dt,
-                          state ? ap : nullptr, dap, c->stream);
+    const auto run = [&] {  // allocates before it does anything else
+        return tan_run(c->tan, c->P, b, 0, prim_dev, dprim0 ? dir_dev : nullptr, deos, nsteps, dt, state ? ap : nullptr,
+                       dap, c->stream);
+    };
+    long long n = run();
+    if (n == TJ_ERR_CUDA && shrink(c)) {
+        b = bufs(c);
+        n = run();
+    }
     if (n < 0) return fail(c, (int)n, "tj_tangent: device allocation failed");
     c->launches += n;
     if (state) TJ_CUDA(c, cudaMemcpyAsync(state, ap, sizeof(double) * aw, cudaMemcpyDefault, c->stream));
@@ -1207,7 +1261,7 @@ int tj_kernel_config(const tj_ctx* c, char* buf, unsigned long len)
 {
     if (!c || !buf || len == 0) return TJ_ERR_ARG;
     if (is_mixed(c)) mixed_describe(c->mixed, buf, len);
-    else std::snprintf(buf, len, "fp64 per-direction kernels");
+    else std::snprintf(buf, len, "fp64 per-direction kernels%s", c->flux_all ? "" : ", updates per direction");
     return TJ_OK;
 }
 

@@ -81,6 +81,8 @@ struct General32 : MixedBase {
     float *A = nullptr, *B = nullptr, *C = nullptr, *UL = nullptr, *UR = nullptr, *FX = nullptr;
     float *uls = nullptr, *urs = nullptr, *gs[3] = {nullptr, nullptr, nullptr};
     int ns32 = 0;
+    int nplans = 0;
+    size_t one_dir = 0;  // words of one direction's fluxes
 
     ~General32() override
     {
@@ -100,11 +102,15 @@ struct General32 : MixedBase {
             return true;
         };
         bool ok = al(&A, ns32 * nt) && al(&B, ns32 * nt) && al(&C, ns32 * nt) &&
-                  al(&UL, face_words(DP) * nt) && al(&UR, face_words(DP) * nt) && al(&FX, flux_words(DP, nftot));
+                  al(&UL, face_words(DP) * nt) && al(&UR, face_words(DP) * nt);
         if (ok && DP.thinc) {
             ok = al(&uls, DP.M * nt) && al(&urs, DP.M * nt);
             for (int d = 0; ok && d < DP.dim; ++d) ok = al(&gs[d], DP.M * (size_t)nftot[d]);
         }
+        // several materials' kernels hold one direction's fluxes
+        one_dir = flux_words(DP, nftot, false);
+        b.all_dirs = DP.M == 1 && al(&FX, flux_words(DP, nftot, true));
+        ok = ok && (b.all_dirs || al(&FX, one_dir));
         if (!ok) return TJ_ERR_CUDA;
         b.A = A;
         b.B = B;
@@ -121,6 +127,19 @@ struct General32 : MixedBase {
         b.ntot = ntot;
         return TJ_OK;
     }
+
+    int shrink() override
+    {
+        if (!b.all_dirs || P.dim == 1 || !FX) return 0;
+        cudaFree(FX);
+        FX = nullptr;
+        b.all_dirs = 0;
+        ++nplans;
+        if (cudaMalloc(&FX, sizeof(float) * one_dir) != cudaSuccess) FX = nullptr;
+        b.FX = FX;
+        return FX ? 1 : -1;
+    }
+    int plan() const override { return nplans; }
 
     // geometry pointers are the binary64 context's
     void sync_geometry(const Fp64Bufs& fb)
@@ -183,7 +202,8 @@ struct General32 : MixedBase {
 
     void describe(char* buf, size_t len) const override
     {
-        std::snprintf(buf, len, "binary32 per-direction kernels (%d-D), binary64 pressure closure and plastic return map", P.dim);
+        std::snprintf(buf, len, "binary32 per-direction kernels (%d-D), binary64 pressure closure and plastic return map%s",
+                      P.dim, P.M == 1 && !b.all_dirs ? ", updates per direction" : "");
     }
 };
 

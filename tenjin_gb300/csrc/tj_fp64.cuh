@@ -1,6 +1,8 @@
 // FP64 reference-faithful kernels of the per-timestep update.
 #pragma once
 
+#include <algorithm>
+
 #include "tj_types.h"
 
 namespace tj {
@@ -9,7 +11,7 @@ template <typename R>
 struct PathBufs {
     R *A, *B, *C;        // state: U^n (and result), stage-1 output, stage-2 partial
     R *UL, *UR;          // reconstructed face states, one per cell
-    R* FX;               // face fluxes, one direction after the other
+    R* FX;               // face fluxes, one direction after the other (all_dirs), or of one
     R *ulstar, *urstar;  // THINC scratch (alpha of the reference's ULStar / URStar)
     R* gstar[3];         // ULStar ghost alpha at box hi+1 faces, per direction
     int* cell_box;            // domain-local box index of each cell
@@ -25,6 +27,7 @@ struct PathBufs {
     // own THINC candidate, 2 a value of the THINC scratch
     R* rec = nullptr;
     int* rec_code = nullptr;
+    int all_dirs = 1;
     int overlap = 0;  // the kernel is launched to overlap the one before it (tj_path_inst.cu)
 };
 using Fp64Bufs = PathBufs<double>;
@@ -56,11 +59,16 @@ inline size_t face_words(const DevParams& P)
     if (P.thinc || P.nmix) return (size_t)P.NF;
     return 2 * (size_t)P.M + 4 + (P.solid ? 9 + (P.any_solid ? 0 : 1) : 0) + (P.plastic ? (size_t)P.M : 0);
 }
-// Words of the flux array: every direction's faces.
-inline size_t flux_words(const DevParams& P, const long long* nftot)
+// Words of the flux array: every direction's faces, for the one update per stage
+// (k_update_all); or the largest direction's, where the device has no room for
+// them: the stage then updates direction by direction (k_update), the same bits
+// (copper 40^3 in binary64, 10 steps 13.7 / 14.0 ms; copper 128^3 in binary32, 5
+// steps 10.9 / 14.5 ms).
+inline size_t flux_words(const DevParams& P, const long long* nftot, bool all_dirs)
 {
     size_t n = 0;
-    for (int d = 0; d < P.dim; ++d) n += (size_t)P.NX * (size_t)nftot[d];
+    for (int d = 0; d < P.dim; ++d)
+        n = all_dirs ? n + (size_t)P.NX * (size_t)nftot[d] : std::max(n, (size_t)P.NX * (size_t)nftot[d]);
     return n;
 }
 

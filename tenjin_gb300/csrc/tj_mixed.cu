@@ -1621,6 +1621,8 @@ int mixed_step(MixedState& ms, const DevParams& DP, const Fp64Bufs& fb, cudaStre
     return ((MixedBase*)ms.impl)->step(DP, fb, st, pr);
 }
 
+int mixed_shrink(MixedState& ms) { return ms.impl ? ((MixedBase*)ms.impl)->shrink() : 0; }
+
 int mixed_plan(const MixedState& ms) { return ms.impl ? ((const MixedBase*)ms.impl)->plan() : 0; }
 
 }  // namespace tj

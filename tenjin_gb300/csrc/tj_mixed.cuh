@@ -35,6 +35,9 @@ struct MixedBase {
     // Another number when the launches of step(), or the buffers that they read,
     // are others than before: a captured graph of steps is stale then.
     virtual int plan() const { return 0; }
+    // Gives back the device memory it can do without: 1, 0 if there was none, -1
+    // if it can compute no more.
+    virtual int shrink() { return 0; }
     // a one-line description of the launch configuration in use
     virtual void describe(char* buf, size_t len) const
     {
@@ -64,6 +67,7 @@ int mixed_from_ap(MixedState& m, const DevParams& P, const Fp64Bufs& b, const do
 int mixed_compute_dt(MixedState& m, const DevParams& P, const Fp64Bufs& b, cudaStream_t st);
 int mixed_step(MixedState& m, const DevParams& P, const Fp64Bufs& b, cudaStream_t st, Prof* pr = nullptr);
 int mixed_plan(const MixedState& m);
+int mixed_shrink(MixedState& m);
 void mixed_describe(const MixedState& m, char* buf, size_t len);
 
 }  // namespace tj

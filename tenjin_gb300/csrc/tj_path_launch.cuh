@@ -55,15 +55,12 @@ inline int path_dir_kind(const Base& P, const PathBufs<typename Base::real>& b, 
                          typename Base::real* Y, int d, int first, int last, int finish, cudaStream_t st, Prof* pr)
 {
 #define TJ_DIR(MC, DC) path_dir<WithM<Base, MC, K>, DC>(WithM<Base, MC, K>(P), b, X, Y, d, first, last, finish, st, pr)
-    switch (P.M * 4 + d) {
-        case 4: return TJ_DIR(1, 0);
-        case 5: return TJ_DIR(1, 1);
-        case 6: return TJ_DIR(1, 2);
-        case 8: return TJ_DIR(2, 0);
-        case 9: return TJ_DIR(2, 1);
-        case 10: return TJ_DIR(2, 2);
-        default: return path_dir<Base, -1>(P, b, X, Y, d, first, last, finish, st, pr);
+    if (P.M == 1) return d == 0 ? TJ_DIR(1, 0) : d == 1 ? TJ_DIR(1, 1) : TJ_DIR(1, 2);
+    if constexpr (kSeveral<Base>) {
+        if (P.M == 2) return d == 0 ? TJ_DIR(2, 0) : d == 1 ? TJ_DIR(2, 1) : TJ_DIR(2, 2);
+        return path_dir<Base, -1>(P, b, X, Y, d, first, last, finish, st, pr);
     }
+    return 0;  // not reached: several materials in binary32 have kernels of their own (tj_multi32.cuh)
 #undef TJ_DIR
 }
 
@@ -88,7 +85,7 @@ inline int path_faces_kind(const Base& P, const PathBufs<typename Base::real>& b
         if (P.M == 2) return d == 0 ? TJ_FACES(2, 0) : d == 1 ? TJ_FACES(2, 1) : TJ_FACES(2, 2);
         return path_faces<Base, -1>(P, b, X, d, st, pr);
     }
-    return 0;
+    return 0;  // not reached, as above
 #undef TJ_FACES
 }
 
@@ -108,6 +105,11 @@ inline int path_stage_kind(const Base& P, const PathBufs<typename Base::real>& b
                            typename Base::real* Y, int finish, cudaStream_t st, Prof* pr)
 {
     int n = 0;
+    if (!b.all_dirs) {
+        for (int d = 0; d < P.dim; ++d)
+            n += path_dir_kind<Base, K>(P, b, X, Y, d, d == 0, d == P.dim - 1, finish, st, pr);
+        return n;
+    }
     PathBufs<typename Base::real> bd = b;
     for (int d = 0; d < P.dim; ++d) {
         n += path_faces_kind<Base, K>(P, bd, X, d, st, pr);
@@ -122,8 +124,8 @@ inline int path_stage_kind(const Base& P, const PathBufs<typename Base::real>& b
 }
 
 // One RK stage: every direction's fluxes from the stage input X, then one
-// update into Y, or with finish into b.A. b.FX holds every direction's fluxes
-// (flux_words).
+// update into Y, or with finish into b.A; direction by direction where b.FX holds
+// one direction's fluxes (flux_words).
 template <class Base>
 inline int path_stage_any(const Base& P, const PathBufs<typename Base::real>& b, const typename Base::real* X,
                           typename Base::real* Y, int finish, cudaStream_t st, Prof* pr)
@@ -144,7 +146,7 @@ inline int path_cfl_kind(const Base& P, const PathBufs<typename Base::real>& b, 
         if (P.M == 2) return path_cfl<WithM<Base, 2, K>>(WithM<Base, 2, K>(P), b, X, st, pr);
         return path_cfl<Base>(P, b, X, st, pr);
     }
-    return 0;
+    return 0;  // not reached, as above
 }
 
 template <class Base>
