@@ -1098,6 +1098,23 @@ int tj_get_stream(tj_ctx* c, void** stream)
     return TJ_OK;
 }
 
+// EOS parameters in place of the context's. Captured steps hold the old ones.
+static void set_eos(tj_ctx* c, const double* eos)
+{
+    bool same = true;
+    for (int m = 0; m < c->P.M; ++m)
+        for (int k = 0; k < c->params.materials[m].nparams && k < TJ_MAX_EOS_PARAMS; ++k) {
+            const double v = eos[m * TJ_MAX_EOS_PARAMS + k];
+            same = same && c->P.prm[m][k] == v;
+            c->P.prm[m][k] = v;
+            c->params.materials[m].params[k] = v;
+        }
+    if (!same && c->graph_exec) {
+        cudaGraphExecDestroy(c->graph_exec);
+        c->graph_exec = nullptr;
+    }
+}
+
 int tj_forward(tj_ctx* c, int q, const double* prim0, const double* eos, int nsteps, const double* dt, int stride)
 {
     if (!c || !prim0 || !dt || nsteps < 1 || stride < 1) return fail(c, TJ_ERR_ARG, "bad tj_forward arguments");
@@ -1113,12 +1130,7 @@ int tj_forward(tj_ctx* c, int q, const double* prim0, const double* eos, int nst
     }
     for (int n = 0; n < nsteps; ++n)
         if (!(dt[n] > 0.0)) return fail(c, TJ_ERR_ARG, "tj_forward: dt must be positive");
-    if (eos)
-        for (int m = 0; m < c->P.M; ++m)
-            for (int k = 0; k < c->params.materials[m].nparams && k < TJ_MAX_EOS_PARAMS; ++k) {
-                c->P.prm[m][k] = eos[m * TJ_MAX_EOS_PARAMS + k];
-                c->params.materials[m].params[k] = eos[m * TJ_MAX_EOS_PARAMS + k];
-            }
+    if (eos) set_eos(c, eos);
     const DevDomain& D = c->doms[0];
     const size_t nprim = 2 * c->P.M + 4 + (c->P.solid ? 9 : 0) + (c->P.plastic ? c->P.M : 0);
     const size_t bytes = sizeof(double) * nprim * (size_t)c->ntot;
@@ -1217,12 +1229,7 @@ int tj_tangent(tj_ctx* c, int q, const double* prim0, const double* dprim0, cons
     if (c->P.nmix) return fail(c, TJ_ERR_ARG, "tj_tangent: no mixtures (the mixture EOS root find)");
     for (int n = 0; n < nsteps; ++n)
         if (!(dt[n] > 0.0)) return fail(c, TJ_ERR_ARG, "tj_tangent: dt must be positive");
-    if (eos)
-        for (int m = 0; m < c->P.M; ++m)
-            for (int k = 0; k < c->params.materials[m].nparams && k < TJ_MAX_EOS_PARAMS; ++k) {
-                c->P.prm[m][k] = eos[m * TJ_MAX_EOS_PARAMS + k];
-                c->params.materials[m].params[k] = eos[m * TJ_MAX_EOS_PARAMS + k];
-            }
+    if (eos) set_eos(c, eos);
     const size_t N = (size_t)c->ntot;
     const size_t nprim = 2 * c->P.M + 4 + (c->P.solid ? 9 : 0) + (c->P.plastic ? c->P.M : 0);
     const size_t pw = nprim * N, aw = (size_t)c->P.NCOMP * N;
