@@ -635,77 +635,68 @@ __device__ __forceinline__ int c2p(const PT& P, CellT<typename PT::real>& c)
         c.vel[r] = quot(c.rhou[r], c.rho);
         ke += R(0.5) * c.rho * c.vel[r] * c.vel[r];
     }
-    if constexpr (sizeof(R) == 4) {
-        if (P.M == 1 && !P.nmix) {
-            // one material: no interface whose stiff cold terms cancel the
-            // energy, so the closure stays binary32, with the numerator
-            // E + Elo - KE - e_cold + p_cold summed without rounding error
-            // into an unevaluated pair (error-free sums)
-            const R ent = eff_e_nonthermal(P, c), pnt = eff_p_nonthermal(P, c), ig = eff_invG(P, c);
-            R sh = c.E, sl = c.Elo;
-            acc_pair32(sh, sl, -ke);
-            acc_pair32(sh, sl, -ent);
-            acc_pair32(sh, sl, pnt);
-            c.p = quot(__fadd_rn(sh, sl), ig);
-            stress(P, c);
-            return err;
-        }
-        // binary32 state with several materials: the closure of the pressure
-        // (and of the mixture densities) in binary64, from the compensated
-        // energy (E, Elo) and binary64 cold terms
-        double rho = 0.0, ent = 0.0, pnt = 0.0, ig = 0.0;
-        for (int m = 0; m < P.M; ++m) rho += (double)c.arho[m];
-        const double ru0 = c.rhou[0], ru1 = c.rhou[1], ru2 = c.rhou[2];
-        const double ked = quot(0.5 * (ru0 * ru0 + ru1 * ru1 + ru2 * ru2), rho);
-        double lam = 0.0, rm0 = 0.0, rm1 = 0.0;
-        if (P.nmix) {
-            lam = quot((double)c.arl, (double)c.arho[0]);
-            CellT<double> cd;
-            for (int m = 0; m < P.M; ++m) {
-                cd.alpha[m] = c.alpha[m];
-                cd.arho[m] = c.arho[m];
-                cd.rhok[m] = c.rhok[m];
-            }
-            cd.hj2 = c.hj2;
-            cd.p = 0.0;
-            cd.E = (double)c.E + (double)c.Elo;
-            cd.lam = lam;
-            cd.rm0 = c.rm0;
-            cd.rm1 = c.rm1;
-            err = mix_root_find(P.d, cd, ked);
-            rm0 = cd.rm0;
-            rm1 = cd.rm1;
-            c.lam = (R)lam;
-            c.rm0 = (R)rm0;
-            c.rm1 = (R)rm1;
-        }
-        for (int m = 0; m < P.M; ++m) {
-            ECellT<double> e;
-            e.alpha = c.alpha[m];
-            e.arho = c.arho[m];
-            e.rhok = c.rhok[m];
-            e.p = 0.0;
-            e.hj2 = c.hj2;
-            e.lam = lam;
-            e.rm0 = rm0;
-            e.rm1 = rm1;
-            if (P.nmix) {
-                ent += eos_e_cold(P.d, m, e) + eos_e_shear(P.d, m, e);
-                pnt += eos_p_cold(P.d, m, e) + eos_p_shear(P.d, m, e);
-                ig += eos_invG(P.d, m, e);
-            } else {
-                closure_terms64(P, m, e, ent, pnt, ig);
-            }
-        }
-        c.p = (R)(quot((double)c.E + (double)c.Elo - ked - ent + pnt, ig));
-    } else {
-        if (P.nmix) {  // :104-113
-            c.lam = quot(c.arl, c.arho[0]);
-            // binary64 only: the tangent instance takes no mixtures
-            if constexpr (std::is_same<R, double>::value) err = mix_root_find(P, c, ke);
-        }
-        c.p = quot(c.E - ke - eff_e_nonthermal(P, c) + eff_p_nonthermal(P, c), eff_invG(P, c));
+    if (P.M == 1 && !P.nmix) {
+        // one material: no interface whose stiff cold terms cancel the
+        // energy, so the closure stays binary32, with the numerator
+        // E + Elo - KE - e_cold + p_cold summed without rounding error
+        // into an unevaluated pair (error-free sums)
+        const R ent = eff_e_nonthermal(P, c), pnt = eff_p_nonthermal(P, c), ig = eff_invG(P, c);
+        R sh = c.E, sl = c.Elo;
+        acc_pair32(sh, sl, -ke);
+        acc_pair32(sh, sl, -ent);
+        acc_pair32(sh, sl, pnt);
+        c.p = quot(__fadd_rn(sh, sl), ig);
+        stress(P, c);
+        return err;
     }
+    // binary32 state with several materials: the closure of the pressure
+    // (and of the mixture densities) in binary64, from the compensated
+    // energy (E, Elo) and binary64 cold terms
+    double rho = 0.0, ent = 0.0, pnt = 0.0, ig = 0.0;
+    for (int m = 0; m < P.M; ++m) rho += (double)c.arho[m];
+    const double ru0 = c.rhou[0], ru1 = c.rhou[1], ru2 = c.rhou[2];
+    const double ked = quot(0.5 * (ru0 * ru0 + ru1 * ru1 + ru2 * ru2), rho);
+    double lam = 0.0, rm0 = 0.0, rm1 = 0.0;
+    if (P.nmix) {
+        lam = quot((double)c.arl, (double)c.arho[0]);
+        CellT<double> cd;
+        for (int m = 0; m < P.M; ++m) {
+            cd.alpha[m] = c.alpha[m];
+            cd.arho[m] = c.arho[m];
+            cd.rhok[m] = c.rhok[m];
+        }
+        cd.hj2 = c.hj2;
+        cd.p = 0.0;
+        cd.E = (double)c.E + (double)c.Elo;
+        cd.lam = lam;
+        cd.rm0 = c.rm0;
+        cd.rm1 = c.rm1;
+        err = mix_root_find(P.d, cd, ked);
+        rm0 = cd.rm0;
+        rm1 = cd.rm1;
+        c.lam = (R)lam;
+        c.rm0 = (R)rm0;
+        c.rm1 = (R)rm1;
+    }
+    for (int m = 0; m < P.M; ++m) {
+        ECellT<double> e;
+        e.alpha = c.alpha[m];
+        e.arho = c.arho[m];
+        e.rhok = c.rhok[m];
+        e.p = 0.0;
+        e.hj2 = c.hj2;
+        e.lam = lam;
+        e.rm0 = rm0;
+        e.rm1 = rm1;
+        if (P.nmix) {
+            ent += eos_e_cold(P.d, m, e) + eos_e_shear(P.d, m, e);
+            pnt += eos_p_cold(P.d, m, e) + eos_p_shear(P.d, m, e);
+            ig += eos_invG(P.d, m, e);
+        } else {
+            closure_terms64(P, m, e, ent, pnt, ig);
+        }
+    }
+    c.p = (R)(quot((double)c.E + (double)c.Elo - ked - ent + pnt, ig));
     stress(P, c);
     return err;
 }

@@ -154,7 +154,7 @@ __device__ inline void load_state(const PT& P, const R* X, long long nt, long lo
         c.rhou[r] = ru;
     }
     c.E = X[P.S_E * nt + g];
-    if constexpr (sizeof(R) == 4) c.Elo = X[P.S_ELO * nt + g];
+    c.Elo = X[P.S_ELO * nt + g];
     c.p = X[P.S_P * nt + g];
     c.hj2 = R(0.0);
     if (P.solid) {
@@ -222,7 +222,7 @@ __device__ inline void store_state(const PT& P, R* X, long long nt, long long g,
         X[(P.S_RHOU + r) * nt + g] = c.rhou[r];
     }
     X[P.S_E * nt + g] = c.E;
-    if constexpr (sizeof(R) == 4) X[P.S_ELO * nt + g] = c.Elo;
+    X[P.S_ELO * nt + g] = c.Elo;
     X[P.S_P * nt + g] = c.p;
     if (P.solid) {
 #pragma unroll
@@ -395,27 +395,6 @@ __device__ __forceinline__ void muscl1(R um, R u0, R up, R& l, R& r)  // hllc.cp
     r = u0 + R(0.5) * grad;
 }
 
-// The same in binary64 with the same bits and fewer operations of that pipe:
-// a ratio that is not positive and finite gives slope 0 without a division;
-// of the limiter's two quotients 2 / (1 + r) and 2 r / (1 + r) the smaller is
-// the one with the smaller numerator (rounding is monotonic), so one is formed;
-// and the factors of one half are exact, so they go into that quotient and
-// into the fused multiply-adds (7 binary64 operations instead of about 45).
-__device__ __forceinline__ void muscl1(double um, double u0, double up, double& l, double& r)
-{
-    const double num = u0 - um, den = up - u0;
-    const int hn = __double2hiint(num), hd = __double2hiint(den);
-    double half = 0.0;
-    if ((hn ^ hd) >= 0 && ((hn << 1) | __double2loint(num)) != 0 && ((hd << 1) | __double2loint(den)) != 0) {
-        const double rr = quot(num, den);
-        if ((__double2hiint(rr) & 0x7ff00000) != 0x7ff00000)  // finite
-            half = quot(__double2hiint(rr) < 0x3ff00000 ? rr : 1.0, 1.0 + rr);
-    }
-    const double grad = half * (up - um);
-    l = fma(-0.5, grad, u0);
-    r = fma(0.5, grad, u0);
-}
-
 // One carried word at a possibly-ghost cell.
 template <typename PT, typename R = typename PT::real>
 __device__ __forceinline__ R gv(const PT& P, const DevDomain& D, const R* X, long long nt, int word,
@@ -493,7 +472,7 @@ __device__ inline void thinc_cand(const PT& P, const DevDomain& D, const R* X, l
 // ---------------------------------------------------------------------------
 // DC >= 0: the direction as a compile-time constant (d is then ignored).
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(256, 2)
     k_recon(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
@@ -637,12 +616,7 @@ template <typename PT, typename R = typename PT::real>
 __device__ inline void star_state(const PT& P, const CellT<R>& U, CellT<R>& Us, R SK, R Ss, int d)  // :12-73
 {
     R ud = U.vel[d];
-    // |(Ss - ud) / Ss| < 1e-20: the difference of two binary64 numbers that
-    // differ is not smaller than 2^-54 of either, so the quotient is that small
-    // only when they are equal (and not zero)
-    bool contact;
-    if constexpr (sizeof(R) == 4) contact = fabs((Ss - ud) / Ss) < R(1E-20);
-    else contact = Ss - ud == R(0.0) && Ss != R(0.0);
+    const bool contact = fabs((Ss - ud) / Ss) < R(1E-20);
     R mult = contact ? R(1.0) : quot(SK - ud, SK - Ss);
     Us.rho = R(0.0);
     for (int m = 0; m < P.M; ++m) {
@@ -905,7 +879,7 @@ __device__ inline int face_flux(const PT& P, const CellT<R>& L, const CellT<R>& 
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_flux(PT P, PathBufs<typename PT::real> b, int dyn_d)
+__global__ void __launch_bounds__(256, 2) k_flux(PT P, PathBufs<typename PT::real> b, int dyn_d)
 {
     const int d = DC >= 0 ? DC : dyn_d;
     if (b.scal->done) return;
@@ -955,56 +929,6 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_flux(PT P, Path
 // ---------------------------------------------------------------------------
 // Plastic radial return (plastic.cpp:83-223) and cleanUpV (:476-528).
 // ---------------------------------------------------------------------------
-template <typename PT, typename R = typename PT::real>
-__device__ inline int plastic_cell(const PT& P, CellT<R>& c)
-{
-    R tsolid = R(0.0);
-    for (int m = 0; m < P.M; ++m)
-        if (P.phase[m] == TJ_PHASE_SOLID) tsolid += c.alpha[m];
-    if (tsolid <= R(0.5)) {  // cellIsMostlyFluid
-        for (int m = 0; m < P.M; ++m) { c.eps[m] = R(0.0); c.are[m] = R(0.0); }
-        return 0;
-    }
-    hencky(P, c);
-    R JT = R(0.0), JB = R(0.0), norm = R(0.0), J, Jn;
-    for (int m = 0; m < P.M; ++m) {
-        ECellT<R> e = ecell_of(c, m);
-        if (P.phase[m] == TJ_PHASE_SOLID) {
-            J = root(c.hj2);
-            R G = eos_G(P, m, e);
-            if (G * J * sqrt(R(3.0)) > P.yield[m]) Jn = quot(P.yield[m], sqrt(R(3.0)) * G);
-            else Jn = J;
-            c.eps[m] += sqrt(R(2.0) / R(3.0)) * (J - Jn);
-            c.are[m] = c.eps[m] * c.arho[m];
-        } else {
-            J = R(0.0);
-            Jn = R(0.0);
-            c.eps[m] = R(0.0);
-            c.are[m] = R(0.0);
-        }
-        JB += (eos_invG(P, m, e)) * J;
-        JT += (eos_invG(P, m, e)) * Jn;
-        norm += (eos_invG(P, m, e));
-    }
-    JB *= quot(R(1.0), norm);
-    JT *= quot(R(1.0), norm);
-    if (JB == R(0.0) && JT == R(0.0)) { JB = R(1.0); JT = R(1.0); }
-    R t1[9], t2[9], t2i[9];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            R& dv = c.devH[3 * r + q];
-            if (dv != R(0.0) && JB == R(0.0) && JT != R(0.0)) return TJ_ERR_PLASTIC;
-            dv *= quot(JT, JB);
-            t1[3 * r + q] = (R)(r == q) + R(0.5) * dv;
-            t2[3 * r + q] = (R)(r == q) - R(0.5) * dv;
-        }
-    invert3(t2, t2i);
-    mm3(t2i, t1, c.V);
-    return 0;
-}
-
 // The radial return of a binary32 cell with its return map in binary64
 // (plastic.cpp:83-223): the Hencky strain of V is binary32; J = sqrt(HJ2),
 // the projection J -> J_new onto the yield surface, the plastic strain and
@@ -1159,8 +1083,7 @@ __device__ inline void radial_source(const PT& P, CellT<R>& c, const R* sg, int 
     R vds = R(0.0);  // vdotsigma (flux.cpp:19-29) along x
 #pragma unroll
     for (int r = 0; r < 3; ++r) vds += c.vel[r] * sg[3 * r];
-    if constexpr (sizeof(R) == 4) dd_add32(c.E, c.Elo, s * ((c.E * u) - vds));
-    else c.E += s * ((c.E * u) - vds);
+    dd_add32(c.E, c.Elo, s * ((c.E * u) - vds));
     if (P.nmix) c.arl += s * (c.arl * u);
     if (P.solid) {
 #pragma unroll
@@ -1206,8 +1129,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
     }
 #pragma unroll
     for (int r = 0; r < 3; ++r) Yc.rhou[r] += dtdx * (FXW(P.X_RHOU + r, 0) - FXW(P.X_RHOU + r, 1));
-    if constexpr (sizeof(R) == 4) dd_add32(Yc.E, Yc.Elo, dtdx * (FXW(P.X_E, 0) - FXW(P.X_E, 1)));
-    else Yc.E += dtdx * (FXW(P.X_E, 0) - FXW(P.X_E, 1));
+    dd_add32(Yc.E, Yc.Elo, dtdx * (FXW(P.X_E, 0) - FXW(P.X_E, 1)));
     if (P.solid)
 #pragma unroll
         for (int qq = 0; qq < 9; ++qq) {
@@ -1242,8 +1164,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
                 Yc.rhou[r] = (A0.rhou[r] * (R(1.0) / R(2.0))) + (Yc.rhou[r] * (R(1.0) / R(2.0)));
                 Yc.vel[r] = (A0.vel[r] * (R(1.0) / R(2.0))) + (Yc.vel[r] * (R(1.0) / R(2.0)));
             }
-            if constexpr (sizeof(R) == 4) avg_pair32(A0.E, A0.Elo, Yc.E, Yc.Elo);
-            else Yc.E = (A0.E * (R(1.0) / R(2.0))) + (Yc.E * (R(1.0) / R(2.0)));
+            avg_pair32(A0.E, A0.Elo, Yc.E, Yc.Elo);
             Yc.p = (A0.p * (R(1.0) / R(2.0))) + (Yc.p * (R(1.0) / R(2.0)));
             if (P.solid) {
 #pragma unroll
@@ -1265,9 +1186,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
                 if (re) set_status(b.scal, re);
             }
             if (P.plastic) {
-                int e;
-                if constexpr (sizeof(R) == 4) e = plastic_cell_proj64(P, Yc);
-                else e = plastic_cell(P, Yc);
+                const int e = plastic_cell_proj64(P, Yc);
                 c2p(P, Yc);
                 if (e) set_status(b.scal, e);
             }
@@ -1303,7 +1222,7 @@ __device__ __forceinline__ void update_cell(const PT& P, const PathBufs<R>& b, c
 }
 
 template <typename PT, int DC = -1, typename R = typename PT::real>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(256, 2)
     k_update(PT P, PathBufs<typename PT::real> b, const R* __restrict__ X, R* Y, int dyn_d, int first, int last,
              int finish)
 {
@@ -1332,7 +1251,7 @@ __global__ void k_cfl(PT P, PathBufs<typename PT::real> b, const R* __restrict__
 {
     if (b.scal->done) return;
     const long long nt = b.ntot;
-    R mn = R(sizeof(R) == 4 ? 3.0e38 : 1.79769313486231570815e+308);
+    R mn = R(3.0e38);
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nt; g += (long long)gridDim.x * blockDim.x) {
         const int q = find_dom(b.doms, b.ndom, g);
         const DevDomain D = b.doms[q];
@@ -1353,7 +1272,7 @@ __global__ void k_cfl(PT P, PathBufs<typename PT::real> b, const R* __restrict__
     if (lane == 0) red[w] = mn;
     __syncthreads();
     if (w == 0) {
-        mn = (lane < (int)(blockDim.x >> 5)) ? red[lane] : R(sizeof(R) == 4 ? 3.0e38 : 1.79769313486231570815e+308);
+        mn = (lane < (int)(blockDim.x >> 5)) ? red[lane] : R(3.0e38);
         for (int s = 16; s > 0; s >>= 1) {
             R o = __shfl_down_sync(0xffffffffu, mn, s);
             if (o < mn) mn = o;
