@@ -762,26 +762,36 @@ TJA_HD void thinc_cand_rev(const double s[3][3], int d, double beta0, double dx,
 // up - u0 when r >= 1, and 0 otherwise (r = (u0-um)/(up-u0), r <= 0, inf or
 // NaN). Returns 1, 2 or 0 for those branches.
 // ---------------------------------------------------------------------------
+// The forward's extrapolation (tj_path.cuh muscl1), the same bits: where the
+// limiter's value and half the slope are normal numbers, the factors of one half
+// are exact.
 TJA_HD void muscl_fwd(double um, double u0, double up, double& l, double& r)
 {
     const double num = u0 - um, den = up - u0;
-    const tj::tjq_u64 bn = tj::tjq_bits(num), bd = tj::tjq_bits(den);
+    const tj::tjq_u64 bn = tj::tjq_bits(num), bd = tj::tjq_bits(den), low = (tj::tjq_u64)4 << 52;
+    const tj::tjq_u64 an = bn & 0x7fffffffffffffffull, ad = bd & 0x7fffffffffffffffull;
     double half = 0.0;  // of the limiter
-    if (!((bn ^ bd) >> 63) && (bn << 1) != 0 && (bd << 1) != 0) {
-        const double rr = quot(num, den);
-        const int er = (int)(tj::tjq_bits(rr) >> 52) & 0x7ff;
-        if (er != 0x7ff) {  // finite
-            half = quot(er < 0x3ff ? rr : er < 0x7fd ? 1.0 : 2.0, 1.0 + rr);
-            if (er >= 0x7fd) half *= 0.5;  // a subnormal half: rounded twice, as the limiter's value is
+    bool rare = false;
+    if (!((bn ^ bd) >> 63)) {
+        if (an >= low && ad >= low) {
+            const double rr = quot(num, den);
+            const unsigned er = (unsigned)(tj::tjq_bits(rr) >> 52);
+            if (er < 0x7fd) half = quot(er < 0x3ff ? rr : 1.0, 1.0 + rr);
+            else rare = er < 0x7ff;
+        } else {
+            rare = an != 0 && ad != 0;
         }
     }
     const double grad = half * (up - um);
     l = fma(-0.5, grad, u0);
     r = fma(0.5, grad, u0);
-    const tj::tjq_u64 bg = tj::tjq_bits(grad) << 1;
-    if (bg != 0 && bg < 0x40000000000000ull) {  // half of it is subnormal: a product that rounds
-        l = u0 - 0.5 * grad;
-        r = u0 + 0.5 * grad;
+    if (rare) {
+        double rr = num / den;
+        if (TJA_NOTFINITE(rr)) rr = 0.0;
+        const double a = 2.0 / (1.0 + rr), b = 2.0 * rr / (1.0 + rr);
+        const double g = (rr <= 0.0 ? 0.0 : (b < a) ? b : a) * 0.5 * (up - um);
+        l = u0 - 0.5 * g;
+        r = u0 + 0.5 * g;
     }
 }
 

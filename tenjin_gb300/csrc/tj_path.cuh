@@ -470,33 +470,49 @@ __device__ __forceinline__ void muscl1(R um, R u0, R up, R& l, R& r)  // hllc.cp
     r = u0 + R(0.5) * grad;
 }
 
+// The limited extrapolation in the order of the reference, out of line: for the
+// values at which the form below would round otherwise.
+static __device__ __noinline__ double2 muscl_rare(double um, double u0, double up)
+{
+    double rr = (u0 - um) / (up - u0);
+    if (isinf(rr) || isnan(rr)) rr = 0.0;
+    const double grad = vanleer(rr) * 0.5 * (up - um);
+    return make_double2(u0 - 0.5 * grad, u0 + 0.5 * grad);
+}
+
 // The same in binary64 with the same bits and fewer operations of that pipe:
 // a ratio that is not positive and finite gives slope 0 without a division;
 // of the limiter's two quotients 2 / (1 + r) and 2 r / (1 + r) the smaller is
 // the one with the smaller numerator (rounding is monotonic), so one is formed;
-// and the factors of one half are exact (but next to the subnormal numbers), so
-// they go into that quotient and into the fused multiply-adds (7 binary64
-// operations instead of about 45).
+// and the factors of one half go into that quotient and into the fused
+// multiply-adds (7 binary64 operations instead of about 45). They are exact where
+// the limiter's value and half the slope, about the smaller difference, are normal
+// numbers: a ratio of 2^1022 or more and a difference below 2^-1019 are left to the
+// general form.
 __device__ __forceinline__ void muscl1(double um, double u0, double up, double& l, double& r)
 {
     const double num = u0 - um, den = up - u0;
     const int hn = __double2hiint(num), hd = __double2hiint(den);
+    const unsigned an = (unsigned)hn & 0x7fffffffu, ad = (unsigned)hd & 0x7fffffffu;
     double half = 0.0;
-    if ((hn ^ hd) >= 0 && ((hn << 1) | __double2loint(num)) != 0 && ((hd << 1) | __double2loint(den)) != 0) {
-        const double rr = quot(num, den);
-        const int er = __double2hiint(rr) & 0x7ff00000;
-        if (er != 0x7ff00000) {  // finite
-            half = quot(er < 0x3ff00000 ? rr : er < 0x7fd00000 ? 1.0 : 2.0, 1.0 + rr);
-            if (er >= 0x7fd00000) half *= 0.5;  // a subnormal half: rounded twice, as the limiter's value is
+    bool rare = false;
+    if ((hn ^ hd) >= 0) {
+        if (min(an, ad) >= 0x00400000u) {
+            const double rr = quot(num, den);
+            const unsigned hr = (unsigned)__double2hiint(rr);
+            if (hr < 0x7fd00000u) half = quot(hr < 0x3ff00000u ? rr : 1.0, 1.0 + rr);
+            else rare = hr < 0x7ff00000u;
+        } else {
+            rare = (an | (unsigned)__double2loint(num)) != 0 && (ad | (unsigned)__double2loint(den)) != 0;
         }
     }
     const double grad = half * (up - um);
     l = fma(-0.5, grad, u0);
     r = fma(0.5, grad, u0);
-    const unsigned hg = (unsigned)__double2hiint(grad) << 1;
-    if (hg < 0x400000u && (hg | __double2loint(grad)) != 0) {  // half of it is subnormal: a product that rounds
-        l = u0 - 0.5 * grad;
-        r = u0 + 0.5 * grad;
+    if (rare) {
+        const double2 x = muscl_rare(um, u0, up);
+        l = x.x;
+        r = x.y;
     }
 }
 
