@@ -75,6 +75,16 @@ struct M3P {
 // the compiler's division by a variable takes about twenty instructions; three
 // per staged cell, face and output cell were a quarter of the kernel.
 __host__ __device__ constexpr unsigned div3(unsigned d) { return ((1u << 20) + d - 1) / d; }
+constexpr unsigned kMaxEntry = 2048, kMaxDiv = 240;
+constexpr bool div3_exact()  // the error of every factor, over every entry
+{
+    for (unsigned d = 1; d <= kMaxDiv; ++d) {
+        const unsigned e = d * div3(d) - (1u << 20);
+        if (e >= d || e * (kMaxEntry - 1) >= (1u << 20)) return false;
+    }
+    return true;
+}
+static_assert(div3_exact(), "t / d == (t * div3(d)) >> 20 for t < 2048, d <= 240");
 
 // one tile of one domain
 struct Work3 {
@@ -127,6 +137,9 @@ template <int M, int TX, int TY, int TZ>
 struct Sm3 {
     static constexpr int SX = TX + 4, SY = TY + 4, SZ = TZ + 4;
     static constexpr int SV = SX * SY * SZ;  // staged cells
+    // the lists that split_t walks: staged cells, faces, output cells
+    static_assert(SV <= (int)kMaxEntry && SX * SY <= (int)kMaxDiv, "staged cells outgrow div3");
+    static_assert((TX + 1) * TY <= (int)kMaxDiv && TX * (TY + 1) <= (int)kMaxDiv, "faces outgrow div3");
     static constexpr int CV = TX * TY * TZ;  // output cells
     // faces of each direction (x faces, y faces, z faces of the tile)
     static constexpr int FV0 = (TX + 1) * TY * TZ, FV1 = TX * (TY + 1) * TZ, FV2 = TX * TY * (TZ + 1);
