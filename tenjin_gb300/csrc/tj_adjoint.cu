@@ -146,8 +146,17 @@ __device__ __forceinline__ void face_prim(const GT& G, const double* X, const do
         for (int m = 0; m < G.M; ++m) x.a[m] = rec[((long long)(d * 2 + side) * G.M + m) * G.N + g];
 }
 
+// (h, l) += x as an unevaluated pair (error-free sum).
+__device__ __forceinline__ void pair_add(double& h, double& l, double x)
+{
+    const double s = h + x, t = s - h;
+    l += (h - (s - t)) + (x - t);
+    h = s;
+}
+
 // Adds the block's sum of g to its slot gpart[blockIdx.x][k], k = m (G),
-// MM + m (p_ref), 2 MM + m (e_ref).
+// MM + m (p_ref), 2 MM + m (e_ref). A slot is a pair: the terms of one parameter
+// cancel to 1e-4 of their size, and a slot takes thousands of them.
 __device__ __forceinline__ void block_add_grad(const tja::GradEos& g, int M, double* gpart)
 {
     __shared__ double red[NT / 32][NG];
@@ -164,12 +173,13 @@ __device__ __forceinline__ void block_add_grad(const tja::GradEos& g, int M, dou
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < NG; ++k) {
-            double s = 0.0;
-            for (int w = 0; w < NT / 32; ++w) s += red[w][k];
-            gpart[(long long)blockIdx.x * NG + k] += s;
-        }
+    if (threadIdx.x < NG) {
+        double* slot = gpart + 2 * ((long long)blockIdx.x * NG + threadIdx.x);
+        double h = slot[0], l = slot[1];
+        for (int w = 0; w < NT / 32; ++w) pair_add(h, l, red[w][threadIdx.x]);
+        slot[0] = h;
+        slot[1] = l;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -615,14 +625,22 @@ __global__ void __launch_bounds__(NT, 8) k_adj_p2c0(AG G0, const double* lam, co
     block_add_grad(gr, M, gpart);
 }
 
-// One warp per parameter: a fixed stride per lane, a fixed tree.
+// One warp per parameter: a fixed stride per lane, a fixed tree, of pairs.
 __global__ void k_adj_gsum(const double* gpart, int nblk, double* out)
 {
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double s = 0.0;
-    for (int b = lane; b < nblk; b += 32) s += gpart[(long long)b * NG + k];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) out[k] = s;
+    double h = 0.0, l = 0.0;
+    for (int b = lane; b < nblk; b += 32) {
+        const double* slot = gpart + 2 * ((long long)b * NG + k);
+        pair_add(h, l, slot[0]);
+        l += slot[1];
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const double oh = __shfl_down_sync(0xffffffffu, h, o), ol = __shfl_down_sync(0xffffffffu, l, o);
+        pair_add(h, l, oh);
+        l += ol;
+    }
+    if (lane == 0) out[k] = h + l;
 }
 
 inline int nb(long long n) { return (int)std::min<long long>((n + NT - 1) / NT, NBLK); }
@@ -759,7 +777,7 @@ static int ensure(AdjState* a, const DevParams& P, const Fp64Bufs& b, const DevD
               dalloc(a, &a->lam, (size_t)ns * N) && dalloc(a, &a->lamA, (size_t)ns * N) &&
               dalloc(a, &a->lamB, (size_t)ns * N) && dalloc(a, &a->mu, NW * N) && dalloc(a, &a->lface, 4 * NW * N) &&
               dalloc(a, &a->limg, 4 * NW * nl) && dalloc(a, &a->sstar, nf0 + nf1) &&
-              dalloc(a, &a->tcon, (size_t)2 * M * 9 * N) && dalloc(a, &a->gpart, (size_t)NBLK * NG) &&
+              dalloc(a, &a->tcon, (size_t)2 * M * 9 * N) && dalloc(a, &a->gpart, (size_t)2 * NBLK * NG) &&
               dalloc(a, &a->gsum, NG) && dalloc(a, &a->sul, (size_t)M * N) && dalloc(a, &a->sur, (size_t)M * N);
     if (!ok) {
         free_all(a);
@@ -839,7 +857,7 @@ long long adj_backward(AdjState* a, const DevParams& P, const Fp64Bufs& b, const
     const size_t nf0 = (size_t)(D.n[0] + 1) * D.n[1];
     long long launches = 0;
     cudaMemcpyAsync(a->lam, lam_final, sizeof(double) * sw, cudaMemcpyDeviceToDevice, st);
-    cudaMemsetAsync(a->gpart, 0, sizeof(double) * NBLK * NG, st);
+    cudaMemsetAsync(a->gpart, 0, sizeof(double) * 2 * NBLK * NG, st);
     cudaMemsetAsync(a->sul, 0, sizeof(double) * M * N, st);
     cudaMemsetAsync(a->sur, 0, sizeof(double) * M * N, st);
     auto S = [&](int k, int which) { return a->seg + (size_t)(3 * k + which) * sw; };
