@@ -338,8 +338,8 @@ def other_configs():
     e = sum(float(np.abs(a - b).sum()) for a, b in zip(r32, r64)) / sum(float(np.abs(b).sum()) for b in r64)
     g32.run(3, 1e300)
     ms32, d32 = _timed_run(g32, 20)
-    buf = ctypes.create_string_buffer(256)
-    g32.L.tj_kernel_config(g32.h, buf, 256)
+    buf = ctypes.create_string_buffer(512)
+    g32.L.tj_kernel_config(g32.h, buf, 512)
     g32.close()
     out["uneven_boxes_3d"] = {
         "workload": f"{len(c.domains)} independent 3-D boxes, edges log-uniform in [8, 64], {c.total_cells} cells, "
@@ -360,7 +360,7 @@ def other_configs():
     g32.run(1, 1e300)
     ms32, d32 = _timed_run(g32, 2)
     r32 = g32.state(0)[c.M:2 * c.M].sum(axis=0)
-    g32.L.tj_kernel_config(g32.h, buf, 256)
+    g32.L.tj_kernel_config(g32.h, buf, 512)
     g32.run(3, 1e300)
     ms32b, d32b = _timed_run(g32, 5)
     g32.close()

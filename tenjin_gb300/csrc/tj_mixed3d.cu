@@ -2,7 +2,7 @@
 // THINC: the reference's 3-D THINC has no interface normal,
 // thinc.cpp:124-127), binary32 with a compensated total energy, over any
 // number of independent domains (AMReX boxes that are each their own
-// domain) in ONE persistent launch per RK stage.
+// domain) in one persistent launch per RK stage and tile shape.
 //
 // Work list: every domain is cut into tiles of at most TX x TY x TZ cells
 // (the split per axis balances the tile extents, so a 27-cell box becomes

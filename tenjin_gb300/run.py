@@ -57,8 +57,8 @@ def main(argv=None) -> dict:
     e1.record(st)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1)
-    buf = ctypes.create_string_buffer(256)
-    g.L.tj_kernel_config(g.h, buf, 256)
+    buf = ctypes.create_string_buffer(512)
+    g.L.tj_kernel_config(g.h, buf, 512)
     out = {"builder": a.builder, "kwargs": kw, "precision": a.precision, "cells": case.total_cells,
            "steps": done, "ms_per_step": ms / max(done, 1),
            "cell_updates_per_s": case.total_cells * done / (ms / 1e3) if ms > 0 else None,
