@@ -46,21 +46,24 @@ constexpr int MH = 3;            // staged halo
 constexpr int MS = MT + 2 * MH;  // staged cells per axis (34)
 constexpr int MP = MS + 1;       // shared-memory pitch (odd: conflict-free columns)
 constexpr int CP = MT + 1;       // pitch of the output-cell arrays (odd)
-// Threads per CTA: eight warps, three CTAs an SM, where there are tiles for it
-// (20 steps with 256 / 288 / 320: 1024^2 5.84 / 6.01 / 5.91 ms, 1500^2 11.44 /
-// 11.83 / 11.45 ms, 640^2 2.93 / 2.97 / 2.87 ms); a grid of fewer tiles leaves
-// SMs with one or two CTAs whose warps walk 28 rows in three rounds or four, so up
-// to two tiles an SM take 14 warps a CTA (two rounds) and up to one takes 28 (one
-// round): 28 warps an SM all the same (333^2 MUSCL, 144 tiles, 40 steps: 1.48 ms
-// with 256, 1.35 with 896). Three and four materials need more registers and
-// binary64 more shared memory: 256 for them at any size.
-constexpr int NTH = 256, NTH_2 = 448, NTH_1 = 896;
+// Threads per CTA: ten warps, three CTAs an SM, where there are tiles for it (a
+// step with 256 / 320: 1024^2 0.1539 / 0.1505 ms, 700^2 0.0857 / 0.0831, 2500^2
+// 0.834 / 0.808; without THINC 1024^2 0.1062 / 0.1067; 20 steps with every cell
+// mixed and 256 / 288 / 320: 1024^2 5.84 / 6.01 / 5.91 ms, 1500^2 11.44 / 11.83 /
+// 11.45); a grid of two to three tiles an SM, all of them at once, eight (520^2, a
+// step 0.0576 / 0.0588 ms). A grid of fewer tiles leaves SMs with one or two CTAs whose
+// warps walk 28 rows in three rounds or four, so up to two tiles an SM take 14 warps a
+// CTA (two rounds) and up to one takes 28 (one round): 28 warps an SM all the same
+// (333^2 MUSCL, 144 tiles, 40 steps: 1.48 ms with 256, 1.35 with 896). Three and
+// four materials need more registers and binary64 more shared memory: 256 for them
+// at any size.
+constexpr int NTH = 320, NTH_2 = 448, NTH_1 = 896, NTH_WIDE = 256;
 
 // The step's scalars (dt from the CFL minimum, the step's end) are handled inside
 // the stage kernels on grids of up to kInside tiles, two an SM, and by launches
 // of one thread on larger ones: there a CTA's slot waits for its block's turn at
-// the counter (last_block) in every wave (2500^2, 20 steps: 30.35 ms inside,
-// 29.63 apart; 300^2: 0.91 ms inside, 1.42 apart). Their launches do not overlap
+// the counter (last_block) in every wave (2500^2, a step: 0.835 ms inside,
+// 0.808 apart; 300^2, 20 steps: 0.91 ms inside, 1.42 apart). Their launches do not overlap
 // either: the next kernel's CTAs take the SMs that drain first and are dealt
 // unevenly (500^2, 324 tiles, 20 steps: 1.90 ms overlapped, 1.81 one after the
 // other).
@@ -820,13 +823,20 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
     // the step's dt: stored by the kernel before (scalars apart), or formed from
     // the CFL minimum that the step before left, by every block's first thread while
     // the tile is staged; the last block to end then stores it
-    __shared__ R dt_over_dx[2];
+    // (binary32: dt / dx as a product with 1 / dx, no binary64 division)
+    const auto over_dx = [&](double dt, int d) { return sizeof(R) == 8 ? (R)(dt / P.dxd[d]) : (R)dt * P.idx[d]; };
+    __shared__ R dt_over_dx[INSIDE ? 2 : 1];
     __shared__ int run_over;
-    if (threadIdx.x == 0) {
-        double dt = b.scal->dt;
-        run_over = INSIDE && stage == 0 && step_dt(b.scal, P.cfl, __longlong_as_double((long long)b.scal->dtmin_bits), dt);
-        // binary32: a product with 1/dx (no binary64 division)
-        for (int d = 0; d < 2; ++d) dt_over_dx[d] = sizeof(R) == 8 ? (R)(dt / P.dxd[d]) : (R)dt * P.idx[d];
+    R dtdx, dtdy;
+    if constexpr (INSIDE) {
+        if (threadIdx.x == 0) {
+            double dt = b.scal->dt;
+            run_over = stage == 0 && step_dt(b.scal, P.cfl, __longlong_as_double((long long)b.scal->dtmin_bits), dt);
+            for (int d = 0; d < 2; ++d) dt_over_dx[d] = over_dx(dt, d);
+        }
+    } else {
+        dtdx = over_dx(b.scal->dt, 0);
+        dtdy = over_dx(b.scal->dt, 1);
     }
     using SM = Smem<R, M, THINC>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -891,10 +901,13 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 4 ? (NT <= NTH ? 3 : NTH_1 / 
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    const R dtdx = dt_over_dx[0], dtdy = dt_over_dx[1];
-    if (INSIDE && run_over) {
-        if (last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
-        return;
+    if constexpr (INSIDE) {
+        dtdx = dt_over_dx[0];
+        dtdy = dt_over_dx[1];
+        if (run_over) {
+            if (last_block(b.scal)) finalize_dt(b.scal, P.cfl, 1);
+            return;
+        }
     }
     // reflect_odd ghosts (FillDomainBoundary): negate the normal velocity of
     // staged cells that mirror across a reflective face
@@ -1470,12 +1483,14 @@ struct MixedImpl : MixedBase {
     {
         const dim3 grid = tiles();
         const long long n = (long long)grid.x * grid.y;
-        if (apart()) return launch_stage_n<MM, TH, NTH, false>(stage, grid, st, overlap);
         if constexpr (sizeof(R) == 4 && MM <= 2) {
-            if (n <= kSMs) launch_stage_n<MM, TH, NTH_1, true>(stage, grid, st, overlap);
+            if (n > 3 * kSMs) launch_stage_n<MM, TH, NTH, false>(stage, grid, st, overlap);
+            else if (apart()) launch_stage_n<MM, TH, NTH_WIDE, false>(stage, grid, st, overlap);
+            else if (n <= kSMs) launch_stage_n<MM, TH, NTH_1, true>(stage, grid, st, overlap);
             else launch_stage_n<MM, TH, NTH_2, true>(stage, grid, st, overlap);
         } else {
-            launch_stage_n<MM, TH, NTH, true>(stage, grid, st, overlap);
+            if (apart()) launch_stage_n<MM, TH, NTH_WIDE, false>(stage, grid, st, overlap);
+            else launch_stage_n<MM, TH, NTH_WIDE, true>(stage, grid, st, overlap);
         }
     }
 
